@@ -158,6 +158,27 @@ def test_act_mul(nat, act):
     assert _rel_err(nat.act_mul(x, 1376, act, gated=False), ref.act_mul(x, 1376, act, gated=False)) < 4e-3
 
 
+@pytest.mark.parametrize("T, V, ld", [(1, 32000, 32000), (1, 128256, 128256), (37, 32000, 32000), (38, 32000, 32000), (75, 32003, 32008), (149, 4096, 4096),
+                                      (3, 50257, 50257), (2, 7, 8), (5, 4097, 4104)])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+def test_argmax_logprob_over_split_rows(nat, T, V, ld, softcap):
+    """Rows over clusters of one to eight CTAs, rows that start off a 16-byte boundary, ties across the parts, masked logits.  The sum of
+    V terms in fp32 in any order is within V * 2^-24 of itself relatively, and so is its logarithm; expf and logf add a few 2^-22."""
+    g = torch.Generator().manual_seed(V + T)
+    logits = (torch.randn(T, ld, generator=g) * 3).to(torch.bfloat16)
+    logits[0, : V // 3] = float("-inf")
+    logits[T - 1, [V // 5, V - 1, V // 2]] = 40.0
+    logits = logits.cuda()[:, :V]
+    i, lp = nat.argmax_logprob(logits, softcap=softcap)
+    x = logits.double()
+    if softcap:
+        x = softcap * torch.tanh(x / softcap)
+    top = x.max(-1).values
+    assert torch.equal(logits.gather(1, i.long()[:, None])[:, 0], logits.max(-1).values)
+    assert torch.equal(i.cpu().long(), (logits == logits.max(-1, keepdim=True).values).int().argmax(-1).cpu())
+    assert torch.allclose(lp.double(), top - torch.logsumexp(x, -1), atol=V * 2 ** -24 + 2 ** -18, rtol=2 ** -20)
+
+
 def test_embed_argmax_advance(nat):
     table = torch.randn(1000, 256, device="cuda", dtype=torch.bfloat16)
     ids = torch.randint(0, 2000, (50,), device="cuda", dtype=torch.int32)
