@@ -155,7 +155,6 @@ LX_DEVICE float fa_block_probs(uint32_t ts, uint8_t* prow, int row, int kb0, int
 template <bool WIDE>
 __global__ void __launch_bounds__(kFaThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const FaParams p) {
-  pdl_trigger();
   using S = FaSmem<WIDE>;
   extern __shared__ uint8_t fa_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~uintptr_t(1023));
@@ -200,6 +199,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
+  pdl_trigger();
 
   const int b = p.tile_seq[tile];
   const int q0 = p.tile_q0[tile];

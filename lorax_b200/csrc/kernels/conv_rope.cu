@@ -105,8 +105,8 @@ struct CvSink {
 // TAPS 1 .. 4: the weights in registers; 0: any number up to kCvMaxTaps; -1: no convolution.
 template <typename T, bool ATTN, int TAPS>
 __global__ void __launch_bounds__(kCvThreads) conv_kernel(const ConvParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) uint8_t cv_raw[];
   const int c0 = blockIdx.y * kCvCols, vec = threadIdx.x % kCvVecs, run = threadIdx.x / kCvVecs, c = c0 + vec * 8;
   const int keep = TAPS < 0 ? 0 : (TAPS > 0 ? TAPS : p.taps) - 1;

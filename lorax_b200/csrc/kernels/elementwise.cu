@@ -25,8 +25,8 @@ norm_residual_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                      __nv_bfloat16* __restrict__ out, int H, long long ldx, long long ldr, long long ldo, float eps,
                      float w_offset, float x_scale) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int row = blockIdx.x;
   const int nvec = H / 8;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
@@ -145,8 +145,8 @@ __global__ void __launch_bounds__(256)
 rope_kvwrite_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const float* __restrict__ cos_sin,
                     __nv_bfloat16* __restrict__ kv_cache, const int* __restrict__ slots, int nh, int nkv, int d, int rot,
                     int page, long long ldq, int apply_rope, int kv_fp8, float k_inv_scale, float v_inv_scale) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int slot = slots ? slots[t] : -1;
@@ -245,8 +245,8 @@ LX_DEVICE float act_fn(float x) {
 template <int ACT, bool GATED>
 __global__ void __launch_bounds__(256)
 act_mul_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int vec_per_row = I / 8;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total_vec; v += (long long)gridDim.x * blockDim.x) {
     const long long t = v / vec_per_row;
@@ -280,8 +280,8 @@ struct EmbedPeerParams {
 };
 
 __global__ void __launch_bounds__(128) embed_peer_kernel(const int* __restrict__ ids, const EmbedPeerParams p, __nv_bfloat16* __restrict__ out) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int t = blockIdx.x;
   const int id = ids[t];
   uint4* o = reinterpret_cast<uint4*>(out + (long long)t * p.H);
@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(128) embed_peer_kernel(const int* __restrict__
 __global__ void __launch_bounds__(128)
 embed_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table, __nv_bfloat16* __restrict__ out, int H,
              int v0, int v1, float mult) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int t = blockIdx.x;
   const int id = ids[t];
   uint4* o = reinterpret_cast<uint4*>(out + (long long)t * H);
@@ -396,8 +396,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(kArgmaxThreads)
 argmax_logprob_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int V, int* __restrict__ ids,
                       float* __restrict__ logprobs, float softcap) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int t = blockIdx.x, part = blockIdx.y, parts = gridDim.y;
   const __nv_bfloat16* row = logits + t * ld;
   const int chunk = ((V + parts - 1) / parts + 7) & ~7;
@@ -468,8 +468,8 @@ argmax_logprob_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, in
 __global__ void advance_decode_kernel(int* __restrict__ input_ids, const int* __restrict__ next_ids, int* __restrict__ positions,
                                       int* __restrict__ ctx_lens, int* __restrict__ slots, const int* __restrict__ block_tables,
                                       int max_blocks, int page, int B) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   if (ctx_lens[b] <= 0) { slots[b] = -1; return; }
@@ -485,8 +485,8 @@ __global__ void __launch_bounds__(256)
 prefill_metadata_kernel(const int* __restrict__ cu_q, const int* __restrict__ cache_lens, const int* __restrict__ seq_slot,
                         const int* __restrict__ block_tables, int max_blocks, int B, int page, int T, int* __restrict__ positions,
                         int* __restrict__ slots, int* __restrict__ tok_slot) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   int lo = 0, hi = B;                     // last sequence whose first token is at or before t

@@ -368,6 +368,7 @@ namespace lx {
 __global__ void __launch_bounds__(256) fp8_block128_dequant_kernel(const uint8_t* __restrict__ q, long long ldq, const float* __restrict__ sw,
                                                                    int lds, __nv_bfloat16* __restrict__ out, long long ldo, int N, int K) {
   pdl_wait();
+  pdl_trigger();
   const long long vecs_per_row = K / 16;
   const long long total = (long long)N * vecs_per_row;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += (long long)gridDim.x * blockDim.x) {

@@ -57,8 +57,8 @@ LX_DEVICE void turn8(float (&f)[8], const float* __restrict__ table, int rot, in
 
 template <typename T>
 __global__ void __launch_bounds__(256) qk_norm_kvwrite_kernel(const QkNormParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const bool values = blockIdx.y == 1;
   const int width = values ? p.DV : p.DK, lanes = width / 8;                      // 8, 16 or 32 threads
   const unsigned heads = values ? p.G : p.H + p.G;
@@ -118,8 +118,8 @@ struct GqaF32Params {
 };
 
 __global__ void __launch_bounds__(32 * kGqaWarps) gqa_attn_f32_kernel(const GqaF32Params p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ __align__(16) float qs[kGqaWarps][kGqaMaxWidth];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x, h = blockIdx.y * kGqaWarps + warp;

@@ -27,8 +27,8 @@ struct LatentPrepParams {
 
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrepParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[4];
   const int t = blockIdx.x;
   const T* dq = reinterpret_cast<const T*>(p.dq) + (long long)t * p.ld_dq;
@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrepParams
 template <typename T>
 __global__ void __launch_bounds__(256) rope_pairs_kernel(T* __restrict__ x, long long ldx, const int* __restrict__ positions,
                                                          const float* __restrict__ cos_sin, int H, int head, int off, int rot) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int t = blockIdx.x, half = rot / 2;
   const float* cs = cos_sin + (long long)positions[t] * rot;
   for (int e = threadIdx.x; e < H * half; e += blockDim.x) {
@@ -144,8 +144,8 @@ constexpr int kLaMaxVec = 5;             // R <= 32 * 8 * 5
 
 template <typename T>
 __global__ void __launch_bounds__(128) latent_attn_kernel(const LatentAttnParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   extern __shared__ float sm[];          // [4 warps][KR] partial sums, then m and l of every warp
   const int t = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int* bt;

@@ -57,8 +57,8 @@ struct LdSmem {
 // KS: 16-wide K steps per slice; KR: latent columns; KEYS: keys per tile; WARPS: per CTA; OCC: CTAs per SM.
 template <int MT, int KS, int KR, int KEYS, int WARPS, int OCC>
 __global__ void __launch_bounds__(32 * WARPS, OCC) latent_decode_kernel(const LatentDecodeParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   using S = LdSmem<MT, KEYS, WARPS>;
   constexpr int kLdThreads = 32 * WARPS, KG = WARPS / 2;      // K slices of the score products
   constexpr int NK2 = KEYS / 32;                   // 16-key steps of a warp's half of the tile
@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(32 * WARPS, OCC) latent_decode_kernel(const La
 // Shares of the keys -> one row: out = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s.
 __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                              __nv_bfloat16* __restrict__ out, long long ldo, int H, int KR, int nsplit) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int t = blockIdx.x, h = blockIdx.y;
   const long long base = ((long long)t * H + h) * nsplit;
   float M = -INFINITY, den = 0.f;

@@ -62,7 +62,6 @@ template <int NK, int NR, int NV>
 __global__ void __launch_bounds__(kLpThreads, 1)
 latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv,
                       const __grid_constant__ CUtensorMap tmap_rot, const LatentPrefillParams p) {
-  pdl_trigger();
   using S = LpSmem<NK, NR, NV>;
   constexpr int NP = NK + NR;
   extern __shared__ uint8_t lp_raw[];
@@ -108,6 +107,7 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;           // columns [0, 128): scores (two buffers of 64), [128, 128 + 64 NV): O
   pdl_wait();
+  pdl_trigger();
 
   const int b = p.tile_seq[tile];
   const int q0 = p.tile_q0[tile];
@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(128) latent_gather_kernel(const __nv_bfloat16*
                                                             const int* __restrict__ ctx_off, const int* __restrict__ cache_lens, int window,
                                                             int B, int page, int KR, int RR,
                                                             __nv_bfloat16* __restrict__ lat, __nv_bfloat16* __restrict__ rot) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int r = blockIdx.x;
   int lo = 0, hi = B;
   while (hi - lo > 1) {

@@ -67,6 +67,7 @@ struct LxLoraFused {
   const void* arena; long long off_a;
   long long off_b, arena_elems;
   int* sync;
+  int w_const;
 };
 int lx_gemm_bf16_lora(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
                       long long ldw, long long ldo, void* ws, long long ws_bytes, int* counters, int* status, int num_sms,
@@ -163,7 +164,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
     f.slot_rank = m.slot_rank; f.slot_base = m.slot_base; f.num_slots = m.num_slots;
     f.nparts = site.nparts; f.n0 = site.n0; f.n1 = site.n1; f.layer = l.layer_index; f.max_rank = m.max_rank;
     f.vimg = m.lora_vimg; f.vimg_bytes = m.lora_vimg_bytes; f.fence_maps = m.lora_fence_maps;
-    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync;
+    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync; f.w_const = 1;
     const int rc = lx_gemm_bf16_lora(x, w, y, bias, s.T, N, K, ldx, ldw, ldy, m.gemm_ws, m.gemm_ws_bytes, m.gemm_counters, m.status, m.num_sms,
                                      &f, stream);
     if (rc != 1) return rc;          // 1: this step does not fit the fused launch, use the separate kernels below
@@ -184,8 +185,8 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
                             s.T, K, m.max_rank, m.status, stream));
     }
   }
-  LX_TRY(lx_gemm_bf16(x, w, y, bias, s.T, N, K, ldx, ldw, ldy, 1.f, m.gemm_ws, m.gemm_ws_bytes, m.gemm_counters, m.status, m.num_sms, 0, 0,
-                      stream));
+  LX_TRY(lx_gemm_bf16(x, w, y, bias, s.T, N, K, ldx, ldw, ldy, 1.f, m.gemm_ws, m.gemm_ws_bytes, m.gemm_counters, m.status, m.num_sms,
+                      1 << 16 /* constant weights */, 0, stream));
   if (lora) {
     if (s.lora_tiles != nullptr) {
       LX_TRY(lx_lora_expand_tiled(m.lora_v, m.ldv, 0, 1, s.lora_tiles, s.num_tiles, s.max_tile_rows, m.arena, m.slot_base, m.slot_rank,

@@ -77,8 +77,8 @@ LX_DEVICE void lt_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
 
 // silu in place over the columns [0, cols) of a row-strided matrix (the projections of prompt rows, read several times below)
 __global__ void __launch_bounds__(256) silu_cols_kernel(__nv_bfloat16* __restrict__ x, long long ld, int cols, long long total) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int per_row = cols / 8;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
     __nv_bfloat16* at = x + (e / per_row) * ld + (e % per_row) * 8;
@@ -101,8 +101,8 @@ struct LtSmem {
 
 template <int D, bool STATES, bool SSD>
 __global__ void __launch_bounds__(kLtThreads, 2) linear_attn_tc_kernel(const LinTcParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   using M = LtSmem<D, STATES>;
   constexpr int LD = D + 8, MT = D / 64;         // 16-row tiles of the state per warp
   extern __shared__ __align__(16) uint8_t lt_sm[];

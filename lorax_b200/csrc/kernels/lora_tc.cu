@@ -62,7 +62,6 @@ struct LtSmem {
 template <int BN>
 __global__ void __launch_bounds__(kLtThreads)
 lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const ShrinkTcParams p) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
   using S = LtSmem<BN>;
   LoraTile tile = p.tiles[blockIdx.x];
@@ -109,6 +108,7 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const ShrinkTc
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
+  pdl_trigger();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -256,8 +256,8 @@ constexpr int kExpRowsInFlight = 4;                  // rows whose y loads are i
 // The grid is a fixed number of CTAs that walk the units; live tiles come first in the table, so the walk stops at
 // the first dead one and padding entries cost nothing.
 __global__ void __launch_bounds__(kExpThreads, 2) lora_expand_tiled_kernel(const ExpandTiledParams p) {
-  pdl_trigger();
   pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   __shared__ __align__(16) float vs[kExpMaxRows * 3 * kExpStage];   // [row][part][16]
   const int nparts = p.n1 < p.N ? 3 : (p.n0 < p.N ? 2 : 1);
   for (int w = blockIdx.x; w < p.num_tiles * p.col_blocks; w += gridDim.x) {

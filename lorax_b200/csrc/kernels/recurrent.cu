@@ -44,8 +44,8 @@ constexpr int kRecStepThreads = 256;
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kRecStepThreads) rec_step_kernel(const RecParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   extern __shared__ float sm[];
   const int t = blockIdx.x, h = blockIdx.y, d = p.d, dv = p.dv;
   float* sq = sm;                 // [d]
@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(kRecStepThreads) rec_step_kernel(const RecPara
 // ------------------------------------------------------------------------------------------------
 template <typename T, int MODE, int RPT, bool STATES>
 __global__ void __launch_bounds__(256) rec_scan_kernel(const RecParams p, int tc) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   extern __shared__ float sm[];
   const int seg = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 64, d = p.d, dv = p.dv;
   const int b = p.seg_seq[seg], q0 = p.seg_q0[seg];
@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(256) rec_scan_kernel(const RecParams p, int tc
 // Second pass: the state in front of every segment of a sequence, from the segments' contributions (in place).
 template <int MODE>
 __global__ void __launch_bounds__(256) rec_carry_kernel(const RecParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x, h = blockIdx.y;
   const int e = (blockIdx.z * blockDim.x + threadIdx.x) * 4;
   const int dd = p.d * p.dv;
@@ -378,8 +378,8 @@ static int rec_launch(const RecParams& p, int what, cudaStream_t s) {
 template <typename T>
 __global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ h, const float* __restrict__ mu, T* __restrict__ shift,
                                                           T* __restrict__ out, int n_mix, int W, int Trows, StepRows rows) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int t = blockIdx.x;
   const T* prev = nullptr;
   T* keep = nullptr;
@@ -414,8 +414,8 @@ __global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ 
 
 template <typename T>
 __global__ void __launch_bounds__(256) shift_store_kernel(const T* __restrict__ h, T* __restrict__ shift, int W, StepRows rows) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x;
   const int end = rows.cu_q[b + 1];
   if (end <= rows.cu_q[b]) return;

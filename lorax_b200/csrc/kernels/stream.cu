@@ -40,8 +40,8 @@ __global__ void __launch_bounds__(128) embed_stream_kernel(const int* __restrict
                                                            int W, int V, float mult, const T* __restrict__ pos,
                                                            const int* __restrict__ positions, int P, T* __restrict__ copy,
                                                            const EmbedPairs pairs) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int t = blockIdx.x;
   const int id = min(max(ids[t], 0), V - 1);
   const int at = pos != nullptr ? min(max(positions[t], 0), P - 1) : 0;
@@ -96,8 +96,8 @@ struct NormStreamParams {
 
 template <typename T, bool PAIRS, int NV>
 __global__ void __launch_bounds__(kNsThreads) norm_stream_kernel(const NormStreamParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[kNsThreads / 32];
   const int t = p.rows != nullptr ? p.rows[blockIdx.x] : (int)blockIdx.x;
   float* res = p.residual + (long long)t * p.W;
@@ -221,8 +221,8 @@ LX_DEVICE float gate_f(float z) {
 
 template <typename T, bool PAIRS, int NV, bool NEXT>
 __global__ void __launch_bounds__(kNsThreads, NEXT && NV <= 2 ? 4 : 1) norm_add_kernel(const NormAddParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[kNsThreads / 32];
   const int t = NEXT && p.rows != nullptr ? p.rows[blockIdx.x] : (int)blockIdx.x;
   const T* y = reinterpret_cast<const T*>(p.y);
@@ -305,8 +305,8 @@ template <typename T>
 __global__ void __launch_bounds__(kNsThreads) norm_rows_kernel(const float* __restrict__ residual, const int* __restrict__ rows,
                                                                const float* __restrict__ w, const float* __restrict__ b, T* __restrict__ out,
                                                                int W, int n, float inv_n, float eps, float w_offset, int layernorm) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[kNsThreads / 32];
   const float* res = residual + (long long)(rows != nullptr ? rows[blockIdx.x] : (int)blockIdx.x) * W;
   float v[kNsMaxVec][8];
@@ -333,8 +333,8 @@ template <typename T, bool WARP>
 __global__ void __launch_bounds__(256) norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ w, const T* __restrict__ gate,
                                                         long long ldg, T* __restrict__ out, long long ldo, int groups, int group, float inv_n,
                                                         float eps, int silu) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[8];
   const int t = blockIdx.x;
   const int lane = WARP ? (threadIdx.x & 31) : threadIdx.x;
@@ -386,8 +386,8 @@ LX_DEVICE float gn_gate(float y, float z) {
 
 template <typename T, bool VEC, bool WARP>
 __global__ void __launch_bounds__(kGnThreads) gate_norm_kernel(const GateNormParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float red[kGnThreads / 32];
   const int t = blockIdx.x, lane = WARP ? threadIdx.x & 31 : threadIdx.x;
   constexpr int width = WARP ? 32 : kGnThreads;
@@ -438,8 +438,8 @@ __global__ void __launch_bounds__(kGnThreads) gate_norm_kernel(const GateNormPar
 
 template <typename T>
 __global__ void __launch_bounds__(256) tanh_kernel(T* __restrict__ x, long long n8) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     float f[8];
     load8(x + i * 8, f);
@@ -452,8 +452,8 @@ __global__ void __launch_bounds__(256) tanh_kernel(T* __restrict__ x, long long 
 // out[t, i] = act(x[t, i]) (* x[t, I + i]) for fp32 rows
 __global__ void __launch_bounds__(256) act_mul_f32_kernel(const float* __restrict__ x, float* __restrict__ out, int I, long long ldx,
                                                           long long ldo, long long total4, int act, int gated) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int per_row = I / 4;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total4; v += (long long)gridDim.x * blockDim.x) {
     const long long t = v / per_row;
@@ -480,8 +480,8 @@ __global__ void __launch_bounds__(256) act_mul_f32_kernel(const float* __restric
 template <typename T>
 __global__ void __launch_bounds__(256) clamped_swiglu_kernel(const T* __restrict__ x, T* __restrict__ out, int I, long long ldx, long long ldo,
                                                              long long total, float alpha, float limit) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int per_row = I / 8;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total; v += (long long)gridDim.x * blockDim.x) {
     const long long t = v / per_row;
@@ -501,8 +501,8 @@ __global__ void __launch_bounds__(256) clamped_swiglu_kernel(const T* __restrict
 // Greedy head over fp32 logits: arg-max (lowest index on ties) and its log-probability.
 __global__ void __launch_bounds__(512) argmax_f32_kernel(const float* __restrict__ logits, long long ld, int V, int* __restrict__ ids,
                                                          float* __restrict__ lps, float softcap) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const float* row = logits + (long long)blockIdx.x * ld;
   __shared__ float sm[16], red[16];
   __shared__ int si[16];
@@ -551,8 +551,8 @@ struct BatchedGemmParams {
 };
 
 __global__ void __launch_bounds__(256) gemm_f32_kernel(const BatchedGemmParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ float xs[16][68], ws[16][68];
   const int b = blockIdx.z, t0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
   const float* x = reinterpret_cast<const float*>(p.x) + b * p.sx;
@@ -612,8 +612,8 @@ LX_DEVICE void ldsm4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uin
 constexpr int kGhK = 64, kGhLd = kGhK + 8;      // row pitch 144 bytes: eight rows of one ldmatrix hit different banks
 
 __global__ void __launch_bounds__(128) gemm_heads_kernel(const BatchedGemmParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   __shared__ __align__(16) __nv_bfloat16 xs[2][64 * kGhLd], ws[2][64 * kGhLd];
   const int b = blockIdx.z, t0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
   const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(p.x) + b * p.sx;

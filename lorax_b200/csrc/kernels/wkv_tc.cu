@@ -90,8 +90,8 @@ struct WkSmem {
 
 template <bool STATES>
 __global__ void __launch_bounds__(kWkThreads, 2) wkv_tc_kernel(const WkvTcParams p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) uint8_t wk_raw[];
   WkSmem& sm = *reinterpret_cast<WkSmem*>(wk_raw);
   const int seg = blockIdx.x, h = blockIdx.y;

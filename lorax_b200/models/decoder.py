@@ -466,11 +466,11 @@ class DecoderModel:
                 return out
             return y if y.dtype == x.dtype else y.to(x.dtype)
         if out is not None and isinstance(w, torch.Tensor):
-            return self.ops.gemm(x, w, bias=b, out=out)
+            return self.ops.gemm(x, w, bias=b, out=out, w_const=True)
         if isinstance(w, Fp8Weight):
             y = self.ops.gemm_fp8(x if x.dtype == torch.bfloat16 or not x.is_cuda else x.to(torch.bfloat16), w.q, w.scale, bias=b)
             return y if y.dtype == x.dtype else y.to(x.dtype)
-        return self.ops.gemm(x, w, bias=b)
+        return self.ops.gemm(x, w, bias=b, w_const=True)
 
     def _linear(self, x, w, b, group: str, layer: int, inp: StepInputs, tok_slot=None, out=None):
         """Base GEMM plus the multi-adapter LoRA delta for the projection group.  On a GPU with the rows grouped by adapter
@@ -486,7 +486,7 @@ class DecoderModel:
             if lf is not None:
                 wb = w if bf16_w else self.ops.fp8_expand(w.q, w.scale)
                 if wb is not None:
-                    y = self.ops.gemm_lora_fused(x, wb, lf, bias=b, out=out)      # shrink, base GEMM and expand: one launch
+                    y = self.ops.gemm_lora_fused(x, wb, lf, bias=b, out=out, w_const=bf16_w)      # shrink, base GEMM and expand: one launch
                     if y is not None:
                         return y
         if self.adapters is not None and ts is not None:
@@ -636,7 +636,7 @@ class DecoderModel:
     def lm_head_forward(self, hidden: torch.Tensor, inp: StepInputs) -> torch.Tensor:
         c = self.config
         scale = c.logit_scale / c.logits_scaling if c.logits_scaling != 1.0 else c.logit_scale
-        logits = self.ops.gemm(hidden, self.lm_head, bias=self.lm_head_b, out_scale=scale)
+        logits = self.ops.gemm(hidden, self.lm_head, bias=self.lm_head_b, out_scale=scale, w_const=True)
         ts = inp.head_tok_slot
         if ts is not None and self.adapters is not None and self.adapters.layout.has_lm_head:
             self.adapters.apply(self.ops, hidden, logits, ts, "lm_head", 0)

@@ -185,7 +185,7 @@ class WkvMixer(Mixer):
         ops = model.ops
         mix = ops.token_shift(h, self.mu, cache["shift"], inp)                 # [5, T, W]
         r, k, v, g = ops.gemm_stack(mix[:4], self.rkvg)
-        z = ops.gemm(ops.tanh_(ops.gemm(mix[4], self.w1)), self.w2)
+        z = ops.gemm(ops.tanh_(ops.gemm(mix[4], self.w1)), self.w2, w_const=True)
         o = ops.wkv(r, k, v, z, self.w0, self.u, self.H, self.dp, cache["S"], inp)
         ops.norm_gate(o, self.dp, self.d, self.norm, g, "silu", model.eps, y)
 
@@ -267,7 +267,7 @@ class LatentAttentionMixer(Mixer):
         prep = lambda dq, norm, **q: ops.latent_prep(dq, proj["dkv"], norm, self.dkv_norm, self.q_rank, self.kv_rank, self.rot, model.eps, self.cos_sin,
                                                      inp.positions, inp.slots, cache, **q)
         if self.q_rank:
-            q = ops.gemm(prep(proj["dq"], self.dq_norm), self.uq)
+            q = ops.gemm(prep(proj["dq"], self.dq_norm), self.uq, w_const=True)
             ops.rope_pairs(q, inp.positions, self.cos_sin, self.H, self.head, self.dp, self.rot)
         else:
             q = proj["q"]
@@ -555,13 +555,13 @@ class MixerLayer:
         ops, m = model.ops, self.mixer
         h = ops.norm_stream(residual, pending, self.norm, model.eps, model.config.norm_weight_offset, model.hidden, model.dtype)
         T = h.shape[0]
-        proj = ops.gemm(h, self.in_w) if self.in_w is not None else None
+        proj = ops.gemm(h, self.in_w, w_const=True) if self.in_w is not None else None
         views = {n: proj[:, a:b] for n, (a, b) in self.parts.items()}
         y = torch.empty(T, m.out_dim + self.ff, dtype=h.dtype, device=h.device)
         m.run(model, h, views, y, inp, cache)
         if self.ff:
             ops.act_mul(views["mlp"], self.ff, model.config.hidden_act, gated=True, out=y[:, m.out_dim:])
-        return ops.gemm(y, self.out_w)
+        return ops.gemm(y, self.out_w, w_const=True)
 
 
 class DenseMlp:
@@ -592,9 +592,9 @@ class DenseMlp:
     def run_beside(self, model, h):
         """-> the same and the projection beside (or None)."""
         ops, n = model.ops, len(self.names) * self.fp
-        u = ops.gemm(h, self.up, bias=self.up_b)
+        u = ops.gemm(h, self.up, bias=self.up_b, w_const=True)
         a = ops.act_mul(u, self.fp, self.act or model.config.hidden_act, gated=self.gated, **self.act_args)
-        return ops.gemm(a, self.down), None, u[:, n:] if self.up_b is not None else None
+        return ops.gemm(a, self.down, w_const=True), None, u[:, n:] if self.up_b is not None else None
 
 
 class MoeMlp:
@@ -672,7 +672,7 @@ class MoeMlp:
         avg = max(1, (h.shape[0] * s.top + s.experts - 1) // s.experts)
         a = ops.moe_grouped_gemm(r.xg, self.up, r.seg, avg, shared=self.slices, tokens=h.shape[0],
                                  act="swiglu" if s.gated else model.config.hidden_act)
-        beside = ops.gemm(h, self.beside[0], bias=self.beside[1]) if self.beside is not None else None
+        beside = ops.gemm(h, self.beside[0], bias=self.beside[1], w_const=True) if self.beside is not None else None
         return ops.moe_grouped_gemm(a, self.down, r.seg, avg), (r.pos, r.topk_w), beside
 
 
@@ -693,10 +693,10 @@ class PreNormLayer:
         ops, m, c = model.ops, self.mixer, model.config
         norm = lambda pending, w: ops.norm_stream(residual, pending[0], w, model.eps, c.norm_weight_offset, model.hidden, model.dtype, pairs=pending[1])
         h = norm(pending, self.norm1)
-        proj = ops.gemm(h, self.in_w, bias=self.in_b)
+        proj = ops.gemm(h, self.in_w, bias=self.in_b, w_const=True)
         y = torch.empty(h.shape[0], m.out_dim, dtype=h.dtype, device=h.device)
         m.run(model, h, {n: proj[:, a:b] for n, (a, b) in self.parts.items()}, y, inp, cache)
-        pending = ops.gemm(y, self.out_w), None
+        pending = ops.gemm(y, self.out_w, w_const=True), None
         return pending if self.mlp is None else self.mlp.run(model, norm(pending, self.norm2))
 
 
@@ -715,12 +715,12 @@ class PostNormLayer:
     def forward(self, model, residual, h, inp, cache):
         """Adds both sublayers to `residual`; -> its new copy."""
         ops, m, c = model.ops, self.mixer, model.config
-        proj = ops.gemm(h, self.in_w)
+        proj = ops.gemm(h, self.in_w, w_const=True)
         y = torch.empty(h.shape[0], m.out_dim, dtype=h.dtype, device=h.device)
         m.run(model, h, {n: proj[:, a:b] for n, (a, b) in self.parts.items()}, y, inp, cache)
         add = lambda rows, norm, pairs=None: ops.norm_add(residual, rows, norm[0], norm[1], c.residual_multiplier, model.eps, model.hidden,
                                                           model.dtype, layernorm=True, pairs=pairs)
-        h = add(ops.gemm(y, self.out_w), self.norm1)
+        h = add(ops.gemm(y, self.out_w, w_const=True), self.norm1)
         if self.mlp is not None:
             rows, pairs = self.mlp.run(model, h)
             h = add(rows, self.norm2, pairs)
@@ -749,11 +749,11 @@ class SandwichLayer:
         ops, m, c = model.ops, self.mixer, model.config
         add = lambda y, w, gate, nxt, rows, pairs=None: ops.norm_add(residual, y, w, None, c.residual_multiplier, model.eps, model.hidden, model.dtype,
                                                                      layernorm=False, pairs=pairs, gate=gate, next_weight=nxt, rows=rows)
-        proj = ops.gemm(h, self.in_w, bias=self.in_b)
+        proj = ops.gemm(h, self.in_w, bias=self.in_b, w_const=True)
         views = {n: proj[:, a:b] for n, (a, b) in self.parts.items()}
         y = torch.empty(h.shape[0], m.out_dim, dtype=h.dtype, device=h.device)
         m.run(model, h, views, y, inp, cache)
-        y, gate = ops.gemm(y, self.out_w), views.get("residual_gate")
+        y, gate = ops.gemm(y, self.out_w, w_const=True), views.get("residual_gate")
         if self.mlp is None:
             return add(y, self.add1, gate, next_norm, rows)
         h = add(y, self.add1, gate, self.norm2, None)

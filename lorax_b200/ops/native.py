@@ -222,6 +222,9 @@ TC_PREFILL = os.environ.get("LORAX_TC_PREFILL", "1") != "0"       # 0: the mma.s
 FP8_EXPAND_MIN_TOKENS = int(os.environ.get("LORAX_FP8_EXPAND_MIN_TOKENS", "512"))
 
 
+MODE_CONST_WEIGHTS = 1 << 16      # of lx_gemm_bf16's mode
+
+
 class LxLoraFused(ctypes.Structure):
     """Mirror of the C struct of the same name (csrc/kernels/gemm_bf16.cu)."""
     _fields_ = [("tiles", ctypes.c_void_p), ("num_tiles", ctypes.c_int),
@@ -232,7 +235,8 @@ class LxLoraFused(ctypes.Structure):
                 ("vimg", ctypes.c_void_p), ("vimg_bytes", ctypes.c_longlong),
                 ("fence_maps", ctypes.c_int),
                 ("arena", ctypes.c_void_p), ("off_a", ctypes.c_longlong),
-                ("off_b", ctypes.c_longlong), ("arena_elems", ctypes.c_longlong), ("sync", ctypes.c_void_p)]
+                ("off_b", ctypes.c_longlong), ("arena_elems", ctypes.c_longlong), ("sync", ctypes.c_void_p),
+                ("w_const", ctypes.c_int)]
 
 
 class LoraFused(NamedTuple):
@@ -271,8 +275,9 @@ def lora_fused_desc(ws: "Workspace", lf: LoraFused, K: int) -> LxLoraFused:
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
-         out_scale: float = 1.0, mode: int = 0, force_split: int = 0) -> torch.Tensor:
-    """out[T, N] = x[T, K] @ w[N, K]^T (+ bias).  bf16 in, fp32 accumulate on tcgen05, bf16 out (fp32 in: true fp32 throughout)."""
+         out_scale: float = 1.0, mode: int = 0, force_split: int = 0, w_const: bool = False) -> torch.Tensor:
+    """out[T, N] = x[T, K] @ w[N, K]^T (+ bias).  bf16 in, fp32 accumulate on tcgen05, bf16 out (fp32 in: true fp32 throughout).
+    `w_const`: the kernel in front on the stream does not write `w` (a model's weights), which is then read while it still runs."""
     if x.dtype == torch.float32:
         return gemm_f32(x, w, out=out, out_scale=out_scale, bias=bias)
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.dim() == 2 and w.dim() == 2
@@ -287,17 +292,17 @@ def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, 
     lib = load()
     rc = lib.lx_gemm_bf16(_ptr(x), _ptr(w), _ptr(out), _ptr(bias), T, N, K, x.stride(0), w.stride(0), out.stride(0),
                           out_scale, _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.gemm_counters), _ptr(ws.status),
-                          ws.num_sms, mode, force_split, _stream())
+                          ws.num_sms, mode | (MODE_CONST_WEIGHTS if w_const else 0), force_split, _stream())
     _check(rc, "lx_gemm_bf16")
     return out
 
 
 def gemm_lora_fused(x: torch.Tensor, w: torch.Tensor, lf: LoraFused, bias: Optional[torch.Tensor] = None,
-                    out: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+                    out: Optional[torch.Tensor] = None, w_const: bool = False) -> Optional[torch.Tensor]:
     """out[T, N] = x @ w^T (+ bias) + the LoRA delta of every row's adapter in one launch of
     `gemm_bf16_tcgen05_kernel<.., true>`: its epilogue warps compute the shrink while the first K loop runs, the expand is
     added by UMMAs after the K loop of every base tile.  None when the step cannot be served this way (rank above 64, part
-    boundaries off the 128 grid, table larger than the scratch): the caller then uses the separate kernels."""
+    boundaries off the 128 grid, table larger than the scratch): the caller then uses the separate kernels.  `w_const` as for `gemm`."""
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1
     T, K = x.shape
     N = w.shape[0]
@@ -309,6 +314,7 @@ def gemm_lora_fused(x: torch.Tensor, w: torch.Tensor, lf: LoraFused, bias: Optio
     if lib.lx_lora_fused_desc_bytes() != ctypes.sizeof(LxLoraFused):
         raise NativeError("LxLoraFused: C++ and ctypes disagree")
     d = lora_fused_desc(ws, lf, K)
+    d.w_const = int(w_const)
     rc = lib.lx_gemm_bf16_lora(_ptr(x), _ptr(w), _ptr(out), _ptr(bias), T, N, K, x.stride(0), w.stride(0), out.stride(0),
                                _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.gemm_counters), _ptr(ws.status), ws.num_sms,
                                ctypes.byref(d), _stream())
