@@ -18,8 +18,9 @@
 //
 // fp8 cache (template flag KV8): pages hold e4m3 bytes in the same layout, written by `rope_kvwrite` as value / scale with one
 // scale for K and one for V per layer (the reference's k_scale / v_scale, server/lorax_server/utils/paged_attention.py:23-47).
-// A page arrives in shared memory as bytes (half the traffic of the bf16 cache, which is what bounds decode attention) and is
-// expanded to a bf16 plane before the MMAs; the K scale is folded into the softmax scale and the V scale into the output.
+// A page arrives in shared memory as bytes (half the traffic of the bf16 cache, which is what bounds decode attention); the decode
+// kernel turns them into f16 operands in registers, the prefill kernel expands them to a bf16 plane before the MMAs.  The K scale is
+// folded into the softmax scale and the V scale into the output.
 #include "attention.cuh"
 
 namespace lx {

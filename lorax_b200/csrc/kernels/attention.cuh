@@ -75,6 +75,149 @@ LX_DEVICE void expand_plane8(uint32_t dst_plane, uint32_t src8, int tid) {
   }
 }
 
+// ---- e4m3 pages in the decode kernel --------------------------------------------------------------------------------------------
+// The bytes go from shared memory straight into f16 operands (every e4m3 value is exact in f16): one conversion per pair of elements
+// and one 16-byte load per 16, no expanded plane.  (The plane cost a store and a second load of twice the bytes and four conversions
+// per pair, which bound the kernel: 32 rows of 1024 to 8192 keys took 272 us a layer, and 97 us now in one part, 83 in four; the pages'
+// bytes alone take 46.)  The orders of k in the two products are permuted the same way for both operands,
+// so that a lane's operands of several steps lie in one 16-byte chunk:
+//   Q K^T: step (h, w) gives lane column c the dimensions 64 h + 16 c + 4 w .. + 3 of a key,
+//   P V:   column n of output tile nd is dimension n * (D / 8) + nd, so a lane's dimensions of one key are contiguous.
+// 16-byte chunk j of row r of a plane of 32 rows x D bytes lies where eight lanes that read together (two keys and four chunks of K, four
+// key pairs and two chunks of V) touch eight different 16-byte bank groups.
+template <int D, bool V>
+LX_DEVICE uint32_t place8(int r, int j) {
+  constexpr int RPL = 128 / D;                                  // rows per 128-byte line
+  const int line = r / RPL, l = (r % RPL) * (D / 16) + j;
+  const int x = V ? ((r >> 1) & 3) << 1 : (D == 128 ? (r & 1) << 2 : 0);
+  return (uint32_t)(line * 128 + ((l ^ x) << 4));
+}
+// Copy one page of a head (key plane, then value plane, 32 x D bytes each, contiguous in global memory).
+template <int D>
+LX_DEVICE void load_page8(uint32_t smem_base, const uint8_t* g, int lane) {
+  constexpr int CPR = D / 16;
+#pragma unroll
+  for (int c = lane; c < kPage * CPR; c += 32) {
+    const int r = c / CPR, j = c % CPR;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_base + place8<D, false>(r, j)), "l"(g + (long long)c * 16) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                 ::"r"(smem_base + kPage * D + place8<D, true>(r, j)), "l"(g + kPage * D + (long long)c * 16) : "memory");
+  }
+}
+LX_DEVICE void mma_f16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+LX_DEVICE uint32_t e4m3x2_to_f16x2(uint32_t two) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(two & 0xffffu), __NV_E4M3);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+LX_DEVICE uint32_t pack_f16x2(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+LX_DEVICE uint4 ld_shared_16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+LX_DEVICE uint2 ld_shared_8(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+
+// The A fragments of Q in f16, each row divided by the power of two below its largest element (back in `unit`): what f16 cannot hold
+// is then below 2^-24 of that element.
+template <int D>
+LX_DEVICE void load_q8(uint32_t (&qf)[D / 16][4], float (&unit)[2], const __nv_bfloat16* q, int grows, int lane) {
+  const int c = lane & 3;
+  uint32_t raw[2][D / 64][8];                                     // (rows start on any 4-byte boundary)
+  float top[2] = {0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int row = (lane >> 2) + 8 * r;
+#pragma unroll
+    for (int h = 0; h < D / 64; ++h) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        raw[r][h][i] = row < grows ? *reinterpret_cast<const uint32_t*>(q + (long long)row * D + 64 * h + 16 * c + 2 * i) : 0u;
+        const float2 f = unpack_bf16x2(raw[r][h][i]);
+        top[r] = fmaxf(top[r], fmaxf(fabsf(f.x), fabsf(f.y)));
+      }
+    }
+    top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
+    top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
+    const uint32_t e = min(max(__float_as_uint(top[r]) >> 23, 1u), 253u);
+    unit[r] = __uint_as_float(e << 23);
+    const float inv = __uint_as_float((254u - e) << 23);
+#pragma unroll
+    for (int h = 0; h < D / 64; ++h) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {                                // word i: dimensions 2 i, 2 i + 1 of the lane's sixteen
+        const float2 f = unpack_bf16x2(raw[r][h][i]);
+        qf[4 * h + (i >> 1)][r + 2 * (i & 1)] = pack_f16x2(f.x * inv, f.y * inv);
+      }
+    }
+  }
+}
+
+// S[16, 32] = Q K^T over one e4m3 page.
+template <int D>
+LX_DEVICE void qk_page8(float (&sacc)[kPage / 8][4], const uint32_t (&qf)[D / 16][4], uint32_t k_smem, int lane) {
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < kPage / 8; ++nt) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sacc[nt][q] = 0.f;
+#pragma unroll
+    for (int h = 0; h < D / 64; ++h) {
+      const uint4 v = ld_shared_16(k_smem + place8<D, false>(nt * 8 + g, 4 * h + c));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mma_f16_16816(sacc[nt], qf[4 * h + i], e4m3x2_to_f16x2(w[i]), e4m3x2_to_f16x2(w[i] >> 16));
+    }
+  }
+}
+
+// O[16, D] += P[16, 32] V over one e4m3 page (columns permuted, see above).
+template <int D>
+LX_DEVICE void pv_page8(float (&oacc)[D / 8][4], const float (&sacc)[kPage / 8][4], uint32_t v_smem, int lane) {
+  constexpr int W = D / 32;                                        // words of a lane's dimensions of one key
+  const int g = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int kk = 0; kk < kPage / 16; ++kk) {
+    uint32_t pa[4];
+    pa[0] = pack_f16x2(sacc[2 * kk][0], sacc[2 * kk][1]);
+    pa[1] = pack_f16x2(sacc[2 * kk][2], sacc[2 * kk][3]);
+    pa[2] = pack_f16x2(sacc[2 * kk + 1][0], sacc[2 * kk + 1][1]);
+    pa[3] = pack_f16x2(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3]);
+    uint32_t v[4][W];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int key = 16 * kk + 2 * c + (q & 1) + 8 * (q >> 1);
+      if constexpr (D == 128) {
+        const uint4 x = ld_shared_16(v_smem + place8<D, true>(key, g));
+        v[q][0] = x.x; v[q][1] = x.y; v[q][2] = x.z; v[q][3] = x.w;
+      } else {
+        const uint2 x = ld_shared_8(v_smem + place8<D, true>(key, g >> 1) + (g & 1) * 8);
+        v[q][0] = x.x; v[q][1] = x.y;
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const uint32_t a0 = __byte_perm(v[0][w], v[1][w], 0x5140), a1 = __byte_perm(v[0][w], v[1][w], 0x7362);
+      const uint32_t b0 = __byte_perm(v[2][w], v[3][w], 0x5140), b1 = __byte_perm(v[2][w], v[3][w], 0x7362);
+      mma_f16_16816(oacc[4 * w], pa, e4m3x2_to_f16x2(a0), e4m3x2_to_f16x2(b0));
+      mma_f16_16816(oacc[4 * w + 1], pa, e4m3x2_to_f16x2(a0 >> 16), e4m3x2_to_f16x2(b0 >> 16));
+      mma_f16_16816(oacc[4 * w + 2], pa, e4m3x2_to_f16x2(a1), e4m3x2_to_f16x2(b1));
+      mma_f16_16816(oacc[4 * w + 3], pa, e4m3x2_to_f16x2(a1 >> 16), e4m3x2_to_f16x2(b1 >> 16));
+    }
+  }
+}
+
 // S[16, NKEYS] (+)= Q[16, D] K[NKEYS, D]^T for one warp.  qf holds the A fragments of Q.
 template <int D, int NKEYS>
 LX_DEVICE void qk_tile(float (&sacc)[NKEYS / 8][4], const uint32_t (&qf)[D / 16][4], uint32_t k_smem, int lane) {
@@ -214,7 +357,7 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
   constexpr int PLANE = kPage * DK * 2, VPLANE = kPage * DV * 2;
   constexpr int PLANE8 = kPage * DK;
   constexpr int STAGE = KV8 ? 2 * PLANE8 : PLANE + VPLANE;
-  constexpr int WARP_BYTES = STAGES * STAGE + (KV8 ? 2 * PLANE : 0);     // fp8: staged bytes + one expanded K and V plane
+  constexpr int WARP_BYTES = STAGES * STAGE;
   const int t = blockIdx.x;
   const int kvh = blockIdx.y / p.gchunks, gc = blockIdx.y % p.gchunks;
   const int split = blockIdx.z;
@@ -229,8 +372,11 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
   const int page_lo = key_lo / kPage;
   const int page_hi = ctx > 0 ? (ctx + kPage - 1) / kPage : 0;
   const int npages = max(page_hi - page_lo, 0);
-  const int per_split = (npages + p.nsplit - 1) / p.nsplit;
-  const int pb = page_lo + split * per_split;
+  // A split has eight pages at least where rows and heads alone give every SM a CTA, otherwise one for every warp: the later splits of a
+  // short context have nothing to do.
+  const int least = p.nsplit == 1 ? 1 : (gridDim.x * gridDim.y >= 148 ? 8 : NW);
+  const int per_split = max((npages + p.nsplit - 1) / p.nsplit, least);
+  const int pb = min(page_lo + split * per_split, page_hi);
   const int pe = min(pb + per_split, page_hi);
 
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
@@ -240,7 +386,10 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
 
   // Q fragments straight from global memory (row = head in group, zero beyond the group).
   uint32_t qf[DK / 16][4];
-  {
+  float unit[2] = {1.f, 1.f};
+  if constexpr (KV8) {
+    load_q8<DK>(qf, unit, p.q + (long long)t * p.ldq + (long long)head0 * DK, grows, lane);
+  } else {
     const int r0 = lane >> 2, r1 = r0 + 8;
     const __nv_bfloat16* q0 = p.q + (long long)t * p.ldq + (long long)(head0 + r0) * DK;
     const __nv_bfloat16* q1 = p.q + (long long)t * p.ldq + (long long)(head0 + r1) * DK;
@@ -255,7 +404,6 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
   }
 
   const uint32_t wbase = smem_u32(dsm) + warp * WARP_BYTES;
-  const uint32_t wwork = wbase + STAGES * STAGE;
   const int* bt = p.block_tables + (long long)t * p.max_blocks;
   float slope0 = 0.f, slope1 = 0.f;
   if (p.alibi != nullptr) {
@@ -273,7 +421,7 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
       const uint32_t sb = wbase + (i % STAGES) * STAGE;
       if constexpr (KV8) {
         const uint8_t* src = reinterpret_cast<const uint8_t*>(p.kv) + ((blk * p.nkv + kvh) * 2) * (long long)(kPage * DK);
-        load_plane8<DK, 2 * kPage, 32>(sb, src, lane, true);            // the K plane and the V plane are one contiguous run
+        load_page8<DK>(sb, src, lane);
       } else {
         const __nv_bfloat16* src = p.kv + (blk * p.nkv + kvh) * (long long)(kPage * (DK + DV));
         load_plane<DK, kPage, 32>(sb, src, lane, true);
@@ -289,18 +437,22 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
     issue(i + STAGES - 1);
     cp_async_wait<STAGES - 1>();
     __syncwarp();
-    uint32_t sb = wbase + (i % STAGES) * STAGE;
-    if constexpr (KV8) {
-      expand_plane8<DK, kPage, 32>(wwork, sb, lane);
-      expand_plane8<DK, kPage, 32>(wwork + PLANE, sb + PLANE8, lane);
-      __syncwarp();
-      sb = wwork;
-    }
+    const uint32_t sb = wbase + (i % STAGES) * STAGE;
     const int page = my_first + NW * i;
     float sacc[kPage / 8][4];
-    qk_tile<DK, kPage>(sacc, qf, sb, lane);
+    if constexpr (KV8) {
+      qk_page8<DK>(sacc, qf, sb, lane);
+#pragma unroll
+      for (int nt = 0; nt < kPage / 8; ++nt) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sacc[nt][q] *= unit[q >> 1];
+      }
+    } else {
+      qk_tile<DK, kPage>(sacc, qf, sb, lane);
+    }
     softmax_tile<DV, kPage>(sacc, oacc, m, l, page * kPage, key_lo, ctx, key_lo, ctx, p.scale, p.softcap, lane, slope0, slope1);
-    pv_tile<DV, kPage, WIDE>(oacc, sacc, sb + PLANE, lane);
+    if constexpr (KV8) pv_page8<DV>(oacc, sacc, sb + PLANE8, lane);
+    else pv_tile<DV, kPage, WIDE>(oacc, sacc, sb + PLANE, lane);
     __syncwarp();
   }
   cp_async_wait<0>();
@@ -340,7 +492,10 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
     for (int w = 0; w < NW; ++w) {
       const float mw = sm[w * 16 + g];
       const float wgt = (mw == -INFINITY) ? 0.f : exp2f((mw - M) * kLog2e);
-      const float2 v = *reinterpret_cast<const float2*>(so + (w * 16 + g) * DV + d);
+      const float* row = so + (w * 16 + g) * DV;
+      float2 v;
+      if constexpr (KV8) v = make_float2(row[(d % (DV / 8)) * 8 + d / (DV / 8)], row[((d + 1) % (DV / 8)) * 8 + d / (DV / 8)]);
+      else v = *reinterpret_cast<const float2*>(row + d);
       num.x += wgt * v.x;
       num.y += wgt * v.y;
       den += wgt * sl[w * 16 + g];
@@ -552,7 +707,7 @@ inline int attn_opt_in(K kernel, int smem, bool (&configured)[64]) {
 
 template <int DK, int DV, int STAGES, bool KV8, int NW, bool WIDE = false>
 static int launch_decode_nw(const DecodeParams& p, int T, cudaStream_t s) {
-  constexpr int SMEM = KV8 ? NW * (STAGES * 2 * kPage * DK + 2 * kPage * DK * 2) : NW * STAGES * kPage * (DK + DV) * 2;
+  constexpr int SMEM = KV8 ? NW * STAGES * 2 * kPage * DK : NW * STAGES * kPage * (DK + DV) * 2;
   static_assert(SMEM >= (NW * 16 * DV + 2 * NW * 16) * 4, "combine buffer must fit in the pipeline buffers");
   static bool configured[64] = {false};          // the shared-memory opt-in is a per-device attribute
   if (int rc = attn_opt_in(attn_decode_kernel<DK, DV, STAGES, KV8, NW, WIDE>, SMEM, configured)) return rc;

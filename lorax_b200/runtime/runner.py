@@ -309,9 +309,7 @@ class ModelRunner:
             tok_slot = cat([st.tok_slot[:nd], p_tok])
             head_slot = cat([st.tok_slot[:nd], p_head])
             tiles = pin.lora_tiles
-        nsplit = 1
-        if self.is_cuda and nd * self.model.nkv < 96:
-            nsplit = max(1, min(8, 192 // max(nd * self.model.nkv, 1)))
+        nsplit = self._attn_splits(nd)
         head = cat([torch.arange(nd, dtype=torch.int32, device=dev), pin.lm_head_indices + nd])
         inp = StepInputs(input_ids=cat([st.input_ids[:nd], pin.input_ids]), positions=cat([st.positions[:nd], pin.positions]),
                          slots=cat([st.slots[:nd], pin.slots]), is_prefill=True, block_tables=pin.block_tables, cu_q=pin.cu_q,
@@ -433,9 +431,7 @@ class ModelRunner:
 
     def _decode_body(self, b: int, lora: bool, need_logits: bool = False):
         st = self.state
-        nsplit = 1
-        if self.is_cuda and b * self.model.nkv < 96:
-            nsplit = max(1, min(8, 192 // max(b * self.model.nkv, 1)))
+        nsplit = self._attn_splits(b)
         # the table always has max_batch rows; a graph launches one CTA per possible tile of the bucket (unused: slot -1)
         tiles = LoraTiles(st.lora_tiles, b, 32, live=st.num_lora_tiles) if (lora and self.tiles_valid) else None
         fused = self.model.tp.fused if self.model.tp.world_size > 1 else None
@@ -452,6 +448,18 @@ class ModelRunner:
         else:
             self.model.ops.argmax_logprob(logits, st.next_ids[:b], st.logprobs[:b], softcap=self.model.config.final_logit_softcapping or 0.0)
         return logits
+
+    def _attn_splits(self, rows: int) -> int:
+        """Parts that decode attention cuts a row's keys into.  Few rows: as many as give the GPU a CTA per SM and more.  From one CTA per
+        (row, KV head) and SM on, contexts of unequal length leave SMs idle at the end: four parts each took 32 rows of 1024 to 8192 keys
+        from 152 to 122 us and 48 rows of 256 to 2048 from 62 to 55 us (parts of fewer than 256 keys are not made).  Where rows and heads
+        alone are several waves (64 rows of 8 heads: 46 us with one part, 52 with four) the second pass over the parts costs more."""
+        if not self.is_cuda:
+            return 1
+        ctas = rows * self.model.nkv
+        if ctas < 96:
+            return max(1, min(8, 192 // max(ctas, 1)))
+        return 4 if 148 <= ctas < 512 else 1
 
     def _advance(self, b: int):
         st = self.state

@@ -337,6 +337,29 @@ def test_attn_prefill_tensor_core(nat, nh, nkv, window, softcap, q_lens, cache_l
         assert torch.isfinite(got.float()).all()
 
 
+@pytest.mark.parametrize("B,nh,nkv,d,window,softcap,nsplit", [(5, 8, 8, 128, 0, 0.0, 1), (3, 32, 8, 128, 50, 0.0, 8), (40, 32, 8, 128, 0, 20.0, 4),
+                                                            (6, 20, 1, 64, 0, 0.0, 2), (38, 16, 8, 64, 33, 0.0, 1), (2, 34, 2, 128, 0, 0.0, 1)])
+def test_attn_decode_fp8_pages(nat, B, nh, nkv, d, window, softcap, nsplit):
+    """Contexts around the edges of pages and of splits, groups of one to twenty heads, both CTA sizes, query rows that start on any 4-byte
+    boundary and of any magnitude.  Weights and results are rounded to bf16 (2^-9 each, relatively)."""
+    max_len = 700
+    wide, bt = _make_cache(B, max_len, nkv, d, seed=B + d)
+    cache = wide.to(torch.float8_e4m3fn)
+    ctx = torch.randint(1, max_len, (B,), device="cuda", dtype=torch.int32)
+    ctx[:2] = torch.tensor([1, 32])
+    ctx[-1] = 33 if B > 2 else 64
+    ldq = nh * d + 6
+    q = torch.randn(B, ldq, device="cuda", dtype=torch.bfloat16)[:, 2: 2 + nh * d]
+    q[0] *= 2.0 ** 20
+    q[1] *= 2.0 ** -60
+    q[-1, ::7] *= 2.0 ** -20
+    got = nat.attn_decode(q, cache, bt, ctx, nh, nkv, d, d ** -0.5, window, softcap, nsplit, kv_scale=(0.5, 0.25))
+    want = ref.attn_decode(q, cache, bt, ctx, nh, nkv, d, d ** -0.5, window, softcap, kv_scale=(0.5, 0.25))
+    assert torch.isfinite(got).all()
+    for b in range(B):
+        assert _rel_err(got[b], want[b]) < 6e-3, (b, int(ctx[b]))
+
+
 @pytest.mark.parametrize("nh,nkv,d,nsplit", [(12, 12, 64, 1), (32, 8, 128, 3), (6, 6, 128, 1)])
 def test_attn_alibi(nat, nh, nkv, d, nsplit):
     """ALiBi slopes in both attention kernels (BLOOM, MPT): bias -slope_h * (query position - key position)."""
