@@ -30,6 +30,7 @@ from .lora import LM_HEAD, BlobLayout, LoraConfig, ModuleMap, check_architecture
 
 TMAP_GROUPS = ("qkv", "o", "gate_up", "down", LM_HEAD)     # index of a group inside a slot's tensor-map row
 TMAP_BYTES = 128
+SHORT_STEP = 512        # rows up to which the shrink is a matter of latency (mma.sync from the blobs) and not of tensor-core rate
 
 
 @dataclass
@@ -311,7 +312,10 @@ class AdapterManager:
         if tiles is not None:
             if tiles.num_tiles == 0:
                 return None
-            if self.is_cuda:
+            if self.is_cuda and x.shape[0] <= SHORT_STEP and tiles.max_rows <= 32:
+                v = ops.lora_shrink_mma(x, tiles.table, tiles.num_tiles, self.arena, self.slot_base, self.slot_rank, offA, nparts, self.max_rank,
+                                        live_tiles=tiles.live)
+            elif self.is_cuda:
                 v = ops.lora_shrink_tiles(x, tiles.table, tiles.num_tiles, tiles.max_rows, self.slot_tmaps, self.groups_per_slot,
                                           TMAP_GROUPS.index(group), self.slot_rank, nparts, 0 if group == LM_HEAD else layer, self.max_rank,
                                           live_tiles=tiles.live)

@@ -326,6 +326,23 @@ LX_DEVICE float warp_max(float v) {
   return v;
 }
 
+// ------------------------------------------------------------------------------------------------
+// thread-block clusters
+// ------------------------------------------------------------------------------------------------
+LX_DEVICE uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Barrier over the cluster's CTAs; what was written to shared memory before it is visible to all of them after it.
+LX_DEVICE void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+LX_DEVICE void cluster_store_f32(uint32_t smem_addr, uint32_t rank, float v) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}"
+               ::"r"(smem_addr), "r"(rank), "f"(v) : "memory");
+}
+
 // cp.async (LDGSTS) 16-byte copy with zero fill when !valid.
 LX_DEVICE void cp_async_16(void* smem_dst, const void* gsrc, bool valid) {
   int sz = valid ? 16 : 0;

@@ -375,20 +375,6 @@ LX_DEVICE void argmax_take(ArgmaxPart& a, float (&x)[N], int i, float softcap) {
   for (int q = 0; q < N; ++q) a.s += __expf(x[q] - m);
 }
 
-LX_DEVICE uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Barrier over the cluster's CTAs; what was written to shared memory before it is visible to all of them after it.
-LX_DEVICE void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-LX_DEVICE void cluster_store_f32(uint32_t smem_addr, uint32_t rank, float v) {
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}"
-               ::"r"(smem_addr), "r"(rank), "f"(v) : "memory");
-}
-
 constexpr int kArgmaxMaxParts = 8;
 
 // VEC: rows start on 16-byte boundaries.

@@ -85,9 +85,24 @@ gemm_fp8_block128_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
+  // The weights' half of the first stages is loaded before the wait for the kernel in front: that is the activations' quantiser, which has
+  // itself waited for whatever may have written the weights.
+  const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
+  int preloaded = 0;
+  if (threadIdx.x == 0 && (int)blockIdx.x < num_tiles * p.ksplit) {
+    const int tile = blockIdx.x / p.ksplit, split = blockIdx.x % p.ksplit;
+    const int kb0 = (int)((long long)kblocks * split / p.ksplit), kb1 = (int)((long long)kblocks * (split + 1) / p.ksplit);
+    preloaded = min(STAGES, kb1 - kb0);
+    for (int s = 0; s < preloaded; ++s) {
+      mbar_expect_tx(&full_bar[s], (uint32_t)(S::kABytes + p.bn * kF8BK));
+      tma_load_2d_hint(smem + s * S::kStageBytes, &tmap_w, &full_bar[s], (kb0 + s) * kF8BK, tile / tiles_b * kF8BM, pol_w);
+    }
+  }
+  pdl_wait();
+  pdl_trigger();
+
   if (warp == 0) {
     if (lane == 0) {
-      const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < num_tiles * p.ksplit && ok; w += gridDim.x) {
@@ -95,10 +110,14 @@ gemm_fp8_block128_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         const int ta = tile / tiles_b, tb = tile % tiles_b;    // token tiles of one weight tile run side by side
         const int kb0 = (int)((long long)kblocks * split / p.ksplit), kb1 = (int)((long long)kblocks * (split + 1) / p.ksplit);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { report_status(p.status, kTimeoutEmptyBarrier, w); *abort_flag = 1; ok = false; break; }
           uint8_t* sa = smem + stage * S::kStageBytes;
-          mbar_expect_tx(&full_bar[stage], (uint32_t)(S::kABytes + p.bn * kF8BK));
-          tma_load_2d_hint(sa, &tmap_w, &full_bar[stage], kb * kF8BK, ta * kF8BM, pol_w);
+          if (preloaded > 0) {
+            --preloaded;
+          } else {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { report_status(p.status, kTimeoutEmptyBarrier, w); *abort_flag = 1; ok = false; break; }
+            mbar_expect_tx(&full_bar[stage], (uint32_t)(S::kABytes + p.bn * kF8BK));
+            tma_load_2d_hint(sa, &tmap_w, &full_bar[stage], kb * kF8BK, ta * kF8BM, pol_w);
+          }
           tma_load_2d_hint(sa + S::kABytes, &tmap_x, &full_bar[stage], kb * kF8BK, tb * p.bn, pol_x);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -214,6 +233,8 @@ gemm_fp8_block128_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 // x[T, K] bf16 -> xq[T, K] e4m3 and sa[kb, t] = amax(x[t, block kb]) / 448.  One warp per (token, K block).
 __global__ void __launch_bounds__(256) quant_act_fp8_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
                                                             long long ldq, float* __restrict__ sa, int ld_sa, int T, int K) {
+  pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const int kblocks = (K + 127) / 128;
   const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (item >= (long long)T * kblocks) return;
@@ -247,6 +268,8 @@ __global__ void __launch_bounds__(256) quant_act_fp8_kernel(const __nv_bfloat16*
 // out[t, n] = bf16(sum_s partial[s, t, n] + bias[n]): the K splits in split order.
 __global__ void __launch_bounds__(256) fp8_splitk_reduce_kernel(const float* __restrict__ partial, int ksplit, int T, int N,
                                                                 const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, long long ldo) {
+  pdl_wait();      // every block waits, also those that return early below
+  pdl_trigger();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= (long long)T * N) return;
   const int t = (int)(i / N), n = (int)(i % N);
@@ -292,7 +315,7 @@ static int launch_fp8(const CUtensorMap& tw, const CUtensorMap& tx, const Fp8Par
     if (e != cudaSuccess) return -(int)e;
     configured = true;
   }
-  gemm_fp8_block128_kernel<BN, STAGES><<<grid, kF8Threads, S::kTotal, stream>>>(tw, tx, p);
+  launch_pdl(gemm_fp8_block128_kernel<BN, STAGES>, dim3(grid), dim3(kF8Threads), (size_t)S::kTotal, stream, tw, tx, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -306,8 +329,8 @@ int lx_quant_act_fp8(const void* x, long long ldx, void* xq, long long ldq, floa
   if (T <= 0) return 0;
   if (K % 4 != 0 || ldx % 4 != 0 || ldq % 4 != 0) return -1;
   const long long items = (long long)T * ((K + 127) / 128);
-  lx::quant_act_fp8_kernel<<<(unsigned)((items + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<uint8_t*>(xq), ldq, sa, ld_sa, T, K);
+  lx::launch_pdl(lx::quant_act_fp8_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+                 reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<uint8_t*>(xq), ldq, sa, ld_sa, T, K);
   return -(int)cudaGetLastError();
 }
 
@@ -350,7 +373,7 @@ int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_
   else rc = launch_fp8<128, 6>(tw, tx, p, grid, stream);
   if (rc != 0 || ks == 1) return rc;
   const long long total = (long long)T * N;
-  fp8_splitk_reduce_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(p.partial, ks, T, N, p.bias, p.out, ldo);
+  launch_pdl(fp8_splitk_reduce_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, p.partial, ks, T, N, p.bias, p.out, ldo);
   return -(int)cudaGetLastError();
 }
 

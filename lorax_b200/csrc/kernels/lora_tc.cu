@@ -223,6 +223,135 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const ShrinkTc
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_d, kCols); }
 }
 
+// ------------------------------------------------------------------------------------------------ shrink of short steps
+// v[row, j] = x[row] . A_cat(slot)[j] for tiles of at most 32 rows, by mma.sync with operands straight from global memory.
+//
+// With a few rows per adapter the work is a chain of latencies: table entry, slot, first bytes, sum.  The tensor-core kernel above adds a
+// descriptor fetch and fence, TMA, UMMA, tensor memory and partial sums that meet in global memory behind a counter (10 us for five rows
+// over three adapters of rank 16, 17 to 23 us for 32 rows over 24 of rank 32).  Here a cluster of up to eight CTAs cuts K, the four warps
+// of a CTA cut its part, every lane has 16 to 24 loads of 16 bytes in flight, and the parts meet in distributed shared memory; A_cat is on its way before the wait for the kernel in front.  Five rows: 4 us; 32 rows: 4 to 9 us.
+//
+// A CTA takes 16 rows of A_cat (j0 ..) and the tile's rows in groups of eight (one group, or four).  The order of k inside a block of 32
+// is permuted the same way for both operands: lane column t holds elements 8 t .. 8 t + 7.
+struct ShrinkRowsParams {
+  const LoraTile* tiles;
+  const __nv_bfloat16* x;
+  long long ldx;
+  const __nv_bfloat16* arena;
+  const long long* slot_base;
+  const int* slot_rank;
+  int num_slots;
+  long long unit_off;
+  int nparts;
+  float* v;
+  int ldv;
+  int K, T;
+  int* status;
+};
+
+constexpr int kSrThreads = 128;
+constexpr int kSrMaxParts = 8;          // CTAs of a cluster
+
+LX_DEVICE void mma_bf16_16816_lora(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Blocks kb0 + warp, + 4, .. below kb1 of the products; sums of this warp into red[warp][16][8 NG].
+template <int NG, int SB>
+LX_DEVICE void shrink_rows_part(const ShrinkRowsParams& p, const __nv_bfloat16* a, int rows_a, int row0, int nrows, int kb0, int kb1, float* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int K8 = p.K >> 3;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const uint4* a0 = reinterpret_cast<const uint4*>(a + (long long)g * p.K);
+  const uint4* a1 = reinterpret_cast<const uint4*>(a + (long long)(g + 8) * p.K);
+  float acc[NG][4];
+#pragma unroll
+  for (int q = 0; q < NG; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
+  bool waited = false;
+  for (int kb = kb0 + warp; kb < kb1 || !waited; kb += 4 * SB) {
+    uint4 ra[SB], rb[SB], rx[NG][SB];
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      const int kk = (kb + 4 * i) * 4 + t;                          // 16-byte index inside a row
+      const bool in = kb + 4 * i < kb1 && kk < K8;
+      ra[i] = in && g < rows_a ? __ldg(a0 + kk) : zero;
+      rb[i] = in && g + 8 < rows_a ? __ldg(a1 + kk) : zero;
+    }
+    if (!waited) {                                                  // (A_cat was written by copies in front of the step; x by the kernel in front)
+      pdl_wait();
+      pdl_trigger();
+      waited = true;
+    }
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      const int kk = (kb + 4 * i) * 4 + t;
+      const bool in = kb + 4 * i < kb1 && kk < K8;
+#pragma unroll
+      for (int q = 0; q < NG; ++q) {
+        const int row = q * 8 + g;
+        rx[q][i] = in && row < nrows ? reinterpret_cast<const uint4*>(p.x + (long long)(row0 + row) * p.ldx)[kk] : zero;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+#pragma unroll
+      for (int q = 0; q < NG; ++q) {
+        mma_bf16_16816_lora(acc[q], ra[i].x, rb[i].x, ra[i].y, rb[i].y, rx[q][i].x, rx[q][i].y);
+        mma_bf16_16816_lora(acc[q], ra[i].z, rb[i].z, ra[i].w, rb[i].w, rx[q][i].z, rx[q][i].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {                                    // (rank g, rows 2t, 2t + 1) and (rank g + 8, the same rows) of every group
+    float* mine = red + (warp * 16 + g) * (8 * NG) + q * 8 + 2 * t;
+    *reinterpret_cast<float2*>(mine) = make_float2(acc[q][0], acc[q][1]);
+    *reinterpret_cast<float2*>(mine + 8 * 8 * NG) = make_float2(acc[q][2], acc[q][3]);
+  }
+}
+
+__global__ void __launch_bounds__(kSrThreads) lora_shrink_mma_kernel(const ShrinkRowsParams p) {
+  __shared__ __align__(16) float red[4 * 16 * 32];
+  __shared__ float gathered[kSrMaxParts][16 * 32];                  // (of the cluster's first CTA)
+  const int part = blockIdx.x, parts = gridDim.x;
+  const LoraTile tile = p.tiles[blockIdx.y];                        // (a cluster has one tile: its CTAs leave together)
+  const int nrows = min(min(tile.nrows, 32), p.T - tile.row0);      // a table may be older than the batch: rows past T are gone
+  const bool known = tile.slot >= 0 && tile.slot < p.num_slots;
+  const int r = known ? p.slot_rank[tile.slot] : 0;
+  const long long base = known ? p.slot_base[tile.slot] : -1;
+  const int j0 = blockIdx.z * 16, rows_a = min(16, r * p.nparts - j0);
+  if (nrows <= 0 || base < 0 || rows_a <= 0) {
+    pdl_wait();      // every block waits
+    if (tile.slot >= p.num_slots && nrows > 0 && threadIdx.x == 0) report_status(p.status, kBadIndex, tile.slot);
+    return;
+  }
+  const __nv_bfloat16* a = p.arena + base + (long long)r * p.unit_off + (long long)j0 * p.K;
+  const int blocks = (p.K + 31) / 32;
+  const int kb0 = (int)((long long)blocks * part / parts), kb1 = (int)((long long)blocks * (part + 1) / parts);
+  const int width = nrows <= 8 ? 8 : 32;                            // rows that `red` holds
+  if (nrows <= 8) shrink_rows_part<1, 8>(p, a, rows_a, tile.row0, nrows, kb0, kb1, red);
+  else shrink_rows_part<4, 4>(p, a, rows_a, tile.row0, nrows, kb0, kb1, red);
+  __syncthreads();
+  if (parts > 1) cluster_sync();                                    // every CTA of the cluster has started: its shared memory may be written
+  const uint32_t to = smem_u32(&gathered[cluster_rank()][0]);
+  for (int e = threadIdx.x; e < 16 * width; e += kSrThreads) {      // e = rank * width + row
+    const float s = red[e] + red[16 * width + e] + red[2 * 16 * width + e] + red[3 * 16 * width + e];
+    if (parts > 1) cluster_store_f32(to + e * 4, 0, s);
+    else gathered[0][e] = s;
+  }
+  if (parts > 1) cluster_sync();
+  else __syncthreads();
+  if (part != 0) return;
+  for (int e = threadIdx.x; e < 16 * width; e += kSrThreads) {      // (neighbouring threads write neighbouring ranks of a row)
+    const int j = e & 15, row = e >> 4;
+    if (j >= rows_a || row >= nrows) continue;
+    float s = 0.f;
+    for (int c = 0; c < parts; ++c) s += gathered[c][j * width + row];
+    p.v[(long long)(tile.row0 + row) * p.ldv + j0 + j] = s;
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ expand
 struct ExpandTiledParams {
   const LoraTile* tiles;
@@ -245,6 +374,7 @@ constexpr int kExpCols = 4;                          // adjacent output features
 constexpr int kExpBlockCols = kExpThreads * kExpCols;
 constexpr int kExpMaxRows = 128;                     // rows of a tile staged at once
 constexpr int kExpStage = 16;                        // ranks per pass
+constexpr int kExpCtas = 2;                          // per SM
 constexpr int kExpRowsInFlight = 4;                  // rows whose y loads are issued together
 
 // One unit of work = one tile (a run of rows of one adapter) x 1024 output features.  A thread keeps the B_cat rows
@@ -255,41 +385,56 @@ constexpr int kExpRowsInFlight = 4;                  // rows whose y loads are i
 //
 // The grid is a fixed number of CTAs that walk the units; live tiles come first in the table, so the walk stops at
 // the first dead one and padding entries cost nothing.
-__global__ void __launch_bounds__(kExpThreads, 2) lora_expand_tiled_kernel(const ExpandTiledParams p) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+//
+// The table, the slots' offsets and B_cat were written by copies in front of the step, so the first unit's are read before the wait for the
+// kernel in front, and the next unit's entry while the current one is multiplied.
+__global__ void __launch_bounds__(kExpThreads, kExpCtas) lora_expand_tiled_kernel(const ExpandTiledParams p) {
   __shared__ __align__(16) float vs[kExpMaxRows * 3 * kExpStage];   // [row][part][16]
   const int nparts = p.n1 < p.N ? 3 : (p.n0 < p.N ? 2 : 1);
-  for (int w = blockIdx.x; w < p.num_tiles * p.col_blocks; w += gridDim.x) {
-    const LoraTile tile = p.tiles[w / p.col_blocks];
+  const int units = p.num_tiles * p.col_blocks;
+  const LoraTile dead{-1, 0, 0, 0};
+  auto known = [&](const LoraTile& t) { return t.slot >= 0 && t.slot < p.num_slots; };
+  // entry, rank and offset of the unit at hand and (two loads that hang on one another) of the next one
+  LoraTile tile = (int)blockIdx.x < units ? p.tiles[blockIdx.x / p.col_blocks] : dead;
+  int r = known(tile) ? p.slot_rank[tile.slot] : 0;
+  long long base = known(tile) ? p.slot_base[tile.slot] : -1;
+  uint4 bw[kExpCols][kExpStage / 8];
+  auto load_b = [&](int n, int jc) {         // ranks jc .. jc + 15 of the thread's features (zeros past the rank)
+    const __nv_bfloat16* B = p.arena + base + (long long)r * p.unit_off + (long long)n * r;
+#pragma unroll
+    for (int c = 0; c < kExpCols; ++c) {
+#pragma unroll
+      for (int h = 0; h < kExpStage / 8; ++h) {
+        bw[c][h] = make_uint4(0u, 0u, 0u, 0u);
+        if (n < p.N && jc + h * 8 < r) bw[c][h] = __ldg(reinterpret_cast<const uint4*>(B + (long long)c * r + jc + h * 8));
+      }
+    }
+  };
+  auto first_col = [&](int w) { return (w % p.col_blocks) * kExpBlockCols + (int)threadIdx.x * kExpCols; };
+  if (base >= 0 && r > 0 && tile.nrows > 0) load_b(first_col(blockIdx.x), 0);
+  pdl_wait();      // every block waits, also those that have nothing to do
+  pdl_trigger();
+  LoraTile ntile = dead;
+  int nr = 0;
+  long long nbase = -1;
+  for (int w = blockIdx.x; w < units; w += gridDim.x, tile = ntile, r = nr, base = nbase) {
     if (tile.slot < 0) break;
-    if (tile.nrows <= 0) continue;
-    if (tile.slot >= p.num_slots) {
-      if (threadIdx.x == 0) report_status(p.status, kBadIndex, tile.slot);
+    ntile = w + (int)gridDim.x < units ? p.tiles[(w + gridDim.x) / p.col_blocks] : dead;
+    if (tile.slot >= p.num_slots && threadIdx.x == 0) report_status(p.status, kBadIndex, tile.slot);
+    const int nrows = min(min(tile.nrows, kExpMaxRows), p.T - tile.row0);
+    if (base < 0 || r <= 0 || nrows <= 0) {
+      nr = known(ntile) ? p.slot_rank[ntile.slot] : 0;
+      nbase = known(ntile) ? p.slot_base[ntile.slot] : -1;
       continue;
     }
-    const int r = p.slot_rank[tile.slot];
-    const long long base = p.slot_base[tile.slot];
-    if (base < 0 || r <= 0) continue;
-    const int n = (w % p.col_blocks) * kExpBlockCols + threadIdx.x * kExpCols;
+    const int n = first_col(w);
     const bool col_ok = n < p.N;                        // N is a multiple of 4: a thread's four features are all in or all out
     const int part = n < p.n0 ? 0 : (n < p.n1 ? 1 : 2);
-    const __nv_bfloat16* B = p.arena + base + (long long)r * p.unit_off + (long long)n * r;
-    const int nrows = min(min(tile.nrows, kExpMaxRows), p.T - tile.row0);
-    if (nrows <= 0) continue;
     __nv_bfloat16* yrow0 = p.y + (long long)tile.row0 * p.ldy + n;
 
     for (int jc = 0; jc < r; jc += kExpStage) {
       const int rs = min(kExpStage, r - jc);            // 8 or 16 live ranks in this pass
-      uint4 bw[kExpCols][kExpStage / 8];
-#pragma unroll
-      for (int c = 0; c < kExpCols; ++c) {
-#pragma unroll
-        for (int h = 0; h < kExpStage / 8; ++h) {
-          bw[c][h] = make_uint4(0u, 0u, 0u, 0u);
-          if (col_ok && h * 8 < rs) bw[c][h] = __ldg(reinterpret_cast<const uint4*>(B + (long long)c * r + jc + h * 8));
-        }
-      }
+      if (jc > 0 || w != (int)blockIdx.x) load_b(n, jc);
       uint2 old[kExpRowsInFlight];
 #pragma unroll
       for (int u = 0; u < kExpRowsInFlight; ++u) {
@@ -301,6 +446,10 @@ __global__ void __launch_bounds__(kExpThreads, 2) lora_expand_tiled_kernel(const
         const int j = e % kExpStage, pr = e / kExpStage;
         const int pp = pr % nparts, m = pr / nparts;
         vs[(m * 3 + pp) * kExpStage + j] = (j < rs) ? p.v[(long long)(tile.row0 + m) * p.ldv + pp * r + jc + j] : 0.f;
+      }
+      if (jc == 0) {
+        nr = known(ntile) ? p.slot_rank[ntile.slot] : 0;
+        nbase = known(ntile) ? p.slot_base[ntile.slot] : -1;
       }
       __syncthreads();
       if (col_ok) {
@@ -451,6 +600,29 @@ int lx_lora_shrink_tc(const void* x, long long ldx, const void* tiles, int num_t
   return launch_shrink_tc<128>(tx, p, num_tiles, chunks, s);
 }
 
+// The same for tiles of at most 32 rows of a short step (see lora_shrink_mma_kernel).  live_tiles: entries that are not padding.
+int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_tiles, int live_tiles, const void* arena, const long long* slot_base,
+                       const int* slot_rank, int num_slots, long long unit_off, int nparts, float* v, int ldv, int T, int K, int max_rank,
+                       int* status, void* stream) {
+  using namespace lx;
+  if (num_tiles <= 0 || max_rank <= 0) return 0;
+  if (K % 8 != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0 || nparts * max_rank > ldv || num_tiles > 65535) return -1;
+  ShrinkRowsParams p{};
+  p.tiles = reinterpret_cast<const LoraTile*>(tiles);
+  p.x = reinterpret_cast<const __nv_bfloat16*>(x); p.ldx = ldx;
+  p.arena = reinterpret_cast<const __nv_bfloat16*>(arena);
+  p.slot_base = slot_base; p.slot_rank = slot_rank; p.num_slots = num_slots; p.unit_off = unit_off;
+  p.nparts = nparts; p.v = v; p.ldv = ldv; p.K = K; p.T = T; p.status = status;
+  const int blocks16 = (nparts * max_rank + 15) / 16;
+  const long long units = (long long)(live_tiles > 0 ? live_tiles : num_tiles) * blocks16;
+  // K is cut while the CTAs stay within four per SM and a warp keeps four blocks of 32 elements
+  int parts = 1;
+  while (parts < kSrMaxParts && units * parts * 2 <= 4 * 148 && K >= parts * 2 * 4 * 4 * 32) parts *= 2;
+  launch_pdl_cluster(lora_shrink_mma_kernel, dim3(parts, num_tiles, blocks16), dim3(kSrThreads), dim3(parts, 1, 1), 0,
+                     reinterpret_cast<cudaStream_t>(stream), p);
+  return -(int)cudaGetLastError();
+}
+
 int lx_lora_expand_tiled(const float* v, int ldv, long long v_split_stride, int ksplit, const void* tiles, int num_tiles,
                          int max_tile_rows, const void* arena, const long long* slot_base, const int* slot_rank, int num_slots,
                          long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1, int* status, void* stream) {
@@ -468,7 +640,7 @@ int lx_lora_expand_tiled(const float* v, int ldv, long long v_split_stride, int 
   p.num_tiles = num_tiles;
   p.col_blocks = (N + kExpBlockCols - 1) / kExpBlockCols;
   const long long work = (long long)num_tiles * p.col_blocks;
-  const int grid = (int)(work < 148 * 2 ? work : 148 * 2);
+  const int grid = (int)(work < 148 * kExpCtas ? work : 148 * kExpCtas);
   launch_pdl(lora_expand_tiled_kernel, dim3(grid), dim3(kExpThreads), 0, reinterpret_cast<cudaStream_t>(stream), p);
   return -(int)cudaGetLastError();
 }

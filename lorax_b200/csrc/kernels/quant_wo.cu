@@ -109,6 +109,7 @@ struct Wq4Params {
   __nv_bfloat16* out;
   long long ldx, ldo;
   int T, N, K, group;
+  int w_const;                 // the kernel in front on the stream does not write the codes: they are read before the wait for it
 };
 
 LX_DEVICE void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -152,8 +153,10 @@ LX_DEVICE Wq4Group wq4_group(__half2 szv) {
   return g;
 }
 
-// Every warp owns the k-blocks warp, warp + 8, ... of the block's 16 * MT weight rows; the next k-block's codes are in flight
-// while the current one is multiplied.  One activation fragment feeds MT row tiles.
+// Every warp owns the k-blocks warp, warp + 8, ... of the block's 16 * MT weight rows; the codes of the next AHEAD k-blocks are in flight
+// while the current one is multiplied, and up to 8 tokens the activations of the next one.  One activation fragment feeds MT row tiles.
+// Bound by the bytes in flight: at five tokens the QKV, O and down projections of a 7B layer take 10, 5 and 15 us (13, 7 and 19 with one
+// k-block ahead and nothing before the wait); gate_up, three waves of blocks, stays at 26.
 // EXACT: every 128-wide k-block lies inside one group and the zero points are integers.  The codes then go to the tensor cores as
 // the exact integers (code - zero); the k-block's partial product is scaled by the group's fp16 scale in fp32 on its way into the
 // accumulator: no fma per pair of weights and no bf16 rounding of the scale.
@@ -174,21 +177,47 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
     for (int j = 0; j < NT; ++j) acc[m][j][0] = acc[m][j][1] = acc[m][j][2] = acc[m][j][3] = 0.f;
 
   const int kblocks = p.K / 128;
-  uint4 nc0[MT], nc1[MT];
-  __half2 nsz0[MT], nsz1[MT];
-  auto fetch = [&](int kb) {
+  constexpr int AHEAD = NT == 1 ? (MT == 1 ? 3 : 2) : 1;
+  uint4 qc0[AHEAD][MT], qc1[AHEAD][MT];
+  __half2 qsz0[AHEAD][MT], qsz1[AHEAD][MT];
+  auto fetch = [&](int kb, int d) {
+    if (kb >= kblocks) return;
     const int grp = (kb * 128 + 32 * t) / p.group;
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
-      nc0[m] = __ldcs(reinterpret_cast<const uint4*>(c_r0 + (16 * m) * row_bytes + (long long)kb * 64));
-      nc1[m] = __ldcs(reinterpret_cast<const uint4*>(c_r0 + (16 * m + 8) * row_bytes + (long long)kb * 64));
-      nsz0[m] = sz_r0[(long long)(16 * m) * G + grp];
-      nsz1[m] = sz_r0[(long long)(16 * m + 8) * G + grp];
+      qc0[d][m] = __ldcs(reinterpret_cast<const uint4*>(c_r0 + (16 * m) * row_bytes + (long long)kb * 64));
+      qc1[d][m] = __ldcs(reinterpret_cast<const uint4*>(c_r0 + (16 * m + 8) * row_bytes + (long long)kb * 64));
+      qsz0[d][m] = sz_r0[(long long)(16 * m) * G + grp];
+      qsz1[d][m] = sz_r0[(long long)(16 * m + 8) * G + grp];
     }
   };
+  auto fetch_x = [&](int kb, int j, uint4 (&xv)[4]) {
+    const int tok = 8 * j + g;
+    const long long kx = (long long)kb * 128 + 32 * t;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      xv[q] = tok < p.T && kb < kblocks ? __ldg(reinterpret_cast<const uint4*>(p.x + tok * p.ldx + kx + 8 * q)) : make_uint4(0, 0, 0, 0);
+  };
   int kb = warp;
-  if (kb < kblocks) fetch(kb);
+  if (!p.w_const) pdl_wait();
+#pragma unroll
+  for (int d = 0; d < AHEAD; ++d) fetch(kb + d * kWqWarps, d);
+  if (p.w_const) pdl_wait();
+  pdl_trigger();
+  uint4 nx[4];
+  if constexpr (NT == 1) fetch_x(kb, 0, nx);
   for (; kb < kblocks; kb += kWqWarps) {
+    uint4 nc0[MT], nc1[MT];
+    __half2 nsz0[MT], nsz1[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      nc0[m] = qc0[0][m]; nc1[m] = qc1[0][m]; nsz0[m] = qsz0[0][m]; nsz1[m] = qsz1[0][m];
+#pragma unroll
+      for (int d = 0; d + 1 < AHEAD; ++d) {
+        qc0[d][m] = qc0[d + 1][m]; qc1[d][m] = qc1[d + 1][m]; qsz0[d][m] = qsz0[d + 1][m]; qsz1[d][m] = qsz1[d + 1][m];
+      }
+    }
+    fetch(kb + AHEAD * kWqWarps, AHEAD - 1);
     uint32_t a0[MT][4][4], a1[MT][4][4];               // [row tile][word][pair]: rows g and g + 8
     float s0[MT], s1[MT];
 #pragma unroll
@@ -217,15 +246,16 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
       wq4_expand(nc1[m].z, g1.bias128z, g1.s2, g1.c2, a1[m][2]);
       wq4_expand(nc1[m].w, g1.bias128z, g1.s2, g1.c2, a1[m][3]);
     }
-    if (kb + kWqWarps < kblocks) fetch(kb + kWqWarps); // next block's codes are in flight while this one is multiplied
-    const long long kx = (long long)kb * 128 + 32 * t;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-      const int tok = 8 * j + g;
       uint4 xv[4];
+      if constexpr (NT == 1) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        xv[q] = tok < p.T ? __ldg(reinterpret_cast<const uint4*>(p.x + tok * p.ldx + kx + 8 * q)) : make_uint4(0, 0, 0, 0);
+        for (int q = 0; q < 4; ++q) xv[q] = nx[q];
+        fetch_x(kb + kWqWarps, 0, nx);
+      } else {
+        fetch_x(kb, j, xv);
+      }
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         float part[4] = {0.f, 0.f, 0.f, 0.f};
@@ -271,8 +301,7 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
 
 template <int NT, int MT>
 int wq4_launch(const Wq4Params& p, bool exact, cudaStream_t s) {
-  if (exact) wq4_mma_kernel<NT, MT, true><<<p.N / (kWqRows * MT), kWqWarps * 32, 0, s>>>(p);
-  else wq4_mma_kernel<NT, MT, false><<<p.N / (kWqRows * MT), kWqWarps * 32, 0, s>>>(p);
+  launch_pdl(exact ? wq4_mma_kernel<NT, MT, true> : wq4_mma_kernel<NT, MT, false>, dim3(p.N / (kWqRows * MT)), dim3(kWqWarps * 32), 0, s, p);
   return -(int)cudaGetLastError();
 }
 
@@ -301,28 +330,29 @@ int lx_wq4_max_tokens() { return 32; }
 // out[T, N] = x[T, K] . W^T (+ bias) for T <= 32 from affine 4-bit codes.  N % 16 == 0, K % 128 == 0, group % 32 == 0, x rows
 // 16-byte aligned.
 int lx_wq4_gemm_ex(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
-                   int K, int group, int integer_zeros, void* stream);
+                   int K, int group, int flags, void* stream);
 
 int lx_wq4_gemm(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
                 int K, int group, void* stream) {
   return lx_wq4_gemm_ex(x, ldx, codes, sz, bias, out, ldo, T, N, K, group, 0, stream);
 }
 
-// `integer_zeros` != 0 promises that every zero point is an integer (GPTQ, AWQ, round-to-nearest; not HQQ): with groups that are
-// multiples of 128 the kernel then multiplies exact integers and scales the partial sums (see EXACT above).
+// `flags` bit 0 promises that every zero point is an integer (GPTQ, AWQ, round-to-nearest; not HQQ): with groups that are
+// multiples of 128 the kernel then multiplies exact integers and scales the partial sums (see EXACT above).  Bit 1: the kernel in front
+// on the stream does not write the codes, scales and zero points, which are then read while it still runs.
 int lx_wq4_gemm_ex(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
-                   int K, int group, int integer_zeros, void* stream) {
+                   int K, int group, int flags, void* stream) {
   using namespace lx;
   if (T <= 0 || T > 32 || N % kWqRows != 0 || K % 128 != 0 || group % 32 != 0 || K % group != 0 || ldx % 8 != 0) return -1;
   Wq4Params p{static_cast<const uint8_t*>(codes), static_cast<const __half2*>(sz), static_cast<const __nv_bfloat16*>(x),
-              static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), ldx, ldo, T, N, K, group};
+              static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), ldx, ldo, T, N, K, group, (flags >> 1) & 1};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // two row tiles per warp halve the re-reads of the activations (every block reads all of x); with few rows and few tokens
   // the larger grid of single tiles fills the machine better
   const bool two = N % (2 * kWqRows) == 0 && (N >= 8192 || T > 8);
   // measured: the exact-integer path wins 6-15 % on the large projections at up to 8 tokens and loses elsewhere (register
   // pressure with two token tiles; small grids)
-  const bool exact = integer_zeros != 0 && group % 128 == 0 && T <= 8 && (N >= 16384 || K >= 8192);
+  const bool exact = (flags & 1) != 0 && group % 128 == 0 && T <= 8 && (N >= 16384 || K >= 8192);
   if (T <= 8) return two ? wq4_launch<1, 2>(p, exact, s) : wq4_launch<1, 1>(p, exact, s);
   if (T <= 16) return two ? wq4_launch<2, 2>(p, exact, s) : wq4_launch<2, 1>(p, exact, s);
   return wq4_launch<4, 1>(p, exact, s);

@@ -460,7 +460,7 @@ class DecoderModel:
     def _gemm(self, x, w, b, out=None):
         if isinstance(w, GroupQuantWeight):
             xb = x if x.dtype == torch.bfloat16 or not x.is_cuda else x.to(torch.bfloat16)
-            y = self.ops.gemm_wq(xb, w, bias=b, out=out if out is not None and out.dtype == xb.dtype else None)
+            y = self.ops.gemm_wq(xb, w, bias=b, out=out if out is not None and out.dtype == xb.dtype else None, w_const=True)
             if out is not None and y is not out:
                 out.copy_(y)
                 return out

@@ -87,6 +87,7 @@ def load() -> ctypes.CDLL:
         "lx_tensormap_bytes": ([], I),
         "lx_lora_encode_tmap": ([P, P, I, I, L, I], I),
         "lx_lora_encode_tmap_b": ([P, P, I, I, L, I], I),
+        "lx_lora_shrink_mma": ([P, L, P, I, I, P, P, P, I, L, I, P, I, I, I, I, P, P], I),
         "lx_lora_shrink_tc": ([P, L, P, I, I, P, I, I, P, I, I, I, P, I, L, I, P, P, I, I, I, I, P, P], I),
         "lx_gemm_bf16_lora": ([P, P, P, P, I, I, I, L, L, L, P, L, P, P, I, P, P], I),
         "lx_lora_fused_desc_bytes": ([], I),
@@ -482,10 +483,10 @@ def wq_dequant(w, out: Optional[torch.Tensor] = None) -> torch.Tensor:
 WQ4_DIRECT_MAX_TOKENS = int(os.environ.get("LORAX_WQ4_DIRECT_TOKENS", "32"))
 
 
-def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, w_const: bool = False) -> torch.Tensor:
     """out[T, N] = x[T, K] @ dequant(w)^T (+ bias) for a weight-only quantised matrix.  Few tokens and affine 4-bit codes:
     the tensor-core kernel that multiplies straight from the packed codes (HBM traffic = the packed weights).  Otherwise
-    the codes are expanded to bf16 once and the tcgen05 GEMM runs on the expansion."""
+    the codes are expanded to bf16 once and the tcgen05 GEMM runs on the expansion.  `w_const` as for `gemm`."""
     assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1
     T, K = x.shape
     N = w.shape[0]
@@ -500,7 +501,7 @@ def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Option
     if (w.bits == 4 and w.table is None and T <= WQ4_DIRECT_MAX_TOKENS and N % 16 == 0 and K % 128 == 0 and w.group % 32 == 0
             and x.stride(0) % 8 == 0):
         rc = load().lx_wq4_gemm_ex(_ptr(x), x.stride(0), _ptr(w.codes), _ptr(w.sz), _ptr(bias), _ptr(out), out.stride(0), T, N, K, w.group,
-                                   1 if getattr(w, "int_zero", False) else 0, _stream())
+                                   (1 if getattr(w, "int_zero", False) else 0) | (2 if w_const else 0), _stream())
         _check(rc, "lx_wq4_gemm")
         return out
     return gemm(x, wq_dequant(w), bias=bias, out=out)
@@ -719,6 +720,18 @@ def lora_shrink_tiles(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, max_
                                   _ptr(vf), _ptr(ws.lora_counters), ws.lora_counters.numel(), T, K, max_rank, _ptr(ws.status), _stream())
     _check(rc, "lx_lora_shrink_tc")
     return vf
+
+
+def lora_shrink_mma(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, arena: torch.Tensor, slot_base: torch.Tensor,
+                    slot_rank: torch.Tensor, unit_off: int, nparts: int, max_rank: int, live_tiles: int = 0) -> torch.Tensor:
+    """Shrink of a short step over a table of tiles of at most 32 rows -> v [rows, cols] fp32, by mma.sync straight from the blobs."""
+    T, K = x.shape
+    ws = workspace(x.device)
+    v = ws.lora_v
+    rc = load().lx_lora_shrink_mma(_ptr(x), x.stride(0), _ptr(tiles), num_tiles, live_tiles, _ptr(arena), _ptr(slot_base), _ptr(slot_rank),
+                                   slot_rank.shape[0], unit_off, nparts, _ptr(v), v.stride(0), T, K, max_rank, _ptr(ws.status), _stream())
+    _check(rc, "lx_lora_shrink_mma")
+    return v
 
 
 def lora_expand_tiles(v, tiles: torch.Tensor, num_tiles: int, max_tile_rows: int, arena: torch.Tensor, slot_base: torch.Tensor,

@@ -62,7 +62,7 @@ def quant_act_fp8(x):
     return q.contiguous(), scale.t().contiguous()
 
 
-def gemm_wq(x, w, bias=None, out=None):
+def gemm_wq(x, w, bias=None, out=None, **_):
     """Oracle of the weight-only quantised GEMM: the packed matrix expanded to the activation dtype, then a plain product."""
     from ..utils.quant_formats import dequantize
     y = x.float() @ dequantize(w, torch.float32).to(x.dtype).float().t()

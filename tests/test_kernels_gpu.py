@@ -360,6 +360,40 @@ def test_attn_decode_fp8_pages(nat, B, nh, nkv, d, window, softcap, nsplit):
         assert _rel_err(got[b], want[b]) < 6e-3, (b, int(ctx[b]))
 
 
+@pytest.mark.parametrize("T, K", [(1, 4096), (7, 64), (9, 1000), (40, 14336), (33, 2056), (300, 512)])
+def test_lora_shrink_short_steps(nat, T, K):
+    """Clusters of one to eight CTAs over K, K off the blocks of 32, one and four row groups, ranks of 8 to 64, rows past the batch, dead entries.
+    bf16 products are exact in fp32; a sum of K terms in fp32 is within K * 2^-24 of the sum of their magnitudes."""
+    g = torch.Generator().manual_seed(T + K)
+    ranks, nparts = [8, 16, 64, 32], 3
+    bases, off = [], 0
+    for r in ranks:
+        bases.append(off)
+        off += (r * (nparts * K + 8) + 63) // 64 * 64
+    arena = (torch.randn(off, generator=g) * 0.05).to(torch.bfloat16)
+    x = torch.randn(T, K + 8, generator=g).to(torch.bfloat16)
+    tl, row = [], 0
+    while row < T:
+        n = min([3, 32, 8, 9, 17][len(tl) % 5], T - row)
+        tl.append((len(tl) % 4, row, n, 0))
+        row += n + len(tl) % 2
+    tl[-1] = (tl[-1][0], tl[-1][1], 32, 0)                             # a table may be older than the batch
+    table = torch.tensor(tl + [(-1, 0, 0, 0)] * 3, dtype=torch.int32)
+    nat.workspace().lora_v.fill_(7.0)
+    v = nat.lora_shrink_mma(x.cuda()[:, :K], table.cuda(), len(table), arena.cuda(), torch.tensor(bases).cuda(),
+                            torch.tensor(ranks, dtype=torch.int32).cuda(), 0, nparts, 64, live_tiles=len(tl))
+    nat.workspace().check_status()
+    v = v[:T].cpu()
+    seen = torch.zeros(T, v.shape[1], dtype=torch.bool)
+    for slot, r0, n, _ in tl:
+        n, R = min(n, T - r0), ranks[slot] * nparts
+        A = arena[bases[slot]: bases[slot] + R * K].view(R, K).double()
+        xs = x[r0: r0 + n, :K].double()
+        assert ((v[r0: r0 + n, :R].double() - xs @ A.t()).abs() <= (xs.abs() @ A.abs().t()) * K * 2 ** -24 + 1e-30).all()
+        seen[r0: r0 + n, :R] = True
+    assert (v[~seen] == 7.0).all()
+
+
 @pytest.mark.parametrize("nh,nkv,d,nsplit", [(12, 12, 64, 1), (32, 8, 128, 3), (6, 6, 128, 1)])
 def test_attn_alibi(nat, nh, nkv, d, nsplit):
     """ALiBi slopes in both attention kernels (BLOOM, MPT): bias -slope_h * (query position - key position)."""
