@@ -13,12 +13,13 @@
 //                               on the next scores while the softmax of this block runs
 //   softmax (warps 2..5)        one thread per row: the 64 scores of a row in registers with one tcgen05.ld, scale / softcap / ALiBi /
 //                               causal and window mask, maximum, exp2, P back to TMEM as bf16.  The sums stand relative to a maximum
-//                               that is only moved when a block exceeds it by more than 2^8: then, and only then, the warp waits for
+//                               that is only moved when a block exceeds it by more than a slack: then, and only then, the warp waits for
 //                               the products so far and rescales O in TMEM
 //
 // Two CTAs share an SM (96 KB of shared memory, 256 TMEM columns each): the softmax of one runs while the other waits for its scores,
 // its pages or its sums.  What bounds it is the exponentials (16 a cycle and SM: 512 cycles a block against 256 for the products).
-// MEASURED_PREFILL
+// One CTA per SM with blocks of 128 keys, weights through shared memory and O folded in registers took 1200 us for 8192 tokens and 32
+// heads, 148 for seven prompts of 4001 tokens, 526 for 6000 tokens with a window of 1024, a cap and WIDE; this takes 933, 129 and 369.
 //
 // WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, and P V is two
 // products into the same accumulator (the layer-by-layer designs ask for it).
@@ -62,7 +63,12 @@ struct FaSmem {
   static constexpr int kTotal = kQBytes + 4 * kBlock + 256 + 1024;
 };
 constexpr int kFaTmemCols = 256;    // scores of two blocks (64 columns each), O (128)
-constexpr float kFaSlack = 8.f;     // how far (log2) a row's scores may exceed the maximum its sums stand relative to
+// How far (log2) a row's scores may exceed the maximum its sums stand relative to.  With two-term weights it costs no precision.  With
+// weights of one bf16 term the largest of a row is exact only while it is the maximum itself: over q and k of size one to three and up to
+// 4000 keys the results are 1.88e-3, 1.95e-3, 2.06e-3 and 1.63e-3 off 64 bits at 1/2 (1.91, 1.96, 2.06 and 1.63 with sums relative to the
+// maximum and divided by those of unrounded weights), but 2.10e-3 and 1.67e-3 at 8, which would take another 7 to 18 % off the time.
+template <bool WIDE>
+constexpr float kFaSlack = WIDE ? 8.f : 0.5f;
 
 // 5-D tiled load: the paged cache {d, slot in page, K|V, kv head, block}.
 LX_DEVICE void tma_load_5d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2, int c3, int c4) {
@@ -94,21 +100,24 @@ struct FaScore {
 // maximum; MASK: keys outside [lo, hi) do not count.
 template <int MODE, bool MASK>
 LX_DEVICE float fa_block_max(float (&s)[kFaKeys], int kb0, int lo, int hi, const FaScore& sc) {
-  float bm = -INFINITY;
+  float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains: two warps a scheduler do not hide one of 64 steps)
 #pragma unroll
   for (int q = 0; q < kFaKeys; ++q) {
     const int key = kb0 + q;
     if (MODE == kFaBias) s[q] = sc.of<MODE>(s[q], key);
     if (MASK) s[q] = (key >= lo && key < hi) ? s[q] : -INFINITY;
-    bm = fmaxf(bm, s[q]);
+    top[q & 3] = fmaxf(top[q & 3], s[q]);
   }
+  const float bm = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
   return MODE == kFaBias || bm == -INFINITY ? bm : sc.of<MODE>(bm, 0);
 }
 
-// p = exp2(score - m) for the 64 keys -> bf16 pairs into the TMEM columns at `tp` (WIDE: the remainders behind them); returns the row sum.
+// p = exp2(score - m) for the 64 keys -> bf16 pairs into the TMEM columns at `tp` (WIDE: the remainders behind them); returns the row sum,
+// of the rounded weights where the products take those: the weight that dominates a row is not 1 (m may lie below its score), and its
+// rounding then cancels in the quotient.
 template <int MODE, bool MASK, bool WIDE>
 LX_DEVICE float fa_block_probs(uint32_t tp, float (&s)[kFaKeys], int kb0, int lo, int hi, float m, const FaScore& sc) {
-  float sum = 0.f;
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
   const bool dead = (m == -INFINITY);
   const float neg_m = dead ? 0.f : -m;
 #pragma unroll
@@ -125,17 +134,16 @@ LX_DEVICE float fa_block_probs(uint32_t tp, float (&s)[kFaKeys], int kb0, int lo
         if (MASK) e = (key >= lo && key < hi && !dead) ? e : 0.f;
         pv[u] = e;
       }
-      sum += pv[0] + pv[1];
       pk[q >> 1] = pack_bf16x2(pv[0], pv[1]);
-      if constexpr (WIDE) {
-        const float2 h = unpack_bf16x2(pk[q >> 1]);
-        lo_pk[q >> 1] = pack_bf16x2(pv[0] - h.x, pv[1] - h.y);
-      }
+      const float2 h = unpack_bf16x2(pk[q >> 1]);
+      if constexpr (WIDE) lo_pk[q >> 1] = pack_bf16x2(pv[0] - h.x, pv[1] - h.y);
+      sum[q & 2] += WIDE ? pv[0] : h.x;
+      sum[(q & 2) + 1] += WIDE ? pv[1] : h.y;
     }
     tmem_st_32x32b_x16(tp + (uint32_t)(c >> 1), pk);
     if constexpr (WIDE) tmem_st_32x32b_x16(tp + 32u + (uint32_t)(c >> 1), lo_pk);
   }
-  return sum;
+  return (sum[0] + sum[1]) + (sum[2] + sum[3]);
 }
 
 template <bool WIDE>
@@ -324,7 +332,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       else if (mode == kFaCap) bm = need_mask ? fa_block_max<kFaCap, true>(s, kb0, lo, hi, sc) : fa_block_max<kFaCap, false>(s, kb0, lo, hi, sc);
       else bm = fa_block_max<kFaBias, true>(s, kb0, lo, hi, sc);
       // a row that has seen no key has added zeros to O: any maximum will do for it
-      const bool move = bm > m + kFaSlack && m > -INFINITY;
+      const bool move = bm > m + kFaSlack<WIDE> && m > -INFINITY;
       if (__any_sync(0xffffffffu, move)) {
         const float alpha = move ? fa_ex2(m - bm) : 1.f;
         if (!mbar_wait(&pv_done[st ^ 1], ((j - 1) >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
