@@ -1536,6 +1536,7 @@ struct GemmPlan {
 constexpr int kOverlapMaxTokens = 512;         // (see pdl_trigger: longer steps lose by it)
 constexpr int kModeConstWeights = 1 << 16;     // of a launch's `mode`: no kernel that may still run writes the weights
 
+constexpr int kClassicSplitTokens = 32;
 static int template_bn(int bn) { return bn <= 16 ? 16 : bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256; }
 
 // Decide how the last, partly filled wave of `tiles` tiles is computed.  sk_policy: 0 = by cost, 1 = never
@@ -1599,6 +1600,19 @@ static GemmPlan choose_plan_swap(int T, int N, int K, int num_sms, long long ws_
     const int work = tiles_a * tt * s;
     pl.grid = work < num_sms ? work : num_sms;
     return pl;
+  }
+  // Few tokens and few weight tiles: the classic split, where that gives 85 % of the SMs a part each.  A tile's last part sums the others
+  // (8 to 16 KB each) as soon as they are there; the stream-K contributors each wait for all of them.  13 tokens, products back to back:
+  // N = K = 4096 14.9 -> 11.3 us (four parts), N = 6144 16.6 -> 14.3 (three), K = 14336 25.9 -> 23.8 (four); at 64 tokens 18.4 -> 18.7,
+  // 18.5 -> 21.4 and 27.8 -> 30.4, the single summing CTA has four times as much to add.
+  if (sk_policy == 0 && !bn_forced && have_counters && t16 <= kClassicSplitTokens) {
+    const int s = num_sms / tiles_a;
+    if (s >= 2 && s <= 4 && tiles_a * s * 100 >= num_sms * 85 && kblocks / s >= 8 && (long long)tiles_a * s * kBM * template_bn(t16) * 4 <= ws_bytes) {
+      GemmPlan pl{};
+      pl.bn = t16; pl.split = s; pl.dp_tiles = tiles_a; pl.sk_ctas = 0;
+      pl.grid = tiles_a * s;
+      return pl;
+    }
   }
   GemmPlan best{};
   best.cost = 1e30;
