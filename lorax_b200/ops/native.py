@@ -71,6 +71,7 @@ def load() -> ctypes.CDLL:
         "lx_rope_kvwrite": ([P, P, P, P, P, I, I, I, I, I, I, L, I, P], I),
         "lx_act_mul": ([P, P, I, I, L, L, I, I, P], I),
         "lx_embed": ([P, P, P, I, I, I, I, F, P], I),
+        "lx_place_rows": ([P, I, I, P, P, P, P, P], I),
         "lx_argmax_logprob": ([P, L, I, I, P, P, F, P], I),
         "lx_advance_decode": ([P, P, P, P, P, P, I, I, I, P], I),
         "lx_prefill_metadata": ([P, P, P, P, I, I, I, I, P, P, P, P], I),
@@ -582,6 +583,13 @@ def argmax_logprob(logits: torch.Tensor, ids: Optional[torch.Tensor] = None, log
     rc = load().lx_argmax_logprob(_ptr(logits), logits.stride(0), T, V, _ptr(ids), _ptr(logprobs), softcap, _stream())
     _check(rc, "lx_argmax_logprob")
     return ids, logprobs
+
+
+def place_rows(job: torch.Tensor, input_ids, positions, ctx_lens, slots):
+    """Points rows of a decode batch at tokens and places; `job` [4, n] int32: rows, input tokens, positions, cache slots."""
+    assert job.dtype == torch.int32 and job.is_contiguous() and job.dim() == 2 and job.shape[0] == 4
+    _check(load().lx_place_rows(_ptr(job), job.shape[1], input_ids.shape[0], _ptr(input_ids), _ptr(positions), _ptr(ctx_lens), _ptr(slots),
+                                _stream()), "lx_place_rows")
 
 
 def advance_decode(input_ids, next_ids, positions, ctx_lens, slots, block_tables, page: int):

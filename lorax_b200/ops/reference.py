@@ -217,6 +217,11 @@ def argmax_logprob(logits, ids=None, logprobs=None, softcap: float = 0.0):
     return i.to(torch.int32), lp
 
 
+def place_rows(job, input_ids, positions, ctx_lens, slots):
+    rows = job[0].long()
+    input_ids[rows], positions[rows], ctx_lens[rows], slots[rows] = job[1], job[2], job[2] + 1, job[3]
+
+
 def advance_decode(input_ids, next_ids, positions, ctx_lens, slots, block_tables, page):
     live = ctx_lens > 0
     input_ids[live] = next_ids[live].to(input_ids.dtype)

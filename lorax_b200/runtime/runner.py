@@ -59,8 +59,10 @@ class DecodeState:
         self.block_tables = torch.zeros(max_batch, max_blocks, **i32)
         self.tok_slot = torch.full((max_batch,), -1, **i32)
         self.state_slots = torch.zeros(max_batch, **i32)       # slot of the row's recurrent state
-        self.next_ids = torch.zeros(max_batch, **i32)
-        self.logprobs = torch.zeros(max_batch, dtype=torch.float32, device=device)
+        # a step's results lie side by side: one copy brings them to the host
+        self.results = torch.zeros(2 * max_batch, **i32)
+        self.next_ids = self.results[:max_batch]
+        self.logprobs = self.results[max_batch:].view(torch.float32)
         # LoRA tile table of the decode batch (rows are kept sorted by adapter slot): [max_batch, 4], unused = slot -1
         self.lora_tiles = torch.full((max_batch, 4), -1, **i32)
         self.row_slot: Dict[int, int] = {}      # row -> adapter slot (host mirror)
@@ -106,8 +108,9 @@ class ModelRunner:
         # pinned result ring (two steps in flight at most)
         self.n_ring = 8
         pin = dict(pin_memory=True) if self.is_cuda else {}
-        self.ring_ids = [torch.zeros(max_batch, dtype=torch.int32, **pin) for _ in range(self.n_ring)]
-        self.ring_lp = [torch.zeros(max_batch, dtype=torch.float32, **pin) for _ in range(self.n_ring)]
+        self.ring = [torch.zeros(2 * max_batch, dtype=torch.int32, **pin) for _ in range(self.n_ring)]
+        self.ring_ids = [r[:max_batch] for r in self.ring]
+        self.ring_lp = [r[max_batch:].view(torch.float32) for r in self.ring]
         # the ring events carry device timestamps: a token's time is the completion of its step on the GPU, on the
         # host's clock through an anchor pair (event, perf_counter) taken at a synchronised moment
         self.ring_ev = [torch.cuda.Event(enable_timing=True) if self.is_cuda else None for _ in range(self.n_ring)]
@@ -399,14 +402,11 @@ class ModelRunner:
         page = self.page
         tabs = [self._table_row(b) for b in blocks]
         slots = [tabs[i][positions[i] // page] * page + positions[i] % page for i in range(len(rows))]
-        n = len(rows)
-        dev = self._to_dev(list(rows) + list(tokens) + list(positions) + [p + 1 for p in positions] + slots)
-        r = dev[:n].long()
         st = self.state
-        st.input_ids.index_copy_(0, r, dev[n:2 * n])
-        st.positions.index_copy_(0, r, dev[2 * n:3 * n])
-        st.ctx_lens.index_copy_(0, r, dev[3 * n:4 * n])
-        st.slots.index_copy_(0, r, dev[4 * n:5 * n])
+        if min(rows) < 0 or max(rows) >= st.max_batch:
+            raise IndexError(f"decode rows {min(rows)} .. {max(rows)} of {st.max_batch}")
+        job = self._to_dev(list(rows) + list(tokens) + list(positions) + slots).view(4, len(rows))
+        self.model.ops.place_rows(job, st.input_ids, st.positions, st.ctx_lens, st.slots)
 
     def retire(self, rows: Sequence[int]):
         """Mark rows as padding: they stop advancing and attention skips them."""
@@ -532,9 +532,8 @@ class ModelRunner:
             sampler(logits, st)
         k = self.ring_pos
         self.ring_pos = (k + 1) % self.n_ring
-        self.ring_ids[k][:b].copy_(st.next_ids[:b], non_blocking=True)
-        self.ring_lp[k][:b].copy_(st.logprobs[:b], non_blocking=True)
-        self.d2h_bytes += b * 8
+        self.ring[k].copy_(st.results, non_blocking=True)
+        self.d2h_bytes += st.results.numel() * 4
         if self.is_cuda:
             self.ring_status[k].copy_(self.status_word, non_blocking=True)
             self.d2h_bytes += 8

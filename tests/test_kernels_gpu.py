@@ -179,6 +179,18 @@ def test_argmax_logprob_over_split_rows(nat, T, V, ld, softcap):
     assert torch.allclose(lp.double(), top - torch.logsumexp(x, -1), atol=V * 2 ** -24 + 2 ** -18, rtol=2 ** -20)
 
 
+@pytest.mark.parametrize("n", [1, 127, 129])
+def test_place_rows(nat, n):
+    g = torch.Generator().manual_seed(n)
+    job = torch.stack([torch.randperm(200, generator=g)[:n]] + [torch.randint(0, 9999, (n,), generator=g) for _ in range(3)]).to(torch.int32)
+    want = [torch.randint(0, 99, (200,), generator=g, dtype=torch.int32) for _ in range(4)]
+    got = [t.clone().cuda() for t in want]
+    ref.place_rows(job, *want)
+    nat.place_rows(job.cuda(), *got)
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu(), b)
+
+
 def test_embed_argmax_advance(nat):
     table = torch.randn(1000, 256, device="cuda", dtype=torch.bfloat16)
     ids = torch.randint(0, 2000, (50,), device="cuda", dtype=torch.int32)
