@@ -46,7 +46,6 @@ __global__ void __launch_bounds__(32 * kRouterWarps) moe_router_logits_kernel(co
                                                                               float* __restrict__ logits, int T, int E, int H, int* counts,
                                                                               int ncounts) {
   pdl_wait();
-  pdl_trigger();
   __shared__ float red[kRouterWarps][16][8 * NT + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
   const int t0 = blockIdx.x * 16 * MT, n0 = blockIdx.y * 8 * NT;
@@ -144,7 +143,6 @@ constexpr int kSelWarps = 8;
 template <int PER>
 __global__ void __launch_bounds__(32 * kSelWarps) moe_select_kernel(const MoeSelectParams p) {
   pdl_wait();
-  pdl_trigger();
   __shared__ float choice_s[kSelWarps][32 * PER];
   __shared__ uint8_t kept_s[kSelWarps][32 * PER];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -266,7 +264,6 @@ struct MoePlaceParams {
 
 __global__ void __launch_bounds__(256) moe_place_kernel(const MoePlaceParams p) {
   pdl_wait();
-  pdl_trigger();
   __shared__ int start[kMoeMaxExperts + 1];
   __shared__ int wsum[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -328,7 +325,6 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* _
                                                           const float* __restrict__ w, int k, __nv_bfloat16* __restrict__ out, long long ldo,
                                                           int T, int H) {
   pdl_wait();
-  pdl_trigger();
   const int lane = threadIdx.x & 31;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < T; t += (gridDim.x * blockDim.x) >> 5) {
     for (int h = lane * 8; h < H; h += 256) {
@@ -467,7 +463,6 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
-  pdl_trigger();
   if (warp == 0) MgIter::build(p.seg, p.runs, p.rows_cap, p.n_w / kMgBM, p.bn, start_s, cum_s);
   __syncthreads();
   const MgIter it{p.runs, p.n_w / kMgBM, p.bn, start_s, cum_s};
@@ -582,7 +577,6 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 __global__ void __launch_bounds__(256) moe_grouped_gemm_f32_kernel(const float* __restrict__ x, long long ldx, const float* __restrict__ w,
                                                                    long long ldw, float* __restrict__ out, const MoeGemmParams p) {
   pdl_wait();
-  pdl_trigger();
   __shared__ float xs[16][68], ws[16][68];
   __shared__ int tile_s[3];
   if (threadIdx.x == 0) {
