@@ -1,28 +1,22 @@
 // Ragged causal prefill attention over the paged KV cache on the 5th-generation tensor cores.
 //
 // One CTA = one 64-query tile of one sequence x TWO query heads of the same KV group: the 128 rows of a tcgen05 M tile are
-// (head, query) pairs, so a K / V block is staged once for both heads.  Keys are walked in blocks of 64 (two cache pages):
+// (head, query) pairs, so a K / V block is staged once for both heads.  Keys are walked in blocks of 128 (four cache pages):
 //
 //   loader  (warp 0, one lane)  Q by TMA from the projection output; K and V pages by TMA straight from the paged cache
 //                               through one 5-D tensor map {d, slot, K|V, kv head, block}: the block table supplies the last
-//                               coordinate, so pages need not be contiguous; a ring of two blocks each for K (free again once its
-//                               scores are formed) and for V
-//   MMA     (warp 1, one lane)  S = Q K^T into TMEM (double buffered), then O += P_j V_j into TMEM; P_j is the A operand from TMEM,
-//                               written by the softmax warps over the scores it came from; V is used as stored (token-major = the
-//                               "MN-major" form of the B operand); S of block j+1 is issued before P_j V_j, so the tensor core works
-//                               on the next scores while the softmax of this block runs
-//   softmax (warps 2..5)        one thread per row: the 64 scores of a row in registers with one tcgen05.ld, scale / softcap / ALiBi /
-//                               causal and window mask, maximum, exp2, P back to TMEM as bf16.  The sums stand relative to a maximum
-//                               that is only moved when a block exceeds it by more than a slack: then, and only then, the warp waits for
-//                               the products so far and rescales O in TMEM
+//                               coordinate, so pages need not be contiguous; a two-stage ring
+//   MMA     (warp 1, one lane)  S = Q K^T into TMEM (double buffered), then O_j = P_j V_j into TMEM (double buffered); P comes
+//                               back from the softmax warps through shared memory as a K-major operand, V is used as stored
+//                               (token-major = the "MN-major" form of the B operand); S of block j+1 is issued before P_j V_j,
+//                               so the tensor core works on the next scores while the softmax of this block runs
+//   softmax (warps 2..5)        one thread per row: scores from TMEM with tcgen05.ld, scale / softcap / ALiBi / causal and
+//                               window mask, running max and sum, exp2, P as bf16 into the swizzled operand tile; the
+//                               per-block products O_j come back from TMEM and are folded into fp32 registers with the
+//                               usual rescaling, so nothing in TMEM ever has to be rescaled
 //
-// Two CTAs share an SM (96 KB of shared memory, 256 TMEM columns each): the softmax of one runs while the other waits for its scores,
-// its pages or its sums.  What bounds it is the exponentials (16 a cycle and SM: 512 cycles a block against 256 for the products).
-// One CTA per SM with blocks of 128 keys, weights through shared memory and O folded in registers took 1200 us for 8192 tokens and 32
-// heads, 148 for seven prompts of 4001 tokens, 526 for 6000 tokens with a window of 1024, a cap and WIDE; this takes 933, 129 and 369.
-//
-// WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, and P V is two
-// products into the same accumulator (the layer-by-layer designs ask for it).
+// WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, in two operand
+// tiles, and P V is two products into the same accumulator (the layer-by-layer designs ask for it).
 //
 // Plain, chunked and prefix-cached prefill are one path: `cache_lens` says how many keys precede the chunk.  It replaces the
 // flash-attn-2 varlen call of the reference (server/lorax_server/utils/flash_attn.py:180-201) and the mma.sync kernel in
@@ -34,7 +28,7 @@ namespace lx {
 
 constexpr int kFaPage = 32;
 constexpr int kFaQ = 64;            // queries per CTA (per head)
-constexpr int kFaKeys = 64;         // keys per block
+constexpr int kFaKeys = 128;        // keys per block
 constexpr int kFaD = 128;
 constexpr int kFaThreads = 192;
 constexpr float kFaLog2e = 1.4426950408889634f;
@@ -56,19 +50,15 @@ struct FaParams {
   AttnTail tail;
 };
 
+template <bool WIDE>
 struct FaSmem {
   static constexpr int kQBytes = 128 * kFaD * 2;             // two 64-wide halves of [128 rows x 64]
-  static constexpr int kHalf = kFaKeys * 64 * 2;             // 64-wide half of a K or V block
-  static constexpr int kBlock = 2 * kHalf;                   // K or V of one block
-  static constexpr int kTotal = kQBytes + 4 * kBlock + 256 + 1024;
+  static constexpr int kKBytes = kFaKeys * kFaD * 2;
+  static constexpr int kVBytes = kFaKeys * kFaD * 2;
+  static constexpr int kPBytes = 128 * kFaKeys * 2;
+  static constexpr int kStage = kKBytes + kVBytes;
+  static constexpr int kTotal = kQBytes + 2 * kStage + (WIDE ? 2 : 1) * kPBytes + 512 + 1024;
 };
-constexpr int kFaTmemCols = 256;    // scores of two blocks (64 columns each), O (128)
-// How far (log2) a row's scores may exceed the maximum its sums stand relative to.  With two-term weights it costs no precision.  With
-// weights of one bf16 term the largest of a row is exact only while it is the maximum itself: over q and k of size one to three and up to
-// 4000 keys the results are 1.88e-3, 1.95e-3, 2.06e-3 and 1.63e-3 off 64 bits at 1/2 (1.91, 1.96, 2.06 and 1.63 with sums relative to the
-// maximum and divided by those of unrounded weights), but 2.10e-3 and 1.67e-3 at 8, which would take another 7 to 18 % off the time.
-template <bool WIDE>
-constexpr float kFaSlack = WIDE ? 8.f : 0.5f;
 
 // 5-D tiled load: the paged cache {d, slot in page, K|V, kv head, block}.
 LX_DEVICE void tma_load_5d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2, int c3, int c4) {
@@ -77,6 +67,7 @@ LX_DEVICE void tma_load_5d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, 
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
+LX_DEVICE void mbar_arrive_cnt(uint64_t* bar) { mbar_arrive(bar); }
 
 LX_DEVICE float fa_ex2(float x) {
   float y;
@@ -96,75 +87,91 @@ struct FaScore {
   }
 };
 
-// The 64 scores of a row of one block.  Without a bias the scores grow with the products (scale > 0), so the largest product gives the
-// maximum; MASK: keys outside [lo, hi) do not count.
+// Maximum over the 128 scores of a row (log2 domain).  Without a bias the scores grow with the products (scale > 0), so the largest product
+// gives it; MASK: keys outside [lo, hi) do not count.
 template <int MODE, bool MASK>
-LX_DEVICE float fa_block_max(float (&s)[kFaKeys], int kb0, int lo, int hi, const FaScore& sc) {
-  float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (four chains: two warps a scheduler do not hide one of 64 steps)
+LX_DEVICE float fa_block_max(uint32_t ts, int kb0, int lo, int hi, const FaScore& sc) {
+  float bm = -INFINITY;
+#pragma unroll 1
+  for (int c = 0; c < kFaKeys; c += 32) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
+    tc_wait_ld();
 #pragma unroll
-  for (int q = 0; q < kFaKeys; ++q) {
-    const int key = kb0 + q;
-    if (MODE == kFaBias) s[q] = sc.of<MODE>(s[q], key);
-    if (MASK) s[q] = (key >= lo && key < hi) ? s[q] : -INFINITY;
-    top[q & 3] = fmaxf(top[q & 3], s[q]);
+    for (int q = 0; q < 32; ++q) {
+      const int key = kb0 + c + q;
+      float t = MODE == kFaBias ? sc.of<MODE>(__uint_as_float(r[q]), key) : __uint_as_float(r[q]);
+      if (MASK) t = (key >= lo && key < hi) ? t : -INFINITY;
+      bm = fmaxf(bm, t);
+    }
   }
-  const float bm = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
   return MODE == kFaBias || bm == -INFINITY ? bm : sc.of<MODE>(bm, 0);
 }
 
-// p = exp2(score - m) for the 64 keys -> bf16 pairs into the TMEM columns at `tp` (WIDE: the remainders behind them); returns the row sum,
-// of the rounded weights where the products take those: the weight that dominates a row is not 1 (m may lie below its score), and its
-// rounding then cancels in the quotient.
+// p = exp2(score - m_new) for the 128 keys of the block -> bf16, written as this row of the K-major, 128-byte-swizzled operand
+// tile (WIDE: the remainders as the same row of the tile behind it); returns the row sum.
 template <int MODE, bool MASK, bool WIDE>
-LX_DEVICE float fa_block_probs(uint32_t tp, float (&s)[kFaKeys], int kb0, int lo, int hi, float m, const FaScore& sc) {
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  const bool dead = (m == -INFINITY);
-  const float neg_m = dead ? 0.f : -m;
-#pragma unroll
+LX_DEVICE float fa_block_probs(uint32_t ts, uint8_t* prow, int row, int kb0, int lo, int hi, float m_new, const FaScore& sc) {
+  float sum = 0.f;
+  const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+  const bool dead = (m_new == -INFINITY);
+#pragma unroll 1
   for (int c = 0; c < kFaKeys; c += 32) {
-    uint32_t pk[16], lo_pk[16];
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
+    tc_wait_ld();
+    uint32_t pk[16], lo_pk[WIDE ? 16 : 1];
 #pragma unroll
     for (int q = 0; q < 32; q += 2) {
       float pv[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
+        const float sraw = __uint_as_float(r[q + u]);
         const int key = kb0 + c + q + u;
-        const float t = s[c + q + u];
-        float e = MODE == kFaPlain ? fa_ex2(fmaf(t, sc.scale_l2, neg_m)) : fa_ex2((MODE == kFaBias ? t : sc.of<MODE>(t, key)) + neg_m);
+        float e = MODE == kFaPlain ? fa_ex2(fmaf(sraw, sc.scale_l2, neg_m)) : fa_ex2(sc.of<MODE>(sraw, key) + neg_m);
         if (MASK) e = (key >= lo && key < hi && !dead) ? e : 0.f;
         pv[u] = e;
       }
+      sum += pv[0] + pv[1];
       pk[q >> 1] = pack_bf16x2(pv[0], pv[1]);
-      const float2 h = unpack_bf16x2(pk[q >> 1]);
-      if constexpr (WIDE) lo_pk[q >> 1] = pack_bf16x2(pv[0] - h.x, pv[1] - h.y);
-      sum[q & 2] += WIDE ? pv[0] : h.x;
-      sum[(q & 2) + 1] += WIDE ? pv[1] : h.y;
+      if constexpr (WIDE) {
+        const float2 h = unpack_bf16x2(pk[q >> 1]);
+        lo_pk[q >> 1] = pack_bf16x2(pv[0] - h.x, pv[1] - h.y);
+      }
     }
-    tmem_st_32x32b_x16(tp + (uint32_t)(c >> 1), pk);
-    if constexpr (WIDE) tmem_st_32x32b_x16(tp + 32u + (uint32_t)(c >> 1), lo_pk);
+    uint8_t* half = prow + (c >> 6) * 16384;
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) {
+      const int chunk = ((c & 63) >> 3) + ch;
+      *reinterpret_cast<uint4*>(half + ((chunk ^ (row & 7)) << 4)) = make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]);
+      if constexpr (WIDE)
+        *reinterpret_cast<uint4*>(half + 32768 + ((chunk ^ (row & 7)) << 4)) =
+            make_uint4(lo_pk[4 * ch], lo_pk[4 * ch + 1], lo_pk[4 * ch + 2], lo_pk[4 * ch + 3]);
+    }
   }
-  return (sum[0] + sum[1]) + (sum[2] + sum[3]);
+  return sum;
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kFaThreads, 2)
+__global__ void __launch_bounds__(kFaThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const FaParams p) {
-  using S = FaSmem;
+  using S = FaSmem<WIDE>;
   extern __shared__ uint8_t fa_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sq = smem;
-  uint8_t* skk = smem + S::kQBytes;           // [2] K blocks
-  uint8_t* svv = skk + 2 * S::kBlock;         // [2] V blocks
-  uint64_t* bars = reinterpret_cast<uint64_t*>(svv + 2 * S::kBlock);
+  uint8_t* skv = smem + S::kQBytes;
+  uint8_t* sp = skv + 2 * S::kStage;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sp + (WIDE ? 2 : 1) * S::kPBytes);
   uint64_t* q_full = bars;            // 1
-  uint64_t* k_full = bars + 1;        // 2
-  uint64_t* k_empty = bars + 3;       // 2
-  uint64_t* v_full = bars + 5;        // 2
-  uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // 2
-  uint64_t* p_full = bars + 11;       // 2  (128 arrivals; the scores have been read too)
-  uint64_t* pv_done = bars + 13;      // 2  (O holds the products up to and including this block's)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* kv_full = bars + 1;       // 2
+  uint64_t* kv_empty = bars + 3;      // 2
+  uint64_t* s_full = bars + 5;        // 2
+  uint64_t* s_empty = bars + 7;       // 2  (128 arrivals)
+  uint64_t* p_full = bars + 9;        // 1  (128 arrivals)
+  uint64_t* p_empty = bars + 10;      // 1
+  uint64_t* pv_full = bars + 11;      // 2
+  uint64_t* pv_empty = bars + 13;     // 2  (128 arrivals)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -175,17 +182,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 128); mbar_init(&pv_done[i], 1);
+      mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128);
+      mbar_init(&pv_full[i], 1); mbar_init(&pv_empty[i], 128);
     }
+    mbar_init(p_full, 128);
+    mbar_init(p_empty, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_kv);
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, kFaTmemCols); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -214,28 +222,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         for (int hf = 0; hf < 2; ++hf)
           tma_load_2d(sq + hf * 16384 + g * 8192, &tmap_q, q_full, (h0 + g) * kFaD + hf * 64, tok_base + q0);
       const int* bt = p.block_tables + (long long)b * p.max_blocks;
-      // K of block j (plane 0) or its V (plane 1) into slot j & 1, once that slot has been read
-      auto load = [&](int j, int plane) -> bool {
+      for (int j = 0; j < nblk; ++j) {
         const int st = j & 1;
-        uint64_t* full = plane ? &v_full[st] : &k_full[st];
-        if (!mbar_wait(plane ? &v_empty[st] : &k_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) {
-          report_status(p.status, kTimeoutEmptyBarrier, tile);
-          *abort_flag = 1;
-          return false;
-        }
-        uint8_t* dst = (plane ? svv : skk) + st * S::kBlock;
-        mbar_expect_tx(full, (uint32_t)S::kBlock);
-        for (int pg = 0; pg < kFaKeys / kFaPage; ++pg) {
-          const int page = (t_lo + j) * (kFaKeys / kFaPage) + pg;
+        if (!mbar_wait(&kv_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) { report_status(p.status, kTimeoutEmptyBarrier, tile); *abort_flag = 1; break; }
+        uint8_t* sk = skv + st * S::kStage;
+        uint8_t* sv = sk + S::kKBytes;
+        mbar_expect_tx(&kv_full[st], (uint32_t)S::kStage);
+        for (int pg = 0; pg < 4; ++pg) {
+          const int page = (t_lo + j) * 4 + pg;
           const int blk = (page < total_pages && page < p.max_blocks) ? bt[page] : 0;      // a page past the keys reads block 0: masked, but finite
-          for (int hf = 0; hf < 2; ++hf) tma_load_5d(dst + hf * S::kHalf + pg * 4096, &tmap_kv, full, hf * 64, 0, plane, kvh, blk);
+          for (int hf = 0; hf < 2; ++hf) {
+            tma_load_5d(sk + hf * 16384 + pg * 4096, &tmap_kv, &kv_full[st], hf * 64, 0, 0, kvh, blk);
+            tma_load_5d(sv + hf * 16384 + pg * 4096, &tmap_kv, &kv_full[st], hf * 64, 0, 1, kvh, blk);
+          }
         }
-        return true;
-      };
-      bool ok = load(0, 0);
-      for (int j = 0; ok && j < nblk; ++j) {
-        if (j + 1 < nblk) ok = load(j + 1, 0);
-        if (ok) ok = load(j, 1);
       }
     }
     __syncwarp();
@@ -243,47 +243,47 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     if (lane == 0 && nblk > 0) {
       const uint32_t idesc_s = make_idesc(128, kFaKeys, kFmtBF16, kFmtBF16);
       const uint32_t idesc_pv = make_idesc(128, kFaD, kFmtBF16, kFmtBF16, 0, 1);          // B (= V) is MN-major
-      const uint32_t sq_a = smem_u32(sq);
-      const uint32_t tmem_o = tmem_base + 128u;
+      const uint32_t sq_a = smem_u32(sq), sp_a = smem_u32(sp);
       bool ok = mbar_wait(q_full, 0, abort_flag);
       if (!ok) { report_status(p.status, kTimeoutFullBarrier, tile); *abort_flag = 1; }
-      auto scores = [&](int j) -> bool {
-        const int st = j & 1;
-        // the buffer holds P of block j - 2 until that block's products are done
-        if (!mbar_wait(&k_full[st], (j >> 1) & 1, abort_flag) || (j > 1 && !mbar_wait(&pv_done[st], ((j - 2) >> 1) & 1, abort_flag))) {
-          report_status(p.status, kTimeoutFullBarrier, tile); *abort_flag = 1; return false;
+      auto do_pv = [&](int i) -> bool {
+        const int st = i & 1;
+        if (!mbar_wait(p_full, i & 1, abort_flag) || !mbar_wait(&pv_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) {
+          report_status(p.status, kTimeoutTmemEmpty, tile); *abort_flag = 1; return false;
         }
         tc_fence_after();
-        const uint32_t sk_a = smem_u32(skk + st * S::kBlock);
+        const uint32_t sv_a = smem_u32(skv + st * S::kStage + S::kKBytes);
+        const uint32_t tmem_o = tmem_base + 256u + (uint32_t)(st * 128);
+#pragma unroll
+        for (int ks = 0; ks < kFaKeys / 16; ++ks) {
+          const uint64_t da = make_desc_k_sw128(sp_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
+          const uint64_t db = make_desc_mn_sw128(sv_a + (uint32_t)(ks * 2048), 16384, 1024);
+          umma_f16_ss(tmem_o, da, db, idesc_pv, ks > 0 ? 1u : 0u);
+          if constexpr (WIDE) umma_f16_ss(tmem_o, da + (uint64_t)(S::kPBytes >> 4), db, idesc_pv, 1u);
+        }
+        tc_commit(&pv_full[st]);
+        tc_commit(p_empty);
+        tc_commit(&kv_empty[st]);
+        return true;
+      };
+      for (int j = 0; ok && j < nblk; ++j) {
+        const int st = j & 1;
+        if (!mbar_wait(&kv_full[st], (j >> 1) & 1, abort_flag) || !mbar_wait(&s_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) {
+          report_status(p.status, kTimeoutFullBarrier, tile); *abort_flag = 1; ok = false; break;
+        }
+        tc_fence_after();
+        const uint32_t sk_a = smem_u32(skv + st * S::kStage);
+        const uint32_t tmem_s = tmem_base + (uint32_t)(st * 128);
 #pragma unroll
         for (int ks = 0; ks < kFaD / 16; ++ks) {
           const uint64_t da = make_desc_k_sw128(sq_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
-          const uint64_t db = make_desc_k_sw128(sk_a + (uint32_t)((ks >> 2) * S::kHalf)) + (uint64_t)((ks & 3) * 2);
-          umma_f16_ss(tmem_base + (uint32_t)(st * 64), da, db, idesc_s, ks > 0 ? 1u : 0u);
+          const uint64_t db = make_desc_k_sw128(sk_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
+          umma_f16_ss(tmem_s, da, db, idesc_s, ks > 0 ? 1u : 0u);
         }
         tc_commit(&s_full[st]);
-        tc_commit(&k_empty[st]);
-        return true;
-      };
-      if (ok) ok = scores(0);
-      for (int j = 0; ok && j < nblk; ++j) {
-        const int st = j & 1;
-        if (j + 1 < nblk && !(ok = scores(j + 1))) break;
-        if (!mbar_wait(&p_full[st], (j >> 1) & 1, abort_flag) || !mbar_wait(&v_full[st], (j >> 1) & 1, abort_flag)) {
-          report_status(p.status, kTimeoutTmemEmpty, tile); *abort_flag = 1; ok = false; break;
-        }
-        tc_fence_after();
-        const uint32_t sv_a = smem_u32(svv + st * S::kBlock);
-        const uint32_t tmem_p = tmem_base + (uint32_t)(st * 64);
-#pragma unroll
-        for (int ks = 0; ks < kFaKeys / 16; ++ks) {
-          const uint64_t db = make_desc_mn_sw128(sv_a + (uint32_t)(ks * 2048), S::kHalf, 1024);
-          umma_f16_ts(tmem_o, tmem_p + (uint32_t)(ks * 8), db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-          if constexpr (WIDE) umma_f16_ts(tmem_o, tmem_p + (uint32_t)(32 + ks * 8), db, idesc_pv, 1u);
-        }
-        tc_commit(&v_empty[st]);
-        tc_commit(&pv_done[st]);
+        if (j > 0) ok = do_pv(j - 1);
       }
+      if (ok) do_pv(nblk - 1);
     }
     __syncwarp();
   } else if (nblk > 0) {
@@ -306,9 +306,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     sc.slope_l2 = p.alibi != nullptr ? p.alibi[head] * kFaLog2e : 0.f;
     const int mode = p.alibi != nullptr ? kFaBias : p.softcap > 0.f ? kFaCap : kFaPlain;
     const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t to = trow + 128u;
+    uint8_t* prow = sp + row * 128;
 
     float m = -INFINITY, l = 0.f;
+    float o[kFaD];
+#pragma unroll
+    for (int i = 0; i < kFaD; ++i) o[i] = 0.f;
     bool alive = true;
 
     for (int j = 0; j < nblk && alive; ++j) {
@@ -317,49 +320,55 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       if (!mbar_wait(&s_full[st], (j >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
       tc_fence_after();
       const bool need_mask = !(rows_all_valid && kb0 + kFaKeys <= hi_min && kb0 >= lo_max);
-      const uint32_t ts = trow + (uint32_t)(st * 64);
-      float s[kFaKeys];
-      {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32b_x32(ts, r0);
-        tmem_ld_32x32b_x32(ts + 32u, r1);
-        tc_wait_ld();
-#pragma unroll
-        for (int q = 0; q < 32; ++q) { s[q] = __uint_as_float(r0[q]); s[32 + q] = __uint_as_float(r1[q]); }
-      }
+      const uint32_t ts = trow + (uint32_t)(st * 128);
+      // pass 1: block maximum of this row (log2 domain)
       float bm;
-      if (mode == kFaPlain) bm = need_mask ? fa_block_max<kFaPlain, true>(s, kb0, lo, hi, sc) : fa_block_max<kFaPlain, false>(s, kb0, lo, hi, sc);
-      else if (mode == kFaCap) bm = need_mask ? fa_block_max<kFaCap, true>(s, kb0, lo, hi, sc) : fa_block_max<kFaCap, false>(s, kb0, lo, hi, sc);
-      else bm = fa_block_max<kFaBias, true>(s, kb0, lo, hi, sc);
-      // a row that has seen no key has added zeros to O: any maximum will do for it
-      const bool move = bm > m + kFaSlack<WIDE> && m > -INFINITY;
-      if (__any_sync(0xffffffffu, move)) {
-        const float alpha = move ? fa_ex2(m - bm) : 1.f;
-        if (!mbar_wait(&pv_done[st ^ 1], ((j - 1) >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
+      if (mode == kFaPlain) bm = need_mask ? fa_block_max<kFaPlain, true>(ts, kb0, lo, hi, sc) : fa_block_max<kFaPlain, false>(ts, kb0, lo, hi, sc);
+      else if (mode == kFaCap) bm = need_mask ? fa_block_max<kFaCap, true>(ts, kb0, lo, hi, sc) : fa_block_max<kFaCap, false>(ts, kb0, lo, hi, sc);
+      else bm = fa_block_max<kFaBias, true>(ts, kb0, lo, hi, sc);
+      const float m_new = fmaxf(m, bm);
+      const float alpha = (m_new == -INFINITY) ? 1.f : fa_ex2(m - m_new);
+      // the P tile is free once the MMAs of the previous block have read it
+      if (!mbar_wait(p_empty, (j & 1) ^ 1, abort_flag)) { report_status(p.status, kTimeoutTmemEmpty, tile); *abort_flag = 1; alive = false; break; }
+      // pass 2: probabilities -> bf16 operand tile, row sum
+      float sum;
+      if (mode == kFaPlain) sum = need_mask ? fa_block_probs<kFaPlain, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc)
+                                            : fa_block_probs<kFaPlain, false, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
+      else if (mode == kFaCap) sum = need_mask ? fa_block_probs<kFaCap, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc)
+                                               : fa_block_probs<kFaCap, false, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
+      else sum = fa_block_probs<kFaBias, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
+      tc_fence_before();
+      mbar_arrive(&s_empty[st]);
+      fence_proxy_async_smem();
+      mbar_arrive(p_full);
+      l = l * alpha + sum;
+      // fold the previous block's product in: o = (o + O_{j-1}) * alpha
+      if (j > 0) {
+        const int ps = (j - 1) & 1;
+        if (!mbar_wait(&pv_full[ps], ((j - 1) >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
         tc_fence_after();
-#pragma unroll 1
+        const bool same_max = __all_sync(0xffffffffu, alpha == 1.f);      // no row of the warp saw a new maximum: nothing to rescale
+#pragma unroll
         for (int c = 0; c < kFaD; c += 32) {
           uint32_t r[32];
-          tmem_ld_32x32b_x32(to + (uint32_t)c, r);
+          tmem_ld_32x32b_x32(trow + (uint32_t)(256 + ps * 128 + c), r);
           tc_wait_ld();
+          if (same_max) {
 #pragma unroll
-          for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(__uint_as_float(r[q]) * alpha);
-          tmem_st_32x32b_x32(to + (uint32_t)c, r);
+            for (int q = 0; q < 32; ++q) o[c + q] += __uint_as_float(r[q]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 32; ++q) o[c + q] = (o[c + q] + __uint_as_float(r[q])) * alpha;
+          }
         }
-        l *= alpha;
+        tc_fence_before();
+        mbar_arrive(&pv_empty[ps]);
       }
-      if (move || m == -INFINITY) m = bm;
-      float sum;
-      if (mode == kFaPlain) sum = need_mask ? fa_block_probs<kFaPlain, true, WIDE>(ts, s, kb0, lo, hi, m, sc) : fa_block_probs<kFaPlain, false, WIDE>(ts, s, kb0, lo, hi, m, sc);
-      else if (mode == kFaCap) sum = need_mask ? fa_block_probs<kFaCap, true, WIDE>(ts, s, kb0, lo, hi, m, sc) : fa_block_probs<kFaCap, false, WIDE>(ts, s, kb0, lo, hi, m, sc);
-      else sum = fa_block_probs<kFaBias, true, WIDE>(ts, s, kb0, lo, hi, m, sc);
-      l += sum;
-      tc_wait_st();
-      tc_fence_before();
-      mbar_arrive(&p_full[st]);
+      m = m_new;
     }
     if (alive) {
-      if (mbar_wait(&pv_done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, abort_flag)) {
+      const int ps = (nblk - 1) & 1;
+      if (mbar_wait(&pv_full[ps], ((nblk - 1) >> 1) & 1, abort_flag)) {
         tc_fence_after();
         const float inv = l > 0.f ? attn_denominator(p.tail, head, m, l) * p.tail.scale : 0.f;
         const __nv_bfloat16* grow = p.tail.gate != nullptr ? p.tail.gate + (long long)(tok_base + qi) * p.tail.ldg + (long long)head * kFaD : nullptr;
@@ -367,7 +376,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 #pragma unroll
         for (int c = 0; c < kFaD; c += 32) {
           uint32_t r[32];
-          tmem_ld_32x32b_x32(to + (uint32_t)c, r);
+          tmem_ld_32x32b_x32(trow + (uint32_t)(256 + ps * 128 + c), r);
           tc_wait_ld();
           if (row_ok) {
 #pragma unroll
@@ -375,7 +384,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
               uint32_t w[4];
               float v[8];
 #pragma unroll
-              for (int u = 0; u < 8; ++u) v[u] = __uint_as_float(r[q + u]) * inv;
+              for (int u = 0; u < 8; ++u) v[u] = (o[c + q + u] + __uint_as_float(r[q + u])) * inv;
               if (p.tail.turn != nullptr) attn_turn_back8(p.tail, v, c + q, cache + qi);
               if (grow != nullptr) {
                 const uint4 g = *reinterpret_cast<const uint4*>(grow + c + q);
@@ -401,7 +410,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, kFaTmemCols); }
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
 typedef CUresult (*FaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -423,11 +432,11 @@ static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const FaPara
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSmem::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSmem<WIDE>::kTotal);
     if (e != cudaSuccess) return -(int)e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_pdl(attn_prefill_tc_kernel<WIDE>, dim3(num_tiles, p.nh / 2), dim3(kFaThreads), (size_t)FaSmem::kTotal, s, tq, tkv, p);
+  launch_pdl(attn_prefill_tc_kernel<WIDE>, dim3(num_tiles, p.nh / 2), dim3(kFaThreads), (size_t)FaSmem<WIDE>::kTotal, s, tq, tkv, p);
   return -(int)cudaGetLastError();
 }
 

@@ -349,6 +349,59 @@ def test_attn_prefill_tensor_core(nat, nh, nkv, window, softcap, q_lens, cache_l
         assert torch.isfinite(got.float()).all()
 
 
+def _by_blocks(q, k, v, first, scale, block=128):
+    """Attention of one head in float64 the way prompt attention forms it: keys in blocks, weights rounded to bf16 relative to the largest
+    score up to and including their block, divided by the sum of the unrounded weights.  q [n, d] at positions first .., k and v [m, d]."""
+    t = q.double() @ k.double().t() * (scale * math.log2(math.e))
+    t = t.masked_fill(torch.arange(k.shape[0], device=t.device) > first + torch.arange(q.shape[0], device=t.device)[:, None], float("-inf"))
+    m = torch.full((q.shape[0], 1), float("-inf"), dtype=torch.float64, device=t.device)
+    total = torch.zeros_like(m)
+    o = torch.zeros(q.shape[0], v.shape[1], dtype=torch.float64, device=t.device)
+    for kb in range(0, k.shape[0], block):
+        s = t[:, kb: kb + block]
+        top = torch.maximum(m, s.max(-1, keepdim=True).values)
+        back, w = torch.exp2(m - top), torch.exp2(s - top)
+        total = total * back + w.sum(-1, keepdim=True)
+        o = o * back + w.to(torch.bfloat16).double() @ v[kb: kb + block].double()
+        m = top
+    return o / total
+
+
+@pytest.mark.parametrize("q_lens,cache_lens,climb", [([137], [0], 0.0), ([700, 64], [0, 331], 0.0), ([500], [0], 0.012), ([300], [450], -0.012)])
+def test_attn_prefill_weights_are_relative_to_the_largest_so_far(nat, q_lens, cache_lens, climb):
+    """The rounding of prompt attention's weights, also where the scores climb or fall by `climb` (log2) from key to key: a near tie that a
+    later layer decides on the last bits (the choice of an expert) comes out as before.  Only sums in fp32 and exp2 separate the kernel from the
+    same in 64 bits: 2^-20 of sums that are up to 2^4 times the result, so that one bf16 word in a hundred rounds the other way, and a few
+    weights in ten thousand.  (Weights relative to anything else are rounded otherwise: a tenth of all words differ and more.)"""
+    nh, nkv, d = 8, 2, 128
+    B, max_len = len(q_lens), max(a + b for a, b in zip(q_lens, cache_lens))
+    cache, bt = _make_cache(B, max_len, nkv, d, seed=len(q_lens))
+    g = torch.Generator().manual_seed(max_len)
+    T = sum(q_lens)
+    q = torch.randn(T, nh * d, generator=g).to(torch.bfloat16)
+    q.view(T, nh, d)[:, :, 0] = 8.0
+    q = q.cuda()
+    cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), device="cuda", dtype=torch.int32)
+    ts, tq = ref.prefill_tiles(q_lens)
+    scale = d ** -0.5
+    for b in range(B):
+        n = -(-max_len // 32)
+        rise = torch.arange(n * 32, device="cuda").view(n, 1, 32) * (climb / (8.0 * scale * math.log2(math.e)))
+        cache[bt[b].long(), :, 0, :, 0] = rise.to(torch.bfloat16)
+    got = nat.attn_prefill(q, cache, bt, cu, torch.tensor(cache_lens, device="cuda", dtype=torch.int32), torch.tensor(ts, device="cuda", dtype=torch.int32),
+                           torch.tensor(tq, device="cuda", dtype=torch.int32), nh, nkv, d, scale)
+    nat.workspace().check_status()
+    at = 0
+    for b in range(B):
+        n, m = q_lens[b], q_lens[b] + cache_lens[b]
+        pages = cache[bt[b].long()]                                            # [pages, nkv, 2, 32, d]
+        for h in range(nh):
+            kv = pages[:, h * nkv // nh].transpose(0, 1).reshape(2, -1, d)[:, :m]
+            want = _by_blocks(q[at: at + n, h * d: (h + 1) * d], kv[0], kv[1], cache_lens[b], scale).to(torch.bfloat16)
+            assert (got[at: at + n, h * d: (h + 1) * d] != want).float().mean() < 0.05, (b, h)
+        at += n
+
+
 @pytest.mark.parametrize("B,nh,nkv,d,window,softcap,nsplit", [(5, 8, 8, 128, 0, 0.0, 1), (3, 32, 8, 128, 50, 0.0, 8), (40, 32, 8, 128, 0, 20.0, 4),
                                                             (6, 20, 1, 64, 0, 0.0, 2), (38, 16, 8, 64, 33, 0.0, 1), (2, 34, 2, 128, 0, 0.0, 1)])
 def test_attn_decode_fp8_pages(nat, B, nh, nkv, d, window, softcap, nsplit):
