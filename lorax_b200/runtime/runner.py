@@ -99,9 +99,9 @@ class ModelRunner:
         self.max_prefill_tokens = max_prefill_tokens
         self.state = DecodeState(max_batch, self.max_blocks, self.device)
         self.use_graphs = use_graphs and self.is_cuda
-        self.graphs: Dict[Tuple[int, bool], object] = {}
+        self.graphs: Dict[tuple, object] = {}
         self.graph_pool = None
-        self.graph_out: Dict[Tuple[int, bool], torch.Tensor] = {}
+        self.graph_out: Dict[tuple, torch.Tensor] = {}
         self.buckets = [b for b in GRAPH_BUCKETS if b <= max_batch]
         if self.buckets[-1] != max_batch:
             self.buckets.append(max_batch)
@@ -133,7 +133,7 @@ class ModelRunner:
         self.steps = 0
         self.h2d_bytes = 0
         self.d2h_bytes = 0
-        self.graph_kernels: Dict[Tuple[int, bool], int] = {}
+        self.graph_kernels: Dict[tuple, int] = {}
         self.keep_logits = False                             # callers that read the logits of mixed steps
         self.last_logits: Optional[torch.Tensor] = None      # of the last mixed step (decode rows, then the prefill's scored rows)
         self.tiles_valid = False
@@ -472,8 +472,13 @@ class ModelRunner:
             return 0
         return min(8, (2 * 148) // max(1, self.state.num_lora_tiles))
 
+    def _graph_key(self, b: int, lora: bool, need_logits: bool):
+        """What the launches of a decode step depend on, apart from what lies in the state's buffers: the adapters' grids cover the largest
+        resident rank."""
+        return b, lora, self.tiles_valid, need_logits, self._ks_class(lora), self.model.adapters.max_rank if lora else 0
+
     def capture(self, b: int, lora: bool, need_logits: bool = False):
-        key = (b, lora, self.tiles_valid, need_logits, self._ks_class(lora))
+        key = self._graph_key(b, lora, need_logits)
         if key in self.graphs:
             return
         # warm up outside capture (lazy cudaFuncSetAttribute calls, workspace allocation)
@@ -519,8 +524,9 @@ class ModelRunner:
         logits = None
         if self.use_graphs:
             variant = need_logits and self.model.tp.world_size > 1      # only TP has two head variants
-            key = (b, lora, self.tiles_valid, variant, self._ks_class(lora))
-            self.capture(b, lora, variant)
+            key = self._graph_key(b, lora, variant)
+            if key not in self.graphs:
+                self.capture(b, lora, variant)
             self.graphs[key].replay()
             self.replayed_launches += self.graph_kernels[key]
             logits = self.graph_out[key] if (need_logits or shards) else None
