@@ -326,6 +326,17 @@ class AdapterManager:
             v = ops.lora_shrink(x, tok_slot, self.arena, self.slot_base, self.slot_rank, offA, nparts, self.max_rank)
         return LoraEpilogue(v, tok_slot, self.arena, self.slot_base, self.slot_rank, offB, n0, n1)
 
+    def launch_class(self, ops, rows: int, tiles: Optional[LoraTiles]) -> Tuple[int, ...]:
+        """What the launches of a step of `rows` rows take from the resident adapters and from the number of live entries, and a captured
+        graph therefore holds: the largest rank, which the grids cover, and the parts that shrinks of their own cut K into."""
+        if tiles is None:
+            return (self.max_rank,)
+        if rows <= SHORT_STEP and tiles.max_rows <= 32:
+            cut = lambda gi: ops.lora_shrink_parts(tiles.live, len(gi.parts), self.max_rank, gi.K)
+        else:
+            cut = lambda gi: ops.lora_shrink_ksplit(ops.workspace(self.device), tiles.live, len(gi.parts), self.max_rank, gi.K)
+        return (self.max_rank, *(cut(gi) for name, gi in self.layout.groups.items() if name != LM_HEAD))
+
     def fused(self, group: str, layer: int, tiles: Optional[LoraTiles]):
         """Descriptor of the projection group's LoRA for the GEMM that carries shrink and expand in its own launch
         (`ops.gemm_lora_fused`); None when the step has no tile table or nothing is resident."""

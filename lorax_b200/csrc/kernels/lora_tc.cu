@@ -600,6 +600,14 @@ int lx_lora_shrink_tc(const void* x, long long ldx, const void* tiles, int num_t
   return launch_shrink_tc<128>(tx, p, num_tiles, chunks, s);
 }
 
+// CTAs (a cluster) over which lx_lora_shrink_mma cuts K: while they stay within four per SM and a warp keeps four blocks of 32 elements.
+int lx_lora_shrink_parts(int live_tiles, int nparts, int max_rank, int K) {
+  const long long units = (long long)live_tiles * ((nparts * max_rank + 15) / 16);
+  int parts = 1;
+  while (parts < lx::kSrMaxParts && units * parts * 2 <= 4 * 148 && K >= parts * 2 * 4 * 4 * 32) parts *= 2;
+  return parts;
+}
+
 // The same for tiles of at most 32 rows of a short step (see lora_shrink_mma_kernel).  live_tiles: entries that are not padding.
 int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_tiles, int live_tiles, const void* arena, const long long* slot_base,
                        const int* slot_rank, int num_slots, long long unit_off, int nparts, float* v, int ldv, int T, int K, int max_rank,
@@ -614,10 +622,7 @@ int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_
   p.slot_base = slot_base; p.slot_rank = slot_rank; p.num_slots = num_slots; p.unit_off = unit_off;
   p.nparts = nparts; p.v = v; p.ldv = ldv; p.K = K; p.T = T; p.status = status;
   const int blocks16 = (nparts * max_rank + 15) / 16;
-  const long long units = (long long)(live_tiles > 0 ? live_tiles : num_tiles) * blocks16;
-  // K is cut while the CTAs stay within four per SM and a warp keeps four blocks of 32 elements
-  int parts = 1;
-  while (parts < kSrMaxParts && units * parts * 2 <= 4 * 148 && K >= parts * 2 * 4 * 4 * 32) parts *= 2;
+  const int parts = lx_lora_shrink_parts(live_tiles > 0 ? live_tiles : num_tiles, nparts, max_rank, K);
   launch_pdl_cluster(lora_shrink_mma_kernel, dim3(parts, num_tiles, blocks16), dim3(kSrThreads), dim3(parts, 1, 1), 0,
                      reinterpret_cast<cudaStream_t>(stream), p);
   return -(int)cudaGetLastError();

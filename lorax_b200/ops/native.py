@@ -88,6 +88,7 @@ def load() -> ctypes.CDLL:
         "lx_tensormap_bytes": ([], I),
         "lx_lora_encode_tmap": ([P, P, I, I, L, I], I),
         "lx_lora_encode_tmap_b": ([P, P, I, I, L, I], I),
+        "lx_lora_shrink_parts": ([I, I, I, I], I),
         "lx_lora_shrink_mma": ([P, L, P, I, I, P, P, P, I, L, I, P, I, I, I, I, P, P], I),
         "lx_lora_shrink_tc": ([P, L, P, I, I, P, I, I, P, I, I, I, P, I, L, I, P, P, I, I, I, I, P, P], I),
         "lx_gemm_bf16_lora": ([P, P, P, P, I, I, I, L, L, L, P, L, P, P, I, P, P], I),
@@ -705,6 +706,21 @@ def lora_encode_tmap_b(out_host: torch.Tensor, base_ptr: int, r: int, N: int, la
         raise NativeError(f"lx_lora_encode_tmap_b failed with code {rc}")
 
 
+def lora_shrink_ksplit(ws: "Workspace", live_tiles: int, nparts: int, max_rank: int, K: int, wanted: Optional[int] = None) -> int:
+    """Parts of K of the tensor-core shrink.  These skinny tiles are latency bound, so K is cut over as many CTAs as the GPU holds at once
+    (two per SM) and no more: a second, partly filled wave doubles the time.  `live_tiles` is the number of entries that are not padding
+    (CTAs of dead entries exit at once)."""
+    kblocks = (K + 63) // 64
+    if wanted is None:
+        wanted = max(1, (2 * ws.num_sms) // max(1, live_tiles * ((nparts * max_rank + 127) // 128)))
+    return max(1, min(ws.lora_v3.shape[0], kblocks // 8 if kblocks >= 8 else 1, wanted))
+
+
+def lora_shrink_parts(live_tiles: int, nparts: int, max_rank: int, K: int) -> int:
+    """Parts of K of the short step's shrink (no GPU needed)."""
+    return load().lx_lora_shrink_parts(live_tiles, nparts, max_rank, K)
+
+
 def lora_shrink_tiles(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, max_tile_rows: int, slot_tmaps: torch.Tensor,
                       groups_per_slot: int, group: int, slot_rank: torch.Tensor, nparts: int, layer: int, max_rank: int,
                       v: Optional[torch.Tensor] = None, ksplit: Optional[int] = None, live_tiles: int = 0):
@@ -715,14 +731,7 @@ def lora_shrink_tiles(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, max_
     vf = ws.lora_v if v is None else v
     v3 = ws.lora_v3
     assert vf.stride(0) == v3.stride(1)
-    kblocks = (K + 63) // 64
-    chunks = (nparts * max_rank + 127) // 128
-    # K split: these skinny tiles are latency bound, so K is cut over as many CTAs as the GPU holds at once (two per SM)
-    # and no more: a second, partly filled wave doubles the time.  `live_tiles` is the number of entries that are not
-    # padding (CTAs of dead entries exit at once).
-    if ksplit is None:
-        ksplit = max(1, (2 * ws.num_sms) // max(1, (live_tiles or num_tiles) * chunks))
-    ksplit = max(1, min(v3.shape[0], kblocks // 8 if kblocks >= 8 else 1, ksplit))
+    ksplit = lora_shrink_ksplit(ws, live_tiles or num_tiles, nparts, max_rank, K, ksplit)
     rc = load().lx_lora_shrink_tc(_ptr(x), x.stride(0), _ptr(tiles), num_tiles, max_tile_rows, _ptr(slot_tmaps), groups_per_slot, group,
                                   _ptr(slot_rank), slot_rank.shape[0], nparts, layer, _ptr(v3), v3.stride(1), v3.stride(0), ksplit,
                                   _ptr(vf), _ptr(ws.lora_counters), ws.lora_counters.numel(), T, K, max_rank, _ptr(ws.status), _stream())

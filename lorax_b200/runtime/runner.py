@@ -432,8 +432,7 @@ class ModelRunner:
     def _decode_body(self, b: int, lora: bool, need_logits: bool = False):
         st = self.state
         nsplit = self._attn_splits(b)
-        # the table always has max_batch rows; a graph launches one CTA per possible tile of the bucket (unused: slot -1)
-        tiles = LoraTiles(st.lora_tiles, b, 32, live=st.num_lora_tiles) if (lora and self.tiles_valid) else None
+        tiles = self._tiles(b, lora)
         fused = self.model.tp.fused if self.model.tp.world_size > 1 else None
         fused_head = (fused is not None and not need_logits and b <= fused.max_rows
                       and not (self.model.config.final_logit_softcapping or 0.0))
@@ -466,16 +465,16 @@ class ModelRunner:
         self.model.ops.advance_decode(st.input_ids[:b], st.next_ids[:b], st.positions[:b], st.ctx_lens[:b], st.slots[:b],
                                       st.block_tables[:b], self.page)
 
-    def _ks_class(self, lora: bool) -> int:
-        """The LoRA shrink's K split is baked into a captured graph; it depends on how many tiles are live."""
-        if not (lora and self.tiles_valid):
-            return 0
-        return min(8, (2 * 148) // max(1, self.state.num_lora_tiles))
+    def _tiles(self, b: int, lora: bool) -> Optional[LoraTiles]:
+        """The table always has max_batch rows; a graph launches one CTA per possible tile of the bucket (unused: slot -1).  A batch without
+        an adapter row counts as one tile: the launches are never sized by the padded table."""
+        st = self.state
+        return LoraTiles(st.lora_tiles, b, 32, live=max(1, st.num_lora_tiles)) if (lora and self.tiles_valid) else None
 
     def _graph_key(self, b: int, lora: bool, need_logits: bool):
-        """What the launches of a decode step depend on, apart from what lies in the state's buffers: the adapters' grids cover the largest
-        resident rank."""
-        return b, lora, self.tiles_valid, need_logits, self._ks_class(lora), self.model.adapters.max_rank if lora else 0
+        """Everything that the launches of a decode step depend on, apart from what lies in the state's buffers."""
+        ad = self.model.adapters
+        return b, lora, self.tiles_valid, need_logits, ad.launch_class(self.model.ops, b, self._tiles(b, lora)) if lora else ()
 
     def capture(self, b: int, lora: bool, need_logits: bool = False):
         key = self._graph_key(b, lora, need_logits)

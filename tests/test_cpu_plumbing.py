@@ -193,6 +193,39 @@ def test_adapter_exchange_under_memory_pressure():
     assert roomy == full and stats3.get("adapter_prefetches", 0) >= 1
 
 
+def test_graph_keys_hold_what_adapter_launches_depend_on():
+    """A captured decode step is used again only where a fresh one would launch the same: the largest resident rank and every projection's cut
+    of K are in its key, and a batch without adapter rows is not sized by the padded table."""
+    from types import SimpleNamespace as NS
+    from lorax_b200.adapters.lora import LM_HEAD
+    from lorax_b200.ops import native
+    from lorax_b200.runtime.runner import ModelRunner
+    groups = {"qkv": NS(parts=(0, 1, 2), K=4096), "o": NS(parts=(0,), K=4096), "gate_up": NS(parts=(0, 1), K=4096), "down": NS(parts=(0,), K=14336),
+              LM_HEAD: NS(parts=(0,), K=4096)}
+    ad = NS(max_rank=16, layout=NS(groups=groups), device=None)
+    ad.launch_class = lambda *a: AdapterManager.launch_class(ad, *a)
+    ops = NS(lora_shrink_parts=native.lora_shrink_parts, workspace=lambda dev: NS(num_sms=148, lora_v3=torch.empty(8, 1)),
+             lora_shrink_ksplit=native.lora_shrink_ksplit)
+    st = NS(lora_tiles=None, num_lora_tiles=0)
+    run = NS(model=NS(adapters=ad, ops=ops), state=st, tiles_valid=True)
+    run._tiles = lambda *a: ModelRunner._tiles(run, *a)
+    for bucket in (8, 256, 1024):
+        seen = {}
+        for ad.max_rank in (8, 16, 24, 64):
+            for st.num_lora_tiles in (*range(0, 70), 100, 200, 256):
+                live = run._tiles(bucket, True).live
+                assert live == max(1, st.num_lora_tiles)
+                if bucket <= 512:
+                    cut = [native.lora_shrink_parts(live, len(g.parts), ad.max_rank, g.K) for n, g in groups.items() if n != LM_HEAD]
+                else:
+                    cut = [native.lora_shrink_ksplit(ops.workspace(None), live, len(g.parts), ad.max_rank, g.K) for n, g in groups.items() if n != LM_HEAD]
+                assert seen.setdefault(ModelRunner._graph_key(run, bucket, True, False), (ad.max_rank, cut)) == (ad.max_rank, cut)
+        assert len({rank for rank, _ in seen.values()}) == 4 and len(seen) <= 4 * 24
+    assert ModelRunner._graph_key(run, 8, False, False) == (8, False, True, False, ())
+    run.tiles_valid = False
+    assert ModelRunner._graph_key(run, 8, True, False)[-1] == (64,)
+
+
 def test_vocabulary_parallel_sampling_equals_sampling_from_the_full_row():
     """Tensor-parallel ranks keep their vocabulary shard, exchange 128 candidates plus (max, sum exp) per row and the best
     (noisy score, log-probability, id) triple: the drawn ids equal those of the sampler that sees the whole row, for
