@@ -518,9 +518,9 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
 }
 
 template <int D>
-__global__ void __launch_bounds__(D) attn_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+__global__ void __launch_bounds__(D) attn_combine_kernel(const float* part_o, const float* part_lse,
                                                          __nv_bfloat16* __restrict__ out, long long ldo, int nh, int nsplit,
-                                                         const AttnTail tail, const int* __restrict__ ctx_lens) {
+                                                         const AttnTail tail, const int* ctx_lens) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
   const int t = blockIdx.x, h = blockIdx.y, d = threadIdx.x;

@@ -118,6 +118,10 @@ LX_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_fla
 //     successor reads before its wait (constant weights, tables that copies wrote) was complete before this kernel began;
 //   * behind the block's tensor memory allocation, if it has one: a successor's block on the same SM might take the columns first, and
 //     would hold them until this kernel has completed.
+// And one on how a kernel reads: what another kernel may write (activations, positions, slots, partial sums) through pointers that are not
+// `const __restrict__`, and never with __ldg.  Those loads (ld.global.nc) ask for memory that is constant while the grid runs, which the output
+// of a kernel that this one was set up under is not, and the compiler may move them in front of the wait.  They are for weights, adapters
+// and tables of constants.
 // ------------------------------------------------------------------------------------------------
 // Grids of more than eight blocks per SM do not trigger: a long kernel's successor gains nothing from a microsecond of set-up, and steps
 // of thousands of rows, which run against the power limit, took 3 to 5 % longer with it (6000 rows: 8.03 -> 8.56 ms a pass).

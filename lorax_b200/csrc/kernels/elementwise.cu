@@ -24,7 +24,7 @@ constexpr int kNormMaxVec = 8;   // 256 threads * 8 vec * 8 elems = 16384 column
 
 template <bool LAYERNORM, int NV>
 __global__ void __launch_bounds__(kNormThreads)
-norm_residual_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
+norm_residual_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ residual,
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                      __nv_bfloat16* __restrict__ out, int H, long long ldx, long long ldr, long long ldo, float eps,
                      float w_offset, float x_scale) {
@@ -154,8 +154,8 @@ LX_DEVICE uint32_t bf16x4_to_e4m3x4(uint2 w, float inv_scale) {
 }
 
 __global__ void __launch_bounds__(256)
-rope_kvwrite_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const float* __restrict__ cos_sin,
-                    __nv_bfloat16* __restrict__ kv_cache, const int* __restrict__ slots, int nh, int nkv, int d, int rot,
+rope_kvwrite_kernel(__nv_bfloat16* __restrict__ qkv, const int* positions, const float* __restrict__ cos_sin,
+                    __nv_bfloat16* __restrict__ kv_cache, const int* slots, int nh, int nkv, int d, int rot,
                     int page, long long ldq, int apply_rope, int kv_fp8, float k_inv_scale, float v_inv_scale) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -256,7 +256,7 @@ LX_DEVICE float act_fn(float x) {
 }
 template <int ACT, bool GATED>
 __global__ void __launch_bounds__(256)
-act_mul_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec) {
+act_mul_kernel(const __nv_bfloat16* in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
   const int vec_per_row = I / 8;
@@ -291,7 +291,7 @@ struct EmbedPeerParams {
   float mult;
 };
 
-__global__ void __launch_bounds__(128) embed_peer_kernel(const int* __restrict__ ids, const EmbedPeerParams p, __nv_bfloat16* __restrict__ out) {
+__global__ void __launch_bounds__(128) embed_peer_kernel(const int* ids, const EmbedPeerParams p, __nv_bfloat16* __restrict__ out) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
   const int t = blockIdx.x;
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(128) embed_peer_kernel(const int* __restrict__
 
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
-embed_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table, __nv_bfloat16* __restrict__ out, int H,
+embed_kernel(const int* ids, const __nv_bfloat16* __restrict__ table, __nv_bfloat16* __restrict__ out, int H,
              int v0, int v1, float mult) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -392,7 +392,7 @@ constexpr int kArgmaxMaxParts = 8;
 // VEC: rows start on 16-byte boundaries.
 template <bool VEC>
 __global__ void __launch_bounds__(kArgmaxThreads)
-argmax_logprob_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int V, int* __restrict__ ids,
+argmax_logprob_kernel(const __nv_bfloat16* logits, long long ld, int V, int* __restrict__ ids,
                       float* __restrict__ logprobs, float softcap) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -463,8 +463,8 @@ argmax_logprob_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, in
 //   input_ids <- next_ids; positions += 1; ctx_lens += 1; slots from the block table.
 // A row with ctx_lens < 0 is padding and is left alone.
 // ------------------------------------------------------------------------------------------------
-__global__ void advance_decode_kernel(int* __restrict__ input_ids, const int* __restrict__ next_ids, int* __restrict__ positions,
-                                      int* __restrict__ ctx_lens, int* __restrict__ slots, const int* __restrict__ block_tables,
+__global__ void advance_decode_kernel(int* __restrict__ input_ids, const int* next_ids, int* __restrict__ positions,
+                                      int* __restrict__ ctx_lens, int* __restrict__ slots, const int* block_tables,
                                       int max_blocks, int page, int B) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -481,7 +481,7 @@ __global__ void advance_decode_kernel(int* __restrict__ input_ids, const int* __
 
 // Points decode rows at given tokens and places: job[0..n) rows, then n input tokens, n positions, n cache slots.  One launch in place of a
 // widening of the indices and four scatters, which cost a step of one row 16 us of small launches and the gaps between them.
-__global__ void place_rows_kernel(const int* __restrict__ job, int n, int max_rows, int* __restrict__ input_ids, int* __restrict__ positions,
+__global__ void place_rows_kernel(const int* job, int n, int max_rows, int* __restrict__ input_ids, int* __restrict__ positions,
                                   int* __restrict__ ctx_lens, int* __restrict__ slots) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -497,8 +497,8 @@ __global__ void place_rows_kernel(const int* __restrict__ job, int n, int max_ro
 }
 
 __global__ void __launch_bounds__(256)
-prefill_metadata_kernel(const int* __restrict__ cu_q, const int* __restrict__ cache_lens, const int* __restrict__ seq_slot,
-                        const int* __restrict__ block_tables, int max_blocks, int B, int page, int T, int* __restrict__ positions,
+prefill_metadata_kernel(const int* cu_q, const int* cache_lens, const int* seq_slot,
+                        const int* block_tables, int max_blocks, int B, int page, int T, int* __restrict__ positions,
                         int* __restrict__ slots, int* __restrict__ tok_slot) {
   pdl_wait();
   pdl_trigger();

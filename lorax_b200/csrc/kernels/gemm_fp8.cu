@@ -231,7 +231,7 @@ gemm_fp8_block128_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
 }
 
 // x[T, K] bf16 -> xq[T, K] e4m3 and sa[kb, t] = amax(x[t, block kb]) / 448.  One warp per (token, K block).
-__global__ void __launch_bounds__(256) quant_act_fp8_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
+__global__ void __launch_bounds__(256) quant_act_fp8_kernel(const __nv_bfloat16* x, long long ldx, uint8_t* __restrict__ xq,
                                                             long long ldq, float* __restrict__ sa, int ld_sa, int T, int K) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) quant_act_fp8_kernel(const __nv_bfloat16*
 }
 
 // out[t, n] = bf16(sum_s partial[s, t, n] + bias[n]): the K splits in split order.
-__global__ void __launch_bounds__(256) fp8_splitk_reduce_kernel(const float* __restrict__ partial, int ksplit, int T, int N,
+__global__ void __launch_bounds__(256) fp8_splitk_reduce_kernel(const float* partial, int ksplit, int T, int N,
                                                                 const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out, long long ldo) {
   pdl_wait();      // every block waits, also those that return early below
   pdl_trigger();

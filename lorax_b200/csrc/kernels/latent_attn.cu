@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrepParams
 
 // Interleaved rotation of columns [off, off + rot) of every head of x [T, H * head], in place.
 template <typename T>
-__global__ void __launch_bounds__(256) rope_pairs_kernel(T* __restrict__ x, long long ldx, const int* __restrict__ positions,
+__global__ void __launch_bounds__(256) rope_pairs_kernel(T* __restrict__ x, long long ldx, const int* positions,
                                                          const float* __restrict__ cos_sin, int H, int head, int off, int rot) {
   pdl_wait();
   pdl_trigger();

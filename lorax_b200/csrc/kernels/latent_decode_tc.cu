@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(32 * WARPS, OCC) latent_decode_kernel(const La
 }
 
 // Shares of the keys -> one row: out = sum_s 2^(m_s - M) o_s / sum_s 2^(m_s - M) l_s.
-__global__ void __launch_bounds__(128) latent_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(128) latent_combine_kernel(const float* part_o, const float* part_ml,
                                                              __nv_bfloat16* __restrict__ out, long long ldo, int H, int KR, int nsplit) {
   pdl_wait();
   pdl_trigger();

@@ -323,8 +323,8 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
 // Rows of the sequences' pages, in order, as one contiguous matrix: latents [N, KR] and shared key parts [N, RR].  With a window a
 // sequence's rows begin window - 1 in front of its portion.
-__global__ void __launch_bounds__(128) latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ bt, int max_blocks,
-                                                            const int* __restrict__ ctx_off, const int* __restrict__ cache_lens, int window,
+__global__ void __launch_bounds__(128) latent_gather_kernel(const __nv_bfloat16* cache, const int* bt, int max_blocks,
+                                                            const int* ctx_off, const int* cache_lens, int window,
                                                             int B, int page, int KR, int RR,
                                                             __nv_bfloat16* __restrict__ lat, __nv_bfloat16* __restrict__ rot) {
   pdl_wait();

@@ -41,7 +41,7 @@ LX_DEVICE void moe_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uin
 }
 
 template <int MT, int NT, int UNROLL>
-__global__ void __launch_bounds__(32 * kRouterWarps) moe_router_logits_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
+__global__ void __launch_bounds__(32 * kRouterWarps) moe_router_logits_kernel(const __nv_bfloat16* x, long long ldx,
                                                                               const __nv_bfloat16* __restrict__ wr, long long ldw,
                                                                               float* __restrict__ logits, int T, int E, int H, int* counts,
                                                                               int ncounts) {
@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(256) moe_place_kernel(const MoePlaceParams p) 
 }
 
 // out[t, :] = sum_j w[t, j] * y[pos[t, j], :] over the experts of the token that this rank owns (fp32 sum in index order).
-__global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* __restrict__ y, long long ldy, const int* __restrict__ pos,
-                                                          const float* __restrict__ w, int k, __nv_bfloat16* __restrict__ out, long long ldo,
+__global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* y, long long ldy, const int* pos,
+                                                          const float* w, int k, __nv_bfloat16* __restrict__ out, long long ldo,
                                                           int T, int H) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -574,7 +574,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 }
 
 // The same product in true fp32: 64 features x 64 rows of one run per CTA.
-__global__ void __launch_bounds__(256) moe_grouped_gemm_f32_kernel(const float* __restrict__ x, long long ldx, const float* __restrict__ w,
+__global__ void __launch_bounds__(256) moe_grouped_gemm_f32_kernel(const float* x, long long ldx, const float* __restrict__ w,
                                                                    long long ldw, float* __restrict__ out, const MoeGemmParams p) {
   pdl_wait();
   __shared__ float xs[16][68], ws[16][68];

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
     const long long kx = (long long)kb * 128 + 32 * t;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      xv[q] = tok < p.T && kb < kblocks ? __ldg(reinterpret_cast<const uint4*>(p.x + tok * p.ldx + kx + 8 * q)) : make_uint4(0, 0, 0, 0);
+      xv[q] = tok < p.T && kb < kblocks ? *reinterpret_cast<const uint4*>(p.x + tok * p.ldx + kx + 8 * q) : make_uint4(0, 0, 0, 0);
   };
   int kb = warp;
   if (!p.w_const) pdl_wait();

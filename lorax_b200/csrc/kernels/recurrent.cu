@@ -376,7 +376,7 @@ static int rec_launch(const RecParams& p, int what, cudaStream_t s) {
 // row has read the old one.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ h, const float* __restrict__ mu, T* __restrict__ shift,
+__global__ void __launch_bounds__(256) token_shift_kernel(const T* h, const float* __restrict__ mu, T* __restrict__ shift,
                                                           T* __restrict__ out, int n_mix, int W, int Trows, StepRows rows) {
   pdl_wait();
   pdl_trigger();
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) shift_store_kernel(const T* __restrict__ h, T* __restrict__ shift, int W, StepRows rows) {
+__global__ void __launch_bounds__(256) shift_store_kernel(const T* h, T* __restrict__ shift, int W, StepRows rows) {
   pdl_wait();
   pdl_trigger();
   const int b = blockIdx.x;

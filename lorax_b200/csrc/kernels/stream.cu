@@ -36,9 +36,9 @@ LX_DEVICE int token_before(const EmbedPairs& e, const int* ids, int t) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) embed_stream_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,
+__global__ void __launch_bounds__(128) embed_stream_kernel(const int* ids, const T* __restrict__ table, float* __restrict__ out,
                                                            int W, int V, float mult, const T* __restrict__ pos,
-                                                           const int* __restrict__ positions, int P, T* __restrict__ copy,
+                                                           const int* positions, int P, T* __restrict__ copy,
                                                            const EmbedPairs pairs) {
   pdl_wait();
   pdl_trigger();
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kNsThreads, NEXT && NV <= 2 ? 4 : 1) norm_add_
 
 // out[i] = norm(residual[rows[i]]) (rows null: every row)
 template <typename T>
-__global__ void __launch_bounds__(kNsThreads) norm_rows_kernel(const float* __restrict__ residual, const int* __restrict__ rows,
+__global__ void __launch_bounds__(kNsThreads) norm_rows_kernel(const float* residual, const int* rows,
                                                                const float* __restrict__ w, const float* __restrict__ b, T* __restrict__ out,
                                                                int W, int n, float inv_n, float eps, float w_offset, int layernorm) {
   pdl_wait();
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kNsThreads) norm_rows_kernel(const float* __re
 // sigmoid(gate) or silu(gate).  WARP: one warp per group (up to 512 columns), else one CTA per group.
 // ------------------------------------------------------------------------------------------------
 template <typename T, bool WARP>
-__global__ void __launch_bounds__(256) norm_gate_kernel(const float* __restrict__ x, const float* __restrict__ w, const T* __restrict__ gate,
+__global__ void __launch_bounds__(256) norm_gate_kernel(const float* x, const float* __restrict__ w, const T* gate,
                                                         long long ldg, T* __restrict__ out, long long ldo, int groups, int group, float inv_n,
                                                         float eps, int silu) {
   pdl_wait();
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(256) tanh_kernel(T* __restrict__ x, long long 
 }
 
 // out[t, i] = act(x[t, i]) (* x[t, I + i]) for fp32 rows
-__global__ void __launch_bounds__(256) act_mul_f32_kernel(const float* __restrict__ x, float* __restrict__ out, int I, long long ldx,
+__global__ void __launch_bounds__(256) act_mul_f32_kernel(const float* x, float* __restrict__ out, int I, long long ldx,
                                                           long long ldo, long long total4, int act, int gated) {
   pdl_wait();
   pdl_trigger();
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(256) act_mul_f32_kernel(const float* __restric
 
 // out[t, i] = g * sigmoid(alpha g) * (u + 1), g = min(x[t, i], limit), u = x[t, I + i] within +-limit.
 template <typename T>
-__global__ void __launch_bounds__(256) clamped_swiglu_kernel(const T* __restrict__ x, T* __restrict__ out, int I, long long ldx, long long ldo,
+__global__ void __launch_bounds__(256) clamped_swiglu_kernel(const T* x, T* __restrict__ out, int I, long long ldx, long long ldo,
                                                              long long total, float alpha, float limit) {
   pdl_wait();
   pdl_trigger();
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(256) clamped_swiglu_kernel(const T* __restrict
 }
 
 // Greedy head over fp32 logits: arg-max (lowest index on ties) and its log-probability.
-__global__ void __launch_bounds__(512) argmax_f32_kernel(const float* __restrict__ logits, long long ld, int V, int* __restrict__ ids,
+__global__ void __launch_bounds__(512) argmax_f32_kernel(const float* logits, long long ld, int V, int* __restrict__ ids,
                                                          float* __restrict__ lps, float softcap) {
   pdl_wait();
   pdl_trigger();

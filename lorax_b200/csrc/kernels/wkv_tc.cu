@@ -135,10 +135,10 @@ __global__ void __launch_bounds__(kWkThreads, 2) wkv_tc_kernel(const WkvTcParams
     const long long t = tok0 + t0 + lt;
     const bool ok = t0 + lt < n;
     const int c = h * kWkD + lc;
-    gk = ok ? __ldg(reinterpret_cast<const uint4*>(p.k + t * p.ldk + c)) : zero4;
-    gv = ok ? __ldg(reinterpret_cast<const uint4*>(p.v + t * p.ldv + c)) : zero4;
-    gz = ok ? __ldg(reinterpret_cast<const uint4*>(p.z + t * p.ldz + c)) : zero4;
-    if (!STATES) gr = ok ? __ldg(reinterpret_cast<const uint4*>(p.r + t * p.ldr + c)) : zero4;
+    gk = ok ? *reinterpret_cast<const uint4*>(p.k + t * p.ldk + c) : zero4;
+    gv = ok ? *reinterpret_cast<const uint4*>(p.v + t * p.ldv + c) : zero4;
+    gz = ok ? *reinterpret_cast<const uint4*>(p.z + t * p.ldz + c) : zero4;
+    if (!STATES) gr = ok ? *reinterpret_cast<const uint4*>(p.r + t * p.ldr + c) : zero4;
   };
   fetch(0);
 

@@ -1,0 +1,45 @@
+"""Rules that the CUDA sources keep and that no run would show reliably."""
+import re
+from pathlib import Path
+
+KERNELS = Path(__file__).resolve().parents[1] / "lorax_b200" / "csrc" / "kernels"
+# what kernels read without any kernel writing it: weights, biases, scales, adapters, embedding tables, tables of angles
+CONSTANT_PARAMS = {"w", "b", "bias", "wr", "mu", "q", "sw", "table", "pos", "cos_sin"}
+CONSTANT_LOADS = re.compile(r"__ldg\((reinterpret_cast<const (uint4|float4)\*>\()?(cs\b|a0 \+|a1 \+|wr \+|B \+|arow \+)")
+
+
+def _sources():
+    for path in sorted([*KERNELS.glob("*.cu"), *KERNELS.glob("*.cuh")]):
+        yield path.name, re.sub(r"//[^\n]*", "", path.read_text())
+
+
+def _kernels():
+    for name, text in _sources():
+        for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\s*\(([^{;]*?)\)\s*\{", text, re.S):
+            depth, end = 1, m.end()
+            while depth:
+                depth += (text[end] == "{") - (text[end] == "}")
+                end += 1
+            yield f"{name}:{m.group(1)}", m.group(2), text[m.end():end]
+
+
+def test_output_of_the_kernel_in_front_is_not_read_as_constant():
+    """A kernel that is set up under its predecessor reads what kernels write with ordinary loads behind its wait: no `const __restrict__`
+    parameter and no __ldg for anything but constants."""
+    seen = 0
+    for kernel, params, body in _kernels():
+        if "pdl_wait" not in body:
+            continue
+        seen += 1
+        read_only = {p.split()[-1] for p in params.split(",") if re.search(r"\bconst\b.*__restrict__", p)}
+        assert read_only <= CONSTANT_PARAMS, (kernel, read_only - CONSTANT_PARAMS)
+    assert seen > 40
+    for name, text in _sources():
+        for line in text.splitlines():
+            assert line.count("__ldg(") == len(CONSTANT_LOADS.findall(line)), (name, line.strip())
+
+
+def test_triggers_stand_behind_the_wait():
+    for kernel, _, body in _kernels():
+        at = [body.find(f) for f in ("pdl_trigger()", "pdl_launch_dependents()") if f in body]
+        assert not at or 0 <= body.find("pdl_wait()") < min(at) or "shrink_rows_part" in body, kernel
