@@ -146,12 +146,12 @@ def bench_lora(results, peaks):
             out = torch.empty(T, N, device="cuda", dtype=torch.bfloat16)
             n0 = parts[0] if nparts > 1 else N
             n1 = parts[0] + parts[1] if nparts > 2 else N
-            lf = native.LoraFused(tiles, tiles.shape[0], len(tl), tmaps, 2 * G, 0, G, slot_rank, slot_base, nparts, n0, n1, 0, r, arena, 0, nparts * K)
+            lf = native.LoraFused(tiles, tiles.shape[0], len(tl), tmaps, 2 * G, 0, G, slot_rank, slot_base, nparts, n0, n1, 0, r, arena, 0, nparts * K, tables_const=True)
 
             def separate(i):
                 v = native.lora_shrink_tiles(x, tiles, tiles.shape[0], 32, tmaps, 2 * G, 0, slot_rank, nparts, 0, r, live_tiles=len(tl))
                 native.gemm(x, ws[i], out=out)
-                native.lora_expand_tiles(v[:T], tiles, tiles.shape[0], 32, arena, slot_base, slot_rank, nparts * K, out, n0, n1)
+                native.lora_expand_tiles(v[:T], tiles, tiles.shape[0], 32, arena, slot_base, slot_rank, nparts * K, out, n0, n1, tables_const=True)
             ms_f = _time(lambda i: native.gemm_lora_fused(x, ws[i], lf, out=out), n_rot)
             ms_s = _time(separate, n_rot)
             ms_b = _time(lambda i: native.gemm(x, ws[i], out=out), n_rot)

@@ -78,7 +78,7 @@ def lora_case(which):
     for _ in range(4):
         v = native.lora_shrink_tiles(x, tiles, T, 32, tmaps, G, 0, slot_rank, 3, 0, r)
         if which == "expand":
-            native.lora_expand_tiles(v[:T], tiles, T, 32, arena, slot_base, slot_rank, 3 * K, y, parts[0], parts[0] + parts[1])
+            native.lora_expand_tiles(v[:T], tiles, T, 32, arena, slot_base, slot_rank, 3 * K, y, parts[0], parts[0] + parts[1], tables_const=True)
 
 
 def gemm_lora_case(T, parts=(4096, 1024, 1024)):
@@ -109,7 +109,7 @@ def gemm_lora_case(T, parts=(4096, 1024, 1024)):
     out = torch.empty(T, N, device="cuda", dtype=torch.bfloat16)
     n0 = parts[0] if nparts > 1 else N
     n1 = parts[0] + parts[1] if nparts > 2 else N
-    lf = native.LoraFused(tiles, tiles.shape[0], len(tl), tmaps, 2 * G, 0, G, slot_rank, slot_base, nparts, n0, n1, 0, r, arena, 0, nparts * K)
+    lf = native.LoraFused(tiles, tiles.shape[0], len(tl), tmaps, 2 * G, 0, G, slot_rank, slot_base, nparts, n0, n1, 0, r, arena, 0, nparts * K, tables_const=True)
     for i in range(4):
         assert native.gemm_lora_fused(x, ws[i], lf, out=out) is not None
 

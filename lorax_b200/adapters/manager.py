@@ -314,7 +314,7 @@ class AdapterManager:
                 return None
             if self.is_cuda and x.shape[0] <= SHORT_STEP and tiles.max_rows <= 32:
                 v = ops.lora_shrink_mma(x, tiles.table, tiles.num_tiles, self.arena, self.slot_base, self.slot_rank, offA, nparts, self.max_rank,
-                                        live_tiles=tiles.live)
+                                        live_tiles=tiles.live, tables_const=True)      # (copies write them, in front of the step)
             elif self.is_cuda:
                 v = ops.lora_shrink_tiles(x, tiles.table, tiles.num_tiles, tiles.max_rows, self.slot_tmaps, self.groups_per_slot,
                                           TMAP_GROUPS.index(group), self.slot_rank, nparts, 0 if group == LM_HEAD else layer, self.max_rank,
@@ -350,7 +350,7 @@ class AdapterManager:
         g = TMAP_GROUPS.index(group)
         return LoraFused(tiles.table, tiles.num_tiles, tiles.live, self.slot_tmaps, self.groups_per_slot, g, len(TMAP_GROUPS) + g,
                          self.slot_rank, self.slot_base, len(gi.parts), n0, n1, 0 if group == LM_HEAD else layer, self.max_rank,
-                         self.arena, self.layout.unit_off(group, layer, "A"), self.layout.unit_off(group, layer, "B"))
+                         self.arena, self.layout.unit_off(group, layer, "A"), self.layout.unit_off(group, layer, "B"), tables_const=True)
 
     def expand(self, ops, epi, y: torch.Tensor, tiles: Optional[LoraTiles] = None):
         """y += v B_cat(slot(t))^T: the second half of the LoRA delta as its own launch (`epi` comes from `shrink`)."""
@@ -358,7 +358,7 @@ class AdapterManager:
             return
         if tiles is not None:
             ops.lora_expand_tiles(epi.v[: y.shape[0]], tiles.table, tiles.num_tiles, tiles.max_rows, epi.arena, epi.slot_base, epi.slot_rank,
-                                  epi.unit_off, y, epi.n0, epi.n1)
+                                  epi.unit_off, y, epi.n0, epi.n1, **(dict(tables_const=True) if self.is_cuda else {}))
         else:
             ops.lora_expand(epi.v, epi.tok_slot, epi.arena, epi.slot_base, epi.slot_rank, epi.unit_off, y, epi.n0, epi.n1)
 

@@ -86,6 +86,7 @@ struct GemmParams {
   int lora_inline_shrink;              // 1: the epilogue warps compute the shrink during the first K loop (0: a launch in front did)
   int* lora_sync;                      // [2] CTAs of this launch that have finished / whose shrink units are done; zero between launches
   int lora_arena_maps;                 // 1: B_cat tiles come through the four arena-wide maps of the launch (LoraBMaps), not the slots' own
+  int lora_tables_const;               // tables and adapters may be read before the wait for the kernel in front
   int lora_fence_maps;                 // 1: acquire-fence a slot's B_cat map before every use (0: never; measurement only)
   int lora_skip;                       // measurement only: bit 0 leaves out the shrink launch, bit 1 the expand stages (results are then wrong)
   int lora_T;                          // rows of the step
@@ -635,9 +636,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
   if constexpr (LORA) {
-    // the table, the slot ranks and the slot offsets are written by copies that the stream orders before every kernel, never by
+    // in a step the table, the slot ranks and the slot offsets are written by copies that the stream orders before every kernel, never by
     // the kernel in front of this one: reading them does not have to wait for that kernel to drain
     if (lora) {
+      if (!p.lora_tables_const) pdl_wait();
       load_lora_entries(p, ents, n_live);
       __syncthreads();
       if (p.lora_inline_shrink && warp == 2) lora_group_prefix(p, ents, gstart);
@@ -1241,6 +1243,7 @@ struct LoraShrinkRowsParams {
   long long off_a;          // A_cat of the projection group and layer starts at slot_base + r * off_a (elements)
   int nparts;
   __nv_bfloat16* vimg;
+  int tables_const;
 };
 
 LX_DEVICE float dot8_bf16(const uint4& a, const uint4& b) {
@@ -1266,7 +1269,8 @@ __global__ void __launch_bounds__(kShrinkRowsThreads) lora_shrink_rows_kernel(co
   __shared__ float s_v[3 * 64 * kShrinkG];
   const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) s_ent[0] = -1;
-  // CTA b -> (entry, group of four rows): groups are numbered entry by entry (a prefix sum over the table).  The table is
+  if (!p.tables_const) pdl_wait();
+  // CTA b -> (entry, group of four rows): groups are numbered entry by entry (a prefix sum over the table).  In a step the table is
   // written by copies that the stream orders before every kernel: it may be read before the wait below.
   int seen = 0;                                                      // groups of the entries before this round
   for (int lt0 = 0; lt0 < p.num_tiles; lt0 += kShrinkRowsThreads) {
@@ -1646,6 +1650,7 @@ struct LxLoraFused {
   long long off_b, arena_elems;            // B_cat likewise; the arena's size bounds the arena-wide maps
   int* sync;                               // two ints, zero before the first launch (see GemmParams::lora_sync)
   int w_const;                             // 1: the kernel in front on the stream does not write w (mode bit 16 of lx_gemm_bf16)
+  int tables_const;                        // 1: nor tiles, slot_rank, slot_base, the maps and the arena (in a step copies do)
 };
 
 static int gemm_impl(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
@@ -1739,6 +1744,7 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     p.lora_nparts = lora->nparts; p.lora_n0 = lora->n0; p.lora_n1 = lora->n1; p.lora_layer = lora->layer;
     p.lora_vimg = reinterpret_cast<__nv_bfloat16*>(lora->vimg);
     p.lora_fence_maps = lora->fence_maps;
+    p.lora_tables_const = lora->tables_const;
     p.lora_off_b = lora->off_b;
     LoraBMaps bm{};
     p.lora_arena_maps = (lora->arena_elems > 0 && make_lora_bmaps(&bm, lora->arena, lora->arena_elems, N) == 0) ? 1 : 0;
@@ -1772,6 +1778,7 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       sp.slot_rank = lora->slot_rank; sp.slot_base = lora->slot_base; sp.num_slots = lora->num_slots;
       sp.off_a = lora->off_a; sp.nparts = lora->nparts;
       sp.vimg = p.lora_vimg;
+      sp.tables_const = lora->tables_const;
       const int rc = launch_lora_shrink_rows(sp, lora->max_rank, num_sms, stream);
       if (rc != 0) return rc;
     }

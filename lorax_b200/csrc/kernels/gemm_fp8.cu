@@ -38,6 +38,7 @@ struct Fp8Params {
   int ksplit;                   // > 1: every tile's K range is cut into ksplit parts, each writes fp32 to `partial`
   float* partial;               // [ksplit][T][N]
   int* status;
+  int w_const;                  // no kernel that may still run writes the weights: their first tiles are loaded before pdl_wait
 };
 
 template <int BN, int STAGES>
@@ -85,8 +86,8 @@ gemm_fp8_block128_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
-  // The weights' half of the first stages is loaded before the wait for the kernel in front: that is the activations' quantiser, which has
-  // itself waited for whatever may have written the weights.
+  // The weights' half of the first stages is loaded before the wait for the kernel in front where the caller allows it.
+  if (!p.w_const) pdl_wait();
   const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
   int preloaded = 0;
   if (threadIdx.x == 0 && (int)blockIdx.x < num_tiles * p.ksplit) {
@@ -335,9 +336,10 @@ int lx_quant_act_fp8(const void* x, long long ldx, void* xq, long long ldq, floa
 }
 
 // out[T, N] (bf16) = block-scaled fp8 product of xq[T, K] (scales sa[kb, t]) and wq[N, K] (scales sw[N/128, K/128]) + bias.
+// w_const: the kernel in front on the stream does not write wq.
 int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_sa, const void* wq, long long ldw, const float* sw,
                          void* out, long long ldo, const void* bias, int T, int N, int K, void* ws, long long ws_bytes, int* status,
-                         int num_sms, void* stream_) {
+                         int num_sms, int w_const, void* stream_) {
   using namespace lx;
   if (T <= 0 || N <= 0) return 0;
   if (K % 16 != 0 || ldq % 16 != 0 || ldw % 16 != 0) return -1000;
@@ -347,6 +349,7 @@ int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_
   p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.status = status;
+  p.w_const = w_const;
   // token tile: the fewest tiles of at most 128 tokens, evenly sized
   const int t16 = (T + 15) / 16 * 16;
   const int ttiles = (t16 + 127) / 128;

@@ -49,14 +49,14 @@ int lx_lora_expand(const float* v, int ldv, const int* tok_slot, const void* are
                    int* status, void* stream);
 int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_tiles, int live_tiles, const void* arena, const long long* slot_base,
                        const int* slot_rank, int num_slots, long long unit_off, int nparts, float* v, int ldv, int T, int K, int max_rank,
-                       int* status, void* stream);
+                       int* status, int tables_const, void* stream);
 int lx_lora_shrink_tc(const void* x, long long ldx, const void* tiles, int num_tiles, int max_tile_rows, const void* slot_tmaps,
                       int groups_per_slot, int group, const int* slot_rank, int num_slots, int nparts, int layer, float* v, int ldv,
                       long long v_split_stride, int ksplit, float* v_final, int* counters, int num_counters, int T, int K, int max_rank,
                       int* status, void* stream);
 int lx_lora_expand_tiled(const float* v, int ldv, long long v_split_stride, int ksplit, const void* tiles, int num_tiles,
                          int max_tile_rows, const void* arena, const long long* slot_base, const int* slot_rank, int num_slots,
-                         long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1, int* status, void* stream);
+                         long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1, int* status, int tables_const, void* stream);
 int lx_gemm_bf16(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
                  long long ldw, long long ldo, float out_scale, void* ws, long long ws_bytes, int* counters,
                  int* status, int num_sms, int mode, int force_split, void* stream_);
@@ -70,7 +70,7 @@ struct LxLoraFused {
   const void* arena; long long off_a;
   long long off_b, arena_elems;
   int* sync;
-  int w_const;
+  int w_const, tables_const;
 };
 int lx_gemm_bf16_lora(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
                       long long ldw, long long ldo, void* ws, long long ws_bytes, int* counters, int* status, int num_sms,
@@ -169,7 +169,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
     f.slot_rank = m.slot_rank; f.slot_base = m.slot_base; f.num_slots = m.num_slots;
     f.nparts = site.nparts; f.n0 = site.n0; f.n1 = site.n1; f.layer = l.layer_index; f.max_rank = m.max_rank;
     f.vimg = m.lora_vimg; f.vimg_bytes = m.lora_vimg_bytes; f.fence_maps = m.lora_fence_maps;
-    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync; f.w_const = 1;
+    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync; f.w_const = f.tables_const = 1;
     const int rc = lx_gemm_bf16_lora(x, w, y, bias, s.T, N, K, ldx, ldw, ldy, m.gemm_ws, m.gemm_ws_bytes, m.gemm_counters, m.status, m.num_sms,
                                      &f, stream);
     if (rc != 1) return rc;          // 1: this step does not fit the fused launch, use the separate kernels below
@@ -177,7 +177,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
   if (lora) {
     if (s.lora_tiles != nullptr && s.T <= kShortStep && s.max_tile_rows <= 32) {
       LX_TRY(lx_lora_shrink_mma(x, ldx, s.lora_tiles, s.num_tiles, s.live_tiles, m.arena, m.slot_base, m.slot_rank, m.num_slots, site.off_a,
-                                site.nparts, m.lora_v, m.ldv, s.T, K, m.max_rank, m.status, stream));
+                                site.nparts, m.lora_v, m.ldv, s.T, K, m.max_rank, m.status, 1, stream));
     } else if (s.lora_tiles != nullptr) {
       const int kblocks = (K + 63) / 64;
       const int chunks = (site.nparts * m.max_rank + 127) / 128;
@@ -198,7 +198,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
   if (lora) {
     if (s.lora_tiles != nullptr) {
       LX_TRY(lx_lora_expand_tiled(m.lora_v, m.ldv, 0, 1, s.lora_tiles, s.num_tiles, s.max_tile_rows, m.arena, m.slot_base, m.slot_rank,
-                                  m.num_slots, site.off_b, y, ldy, s.T, N, site.n0, site.n1, m.status, stream));
+                                  m.num_slots, site.off_b, y, ldy, s.T, N, site.n0, site.n1, m.status, 1, stream));
     } else {
       LX_TRY(lx_lora_expand(m.lora_v, m.ldv, s.tok_slot, m.arena, m.slot_base, m.slot_rank, m.num_slots, site.off_b, y, ldy, s.T, N,
                             site.n0, site.n1, m.status, stream));

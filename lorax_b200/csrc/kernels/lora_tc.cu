@@ -247,6 +247,7 @@ struct ShrinkRowsParams {
   int ldv;
   int K, T;
   int* status;
+  int tables_const;                // no kernel that may still run writes tiles, slot tables and arena: they are read before the wait
 };
 
 constexpr int kSrThreads = 128;
@@ -279,7 +280,7 @@ LX_DEVICE void shrink_rows_part(const ShrinkRowsParams& p, const __nv_bfloat16* 
       ra[i] = in && g < rows_a ? __ldg(a0 + kk) : zero;
       rb[i] = in && g + 8 < rows_a ? __ldg(a1 + kk) : zero;
     }
-    if (!waited) {                                                  // (A_cat was written by copies in front of the step; x by the kernel in front)
+    if (!waited) {                                                  // (x comes from the kernel in front)
       pdl_wait();
       pdl_trigger();
       waited = true;
@@ -315,6 +316,7 @@ __global__ void __launch_bounds__(kSrThreads) lora_shrink_mma_kernel(const Shrin
   __shared__ __align__(16) float red[4 * 16 * 32];
   __shared__ float gathered[kSrMaxParts][16 * 32];                  // (of the cluster's first CTA)
   const int part = blockIdx.x, parts = gridDim.x;
+  if (!p.tables_const) pdl_wait();
   const LoraTile tile = p.tiles[blockIdx.y];                        // (a cluster has one tile: its CTAs leave together)
   const int nrows = min(min(tile.nrows, 32), p.T - tile.row0);      // a table may be older than the batch: rows past T are gone
   const bool known = tile.slot >= 0 && tile.slot < p.num_slots;
@@ -367,6 +369,7 @@ struct ExpandTiledParams {
   int n0, n1, N, T;
   int num_tiles, col_blocks;
   int* status;
+  int tables_const;                // as for the shrink
 };
 
 constexpr int kExpThreads = 256;
@@ -386,13 +389,14 @@ constexpr int kExpRowsInFlight = 4;                  // rows whose y loads are i
 // The grid is a fixed number of CTAs that walk the units; live tiles come first in the table, so the walk stops at
 // the first dead one and padding entries cost nothing.
 //
-// The table, the slots' offsets and B_cat were written by copies in front of the step, so the first unit's are read before the wait for the
-// kernel in front, and the next unit's entry while the current one is multiplied.
+// Where the caller says that no kernel in front writes the table, the slots' offsets and B_cat (in a step copies do), the first unit's are read
+// before the wait for the kernel in front.  The next unit's entry is read while the current one is multiplied.
 __global__ void __launch_bounds__(kExpThreads, kExpCtas) lora_expand_tiled_kernel(const ExpandTiledParams p) {
   __shared__ __align__(16) float vs[kExpMaxRows * 3 * kExpStage];   // [row][part][16]
   const int nparts = p.n1 < p.N ? 3 : (p.n0 < p.N ? 2 : 1);
   const int units = p.num_tiles * p.col_blocks;
   const LoraTile dead{-1, 0, 0, 0};
+  if (!p.tables_const) pdl_wait();
   auto known = [&](const LoraTile& t) { return t.slot >= 0 && t.slot < p.num_slots; };
   // entry, rank and offset of the unit at hand and (two loads that hang on one another) of the next one
   LoraTile tile = (int)blockIdx.x < units ? p.tiles[blockIdx.x / p.col_blocks] : dead;
@@ -608,10 +612,11 @@ int lx_lora_shrink_parts(int live_tiles, int nparts, int max_rank, int K) {
   return parts;
 }
 
-// The same for tiles of at most 32 rows of a short step (see lora_shrink_mma_kernel).  live_tiles: entries that are not padding.
+// The same for tiles of at most 32 rows of a short step (see lora_shrink_mma_kernel).  tables_const: the kernel in front on the stream writes
+// neither the tiles nor the slots' tables nor the arena.  live_tiles: entries that are not padding.
 int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_tiles, int live_tiles, const void* arena, const long long* slot_base,
                        const int* slot_rank, int num_slots, long long unit_off, int nparts, float* v, int ldv, int T, int K, int max_rank,
-                       int* status, void* stream) {
+                       int* status, int tables_const, void* stream) {
   using namespace lx;
   if (num_tiles <= 0 || max_rank <= 0) return 0;
   if (K % 8 != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0 || nparts * max_rank > ldv || num_tiles > 65535) return -1;
@@ -620,7 +625,7 @@ int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_
   p.x = reinterpret_cast<const __nv_bfloat16*>(x); p.ldx = ldx;
   p.arena = reinterpret_cast<const __nv_bfloat16*>(arena);
   p.slot_base = slot_base; p.slot_rank = slot_rank; p.num_slots = num_slots; p.unit_off = unit_off;
-  p.nparts = nparts; p.v = v; p.ldv = ldv; p.K = K; p.T = T; p.status = status;
+  p.nparts = nparts; p.v = v; p.ldv = ldv; p.K = K; p.T = T; p.status = status; p.tables_const = tables_const;
   const int blocks16 = (nparts * max_rank + 15) / 16;
   const int parts = lx_lora_shrink_parts(live_tiles > 0 ? live_tiles : num_tiles, nparts, max_rank, K);
   launch_pdl_cluster(lora_shrink_mma_kernel, dim3(parts, num_tiles, blocks16), dim3(kSrThreads), dim3(parts, 1, 1), 0,
@@ -630,7 +635,8 @@ int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_
 
 int lx_lora_expand_tiled(const float* v, int ldv, long long v_split_stride, int ksplit, const void* tiles, int num_tiles,
                          int max_tile_rows, const void* arena, const long long* slot_base, const int* slot_rank, int num_slots,
-                         long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1, int* status, void* stream) {
+                         long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1, int* status, int tables_const,
+                         void* stream) {
   using namespace lx;
   (void)v_split_stride;
   if (num_tiles <= 0) return 0;
@@ -642,6 +648,7 @@ int lx_lora_expand_tiled(const float* v, int ldv, long long v_split_stride, int 
   p.slot_base = slot_base; p.slot_rank = slot_rank; p.num_slots = num_slots; p.unit_off = unit_off;
   p.v = v; p.ldv = ldv; p.y = reinterpret_cast<__nv_bfloat16*>(y); p.ldy = ldy; p.n0 = n0; p.n1 = n1; p.N = N; p.T = T;
   p.status = status;
+  p.tables_const = tables_const;
   p.num_tiles = num_tiles;
   p.col_blocks = (N + kExpBlockCols - 1) / kExpBlockCols;
   const long long work = (long long)num_tiles * p.col_blocks;

@@ -89,17 +89,17 @@ def load() -> ctypes.CDLL:
         "lx_lora_encode_tmap": ([P, P, I, I, L, I], I),
         "lx_lora_encode_tmap_b": ([P, P, I, I, L, I], I),
         "lx_lora_shrink_parts": ([I, I, I, I], I),
-        "lx_lora_shrink_mma": ([P, L, P, I, I, P, P, P, I, L, I, P, I, I, I, I, P, P], I),
+        "lx_lora_shrink_mma": ([P, L, P, I, I, P, P, P, I, L, I, P, I, I, I, I, P, I, P], I),
         "lx_lora_shrink_tc": ([P, L, P, I, I, P, I, I, P, I, I, I, P, I, L, I, P, P, I, I, I, I, P, P], I),
         "lx_gemm_bf16_lora": ([P, P, P, P, I, I, I, L, L, L, P, L, P, P, I, P, P], I),
         "lx_lora_fused_desc_bytes": ([], I),
         "lx_quant_act_fp8": ([P, L, P, L, P, I, I, I, P], I),
-        "lx_gemm_fp8_block128": ([P, L, P, I, P, L, P, P, L, P, I, I, I, P, L, P, I, P], I),
+        "lx_gemm_fp8_block128": ([P, L, P, I, P, L, P, P, L, P, I, I, I, P, L, P, I, I, P], I),
         "lx_fp8_block128_dequant": ([P, L, P, I, P, L, I, I, P], I),
         "lx_wq_dequant": ([P, P, P, P, L, I, I, I, I, P], I),
         "lx_wq4_gemm": ([P, L, P, P, P, P, L, I, I, I, I, P], I),
         "lx_wq4_gemm_ex": ([P, L, P, P, P, P, L, I, I, I, I, I, P], I),
-        "lx_lora_expand_tiled": ([P, I, L, I, P, I, I, P, P, P, I, L, P, L, I, I, I, I, P, P], I),
+        "lx_lora_expand_tiled": ([P, I, L, I, P, I, I, P, P, P, I, L, P, L, I, I, I, I, P, I, P], I),
         "lx_attn_prefill_tc_supported": ([I, I, I, L, L], I),
         "lx_attn_prefill_tc": ([P, L, I, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, F, F, P, I, P, P], I),
         "lx_moe_router_logits": ([P, L, P, L, P, I, I, I, P, I, P], I),
@@ -239,7 +239,7 @@ class LxLoraFused(ctypes.Structure):
                 ("fence_maps", ctypes.c_int),
                 ("arena", ctypes.c_void_p), ("off_a", ctypes.c_longlong),
                 ("off_b", ctypes.c_longlong), ("arena_elems", ctypes.c_longlong), ("sync", ctypes.c_void_p),
-                ("w_const", ctypes.c_int)]
+                ("w_const", ctypes.c_int), ("tables_const", ctypes.c_int)]
 
 
 class LoraFused(NamedTuple):
@@ -261,6 +261,7 @@ class LoraFused(NamedTuple):
     arena: Optional[torch.Tensor] = None      # the slots' blobs; A_cat of the group and layer at slot_base + rank * off_a (elements)
     off_a: int = 0
     off_b: int = 0                            # B_cat likewise
+    tables_const: bool = False                # the kernel in front on the stream writes nothing of all this: it may be read while that one runs
 
 
 def lora_fused_desc(ws: "Workspace", lf: LoraFused, K: int) -> LxLoraFused:
@@ -274,6 +275,7 @@ def lora_fused_desc(ws: "Workspace", lf: LoraFused, K: int) -> LxLoraFused:
     d.off_b, d.arena_elems = lf.off_b, (lf.arena.numel() if lf.arena is not None else 0)
     d.sync = ws.lora_sync.data_ptr()
     d.fence_maps = LORA_FENCE_MAPS
+    d.tables_const = int(lf.tables_const)
     return d
 
 
@@ -465,7 +467,7 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
     xq, sa = quant_act_fp8(x)
     rc = load().lx_gemm_fp8_block128(_ptr(xq), xq.stride(0), _ptr(sa), sa.stride(0), _ptr(wq), wq.stride(0), _ptr(w_scale), _ptr(out),
                                      out.stride(0), _ptr(bias), T, N, K, _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.status),
-                                     ws.num_sms, _stream())
+                                     ws.num_sms, 1, _stream())      # (the kernel in front is the quantiser, which has waited for whatever wrote wq)
     _check(rc, "lx_gemm_fp8_block128")
     return out
 
@@ -740,25 +742,29 @@ def lora_shrink_tiles(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, max_
 
 
 def lora_shrink_mma(x: torch.Tensor, tiles: torch.Tensor, num_tiles: int, arena: torch.Tensor, slot_base: torch.Tensor,
-                    slot_rank: torch.Tensor, unit_off: int, nparts: int, max_rank: int, live_tiles: int = 0) -> torch.Tensor:
-    """Shrink of a short step over a table of tiles of at most 32 rows -> v [rows, cols] fp32, by mma.sync straight from the blobs."""
+                    slot_rank: torch.Tensor, unit_off: int, nparts: int, max_rank: int, live_tiles: int = 0, tables_const: bool = False) -> torch.Tensor:
+    """Shrink of a short step over a table of tiles of at most 32 rows -> v [rows, cols] fp32, by mma.sync straight from the blobs.
+    `tables_const`: the kernel in front on the stream writes none of `tiles`, `arena`, `slot_base` and `slot_rank` (in a step, copies do), which
+    are then read while it still runs."""
     T, K = x.shape
     ws = workspace(x.device)
     v = ws.lora_v
     rc = load().lx_lora_shrink_mma(_ptr(x), x.stride(0), _ptr(tiles), num_tiles, live_tiles, _ptr(arena), _ptr(slot_base), _ptr(slot_rank),
-                                   slot_rank.shape[0], unit_off, nparts, _ptr(v), v.stride(0), T, K, max_rank, _ptr(ws.status), _stream())
+                                   slot_rank.shape[0], unit_off, nparts, _ptr(v), v.stride(0), T, K, max_rank, _ptr(ws.status), int(tables_const),
+                                   _stream())
     _check(rc, "lx_lora_shrink_mma")
     return v
 
 
 def lora_expand_tiles(v, tiles: torch.Tensor, num_tiles: int, max_tile_rows: int, arena: torch.Tensor, slot_base: torch.Tensor,
-                      slot_rank: torch.Tensor, unit_off: int, y: torch.Tensor, n0: int, n1: int):
+                      slot_rank: torch.Tensor, unit_off: int, y: torch.Tensor, n0: int, n1: int, tables_const: bool = False):
+    """y += v B_cat(slot)^T over a tile table.  `tables_const` as for `lora_shrink_mma`."""
     v3, ksplit = v.unsqueeze(0), 1
     T, N = y.shape
     ws = workspace(y.device)
     rc = load().lx_lora_expand_tiled(_ptr(v3), v3.stride(1), v3.stride(0), ksplit, _ptr(tiles), num_tiles, max_tile_rows, _ptr(arena),
                                      _ptr(slot_base), _ptr(slot_rank), slot_rank.shape[0], unit_off, _ptr(y), y.stride(0), T, N, n0, n1,
-                                     _ptr(ws.status), _stream())
+                                     _ptr(ws.status), int(tables_const), _stream())
     _check(rc, "lx_lora_expand_tiled")
 
 

@@ -459,6 +459,64 @@ def test_lora_shrink_short_steps(nat, T, K):
     assert (v[~seen] == 7.0).all()
 
 
+@pytest.mark.parametrize("T", [7, 200])
+def test_adapter_tables_of_the_kernel_in_front(nat, T):
+    """Without `tables_const` table and ranks may come from the kernel directly in front, one that lets its successor start early; with it, and
+    tables that lie there, the bits are the same."""
+    g = torch.Generator().manual_seed(T)
+    K, N, ranks, nparts = 1024, 1024, [16, 32, 48, 64], 2
+    bases, off = [], 0
+    for r in ranks:
+        bases.append(off)
+        off += r * (nparts * K + N)
+    arena = (torch.randn(off, generator=g) * 0.05).to(torch.bfloat16).cuda()
+    base = torch.tensor(bases).cuda()
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, K, generator=g) / 32).to(torch.bfloat16).cuda()
+    G = 5
+    host = torch.zeros(len(ranks) * 2 * G * 128, dtype=torch.uint8).pin_memory()
+    for s, r in enumerate(ranks):
+        nat.lora_encode_tmap(host[s * 2 * G * 128:], arena.data_ptr() + bases[s] * 2, K, nparts * r, r * (nparts * K + N), 1)
+        nat.lora_encode_tmap_b(host[(s * 2 * G + G) * 128:], arena.data_ptr() + (bases[s] + r * nparts * K) * 2, r, N, r * (nparts * K + N), 1)
+    maps = host.cuda()
+    tables = [torch.tensor(ref.build_lora_tiles([(t // 5 + i) % 4 for t in range(T)], 32), dtype=torch.int32) for i in range(2)]
+    n = tables[0].numel()
+    assert tables[1].numel() == n and not torch.equal(*tables)
+    size = max(n, 4)
+    ints = [torch.zeros(size, device="cuda", dtype=torch.int32) for _ in range(4)]
+    jobs = [torch.stack([torch.arange(n), t.flatten().long(), torch.tensor((ranks * n)[:n]), torch.zeros(n, dtype=torch.long)]).to(torch.int32).cuda() for t in tables]
+
+    def passes(write):
+        outs = []
+        for i in range(6):
+            table, rank = (ints[0][:n].view(-1, 4), ints[1][:4]) if write else (tables[i % 2].cuda(), torch.tensor(ranks, dtype=torch.int32).cuda())
+            place = (lambda: nat.place_rows(jobs[i % 2], *ints)) if write else (lambda: torch.cuda.synchronize())
+            known = dict(tables_const=not write)
+            place()
+            v = nat.lora_shrink_mma(x, table, len(table), arena, base, rank, 0, nparts, 64, **known)[:T].clone()
+            y = torch.zeros(T, N, device="cuda", dtype=torch.bfloat16)
+            v2 = v.nan_to_num(0.0)
+            place()
+            nat.lora_expand_tiles(v2, table, len(table), 32, arena, base, rank, nparts * K, y, N // 2, N, **known)
+            place()
+            z = nat.gemm_lora_fused(x, w, nat.LoraFused(table, len(table), len(table), maps, 2 * G, 0, G, rank, base, nparts, N // 2, N, 0, 64, arena, 0,
+                                                        nparts * K, **known))
+            outs.append((v, y, z))
+        torch.cuda.synchronize()
+        return outs
+
+    nat.place_rows(jobs[1], *ints)
+    torch.cuda.synchronize()
+    nat.workspace().lora_v.zero_()
+    want = passes(False)
+    nat.workspace().lora_v.zero_()
+    got = passes(True)
+    nat.workspace().check_status()
+    for a, b in zip(got, want):
+        assert all(torch.equal(p, q) for p, q in zip(a, b))
+        assert a[1].abs().sum() > 0
+
+
 @pytest.mark.parametrize("nh,nkv,d,nsplit", [(12, 12, 64, 1), (32, 8, 128, 3), (6, 6, 128, 1)])
 def test_attn_alibi(nat, nh, nkv, d, nsplit):
     """ALiBi slopes in both attention kernels (BLOOM, MPT): bias -slope_h * (query position - key position)."""
