@@ -459,6 +459,58 @@ def test_lora_shrink_short_steps(nat, T, K):
     assert (v[~seen] == 7.0).all()
 
 
+def _after_a_kernel(nat, product, T, K, rounds=6):
+    """`product(x)` over inputs that a kernel which lets its successor start early has written directly in front: different ones in turn through
+    one buffer, without a synchronisation in between.  -> the outputs, and the inputs they belong to."""
+    srcs = [torch.randn(T, 2 * K, device="cuda", dtype=torch.bfloat16) * (1 + i) for i in range(2)]
+    x = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16)
+    outs = []
+    for i in range(rounds):
+        nat.act_mul(srcs[i % 2], K, "silu", out=x)
+        outs.append(product(x))
+    torch.cuda.synchronize()
+    return outs, [nat.act_mul(s, K, "silu") for s in srcs]
+
+
+@pytest.mark.parametrize("T,N,K,mode,split", [
+    (1, 4096, 4096, 0, 0), (13, 6144, 4096, 0, 0), (32, 4096, 14336, 0, 0),                # parts of K: a CTA's first block is not block 0
+    (32, 512, 64, 0, 0), (33, 1024, 448, 0, 0), (33, 1024, 512, 0, 0), (33, 1000, 520, 0, 0),      # one, seven, eight and nine blocks in a ring of eight
+    (129, 2048, 1024, 0, 0), (200, 1024, 256, 1, 0), (512, 1536, 1024, 2, 0), (300, 4096, 192, 2, 0),      # both orientations, rings of four and six
+    (16, 1024, 4096, 1, 3), (64, 4096, 4096, 1 | 2 << 8, 0), (512, 6144, 2048, 2 | 2 << 8, 0), (513, 1024, 512, 0, 0)])
+def test_gemm_reads_constant_weights_early(nat, T, N, K, mode, split):
+    """Weights loaded in front of the wait: the same bits as behind it, however the product is cut."""
+    torch.manual_seed(T + N)
+    w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16) / math.sqrt(K)
+    b = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    outs, xs = _after_a_kernel(nat, lambda x: nat.gemm(x, w, bias=b, mode=mode, force_split=split, w_const=True), T, K)
+    want = [nat.gemm(x, w, bias=b, mode=mode, force_split=split) for x in xs]
+    assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(outs))
+    assert _rel_err(want[1], xs[1].float() @ w.float().t() + b.float()) < 5e-3
+    nat.workspace().check_status()
+
+
+@pytest.mark.parametrize("T,N,K,group", [(1, 4096, 1024, 128), (5, 28672, 4096, 128), (8, 8192, 384, 64), (9, 512, 2048, 128), (17, 1024, 256, 32), (32, 256, 128, 128)])
+def test_packed_products_read_constant_codes_early(nat, T, N, K, group):
+    from lorax_b200.utils.quant_formats import quantize_rtn
+    torch.manual_seed(T + N)
+    q = quantize_rtn(torch.randn(N, K, device="cuda") / math.sqrt(K), 4, group)
+    outs, xs = _after_a_kernel(nat, lambda x: nat.gemm_wq(x, q, w_const=True), T, K)
+    want = [nat.gemm_wq(x, q) for x in xs]
+    assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(outs))
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 512, 1024), (5, 640, 4096), (33, 1024, 384), (100, 256, 128), (300, 512, 1024)])
+def test_fp8_products_read_weights_early(nat, T, N, K):
+    torch.manual_seed(T + N)
+    wq, sw = ref.quantize_weight_fp8_block128(torch.randn(N, K, device="cuda") / math.sqrt(K))
+    outs, xs = _after_a_kernel(nat, lambda x: nat.gemm_fp8(x, wq, sw), T, K)
+    want = []
+    for x in xs:
+        want.append(nat.gemm_fp8(x, wq, sw))
+        torch.cuda.synchronize()
+    assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(outs))
+
+
 @pytest.mark.parametrize("T", [7, 200])
 def test_adapter_tables_of_the_kernel_in_front(nat, T):
     """Without `tables_const` table and ranks may come from the kernel directly in front, one that lets its successor start early; with it, and
