@@ -129,8 +129,11 @@ LX_DEVICE uint2 ld_shared_8(uint32_t addr) {
   return v;
 }
 
-// The A fragments of Q in f16, each row divided by the power of two below its largest element (back in `unit`): what f16 cannot hold
-// is then below 2^-24 of that element.
+// Both operands that are not e4m3 are scaled so that f16 holds what bf16 held.  f16 keeps bf16's eight bits down to 2^-17 and something down to
+// 2^-25: with the largest element of a query row in [2^15, 2^16) and weights of up to 2^15, that is 2^-32 and 2^-40 of the largest.
+constexpr float kWeightUnit8 = 32768.f;
+
+// The A fragments of Q in f16, each row divided by the power of two that brings its largest element to 2^15 .. 2^16 (back in `unit`).
 template <int D>
 LX_DEVICE void load_q8(uint32_t (&qf)[D / 16][4], float (&unit)[2], const __nv_bfloat16* q, int grows, int lane) {
   const int c = lane & 3;
@@ -150,9 +153,9 @@ LX_DEVICE void load_q8(uint32_t (&qf)[D / 16][4], float (&unit)[2], const __nv_b
     }
     top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
     top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
-    const uint32_t e = min(max(__float_as_uint(top[r]) >> 23, 1u), 253u);
-    unit[r] = __uint_as_float(e << 23);
-    const float inv = __uint_as_float((254u - e) << 23);
+    const uint32_t e = min(max(__float_as_uint(top[r]) >> 23, 16u), 254u);
+    unit[r] = __uint_as_float((e - 15u) << 23);
+    const float inv = __uint_as_float((269u - e) << 23);
 #pragma unroll
     for (int h = 0; h < D / 64; ++h) {
 #pragma unroll
@@ -182,7 +185,7 @@ LX_DEVICE void qk_page8(float (&sacc)[kPage / 8][4], const uint32_t (&qf)[D / 16
   }
 }
 
-// O[16, D] += P[16, 32] V over one e4m3 page (columns permuted, see above).
+// O[16, D] += kWeightUnit8 P[16, 32] V over one e4m3 page (columns permuted, see above).
 template <int D>
 LX_DEVICE void pv_page8(float (&oacc)[D / 8][4], const float (&sacc)[kPage / 8][4], uint32_t v_smem, int lane) {
   constexpr int W = D / 32;                                        // words of a lane's dimensions of one key
@@ -190,10 +193,10 @@ LX_DEVICE void pv_page8(float (&oacc)[D / 8][4], const float (&sacc)[kPage / 8][
 #pragma unroll
   for (int kk = 0; kk < kPage / 16; ++kk) {
     uint32_t pa[4];
-    pa[0] = pack_f16x2(sacc[2 * kk][0], sacc[2 * kk][1]);
-    pa[1] = pack_f16x2(sacc[2 * kk][2], sacc[2 * kk][3]);
-    pa[2] = pack_f16x2(sacc[2 * kk + 1][0], sacc[2 * kk + 1][1]);
-    pa[3] = pack_f16x2(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3]);
+    pa[0] = pack_f16x2(sacc[2 * kk][0] * kWeightUnit8, sacc[2 * kk][1] * kWeightUnit8);
+    pa[1] = pack_f16x2(sacc[2 * kk][2] * kWeightUnit8, sacc[2 * kk][3] * kWeightUnit8);
+    pa[2] = pack_f16x2(sacc[2 * kk + 1][0] * kWeightUnit8, sacc[2 * kk + 1][1] * kWeightUnit8);
+    pa[3] = pack_f16x2(sacc[2 * kk + 1][2] * kWeightUnit8, sacc[2 * kk + 1][3] * kWeightUnit8);
     uint32_t v[4][W];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -481,6 +484,7 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
     }
   }
   __syncthreads();
+  const float v_unit = KV8 ? p.v_scale / kWeightUnit8 : 1.f;
   for (int idx = threadIdx.x * 2; idx < grows * DV; idx += 64 * NW) {
     const int g = idx / DV, d = idx % DV;
     float M = -INFINITY;
@@ -502,14 +506,14 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
     }
     const int head = head0 + g;
     if (p.nsplit == 1) {                         // (of several splits the tail joins where they are combined)
-      const float f = (den > 0.f ? attn_denominator(p.tail, head, M * kLog2e, den) : 0.f) * (KV8 ? p.v_scale : 1.f);
+      const float f = (den > 0.f ? attn_denominator(p.tail, head, M * kLog2e, den) : 0.f) * v_unit;
       const float2 o = attn_turn_back(p.tail, make_float2(num.x * f, num.y * f), d, ctx - 1);
       const int col = head * DV + d;
       __nv_bfloat16* dst = p.out + (long long)t * p.ldo + col;
       dst[0] = __float2bfloat16(attn_tail(p.tail, o.x, t, col));
       dst[1] = __float2bfloat16(attn_tail(p.tail, o.y, t, col + 1));
     } else {
-      const float f = (den > 0.f ? 1.f / den : 0.f) * (KV8 ? p.v_scale : 1.f);
+      const float f = (den > 0.f ? 1.f / den : 0.f) * v_unit;
       const long long pi = ((long long)t * p.nh + head) * p.nsplit + split;
       *reinterpret_cast<float2*>(p.part_o + pi * DV + d) = make_float2(num.x * f, num.y * f);
       if (d == 0) p.part_lse[pi] = den > 0.f ? M + __logf(den) : -INFINITY;

@@ -425,6 +425,37 @@ def test_attn_decode_fp8_pages(nat, B, nh, nkv, d, window, softcap, nsplit):
         assert _rel_err(got[b], want[b]) < 6e-3, (b, int(ctx[b]))
 
 
+@pytest.mark.parametrize("nsplit,d", [(1, 128), (4, 128), (1, 64)])
+def test_attn_decode_fp8_pages_keep_what_is_faint(nat, nsplit, d):
+    """One key that takes nearly all of a row's weight, its value zero, beside 8000 of 2^-26 of it; and query rows whose largest element, 2^24
+    times the others, meets zeros in every key.  The result hangs on what f16 loses without a scale.  Weights and results are rounded to 8
+    bits at least, 2^-9 relatively, as over bf16 pages; the scores' sums in fp32 add 2^-22 of the scores (up to 20)."""
+    nh, nkv, B, ctx = 8, 2, 3, 8001
+    wide, bt = _make_cache(B, ctx, nkv, d, seed=d + nsplit)
+    wide[:, :, 0] = 0.0
+    wide[:, :, 1] = wide[:, :, 1].abs()
+    q = torch.zeros(B, nh * d, device="cuda", dtype=torch.bfloat16)
+    scale = d ** -0.5
+    for b, at in ((0, 0), (1, 5000)):                                          # before and between the faint ones
+        page = bt[b, at // 32].long()
+        wide[page, :, 0, at % 32, 0] = round(18.3 / (8 * scale))
+        wide[page, :, 1, at % 32] = 0.0
+        q.view(B, nh, d)[b, :, 0] = 8.0
+    wide[bt[2].long(), :, 0] = torch.randn_like(wide[bt[2].long(), :, 0])
+    wide[bt[2].long(), :, 0, :, 0] = 0.0
+    q[2] = torch.randn(nh * d, device="cuda") * 2
+    q.view(B, nh, d)[2, :, 0] = 2.0 ** 24
+    cache = wide.to(torch.float8_e4m3fn)
+    lens = torch.full((B,), ctx, device="cuda", dtype=torch.int32)
+    got = nat.attn_decode(q, cache, bt, lens, nh, nkv, d, scale, 0, 0.0, nsplit, kv_scale=(1.0, 0.5))
+    for b in range(B):
+        pages = cache[bt[b].long()].double()
+        for h in range(nh):
+            k, v = pages[:, h * nkv // nh].transpose(0, 1).reshape(2, -1, d)[:, :ctx]
+            want = torch.softmax(q[b, h * d: (h + 1) * d].double() @ k.t() * scale, -1) @ v * 0.5
+            assert want.abs().min() > 0 and _rel_err(got[b, h * d: (h + 1) * d], want) < 6e-3, (b, h)
+
+
 @pytest.mark.parametrize("T, K", [(1, 4096), (7, 64), (9, 1000), (40, 14336), (33, 2056), (300, 512)])
 def test_lora_shrink_short_steps(nat, T, K):
     """Clusters of one to eight CTAs over K, K off the blocks of 32, one and four row groups, ranks of 8 to 64, rows past the batch, dead entries.
