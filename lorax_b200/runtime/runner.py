@@ -70,6 +70,8 @@ class DecodeState:
         self.tile_list: List[Tuple[int, int, int, int]] = []      # host copy of the live part of lora_tiles
         self.free_rows = list(range(max_batch - 1, -1, -1))
         self.live: Dict[int, int] = {}          # row -> request id
+        self.context: Dict[int, int] = {}       # row -> keys that its next step reads, less the steps taken so far (host mirror)
+        self.steps = 0
         self.high_water = 0
 
     def take_row(self, request_id: int) -> int:
@@ -82,6 +84,7 @@ class DecodeState:
     def drop_row(self, row: int):
         self.live.pop(row, None)
         self.row_slot.pop(row, None)
+        self.context.pop(row, None)
         self.free_rows.append(row)
         self.high_water = (max(self.live) + 1) if self.live else 0
 
@@ -94,6 +97,8 @@ class ModelRunner:
         self.device = model.device
         self.is_cuda = self.device.type == "cuda"
         self.page = kv.page
+        pages = kv.layers[0] if kv.layers else None
+        self.kv_bytes = pages.element_size() if isinstance(pages, torch.Tensor) else 2      # of an element of the cache
         self.max_blocks = (max_seq_tokens + self.page - 1) // self.page + 1
         self.max_batch = max_batch
         self.max_prefill_tokens = max_prefill_tokens
@@ -328,6 +333,7 @@ class ModelRunner:
         st.next_ids[:nd].copy_(ids[:nd])
         st.logprobs[:nd].copy_(lps[:nd])
         self._advance(nd)
+        st.steps += 1
         k = self.stash(st.next_ids[:nd], st.logprobs[:nd])
         self.steps += 1
         return k, nd, ids[nd:], lps[nd:]
@@ -360,8 +366,9 @@ class ModelRunner:
         st.tok_slot.index_copy_(0, r, dev[5 * n:6 * n])
         st.state_slots.index_copy_(0, r, dev[6 * n:7 * n])
         st.block_tables.index_copy_(0, r, dev[7 * n:].view(n, self.max_blocks))
-        for row, sl in zip(rows, tslot):
+        for row, sl, c in zip(rows, tslot, ctx):
             st.row_slot[row] = sl
+            st.context[row] = c - st.steps
         self.tiles_valid = False        # rows are no longer grouped by adapter until resort() runs
 
     def resort(self) -> Dict[int, int]:
@@ -383,6 +390,7 @@ class ModelRunner:
             st.tok_slot[n:hw] = -1
         st.live = {mapping[o]: rid for o, rid in st.live.items()}
         st.row_slot = {mapping[o]: sl for o, sl in st.row_slot.items() if o in mapping}
+        st.context = {mapping[o]: c for o, c in st.context.items() if o in mapping}
         st.free_rows = list(range(st.max_batch - 1, n - 1, -1))
         st.high_water = n
         # tile table: decode tiles hold at most 32 rows
@@ -407,6 +415,8 @@ class ModelRunner:
             raise IndexError(f"decode rows {min(rows)} .. {max(rows)} of {st.max_batch}")
         job = self._to_dev(list(rows) + list(tokens) + list(positions) + slots).view(4, len(rows))
         self.model.ops.place_rows(job, st.input_ids, st.positions, st.ctx_lens, st.slots)
+        for row, p in zip(rows, positions):
+            st.context[row] = p + 1 - st.steps
 
     def retire(self, rows: Sequence[int]):
         """Mark rows as padding: they stop advancing and attention skips them."""
@@ -449,16 +459,23 @@ class ModelRunner:
         return logits
 
     def _attn_splits(self, rows: int) -> int:
-        """Parts that decode attention cuts a row's keys into.  Few rows: as many as give the GPU a CTA per SM and more.  From one CTA per
-        (row, KV head) and SM on, contexts of unequal length leave SMs idle at the end: four parts each took 32 rows of 1024 to 8192 keys
-        from 152 to 122 us and 48 rows of 256 to 2048 from 62 to 55 us (parts of fewer than 256 keys are not made).  Where rows and heads
-        alone are several waves (64 rows of 8 heads: 46 us with one part, 52 with four) the second pass over the parts costs more."""
+        """Parts that decode attention cuts a row's keys into.  Up to 96 CTAs of a row and a KV head: as many as give the GPU a CTA per SM and
+        more.  Up to 512, contexts that are long and differ leave SMs idle at the end, and four parts (of 256 keys at least) and a second pass
+        over them are quicker: bf16 pages, 13, 32 and 48 rows of 8 heads and 1024 to 8192 keys 94, 162 and 218 us with one part, 85, 130 and 169
+        with four; e4m3 pages 78, 100 and 195 against 60, 97 and 122.  With short contexts the parts are empty and the second pass is lost (48 rows of 16 to
+        64 keys 14 us against 26), and with equal ones there is little to even out (32 rows of 1024 42 against 48, of 4096 e4m3 keys 66 against
+        73), so the longest has to be 4 KB of keys a dimension and the mean at most three quarters of it: around those lines both are within a tenth of one
+        another.  Beyond 512 CTAs rows alone are several waves (64 rows: 46 us with one part, 52 with four)."""
         if not self.is_cuda:
             return 1
-        ctas = rows * self.model.nkv
+        ctas, st = rows * self.model.nkv, self.state
         if ctas < 96:
             return max(1, min(8, 192 // max(ctas, 1)))
-        return 4 if 148 <= ctas < 512 else 1
+        if ctas >= 512 or not st.context:
+            return 1
+        window = self.model.config.sliding_window or 1 << 30
+        keys = [min(c + st.steps, window) for c in st.context.values()]
+        return 4 if max(keys) * self.kv_bytes >= 4096 and 4 * sum(keys) <= 3 * max(keys) * len(keys) else 1
 
     def _advance(self, b: int):
         st = self.state
@@ -474,7 +491,8 @@ class ModelRunner:
     def _graph_key(self, b: int, lora: bool, need_logits: bool):
         """Everything that the launches of a decode step depend on, apart from what lies in the state's buffers."""
         ad = self.model.adapters
-        return b, lora, self.tiles_valid, need_logits, ad.launch_class(self.model.ops, b, self._tiles(b, lora)) if lora else ()
+        return (b, lora, self.tiles_valid, need_logits, self._attn_splits(b),
+                ad.launch_class(self.model.ops, b, self._tiles(b, lora)) if lora else ())
 
     def capture(self, b: int, lora: bool, need_logits: bool = False):
         key = self._graph_key(b, lora, need_logits)
@@ -532,6 +550,7 @@ class ModelRunner:
         else:
             logits = self._decode_body(b, lora, need_logits)
             self._advance(b)
+        st.steps += 1
         logits = self._cap(logits)
         if sampler is not None:
             sampler(logits, st)

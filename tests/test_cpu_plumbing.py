@@ -207,7 +207,7 @@ def test_graph_keys_hold_what_adapter_launches_depend_on():
     ops = NS(lora_shrink_parts=native.lora_shrink_parts, workspace=lambda dev: NS(num_sms=148, lora_v3=torch.empty(8, 1)),
              lora_shrink_ksplit=native.lora_shrink_ksplit)
     st = NS(lora_tiles=None, num_lora_tiles=0)
-    run = NS(model=NS(adapters=ad, ops=ops), state=st, tiles_valid=True)
+    run = NS(model=NS(adapters=ad, ops=ops), state=st, tiles_valid=True, _attn_splits=lambda b: 1)
     run._tiles = lambda *a: ModelRunner._tiles(run, *a)
     for bucket in (8, 256, 1024):
         seen = {}
@@ -221,9 +221,53 @@ def test_graph_keys_hold_what_adapter_launches_depend_on():
                     cut = [native.lora_shrink_ksplit(ops.workspace(None), live, len(g.parts), ad.max_rank, g.K) for n, g in groups.items() if n != LM_HEAD]
                 assert seen.setdefault(ModelRunner._graph_key(run, bucket, True, False), (ad.max_rank, cut)) == (ad.max_rank, cut)
         assert len({rank for rank, _ in seen.values()}) == 4 and len(seen) <= 4 * 24
-    assert ModelRunner._graph_key(run, 8, False, False) == (8, False, True, False, ())
+    assert ModelRunner._graph_key(run, 8, False, False) == (8, False, True, False, 1, ())
     run.tiles_valid = False
     assert ModelRunner._graph_key(run, 8, True, False)[-1] == (64,)
+
+
+def test_parts_of_decode_attention_follow_the_contexts():
+    """The host's mirror of the rows' contexts is what the device holds, through decode steps, repositioning, sorting and leaving rows; short
+    or equal contexts keep one part where rows and heads fill the GPU."""
+    from types import SimpleNamespace as NS
+    from lorax_b200.runtime.kv_cache import KVCache
+    from lorax_b200.runtime.runner import ModelRunner, PrefillItem
+    cfg = tiny_llama()
+    m = DecoderModel.random_init(cfg, torch.device("cpu"), torch.float32, seed=0)
+    r = ModelRunner(m, KVCache(cfg.num_hidden_layers, 16, m.nkv, m.d, m.dtype, m.device), max_batch=4, max_seq_tokens=96, max_prefill_tokens=128)
+    st = r.state
+
+    def same():
+        assert {row: c + st.steps for row, c in st.context.items()} == {row: int(st.ctx_lens[row]) for row in st.live}
+
+    blocks = [[1 + 3 * i, 2 + 3 * i, 3 + 3 * i] for i in range(4)]
+    prompts = [[5] * n for n in (7, 31, 20)]
+    ids, _, _ = r.prefill([PrefillItem(p, 0, b) for p, b in zip(prompts, blocks)])
+    r.install([st.take_row(i) for i in range(3)], ids.tolist(), [len(p) for p in prompts], blocks[:3], [0, 0, 0])
+    same()
+    r.decode()
+    r.decode()
+    same()
+    r.reposition([1], [9], [40], [blocks[1]])
+    r.decode()
+    same()
+    r.retire([0])
+    st.drop_row(0)
+    mapping = r.resort()
+    assert mapping == {1: 0, 2: 1}
+    same()
+    r.mixed_step([PrefillItem([3] * 9, 0, blocks[3])])
+    r.install([st.take_row(3)], [4], [9], [blocks[3]], [0])
+    r.decode()
+    same()
+
+    splits = lambda keys, rows=32, heads=8, kv_bytes=2, window=None: ModelRunner._attn_splits(
+        NS(is_cuda=True, model=NS(nkv=heads, config=NS(sliding_window=window)), kv_bytes=kv_bytes, state=NS(context=dict(enumerate(keys)), steps=100)), rows)
+    long = [924 + 300 * i for i in range(25)]
+    assert splits(long) == splits(long, rows=13) == splits(long, kv_bytes=1) == 4
+    assert splits(long, rows=64) == splits([], rows=32) == splits([8000] * 32) == splits([0] * 32) == splits([i * 60 for i in range(32)]) == 1
+    assert splits([i * 100 for i in range(32)]) == 4 and splits([i * 100 for i in range(32)], kv_bytes=1) == 1
+    assert splits(long, window=1024) == 1 and splits([8000] * 4, rows=4) == 6 and splits([], rows=1, heads=4) == 8
 
 
 def test_vocabulary_parallel_sampling_equals_sampling_from_the_full_row():
