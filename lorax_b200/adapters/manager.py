@@ -30,7 +30,6 @@ from .lora import LM_HEAD, BlobLayout, LoraConfig, ModuleMap, check_architecture
 
 TMAP_GROUPS = ("qkv", "o", "gate_up", "down", LM_HEAD)     # index of a group inside a slot's tensor-map row
 TMAP_BYTES = 128
-SHORT_STEP = 512        # rows up to which the shrink is a matter of latency (mma.sync from the blobs) and not of tensor-core rate
 
 
 @dataclass
@@ -312,7 +311,7 @@ class AdapterManager:
         if tiles is not None:
             if tiles.num_tiles == 0:
                 return None
-            if self.is_cuda and x.shape[0] <= SHORT_STEP and tiles.max_rows <= 32:
+            if self.is_cuda and ops.lora_short_step(x.shape[0], tiles.max_rows):
                 v = ops.lora_shrink_mma(x, tiles.table, tiles.num_tiles, self.arena, self.slot_base, self.slot_rank, offA, nparts, self.max_rank,
                                         live_tiles=tiles.live, tables_const=True)      # (copies write them, in front of the step)
             elif self.is_cuda:
@@ -331,7 +330,7 @@ class AdapterManager:
         graph therefore holds: the largest rank, which the grids cover, and the parts that shrinks of their own cut K into."""
         if tiles is None:
             return (self.max_rank,)
-        if rows <= SHORT_STEP and tiles.max_rows <= 32:
+        if ops.lora_short_step(rows, tiles.max_rows):
             cut = lambda gi: ops.lora_shrink_parts(tiles.live, len(gi.parts), self.max_rank, gi.K)
         else:
             cut = lambda gi: ops.lora_shrink_ksplit(ops.workspace(self.device), tiles.live, len(gi.parts), self.max_rank, gi.K)

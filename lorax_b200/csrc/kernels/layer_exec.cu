@@ -47,6 +47,7 @@ int lx_lora_shrink(const void* x, long long ldx, const int* tok_slot, const void
 int lx_lora_expand(const float* v, int ldv, const int* tok_slot, const void* arena, const long long* slot_base,
                    const int* slot_rank, int num_slots, long long unit_off, void* y, long long ldy, int T, int N, int n0, int n1,
                    int* status, void* stream);
+int lx_lora_short_step(int T, int max_tile_rows);
 int lx_lora_shrink_mma(const void* x, long long ldx, const void* tiles, int num_tiles, int live_tiles, const void* arena, const long long* slot_base,
                        const int* slot_rank, int num_slots, long long unit_off, int nparts, float* v, int ldv, int T, int K, int max_rank,
                        int* status, int tables_const, void* stream);
@@ -154,8 +155,6 @@ namespace {
     if (rc_ != 0) return rc_;   \
   } while (0)
 
-constexpr int kShortStep = 512;      // rows up to which the stand-alone shrink is a matter of latency (adapters/manager.py has the same line)
-
 // y[T, N] = x[T, K] w^T (+ bias) (+ LoRA delta of the site)
 int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDesc& s, int site_idx, const void* x, long long ldx,
                      const void* w, long long ldw, const void* bias, void* y, long long ldy, int N, int K, void* stream) {
@@ -175,7 +174,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
     if (rc != 1) return rc;          // 1: this step does not fit the fused launch, use the separate kernels below
   }
   if (lora) {
-    if (s.lora_tiles != nullptr && s.T <= kShortStep && s.max_tile_rows <= 32) {
+    if (s.lora_tiles != nullptr && lx_lora_short_step(s.T, s.max_tile_rows)) {
       LX_TRY(lx_lora_shrink_mma(x, ldx, s.lora_tiles, s.num_tiles, s.live_tiles, m.arena, m.slot_base, m.slot_rank, m.num_slots, site.off_a,
                                 site.nparts, m.lora_v, m.ldv, s.T, K, m.max_rank, m.status, 1, stream));
     } else if (s.lora_tiles != nullptr) {

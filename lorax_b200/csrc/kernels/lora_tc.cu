@@ -604,6 +604,10 @@ int lx_lora_shrink_tc(const void* x, long long ldx, const void* tiles, int num_t
   return launch_shrink_tc<128>(tx, p, num_tiles, chunks, s);
 }
 
+// Which shrink a step of T rows over tiles of at most max_tile_rows takes: lx_lora_shrink_mma (1), up to 512 rows, where it is a matter of latency, or
+// lx_lora_shrink_tc (0), where it is one of tensor-core rate.
+int lx_lora_short_step(int T, int max_tile_rows) { return T <= 512 && max_tile_rows <= 32; }
+
 // CTAs (a cluster) over which lx_lora_shrink_mma cuts K: while they stay within four per SM and a warp keeps four blocks of 32 elements.
 int lx_lora_shrink_parts(int live_tiles, int nparts, int max_rank, int K) {
   const long long units = (long long)live_tiles * ((nparts * max_rank + 15) / 16);

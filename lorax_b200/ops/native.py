@@ -88,6 +88,7 @@ def load() -> ctypes.CDLL:
         "lx_tensormap_bytes": ([], I),
         "lx_lora_encode_tmap": ([P, P, I, I, L, I], I),
         "lx_lora_encode_tmap_b": ([P, P, I, I, L, I], I),
+        "lx_lora_short_step": ([I, I], I),
         "lx_lora_shrink_parts": ([I, I, I, I], I),
         "lx_lora_shrink_mma": ([P, L, P, I, I, P, P, P, I, L, I, P, I, I, I, I, P, I, P], I),
         "lx_lora_shrink_tc": ([P, L, P, I, I, P, I, I, P, I, I, I, P, I, L, I, P, P, I, I, I, I, P, P], I),
@@ -716,6 +717,11 @@ def lora_shrink_ksplit(ws: "Workspace", live_tiles: int, nparts: int, max_rank: 
     if wanted is None:
         wanted = max(1, (2 * ws.num_sms) // max(1, live_tiles * ((nparts * max_rank + 127) // 128)))
     return max(1, min(ws.lora_v3.shape[0], kblocks // 8 if kblocks >= 8 else 1, wanted))
+
+
+def lora_short_step(rows: int, max_tile_rows: int) -> bool:
+    """Whether a step takes `lora_shrink_mma` (few rows: latency) or `lora_shrink_tiles` (no GPU needed)."""
+    return load().lx_lora_short_step(rows, max_tile_rows) != 0
 
 
 def lora_shrink_parts(live_tiles: int, nparts: int, max_rank: int, K: int) -> int:

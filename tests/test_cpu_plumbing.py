@@ -204,7 +204,7 @@ def test_graph_keys_hold_what_adapter_launches_depend_on():
               LM_HEAD: NS(parts=(0,), K=4096)}
     ad = NS(max_rank=16, layout=NS(groups=groups), device=None)
     ad.launch_class = lambda *a: AdapterManager.launch_class(ad, *a)
-    ops = NS(lora_shrink_parts=native.lora_shrink_parts, workspace=lambda dev: NS(num_sms=148, lora_v3=torch.empty(8, 1)),
+    ops = NS(lora_short_step=native.lora_short_step, lora_shrink_parts=native.lora_shrink_parts, workspace=lambda dev: NS(num_sms=148, lora_v3=torch.empty(8, 1)),
              lora_shrink_ksplit=native.lora_shrink_ksplit)
     st = NS(lora_tiles=None, num_lora_tiles=0)
     run = NS(model=NS(adapters=ad, ops=ops), state=st, tiles_valid=True, _attn_splits=lambda b: 1)
