@@ -402,6 +402,37 @@ def test_attn_prefill_weights_are_relative_to_the_largest_so_far(nat, q_lens, ca
         at += n
 
 
+@pytest.mark.parametrize("climb,softcap,window,cached", [(0.0, 0.0, 0, 0), (0.02, 0.0, 0, 300), (1.5, 0.0, 0, 0), (-0.3, 0.0, 0, 70), (0.4, 60.0, 200, 0)])
+def test_attn_prefill_wide_weights_under_moving_maxima(nat, climb, softcap, window, cached):
+    """Softmax weights of two bf16 terms where the largest score grows or falls by `climb` (log2) from key to key: from block to block the sums
+    are rescaled by up to 2^192.  What remains is the rounding of the result: 2^-9 at most, 2^-9 / sqrt(3) = 1.1e-3 over all for evenly spread
+    mantissas, up to 1.7e-3 where they gather above a power of two; the weights' two terms add 2^-17."""
+    nh, nkv, d, n = 4, 2, 128, 700
+    m = n + cached
+    cache, bt = _make_cache(1, m, nkv, d, seed=n)
+    scale = d ** -0.5
+    pages = bt.shape[1]
+    rise = torch.arange(pages * 32, device="cuda").view(pages, 1, 32) * (climb / (8.0 * scale * math.log2(math.e)))
+    cache[bt[0].long(), :, 0, :, 0] = rise.to(torch.bfloat16)
+    q = torch.randn(n, nh * d, device="cuda", dtype=torch.bfloat16)
+    q.view(n, nh, d)[:, :, 0] = 8.0
+    ints = lambda *v: torch.tensor(v, device="cuda", dtype=torch.int32)
+    ts, tq = (ints(*t) for t in ref.prefill_tiles([n]))
+    cu, cl, out, p = ints(0, n), ints(cached), torch.empty_like(q), nat._ptr
+    rc = nat.load().lx_attn_prefill_tc(p(q), q.stride(0), n, p(cache), cache.shape[0], p(bt), bt.shape[1], p(cu), p(cl), p(ts), p(tq), ts.shape[0], p(out),
+                                       out.stride(0), nh, nkv, d, window, scale, softcap, None, 1, p(nat.workspace().status), nat._stream())
+    assert rc == 0
+    nat.workspace().check_status()
+    at = cached + torch.arange(n, device="cuda")[:, None]
+    key = torch.arange(m, device="cuda")
+    for h in range(nh):
+        k, v = cache[bt[0].long()][:, h * nkv // nh].transpose(0, 1).reshape(2, -1, d)[:, :m].double()
+        s = q[:, h * d: (h + 1) * d].double() @ k.t() * scale
+        s = softcap * torch.tanh(s / softcap) if softcap else s
+        s = s.masked_fill((key > at) | ((at - key >= window) if window else (key < 0)), float("-inf"))
+        assert _rel_err(out[:, h * d: (h + 1) * d], torch.softmax(s, -1) @ v) < 1.8e-3
+
+
 @pytest.mark.parametrize("B,nh,nkv,d,window,softcap,nsplit", [(5, 8, 8, 128, 0, 0.0, 1), (3, 32, 8, 128, 50, 0.0, 8), (40, 32, 8, 128, 0, 20.0, 4),
                                                             (6, 20, 1, 64, 0, 0.0, 2), (38, 16, 8, 64, 33, 0.0, 1), (2, 34, 2, 128, 0, 0.0, 1)])
 def test_attn_decode_fp8_pages(nat, B, nh, nkv, d, window, softcap, nsplit):
