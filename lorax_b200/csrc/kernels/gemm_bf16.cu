@@ -1606,12 +1606,17 @@ static GemmPlan choose_plan_swap(int T, int N, int K, int num_sms, long long ws_
     return pl;
   }
   // Few tokens and few weight tiles: the classic split, where that gives 85 % of the SMs a part each.  A tile's last part sums the others
-  // (8 to 16 KB each) as soon as they are there; the stream-K contributors each wait for all of them.  13 tokens, products back to back:
-  // N = K = 4096 14.9 -> 11.3 us (four parts), N = 6144 16.6 -> 14.3 (three), K = 14336 25.9 -> 23.8 (four); at 64 tokens 18.4 -> 18.7,
-  // 18.5 -> 21.4 and 27.8 -> 30.4, the single summing CTA has four times as much to add.
+  // (8 to 16 KB each) as soon as they are there; the stream-K contributors each wait for all of them.  Products back to back, constant weights:
+  // 13 tokens, N = K = 4096 15.2 -> 11.9 us (four parts), N = 6144 17.4 -> 15.1 (three), N = 8192 19.8 -> 17.6 (two), K = 14336 28.7 -> 26.2; at 64 tokens
+  // 18.4 -> 18.7, the single summing CTA has four times as much to add.  Not where
+  //   * the parts are as many as the SMs: stream-K's ranges are then whole parts too, and its sums shared (N = 4736, K = 4096, 32 tokens: 13.3 against 16.6);
+  //   * whole tiles of a short K are quicker than any sum: two parts of K below 2048 (N = 8064, K = 1024: 7.2 against 8.9), and from 17 tokens on, where
+  //     they are two token tiles side by side, two and three parts of K below 3072 (N = 8192, K = 2048, 32 tokens: 13.0 against 14.4).
   if (sk_policy == 0 && !bn_forced && have_counters && t16 <= kClassicSplitTokens) {
     const int s = num_sms / tiles_a;
-    if (s >= 2 && s <= 4 && tiles_a * s * 100 >= num_sms * 85 && kblocks / s >= 8 && (long long)tiles_a * s * kBM * template_bn(t16) * 4 <= ws_bytes) {
+    const int least = s == 4 ? 32 : t16 > 16 ? 48 : s == 3 ? 24 : 32;      // k-blocks of 64
+    if (s >= 2 && s <= 4 && tiles_a * s * 100 >= num_sms * 85 && tiles_a * s < num_sms && kblocks >= least &&
+        (long long)tiles_a * s * kBM * template_bn(t16) * 4 <= ws_bytes) {
       GemmPlan pl{};
       pl.bn = t16; pl.split = s; pl.dp_tiles = tiles_a; pl.sk_ctas = 0;
       pl.grid = tiles_a * s;

@@ -2,6 +2,8 @@
 import re
 from pathlib import Path
 
+import pytest
+
 KERNELS = Path(__file__).resolve().parents[1] / "lorax_b200" / "csrc" / "kernels"
 # what kernels read without any kernel writing it: weights, biases, scales, adapters, embedding tables, tables of angles
 CONSTANT_PARAMS = {"w", "b", "bias", "wr", "mu", "q", "sw", "table", "pos", "cos_sin"}
@@ -43,3 +45,12 @@ def test_triggers_stand_behind_the_wait():
     for kernel, _, body in _kernels():
         at = [body.find(f) for f in ("pdl_trigger()", "pdl_launch_dependents()") if f in body]
         assert not at or 0 <= body.find("pdl_wait()") < min(at) or "shrink_rows_part" in body, kernel
+
+
+@pytest.mark.parametrize("T,N,K,parts", [
+    (13, 4096, 4096, 4), (32, 4096, 2048, 4), (1, 4096, 1984, 1), (13, 6144, 4096, 3), (16, 5504, 1536, 3), (16, 5504, 1472, 1), (17, 5504, 3072, 3),
+    (17, 5504, 3008, 1), (13, 8192, 2048, 2), (13, 9216, 1984, 1), (32, 8192, 3072, 2), (32, 8192, 3008, 1),
+    (32, 4736, 4096, 1), (1, 9472, 4096, 1), (33, 4096, 4096, 1), (1, 4864, 4096, 1)])      # as many parts as SMs; 33 tokens; 114 of 148 SMs
+def test_classic_split_only_where_it_measured_quicker(T, N, K, parts):
+    from lorax_b200.ops import native
+    assert native.gemm_plan(T, N, K)["split"] == parts
