@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from pathlib import Path
@@ -719,11 +720,13 @@ def lora_shrink_ksplit(ws: "Workspace", live_tiles: int, nparts: int, max_rank: 
     return max(1, min(ws.lora_v3.shape[0], kblocks // 8 if kblocks >= 8 else 1, wanted))
 
 
+@functools.lru_cache(maxsize=4096)      # (asked for every decode step)
 def lora_short_step(rows: int, max_tile_rows: int) -> bool:
     """Whether a step takes `lora_shrink_mma` (few rows: latency) or `lora_shrink_tiles` (no GPU needed)."""
     return load().lx_lora_short_step(rows, max_tile_rows) != 0
 
 
+@functools.lru_cache(maxsize=4096)
 def lora_shrink_parts(live_tiles: int, nparts: int, max_rank: int, K: int) -> int:
     """Parts of K of the short step's shrink (no GPU needed)."""
     return load().lx_lora_shrink_parts(live_tiles, nparts, max_rank, K)

@@ -473,9 +473,11 @@ class ModelRunner:
             return max(1, min(8, 192 // max(ctas, 1)))
         if ctas >= 512 or not st.context:
             return 1
-        window = self.model.config.sliding_window or 1 << 30
+        longest, window = max(st.context.values()) + st.steps, self.model.config.sliding_window or 1 << 30
+        if min(longest, window) * self.kv_bytes < 4096:
+            return 1
         keys = [min(c + st.steps, window) for c in st.context.values()]
-        return 4 if max(keys) * self.kv_bytes >= 4096 and 4 * sum(keys) <= 3 * max(keys) * len(keys) else 1
+        return 4 if 4 * sum(keys) <= 3 * max(keys) * len(keys) else 1
 
     def _advance(self, b: int):
         st = self.state
