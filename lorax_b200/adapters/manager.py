@@ -155,7 +155,11 @@ class AdapterManager:
         self.key_of_index: Dict[int, str] = {}
         self.max_rank = 0
         self.is_cuda = self.device.type == "cuda"
-        self.copy_stream = torch.cuda.Stream(device=self.device) if self.is_cuda else None
+        # Of the pool of high priority, which graphs are not captured on: torch hands out 32 streams of a priority in turn, and a copy stream
+        # that is the capture's too would carry copies into a graph, and the release of a pinned block that was copied on it, while a graph
+        # is captured, would leave an event in that graph, at which every later pinned allocation of the block's size fails
+        # ("invalid argument").
+        self.copy_stream = torch.cuda.Stream(device=self.device, priority=-1) if self.is_cuda else None
         self._pending_events: List[object] = []
         self.stats = dict(h2d_bytes=0, loads=0, evictions=0, host_hits=0, host_misses=0)
         # staging for slot-table updates (pinned so the H2D is async)

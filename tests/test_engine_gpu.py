@@ -186,6 +186,34 @@ def test_captured_steps_follow_the_largest_rank(weights):
     assert torch.equal(seen[0], seen[3]) and (seen[1] - seen[0]).norm() > 0.05 * seen[0].norm()
 
 
+def test_adapter_copies_stay_out_of_captures():
+    """However many managers a process makes, none copies on the stream that graphs are captured on: a pinned block of its copies may be
+    released while a graph is captured, and pinned memory of its size is to be had afterwards."""
+    cfg, gm, mgr = _build("cuda", torch.bfloat16, 1)
+    r = ModelRunner(gm, KVCache(cfg.num_hidden_layers, 8, gm.nkv, gm.d, gm.dtype, gm.device), max_batch=4, max_seq_tokens=64, max_prefill_tokens=64)
+    r.prefill([PrefillItem([1, 2, 3], 0, [1])])
+    r.install([r.state.take_row(0)], [4], [3], [[1]], [1])
+    r.resort()
+    r.decode()                                   # (captures)
+    on = torch.cuda.graph.default_capture_stream
+    a = torch.zeros(8, device="cuda")
+    for i in range(40):
+        m = AdapterManager(gm, arena_bytes=1 << 20, host_bytes=1 << 20, max_slots=4)
+        assert m.copy_stream.cuda_stream != on.cuda_stream, i
+        if i % 8 == 0:
+            size = 3000 + 4096 * i
+            block = torch.zeros(size, dtype=torch.uint8).pin_memory()
+            with torch.cuda.stream(m.copy_stream):
+                block.to("cuda", non_blocking=True)
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+                a.add_(1)
+                del block
+            for _ in range(2):
+                torch.zeros(size, dtype=torch.uint8).pin_memory()
+
+
 def test_engine_generate_runs_with_graphs():
     cfg, gm, _ = _build("cuda", torch.bfloat16)
     g = torch.Generator().manual_seed(5)
