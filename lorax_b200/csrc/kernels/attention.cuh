@@ -78,8 +78,8 @@ LX_DEVICE void expand_plane8(uint32_t dst_plane, uint32_t src8, int tid) {
 // ---- e4m3 pages in the decode kernel --------------------------------------------------------------------------------------------
 // The bytes go from shared memory straight into f16 operands (every e4m3 value is exact in f16): one conversion per pair of elements
 // and one 16-byte load per 16, no expanded plane.  (The plane cost a store and a second load of twice the bytes and four conversions
-// per pair, which bound the kernel: 32 rows of 1024 to 8192 keys took 272 us a layer, and 97 us now in one part, 83 in four; the pages'
-// bytes alone take 46.)  The orders of k in the two products are permuted the same way for both operands,
+// per pair, which bound the kernel: 32 rows of 1024 to 8192 keys took 272 us a layer, and take 83 to 100 now by
+// the contexts' spread; the pages' bytes alone take 46.)  The orders of k in the two products are permuted the same way for both operands,
 // so that a lane's operands of several steps lie in one 16-byte chunk:
 //   Q K^T: step (h, w) gives lane column c the dimensions 64 h + 16 c + 4 w .. + 3 of a key,
 //   P V:   column n of output tile nd is dimension n * (D / 8) + nd, so a lane's dimensions of one key are contiguous.

@@ -124,7 +124,7 @@ LX_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_fla
 // and tables of constants.
 // ------------------------------------------------------------------------------------------------
 // Grids of more than eight blocks per SM do not trigger: a long kernel's successor gains nothing from a microsecond of set-up, and steps
-// of thousands of rows, which run against the power limit, took 3 to 5 % longer with it (6000 rows: 8.03 -> 8.56 ms a pass).
+// of thousands of rows, which run against the power limit, took up to 7 % longer with it (6000 rows: 8.03 -> 8.56 ms a pass).
 constexpr unsigned kTriggerBlocks = 8 * 148;
 LX_DEVICE void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 LX_DEVICE void pdl_trigger() {

@@ -229,7 +229,8 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const ShrinkTc
 // With a few rows per adapter the work is a chain of latencies: table entry, slot, first bytes, sum.  The tensor-core kernel above adds a
 // descriptor fetch and fence, TMA, UMMA, tensor memory and partial sums that meet in global memory behind a counter (10 us for five rows
 // over three adapters of rank 16, 17 to 23 us for 32 rows over 24 of rank 32).  Here a cluster of up to eight CTAs cuts K, the four warps
-// of a CTA cut its part, every lane has 16 to 24 loads of 16 bytes in flight, and the parts meet in distributed shared memory; A_cat is on its way before the wait for the kernel in front.  Five rows: 4 us; 32 rows: 4 to 9 us.
+// of a CTA cut its part, every lane has 16 to 24 loads of 16 bytes in flight, and the parts meet in distributed shared memory; A_cat is on
+// its way before the wait for the kernel in front, where the caller allows it.  Five rows: 4 us; 32 rows: 4 to 9 us.
 //
 // A CTA takes 16 rows of A_cat (j0 ..) and the tile's rows in groups of eight (one group, or four).  The order of k inside a block of 32
 // is permuted the same way for both operands: lane column t holds elements 8 t .. 8 t + 7.
