@@ -202,7 +202,7 @@ class NativeExecutor:
             s.block_tables, s.max_blocks = _p(inp.block_tables), inp.block_tables.shape[1]
             s.cu_q, s.cache_lens, s.tile_seq, s.tile_q0 = _p(inp.cu_q), _p(inp.cache_lens), _p(inp.tile_seq), _p(inp.tile_q0)
             s.n_attn_tiles = inp.tile_seq.shape[0]
-        s.nsplit = inp.attn_nsplit
+        s.nsplit = native.workspace(dev).attn_parts(inp.attn_nsplit, s.n_decode, m.nh, m.d)
         if inp.tok_slot is not None and m.max_rank > 0:
             s.tok_slot = _p(inp.tok_slot)
             if inp.lora_tiles is not None:

@@ -177,6 +177,11 @@ class Workspace:
         self.attn_part_lse = torch.empty(self.attn_part_tokens * num_heads * attn_splits, dtype=torch.float32, device=device)
         self.num_sms = torch.cuda.get_device_properties(device).multi_processor_count
 
+    def attn_parts(self, wanted: int, rows: int, heads: int, d: int) -> int:
+        """Parts of a row's keys (at most `wanted`) whose sums the scratch holds for `rows` rows of `heads` heads of `d`."""
+        held = min(self.attn_part_lse.numel(), self.attn_part_o.numel() // d) // max(1, rows * heads)
+        return max(1, min(wanted, self.attn_splits, held)) if rows <= self.attn_part_tokens else 1
+
     def check_status(self):
         """Raise if a bounded device-side wait ran out since the last check (one D2H of 8 bytes)."""
         st = self.status.tolist()
@@ -625,10 +630,7 @@ def attn_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_tables: torch.Ten
     if out is None:
         out = torch.empty(T, nh * d, dtype=q.dtype, device=q.device)
     ws = workspace(q.device)
-    if nsplit > 1:
-        nsplit = min(nsplit, ws.attn_splits)
-        if T > ws.attn_part_tokens:
-            nsplit = 1
+    nsplit = ws.attn_parts(nsplit, T, nh, d)
     if kv_cache.dtype == torch.float8_e4m3fn:
         ks, vs = kv_scale or (1.0, 1.0)
         rc = load().lx_attn_decode_kv8(_ptr(q), q.stride(0), _ptr(kv_cache), _ptr(block_tables), block_tables.shape[1], _ptr(ctx_lens),

@@ -270,6 +270,26 @@ def test_parts_of_decode_attention_follow_the_contexts():
     assert splits(long, window=1024) == 1 and splits([8000] * 4, rows=4) == 6 and splits([], rows=1, heads=4) == 8
 
 
+def test_parts_of_decode_attention_fit_the_scratch():
+    """Whatever a caller asks for, the parts' sums stay inside the scratch, in widths, rows and heads; what fits is cut as wanted."""
+    from types import SimpleNamespace as NS
+    from lorax_b200.ops.native import Workspace
+    ws = NS(attn_splits=8, attn_part_tokens=256, attn_part_lse=torch.empty(256 * 64 * 8, device="meta"),
+            attn_part_o=torch.empty(256 * 64 * 8 * 128, device="meta"))
+    for d in (64, 128):
+        for heads in (1, 8, 64, 71, 96, 128, 256, 1000):
+            for rows in (1, 13, 95, 129, 255, 256, 257, 511):
+                for wanted in (0, 1, 2, 4, 8, 32):
+                    n = Workspace.attn_parts(ws, wanted, rows, heads, d)
+                    assert 1 <= n <= max(1, min(wanted, 8))
+                    if n > 1:
+                        assert rows * heads * n <= ws.attn_part_lse.numel() and rows * heads * n * d <= ws.attn_part_o.numel()
+                    if wanted and rows <= 256 and heads <= 64:
+                        assert n == min(wanted, 8)
+    assert Workspace.attn_parts(ws, 4, 256, 128, 128) == 4 and Workspace.attn_parts(ws, 4, 256, 256, 128) == 2
+    assert Workspace.attn_parts(ws, 4, 0, 32, 128) == 4
+
+
 def test_vocabulary_parallel_sampling_equals_sampling_from_the_full_row():
     """Tensor-parallel ranks keep their vocabulary shard, exchange 128 candidates plus (max, sum exp) per row and the best
     (noisy score, log-probability, id) triple: the drawn ids equal those of the sampler that sees the whole row, for
