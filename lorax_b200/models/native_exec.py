@@ -132,12 +132,12 @@ class NativeExecutor:
         m.attn_splits, m.attn_part_tokens = ws.attn_splits, ws.attn_part_tokens
         self.max_tokens = ws.lora_v.shape[0]
         ad = self.adapters
-        lora = ad is not None and ad.max_rank > 0 and ad.is_cuda
+        lora = ad is not None and ad.is_cuda      # (adapters may come after the first step)
         if lora:
             from ..adapters.manager import TMAP_GROUPS
             m.arena, m.slot_base, m.slot_rank, m.slot_tmaps = (ad.arena.data_ptr(), ad.slot_base.data_ptr(), ad.slot_rank.data_ptr(),
                                                                ad.slot_tmaps.data_ptr())
-            m.num_slots, m.max_rank, m.groups_per_slot = ad.slot_rank.shape[0], ad.max_rank, ad.groups_per_slot
+            m.num_slots, m.groups_per_slot = ad.slot_rank.shape[0], ad.groups_per_slot
             m.fused_lora = int(model.fused_lora_max_tokens)        # rows up to which LoRA rides inside the GEMM launch
             m.lora_vimg, m.lora_vimg_bytes = ws.lora_vimg.data_ptr(), ws.lora_vimg.numel() * 2
             m.arena_elems = ad.arena.numel()
@@ -203,14 +203,13 @@ class NativeExecutor:
             s.cu_q, s.cache_lens, s.tile_seq, s.tile_q0 = _p(inp.cu_q), _p(inp.cache_lens), _p(inp.tile_seq), _p(inp.tile_q0)
             s.n_attn_tiles = inp.tile_seq.shape[0]
         s.nsplit = native.workspace(dev).attn_parts(inp.attn_nsplit, s.n_decode, m.nh, m.d)
+        m.max_rank = self.adapters.max_rank if self.adapters is not None and self.adapters.is_cuda else 0      # changes as adapters come and go
         if inp.tok_slot is not None and m.max_rank > 0:
             s.tok_slot = _p(inp.tok_slot)
             if inp.lora_tiles is not None:
                 s.lora_tiles, s.num_tiles, s.max_tile_rows = _p(inp.lora_tiles.table), inp.lora_tiles.num_tiles, inp.lora_tiles.max_rows
                 s.live_tiles = inp.lora_tiles.live
         s.normed, s.qkv, s.attn, s.gate_up, s.act = normed.data_ptr(), qkv.data_ptr(), attn.data_ptr(), gate_up.data_ptr(), act.data_ptr()
-        if self.adapters is not None:
-            m.max_rank = self.adapters.max_rank if self.adapters.is_cuda else 0      # changes as adapters come and go
         stream = torch.cuda.current_stream().cuda_stream
         tp = model.tp
         rm = float(c.residual_multiplier)

@@ -46,6 +46,41 @@ def test_prefill_logits_match_cpu_oracle():
     assert (outs[1][1] - outs[1][0]).norm() > 0
 
 
+def test_native_layers_take_adapters_that_come_after_the_first_step():
+    """Prompts before any adapter is resident, with adapters, after the last one has left and with one again: the native layers give what
+    the per-kernel path gives."""
+    cfg, gm, mgr = _build("cuda", torch.bfloat16, 0)
+    for i, r in enumerate([16, 32]):
+        c, mm = random_adapter(cfg, r=r, alpha=16, target_modules=TARGETS, seed=40 + i, std_a=0.05, std_b=0.05)
+        mgr.register(f"a{i}", c, mm)
+    g = torch.Generator().manual_seed(12)
+    prompts = [torch.randint(0, cfg.vocab_size, (n,), generator=g).tolist() for n in (17, 64, 33)]
+    kv = KVCache(cfg.num_hidden_layers, 16, gm.nkv, gm.d, gm.dtype, gm.device)
+    r = ModelRunner(gm, kv, max_batch=4, max_seq_tokens=128, max_prefill_tokens=256, use_graphs=False)
+    blocks = [[1 + 3 * i + j for j in range(3)] for i in range(3)]
+
+    def both(ads):
+        out = []
+        for gm.use_native_layers in (True, False):
+            out.append(r.prefill([PrefillItem(p, 0, b, adapter_index=a) for p, b, a in zip(prompts, blocks, ads)])[2].clone())
+        torch.cuda.synchronize()
+        assert torch.equal(*out), ads
+        return out[0]
+
+    plain = both([0, 0, 0])
+    executor = gm._native
+    assert executor is not None and mgr.load(1, "a0") and mgr.load(2, "a1")
+    with_adapters = both([1, 0, 2])
+    assert torch.equal(with_adapters[1], plain[1])
+    assert all((with_adapters[i] - plain[i]).norm() > 0.01 * plain[i].norm() for i in (0, 2))
+    mgr.offload(1)
+    mgr.offload(2)
+    assert mgr.max_rank == 0 and torch.equal(both([0, 0, 0]), plain)
+    assert mgr.load(2, "a1")
+    again = both([2, 0, 0])
+    assert gm._native is executor and (again[0] - plain[0]).norm() > 0.01 * plain[0].norm()
+
+
 def test_native_layer_executor_equals_python_path():
     """The C++ layer executor issues the same kernels with the same arguments as the per-kernel Python path: prefill
     logits and a mixed prefill + decode step must be bit-identical."""
