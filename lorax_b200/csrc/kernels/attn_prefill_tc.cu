@@ -1,22 +1,27 @@
 // Ragged causal prefill attention over the paged KV cache on the 5th-generation tensor cores.
 //
-// One CTA = one 64-query tile of one sequence x TWO query heads of the same KV group: the 128 rows of a tcgen05 M tile are
-// (head, query) pairs, so a K / V block is staged once for both heads.  Keys are walked in blocks of 128 (four cache pages):
+// One CTA = one 64-query tile of one sequence x TWO or FOUR query heads of the same KV group: the 128 rows of a tcgen05 M tile are
+// (head, query) pairs of two heads, a CTA has NT = 1 or 2 such tiles (two where the group's heads divide by four), and a K / V block is
+// staged once for all of them.  Keys are walked in blocks of 128 (four cache pages):
 //
 //   loader  (warp 0, one lane)  Q by TMA from the projection output; K and V pages by TMA straight from the paged cache
 //                               through one 5-D tensor map {d, slot, K|V, kv head, block}: the block table supplies the last
-//                               coordinate, so pages need not be contiguous; a two-stage ring
-//   MMA     (warp 1, one lane)  S = Q K^T into TMEM (double buffered), then O_j = P_j V_j into TMEM (double buffered); P comes
-//                               back from the softmax warps through shared memory as a K-major operand, V is used as stored
-//                               (token-major = the "MN-major" form of the B operand); S of block j+1 is issued before P_j V_j,
-//                               so the tensor core works on the next scores while the softmax of this block runs
-//   softmax (warps 2..5)        one thread per row: scores from TMEM with tcgen05.ld, scale / softcap / ALiBi / causal and
-//                               window mask, running max and sum, exp2, P as bf16 into the swizzled operand tile; the
-//                               per-block products O_j come back from TMEM and are folded into fp32 registers with the
-//                               usual rescaling, so nothing in TMEM ever has to be rescaled
+//                               coordinate, so pages need not be contiguous; rings of two stages for K and for V
+//   MMA     (warp 1)            S = Q K^T into TMEM, O_j = P_j V_j into TMEM; P is a TMEM operand in the columns that its scores had.
+//                               The tiles take turns: P V and the next S of one run while the other's softmax does
+//   softmax (a warpgroup per tile)  one thread per row: scores from TMEM with tcgen05.ld, scale / softcap / ALiBi / causal and
+//                               window mask, running max and sum, exp2, P as bf16 back into TMEM; the per-block products O_j come
+//                               from TMEM and are folded into fp32 registers with the usual rescaling, so nothing in TMEM ever has
+//                               to be rescaled.  O_j is folded while the tensor core forms S_{j+1}
 //
-// WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, in two operand
-// tiles, and P V is two products into the same accumulator (the layer-by-layer designs ask for it).
+// What bounds it: per tile and block 128 x 128 exponentials take 1024 cycles of the special function units and the products about 1550 of
+// the tensor core (S 950: at N = 128 both operands come from shared memory at its full rate; P V 600).  One tile per CTA has them in a chain
+// (S, softmax, P V, S, ...), 4700 cycles with P through shared memory; two tiles fill each other's gaps, and P in TMEM spares the stores and
+// half of P V's shared memory.  32 heads, 8 KV heads, one tile per CTA and P in shared memory -> this: 8192 tokens 1021 -> 579 us, seven prompts
+// of together 4001 134 -> 70, three of 1700 57 -> 31, 137 tokens 15.9 -> 14.0 (products alone: 368 us of the 579).
+//
+// WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, side by side in
+// TMEM, and P V is two products into the same accumulator (the layer-by-layer designs ask for it).
 //
 // Plain, chunked and prefix-cached prefill are one path: `cache_lens` says how many keys precede the chunk.  It replaces the
 // flash-attn-2 varlen call of the reference (server/lorax_server/utils/flash_attn.py:180-201) and the mma.sync kernel in
@@ -30,7 +35,6 @@ constexpr int kFaPage = 32;
 constexpr int kFaQ = 64;            // queries per CTA (per head)
 constexpr int kFaKeys = 128;        // keys per block
 constexpr int kFaD = 128;
-constexpr int kFaThreads = 192;
 constexpr float kFaLog2e = 1.4426950408889634f;
 
 struct FaParams {
@@ -50,14 +54,14 @@ struct FaParams {
   AttnTail tail;
 };
 
-template <bool WIDE>
-struct FaSmem {
-  static constexpr int kQBytes = 128 * kFaD * 2;             // two 64-wide halves of [128 rows x 64]
+template <int NT>
+struct FaShape {
+  static constexpr int kThreads = 128 * (1 + NT);            // loader, MMA and two idle warps; four softmax warps per tile
+  static constexpr int kQBytes = 128 * kFaD * 2;             // of a tile: two 64-wide halves of [128 rows x 64]
   static constexpr int kKBytes = kFaKeys * kFaD * 2;
   static constexpr int kVBytes = kFaKeys * kFaD * 2;
-  static constexpr int kPBytes = 128 * kFaKeys * 2;
-  static constexpr int kStage = kKBytes + kVBytes;
-  static constexpr int kTotal = kQBytes + 2 * kStage + (WIDE ? 2 : 1) * kPBytes + 512 + 1024;
+  static constexpr int kTotal = NT * kQBytes + 2 * (kKBytes + kVBytes) + 512 + 1024;
+  static constexpr uint32_t kTmemCols = NT * 256;            // S (later P) of every tile, then O of every tile
 };
 
 // 5-D tiled load: the paged cache {d, slot in page, K|V, kv head, block}.
@@ -67,13 +71,64 @@ LX_DEVICE void tma_load_5d(void* smem_dst, const CUtensorMap* m, uint64_t* bar, 
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
-LX_DEVICE void mbar_arrive_cnt(uint64_t* bar) { mbar_arrive(bar); }
 
 LX_DEVICE float fa_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+LX_DEVICE float fa_max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+// Two fp32 numbers in one 64-bit register: one instruction adds or multiplies both (the same roundings as two).
+LX_DEVICE unsigned long long fa_pair(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+LX_DEVICE float2 fa_unpair(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+LX_DEVICE unsigned long long fa_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+LX_DEVICE unsigned long long fa_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+LX_DEVICE unsigned long long fa_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// The wait for tcgen05.ld as something the loaded registers pass through: their first use stays behind it while other loads are in flight.
+LX_DEVICE void fa_wait_ld(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+LX_DEVICE void fa_wait_ld(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
+                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]),
+                 "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]),
+                 "+r"(r[31])
+               :
+               : "memory");
+}
+template <int N>
+LX_DEVICE void fa_regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+LX_DEVICE void fa_regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // How a raw product becomes a score in the log2 domain (the softmax uses exp2): scaled; scaled and capped; also with an ALiBi bias.
 enum FaScores : int { kFaPlain = 0, kFaCap = 1, kFaBias = 2 };
@@ -87,113 +142,187 @@ struct FaScore {
   }
 };
 
-// Maximum over the 128 scores of a row (log2 domain).  Without a bias the scores grow with the products (scale > 0), so the largest product
-// gives it; MASK: keys outside [lo, hi) do not count.
-template <int MODE, bool MASK>
-LX_DEVICE float fa_block_max(uint32_t ts, int kb0, int lo, int hi, const FaScore& sc) {
-  float bm = -INFINITY;
+// The keys a row sees, [lo, hi), and what that is over the rows of its warp: chunks of keys that all of them see, or none, need no mask.
+struct FaBounds {
+  int lo, hi, lo_max, lo_min, hi_min, hi_max;
+  LX_DEVICE bool all(int key, int n) const { return key >= lo_max && key + n <= hi_min; }
+  LX_DEVICE bool none(int key, int n) const { return key >= hi_max || key + n <= lo_min; }
+};
+
+// Products of keys a row does not see become -inf where they lie: their weights are exact zeros without a mask in the passes that follow
+// (a block at a tile's edges only, so its code is small rather than quick: a CTA of a short prompt fetches all its code for a block or two).
+LX_DEVICE void fa_block_mask(uint32_t ts, int kb0, const FaBounds& bd) {
 #pragma unroll 1
-  for (int c = 0; c < kFaKeys; c += 32) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
-    tc_wait_ld();
+  for (int c = 0; c < kFaKeys; c += 16) {
+    if (bd.all(kb0 + c, 16)) continue;
+    const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
+    uint32_t r[16];
+    if (!bd.none(kb0 + c, 16)) {
+      tmem_ld_32x32b_x16(ts + (uint32_t)c, r);
+      fa_wait_ld(r);
+    }
+    uint32_t w[8];
 #pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const int key = kb0 + c + q;
-      float t = MODE == kFaBias ? sc.of<MODE>(__uint_as_float(r[q]), key) : __uint_as_float(r[q]);
-      if (MASK) t = (key >= lo && key < hi) ? t : -INFINITY;
-      bm = fmaxf(bm, t);
+    for (int h = 0; h < 16; h += 8) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) w[q] = (h + q >= lo && h + q < hi) ? r[h + q] : 0xff800000u;
+      tmem_st_32x32b_x8(ts + (uint32_t)(c + h), w);
     }
   }
-  return MODE == kFaBias || bm == -INFINITY ? bm : sc.of<MODE>(bm, 0);
+  tc_wait_st();
 }
 
-// p = exp2(score - m_new) for the 128 keys of the block -> bf16, written as this row of the K-major, 128-byte-swizzled operand
-// tile (WIDE: the remainders as the same row of the tile behind it); returns the row sum.
-template <int MODE, bool MASK, bool WIDE>
-LX_DEVICE float fa_block_probs(uint32_t ts, uint8_t* prow, int row, int kb0, int lo, int hi, float m_new, const FaScore& sc) {
-  float sum = 0.f;
-  const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
-  const bool dead = (m_new == -INFINITY);
-#pragma unroll 1
-  for (int c = 0; c < kFaKeys; c += 32) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
-    tc_wait_ld();
-    uint32_t pk[16], lo_pk[WIDE ? 16 : 1];
+// Maximum over the 128 scores of a row (log2 domain).  Without a bias the scores grow with the products (scale > 0), so the largest product
+// gives it; MASK: keys outside the bounds do not count.
+template <int MODE, bool MASK>
+LX_DEVICE float fa_block_max(uint32_t ts, int kb0, const FaBounds& bd, const FaScore& sc) {
+  float bm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  auto take = [&](const uint32_t (&r)[32], int c, bool mask) {
+    const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
 #pragma unroll
     for (int q = 0; q < 32; q += 2) {
-      float pv[2];
+      float t[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const float sraw = __uint_as_float(r[q + u]);
-        const int key = kb0 + c + q + u;
-        float e = MODE == kFaPlain ? fa_ex2(fmaf(sraw, sc.scale_l2, neg_m)) : fa_ex2(sc.of<MODE>(sraw, key) + neg_m);
-        if (MASK) e = (key >= lo && key < hi && !dead) ? e : 0.f;
-        pv[u] = e;
+        t[u] = MODE == kFaBias ? sc.of<MODE>(__uint_as_float(r[q + u]), kb0 + c + q + u) : __uint_as_float(r[q + u]);
+        if (mask) t[u] = (q + u >= lo && q + u < hi) ? t[u] : -INFINITY;
       }
-      sum += pv[0] + pv[1];
-      pk[q >> 1] = pack_bf16x2(pv[0], pv[1]);
+      bm[(q >> 1) & 3] = fa_max3(bm[(q >> 1) & 3], t[0], t[1]);
+    }
+  };
+  auto chunk = [&](const uint32_t (&r)[32], int c) {
+    if (!MASK || bd.all(kb0 + c, 32)) take(r, c, false);
+    else if (!bd.none(kb0 + c, 32)) take(r, c, true);
+  };
+  uint32_t ra[32], rb[32];
+  tmem_ld_32x32b_x32(ts, ra);
+  fa_wait_ld(ra);
+  tmem_ld_32x32b_x32(ts + 32u, rb);
+  chunk(ra, 0);
+  fa_wait_ld(rb);
+  tmem_ld_32x32b_x32(ts + 64u, ra);
+  chunk(rb, 32);
+  fa_wait_ld(ra);
+  tmem_ld_32x32b_x32(ts + 96u, rb);
+  chunk(ra, 64);
+  fa_wait_ld(rb);
+  chunk(rb, 96);
+  const float m = fmaxf(fa_max3(bm[0], bm[1], bm[2]), bm[3]);
+  return MODE == kFaBias || m == -INFINITY ? m : sc.of<MODE>(m, 0);
+}
+
+// p = exp2(score - m_new) for the 128 keys of the block -> bf16 as a TMEM operand in the columns of the scores: those of 16 keys give
+// eight columns of weights (WIDE: and eight of the remainders).  Returns the row sum.  The exponentials of the next 16 keys are under way
+// while those before are summed, rounded and stored (one after the other 2360 cycles a block, 1024 of them the special function unit's).
+template <int MODE, bool MASK, bool WIDE>
+LX_DEVICE float fa_block_probs(uint32_t ts, int kb0, const FaBounds& bd, float m_new, const FaScore& sc) {
+  float sum = 0.f;
+  const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+  const unsigned long long scale2 = fa_pair(sc.scale_l2, sc.scale_l2), neg2 = fa_pair(neg_m, neg_m);
+  auto exps = [&](const uint32_t (&r)[16], int c, float (&e)[16]) {
+#pragma unroll
+    for (int q = 0; q < 16; q += 2) {
+      const float s0 = __uint_as_float(r[q]), s1 = __uint_as_float(r[q + 1]);
+      if (MODE == kFaPlain) {
+        const float2 x = fa_unpair(fa_fma2(fa_pair(s0, s1), scale2, neg2));
+        e[q] = fa_ex2(x.x);
+        e[q + 1] = fa_ex2(x.y);
+      } else {
+        e[q] = fa_ex2(sc.of<MODE>(s0, kb0 + c + q) + neg_m);
+        e[q + 1] = fa_ex2(sc.of<MODE>(s1, kb0 + c + q + 1) + neg_m);
+      }
+    }
+  };
+  auto chunk = [&](const uint32_t (&r)[16], int c, float (&e)[16]) {
+    if (MASK && bd.none(kb0 + c, 16)) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) e[q] = 0.f;
+      return;
+    }
+    exps(r, c, e);
+    if (MASK && !bd.all(kb0 + c, 16)) {
+      const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) e[q] = (q >= lo && q < hi) ? e[q] : 0.f;
+    }
+  };
+  auto finish = [&](const float (&e)[16], int c) {
+    uint32_t pk[8], rest[8];
+#pragma unroll
+    for (int q = 0; q < 16; q += 2) {
+      sum += e[q] + e[q + 1];
+      pk[q >> 1] = pack_bf16x2(e[q], e[q + 1]);
       if constexpr (WIDE) {
         const float2 h = unpack_bf16x2(pk[q >> 1]);
-        lo_pk[q >> 1] = pack_bf16x2(pv[0] - h.x, pv[1] - h.y);
+        rest[q >> 1] = pack_bf16x2(e[q] - h.x, e[q + 1] - h.y);
       }
     }
-    uint8_t* half = prow + (c >> 6) * 16384;
-#pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
-      const int chunk = ((c & 63) >> 3) + ch;
-      *reinterpret_cast<uint4*>(half + ((chunk ^ (row & 7)) << 4)) = make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]);
-      if constexpr (WIDE)
-        *reinterpret_cast<uint4*>(half + 32768 + ((chunk ^ (row & 7)) << 4)) =
-            make_uint4(lo_pk[4 * ch], lo_pk[4 * ch + 1], lo_pk[4 * ch + 2], lo_pk[4 * ch + 3]);
-    }
+    tmem_st_32x32b_x8(ts + (uint32_t)c, pk);
+    if constexpr (WIDE) tmem_st_32x32b_x8(ts + (uint32_t)(c + 8), rest);
+  };
+  uint32_t ra[16], rb[16];
+  float ea[16], eb[16];
+  tmem_ld_32x32b_x16(ts, ra);
+  fa_wait_ld(ra);
+  tmem_ld_32x32b_x16(ts + 16u, rb);
+  chunk(ra, 0, ea);
+#pragma unroll 1
+  for (int c = 0; c < kFaKeys - 32; c += 32) {
+    fa_wait_ld(rb);
+    tmem_ld_32x32b_x16(ts + (uint32_t)(c + 32), ra);
+    chunk(rb, c + 16, eb);
+    finish(ea, c);
+    fa_wait_ld(ra);
+    tmem_ld_32x32b_x16(ts + (uint32_t)(c + 48), rb);
+    chunk(ra, c + 32, ea);
+    finish(eb, c + 16);
   }
+  fa_wait_ld(rb);
+  chunk(rb, kFaKeys - 16, eb);
+  finish(ea, kFaKeys - 32);
+  finish(eb, kFaKeys - 16);
   return sum;
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(kFaThreads, 1)
+template <bool WIDE, int NT>
+__global__ void __launch_bounds__(FaShape<NT>::kThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_kv, const FaParams p) {
-  using S = FaSmem<WIDE>;
+  using S = FaShape<NT>;
   extern __shared__ uint8_t fa_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sq = smem;
-  uint8_t* skv = smem + S::kQBytes;
-  uint8_t* sp = skv + 2 * S::kStage;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sp + (WIDE ? 2 : 1) * S::kPBytes);
+  uint8_t* sk = sq + NT * S::kQBytes;
+  uint8_t* sv = sk + 2 * S::kKBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sv + 2 * S::kVBytes);
   uint64_t* q_full = bars;            // 1
-  uint64_t* kv_full = bars + 1;       // 2
-  uint64_t* kv_empty = bars + 3;      // 2
-  uint64_t* s_full = bars + 5;        // 2
-  uint64_t* s_empty = bars + 7;       // 2  (128 arrivals)
-  uint64_t* p_full = bars + 9;        // 1  (128 arrivals)
-  uint64_t* p_empty = bars + 10;      // 1
-  uint64_t* pv_full = bars + 11;      // 2
-  uint64_t* pv_empty = bars + 13;     // 2  (128 arrivals)
+  uint64_t* k_full = bars + 1;        // 2
+  uint64_t* k_empty = bars + 3;       // 2
+  uint64_t* v_full = bars + 5;        // 2
+  uint64_t* v_empty = bars + 7;       // 2
+  uint64_t* s_full = bars + 9;        // per tile
+  uint64_t* p_full = bars + 11;       // per tile, an arrival per softmax warp: weights written, the product before them folded
+  uint64_t* pv_full = bars + 13;      // per tile
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = (int)gridDim.x - 1 - (int)blockIdx.x;      // later tiles of a sequence see more keys: start the long ones first
-  const int h0 = blockIdx.y * 2;                 // first of the two query heads
-  const int kvh = h0 / p.group;
+  const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;      // later tiles of a sequence see more keys: start the long ones first
+  const int hc = blockIdx.x * 2 * NT;            // first of the CTA's query heads
+  const int kvh = hc / p.group;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128);
-      mbar_init(&pv_full[i], 1); mbar_init(&pv_empty[i], 128);
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&pv_full[i], 1);
     }
-    mbar_init(p_full, 128);
-    mbar_init(p_empty, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_kv);
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_slot, S::kTmemCols); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -214,177 +343,207 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   const int nblk = max((key_hi + kFaKeys - 1) / kFaKeys - t_lo, 0);
   const int total_pages = (key_hi + kFaPage - 1) / kFaPage;
 
-  if (warp == 0) {
-    if (lane == 0 && nblk > 0) {
-      // Q: rows 0..63 = head h0, rows 64..127 = head h0 + 1; two 64-wide halves of d
-      mbar_expect_tx(q_full, (uint32_t)S::kQBytes);
-      for (int g = 0; g < 2; ++g)
+  if (warp < 4) {
+    if constexpr (NT == 2) fa_regs_dec<56>();      // 128 * 56 + 256 * 224 = 384 * 168: what the block was launched with
+    if (warp == 0 && lane == 0 && nblk > 0) {
+      // Q: rows 0..63 of a tile = its first head, rows 64..127 = its second; two 64-wide halves of d
+      mbar_expect_tx(q_full, (uint32_t)(NT * S::kQBytes));
+      for (int g = 0; g < 2 * NT; ++g)
         for (int hf = 0; hf < 2; ++hf)
-          tma_load_2d(sq + hf * 16384 + g * 8192, &tmap_q, q_full, (h0 + g) * kFaD + hf * 64, tok_base + q0);
+          tma_load_2d(sq + (g >> 1) * S::kQBytes + hf * 16384 + (g & 1) * 8192, &tmap_q, q_full, (hc + g) * kFaD + hf * 64, tok_base + q0);
       const int* bt = p.block_tables + (long long)b * p.max_blocks;
       for (int j = 0; j < nblk; ++j) {
         const int st = j & 1;
-        if (!mbar_wait(&kv_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) { report_status(p.status, kTimeoutEmptyBarrier, tile); *abort_flag = 1; break; }
-        uint8_t* sk = skv + st * S::kStage;
-        uint8_t* sv = sk + S::kKBytes;
-        mbar_expect_tx(&kv_full[st], (uint32_t)S::kStage);
+        int blk[4];
         for (int pg = 0; pg < 4; ++pg) {
           const int page = (t_lo + j) * 4 + pg;
-          const int blk = (page < total_pages && page < p.max_blocks) ? bt[page] : 0;      // a page past the keys reads block 0: masked, but finite
-          for (int hf = 0; hf < 2; ++hf) {
-            tma_load_5d(sk + hf * 16384 + pg * 4096, &tmap_kv, &kv_full[st], hf * 64, 0, 0, kvh, blk);
-            tma_load_5d(sv + hf * 16384 + pg * 4096, &tmap_kv, &kv_full[st], hf * 64, 0, 1, kvh, blk);
+          blk[pg] = (page < total_pages && page < p.max_blocks) ? bt[page] : 0;      // a page past the keys reads block 0: masked, but finite
+        }
+        for (int kv = 0; kv < 2; ++kv) {
+          uint64_t* full = kv ? &v_full[st] : &k_full[st];
+          if (!mbar_wait(kv ? &v_empty[st] : &k_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) {
+            report_status(p.status, kTimeoutEmptyBarrier, tile);
+            *abort_flag = 1;
+            j = nblk;
+            break;
+          }
+          uint8_t* dst = kv ? sv + st * S::kVBytes : sk + st * S::kKBytes;
+          mbar_expect_tx(full, (uint32_t)S::kKBytes);
+          for (int pg = 0; pg < 4; ++pg)
+            for (int hf = 0; hf < 2; ++hf) tma_load_5d(dst + hf * 16384 + pg * 4096, &tmap_kv, full, hf * 64, 0, kv, kvh, blk[pg]);
+        }
+      }
+    } else if (warp == 1 && nblk > 0) {
+      // The whole warp walks the blocks and one lane issues: addresses and descriptors stay uniform, so that MMAs of 64 cycles each
+      // are not held up by their issue (all of it by one lane of a divergent warp: 8192 tokens 615 us instead of 579).
+      const uint32_t idesc_s = make_idesc(128, kFaKeys, kFmtBF16, kFmtBF16);
+      const uint32_t idesc_pv = make_idesc(128, kFaD, kFmtBF16, kFmtBF16, 0, 1);          // B (= V) is MN-major
+      const uint64_t dq = make_desc_k_sw128(smem_u32(sq)), dk = make_desc_k_sw128(smem_u32(sk)), dv = make_desc_mn_sw128(smem_u32(sv), 16384, 1024);
+      const bool leader = elect_one();
+      auto give_up = [&](int code) {
+        if (leader) report_status(p.status, code, tile);
+        *abort_flag = 1;
+      };
+      // S of tile t and block j.  It takes the columns of the weights that the product issued before it reads: one thread's MMAs run in order.
+      auto issue_s = [&](int t, int j) {
+        const uint64_t da = dq + (uint64_t)((t * S::kQBytes) >> 4), db = dk + (uint64_t)(((j & 1) * S::kKBytes) >> 4);
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < kFaD / 16; ++ks) {
+            const uint64_t at = (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * 2);
+            umma_f16_ss(tmem_base + (uint32_t)(t * 128), da + at, db + at, idesc_s, ks > 0 ? 1u : 0u);
+          }
+          tc_commit(&s_full[t]);
+          if (t == NT - 1) tc_commit(&k_empty[j & 1]);
+        }
+        __syncwarp();
+      };
+      bool ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&k_full[0], 0, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) give_up(kTimeoutFullBarrier);
+      tc_fence_after();
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+        if (ok) issue_s(t, 0);
+      for (int j = 0; ok && j < nblk; ++j) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag));
+        if (!ok) { give_up(kTimeoutFullBarrier); break; }
+        const uint64_t dvj = dv + (uint64_t)(((j & 1) * S::kVBytes) >> 4);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&p_full[t], j & 1, abort_flag));
+          if (!ok) { give_up(kTimeoutTmemEmpty); break; }
+          tc_fence_after();
+          const uint32_t tmem_p = tmem_base + (uint32_t)(t * 128), tmem_o = tmem_base + (uint32_t)(NT * 128 + t * 128);
+          if (leader) {
+#pragma unroll
+            for (int ks = 0; ks < kFaKeys / 16; ++ks) {
+              const uint64_t db = dvj + (uint64_t)(ks * (2048 >> 4));
+              umma_f16_ts(tmem_o, tmem_p + (uint32_t)(ks * 16), db, idesc_pv, ks > 0 ? 1u : 0u);
+              if constexpr (WIDE) umma_f16_ts(tmem_o, tmem_p + (uint32_t)(ks * 16 + 8), db, idesc_pv, 1u);
+            }
+            tc_commit(&pv_full[t]);
+            if (t == NT - 1) tc_commit(&v_empty[j & 1]);
+          }
+          __syncwarp();
+          if (j + 1 < nblk) {
+            if (t == 0) {
+              ok = __all_sync(0xffffffffu, mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag));
+              if (!ok) { give_up(kTimeoutFullBarrier); break; }
+              tc_fence_after();
+            }
+            issue_s(t, j + 1);
           }
         }
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0 && nblk > 0) {
-      const uint32_t idesc_s = make_idesc(128, kFaKeys, kFmtBF16, kFmtBF16);
-      const uint32_t idesc_pv = make_idesc(128, kFaD, kFmtBF16, kFmtBF16, 0, 1);          // B (= V) is MN-major
-      const uint32_t sq_a = smem_u32(sq), sp_a = smem_u32(sp);
-      bool ok = mbar_wait(q_full, 0, abort_flag);
-      if (!ok) { report_status(p.status, kTimeoutFullBarrier, tile); *abort_flag = 1; }
-      auto do_pv = [&](int i) -> bool {
-        const int st = i & 1;
-        if (!mbar_wait(p_full, i & 1, abort_flag) || !mbar_wait(&pv_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) {
-          report_status(p.status, kTimeoutTmemEmpty, tile); *abort_flag = 1; return false;
-        }
-        tc_fence_after();
-        const uint32_t sv_a = smem_u32(skv + st * S::kStage + S::kKBytes);
-        const uint32_t tmem_o = tmem_base + 256u + (uint32_t)(st * 128);
-#pragma unroll
-        for (int ks = 0; ks < kFaKeys / 16; ++ks) {
-          const uint64_t da = make_desc_k_sw128(sp_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
-          const uint64_t db = make_desc_mn_sw128(sv_a + (uint32_t)(ks * 2048), 16384, 1024);
-          umma_f16_ss(tmem_o, da, db, idesc_pv, ks > 0 ? 1u : 0u);
-          if constexpr (WIDE) umma_f16_ss(tmem_o, da + (uint64_t)(S::kPBytes >> 4), db, idesc_pv, 1u);
-        }
-        tc_commit(&pv_full[st]);
-        tc_commit(p_empty);
-        tc_commit(&kv_empty[st]);
-        return true;
-      };
-      for (int j = 0; ok && j < nblk; ++j) {
-        const int st = j & 1;
-        if (!mbar_wait(&kv_full[st], (j >> 1) & 1, abort_flag) || !mbar_wait(&s_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) {
-          report_status(p.status, kTimeoutFullBarrier, tile); *abort_flag = 1; ok = false; break;
-        }
-        tc_fence_after();
-        const uint32_t sk_a = smem_u32(skv + st * S::kStage);
-        const uint32_t tmem_s = tmem_base + (uint32_t)(st * 128);
-#pragma unroll
-        for (int ks = 0; ks < kFaD / 16; ++ks) {
-          const uint64_t da = make_desc_k_sw128(sq_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
-          const uint64_t db = make_desc_k_sw128(sk_a + (uint32_t)((ks >> 2) * 16384)) + (uint64_t)((ks & 3) * 2);
-          umma_f16_ss(tmem_s, da, db, idesc_s, ks > 0 ? 1u : 0u);
-        }
-        tc_commit(&s_full[st]);
-        if (j > 0) ok = do_pv(j - 1);
-      }
-      if (ok) do_pv(nblk - 1);
-    }
-    __syncwarp();
-  } else if (nblk > 0) {
+  } else {
     // ------------------------------------------------------------------ softmax warps: one row per thread
+    if constexpr (NT == 2) fa_regs_inc<224>();
+    const int t = (warp >> 2) - 1;
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
-    const int head = h0 + (row >> 6);
+    const int head = hc + 2 * t + (row >> 6);
     const int qi = q0 + (row & 63);
     const bool row_ok = qi < qlen;
-    const int hi = row_ok ? cache + qi + 1 : 0;
+    const int hi = cache + min(qi, qlen - 1) + 1;      // (a row past the sequence's end sees what its last one does, and is not stored)
     const int lo = (p.window > 0 && hi > p.window) ? hi - p.window : 0;
-    // block-level bounds: a block whose keys every row of the tile sees needs no mask
-    const int hi_min = cache + q0 + 1;
-    const int lo_max = (p.window > 0 && key_hi > p.window) ? key_hi - p.window : 0;
-    const bool rows_all_valid = (q0 + kFaQ <= qlen);
+    const FaBounds bd{lo, hi, __reduce_max_sync(0xffffffffu, lo), __reduce_min_sync(0xffffffffu, lo), __reduce_min_sync(0xffffffffu, hi),
+                      __reduce_max_sync(0xffffffffu, hi)};
     FaScore sc;
     sc.scale_l2 = p.scale * kFaLog2e;
     sc.cap_l2 = p.softcap > 0.f ? p.softcap * kFaLog2e : 0.f;
     sc.cap_k = p.softcap > 0.f ? 2.f * sc.scale_l2 / p.softcap : 0.f;
     sc.slope_l2 = p.alibi != nullptr ? p.alibi[head] * kFaLog2e : 0.f;
-    const int mode = p.alibi != nullptr ? kFaBias : p.softcap > 0.f ? kFaCap : kFaPlain;
+    // (the plain forms take the largest product for the largest score)
+    const int mode = p.alibi != nullptr || !(p.scale > 0.f) ? kFaBias : p.softcap > 0.f ? kFaCap : kFaPlain;
     const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16);
-    uint8_t* prow = sp + row * 128;
+    const uint32_t ts = trow + (uint32_t)(t * 128), to = trow + (uint32_t)(NT * 128 + t * 128);
 
     float m = -INFINITY, l = 0.f;
-    float o[kFaD];
+    unsigned long long o[kFaD / 2];           // pairs of columns
 #pragma unroll
-    for (int i = 0; i < kFaD; ++i) o[i] = 0.f;
-    bool alive = true;
+    for (int i = 0; i < kFaD / 2; ++i) o[i] = 0ull;
+    // o += the product of the block before, while the tensor core forms the next scores
+    auto fold = [&]() {
+      auto add = [&](const uint32_t (&r)[32], int c) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 2) o[(c + q) >> 1] = fa_add2(o[(c + q) >> 1], fa_pair(__uint_as_float(r[q]), __uint_as_float(r[q + 1])));
+      };
+      uint32_t ra[32], rb[32];
+      tmem_ld_32x32b_x32(to, ra);
+      fa_wait_ld(ra);
+      tmem_ld_32x32b_x32(to + 32u, rb);
+      add(ra, 0);
+      fa_wait_ld(rb);
+      tmem_ld_32x32b_x32(to + 64u, ra);
+      add(rb, 32);
+      fa_wait_ld(ra);
+      tmem_ld_32x32b_x32(to + 96u, rb);
+      add(ra, 64);
+      fa_wait_ld(rb);
+      add(rb, 96);
+    };
+    bool alive = nblk > 0;
 
     for (int j = 0; j < nblk && alive; ++j) {
-      const int st = j & 1;
       const int kb0 = (t_lo + j) * kFaKeys;
-      if (!mbar_wait(&s_full[st], (j >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
+      if (j > 0) {
+        if (!mbar_wait(&pv_full[t], (j - 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
+        tc_fence_after();
+        fold();
+      }
+      if (!mbar_wait(&s_full[t], j & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
       tc_fence_after();
-      const bool need_mask = !(rows_all_valid && kb0 + kFaKeys <= hi_min && kb0 >= lo_max);
-      const uint32_t ts = trow + (uint32_t)(st * 128);
-      // pass 1: block maximum of this row (log2 domain)
+      // pass 1: block maximum of this row (log2 domain).  Plain scores have their masked keys set to -inf first, the others are masked chunk
+      // by chunk: a capped -inf is finite
+      if (mode == kFaPlain && !bd.all(kb0, kFaKeys)) fa_block_mask(ts, kb0, bd);
       float bm;
-      if (mode == kFaPlain) bm = need_mask ? fa_block_max<kFaPlain, true>(ts, kb0, lo, hi, sc) : fa_block_max<kFaPlain, false>(ts, kb0, lo, hi, sc);
-      else if (mode == kFaCap) bm = need_mask ? fa_block_max<kFaCap, true>(ts, kb0, lo, hi, sc) : fa_block_max<kFaCap, false>(ts, kb0, lo, hi, sc);
-      else bm = fa_block_max<kFaBias, true>(ts, kb0, lo, hi, sc);
+      if (mode == kFaPlain) bm = fa_block_max<kFaPlain, false>(ts, kb0, bd, sc);
+      else if (mode == kFaCap) bm = fa_block_max<kFaCap, true>(ts, kb0, bd, sc);
+      else bm = fa_block_max<kFaBias, true>(ts, kb0, bd, sc);
       const float m_new = fmaxf(m, bm);
       const float alpha = (m_new == -INFINITY) ? 1.f : fa_ex2(m - m_new);
-      // the P tile is free once the MMAs of the previous block have read it
-      if (!mbar_wait(p_empty, (j & 1) ^ 1, abort_flag)) { report_status(p.status, kTimeoutTmemEmpty, tile); *abort_flag = 1; alive = false; break; }
-      // pass 2: probabilities -> bf16 operand tile, row sum
+      // pass 2: weights -> bf16 operand, row sum
       float sum;
-      if (mode == kFaPlain) sum = need_mask ? fa_block_probs<kFaPlain, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc)
-                                            : fa_block_probs<kFaPlain, false, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
-      else if (mode == kFaCap) sum = need_mask ? fa_block_probs<kFaCap, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc)
-                                               : fa_block_probs<kFaCap, false, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
-      else sum = fa_block_probs<kFaBias, true, WIDE>(ts, prow, row, kb0, lo, hi, m_new, sc);
+      if (mode == kFaPlain) sum = fa_block_probs<kFaPlain, false, WIDE>(ts, kb0, bd, m_new, sc);
+      else if (mode == kFaCap) sum = fa_block_probs<kFaCap, true, WIDE>(ts, kb0, bd, m_new, sc);
+      else sum = fa_block_probs<kFaBias, true, WIDE>(ts, kb0, bd, m_new, sc);
+      tc_wait_st();
       tc_fence_before();
-      mbar_arrive(&s_empty[st]);
-      fence_proxy_async_smem();
-      mbar_arrive(p_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[t]);
       l = l * alpha + sum;
-      // fold the previous block's product in: o = (o + O_{j-1}) * alpha
-      if (j > 0) {
-        const int ps = (j - 1) & 1;
-        if (!mbar_wait(&pv_full[ps], ((j - 1) >> 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
-        tc_fence_after();
-        const bool same_max = __all_sync(0xffffffffu, alpha == 1.f);      // no row of the warp saw a new maximum: nothing to rescale
+      if (j > 0 && !__all_sync(0xffffffffu, alpha == 1.f)) {      // some row of the warp saw a new maximum
+        const unsigned long long alpha2 = fa_pair(alpha, alpha);
 #pragma unroll
-        for (int c = 0; c < kFaD; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(trow + (uint32_t)(256 + ps * 128 + c), r);
-          tc_wait_ld();
-          if (same_max) {
-#pragma unroll
-            for (int q = 0; q < 32; ++q) o[c + q] += __uint_as_float(r[q]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < 32; ++q) o[c + q] = (o[c + q] + __uint_as_float(r[q])) * alpha;
-          }
-        }
-        tc_fence_before();
-        mbar_arrive(&pv_empty[ps]);
+        for (int i = 0; i < kFaD / 2; ++i) o[i] = fa_mul2(o[i], alpha2);
       }
       m = m_new;
     }
     if (alive) {
-      const int ps = (nblk - 1) & 1;
-      if (mbar_wait(&pv_full[ps], ((nblk - 1) >> 1) & 1, abort_flag)) {
+      if (mbar_wait(&pv_full[t], (nblk - 1) & 1, abort_flag)) {
         tc_fence_after();
         const float inv = l > 0.f ? attn_denominator(p.tail, head, m, l) * p.tail.scale : 0.f;
         const __nv_bfloat16* grow = p.tail.gate != nullptr ? p.tail.gate + (long long)(tok_base + qi) * p.tail.ldg + (long long)head * kFaD : nullptr;
         __nv_bfloat16* orow = p.out + (long long)(tok_base + qi) * p.ldo + (long long)head * kFaD;
 #pragma unroll
-        for (int c = 0; c < kFaD; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(trow + (uint32_t)(256 + ps * 128 + c), r);
-          tc_wait_ld();
+        for (int c = 0; c < kFaD; c += 16) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(to + (uint32_t)c, r);
+          fa_wait_ld(r);
           if (row_ok) {
 #pragma unroll
-            for (int q = 0; q < 32; q += 8) {
+            for (int q = 0; q < 16; q += 8) {
               uint32_t w[4];
               float v[8];
 #pragma unroll
-              for (int u = 0; u < 8; ++u) v[u] = (o[c + q + u] + __uint_as_float(r[q + u])) * inv;
+              for (int u = 0; u < 8; u += 2) {
+                const float2 s = fa_unpair(o[(c + q + u) >> 1]);
+                v[u] = (s.x + __uint_as_float(r[q + u])) * inv;
+                v[u + 1] = (s.y + __uint_as_float(r[q + u + 1])) * inv;
+              }
               if (p.tail.turn != nullptr) attn_turn_back8(p.tail, v, c + q, cache + qi);
               if (grow != nullptr) {
                 const uint4 g = *reinterpret_cast<const uint4*>(grow + c + q);
@@ -410,7 +569,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, S::kTmemCols); }
 }
 
 typedef CUresult (*FaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -426,18 +585,24 @@ static FaEncodeFn fa_encode_fn() {
   return fn;
 }
 
-template <bool WIDE>
-static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const FaParams& p, int num_tiles, cudaStream_t s) {
+template <bool WIDE, int NT>
+static int launch_fa_t(const CUtensorMap& tq, const CUtensorMap& tkv, const FaParams& p, int num_tiles, cudaStream_t s) {
+  using S = FaShape<NT>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSmem<WIDE>::kTotal);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<WIDE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal);
     if (e != cudaSuccess) return -(int)e;
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  launch_pdl(attn_prefill_tc_kernel<WIDE>, dim3(num_tiles, p.nh / 2), dim3(kFaThreads), (size_t)FaSmem<WIDE>::kTotal, s, tq, tkv, p);
+  // the heads of a query tile run side by side (they share its keys' pages where they share a KV head), long tiles first
+  launch_pdl(attn_prefill_tc_kernel<WIDE, NT>, dim3(p.nh / (2 * NT), num_tiles), dim3(S::kThreads), (size_t)S::kTotal, s, tq, tkv, p);
   return -(int)cudaGetLastError();
+}
+template <bool WIDE>
+static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const FaParams& p, int num_tiles, cudaStream_t s) {
+  return p.group % 4 == 0 ? launch_fa_t<WIDE, 2>(tq, tkv, p, num_tiles, s) : launch_fa_t<WIDE, 1>(tq, tkv, p, num_tiles, s);
 }
 
 static int attn_prefill_tc(const void* q, long long ldq, int T, const void* kv, int num_blocks, const int* block_tables, int max_blocks,

@@ -349,6 +349,41 @@ def test_attn_prefill_tensor_core(nat, nh, nkv, window, softcap, q_lens, cache_l
         assert torch.isfinite(got.float()).all()
 
 
+@pytest.mark.parametrize("wide", [0, 1])
+@pytest.mark.parametrize("nh,nkv,window,softcap,bias,q_lens,cache_lens", [
+    (8, 1, 0, 0.0, False, [1, 63, 64, 65], [0, 0, 127, 128]),      # two tiles a CTA; queries and keys around the edges of tiles and blocks
+    (12, 2, 0, 0.0, False, [129, 192], [1, 300]),                  # six heads a group: one tile a CTA
+    (4, 1, 1, 0.0, False, [130], [0]), (16, 4, 33, 0.0, False, [200, 5], [31, 700]), (4, 2, 128, 0.0, False, [257], [0]),
+    (8, 2, 100, 20.0, False, [190, 66], [0, 250]), (8, 2, 0, 0.0, True, [150, 33], [0, 96]), (4, 2, 40, 15.0, True, [140], [64])])
+def test_attn_prefill_tensor_core_tiles_and_masks(nat, nh, nkv, window, softcap, bias, q_lens, cache_lens, wide):
+    """Every form of the scores and of their mask, with one and two tiles a CTA.  Weights are rounded to bf16 unless `wide`, results always:
+    2^-9 each at most, relatively."""
+    d, B, T = 128, len(q_lens), sum(q_lens)
+    cache, bt = _make_cache(B, max(a + b for a, b in zip(q_lens, cache_lens)), nkv, d, seed=nh)
+    q = torch.randn(T, nh * d, generator=torch.Generator("cuda").manual_seed(T), device="cuda").to(torch.bfloat16)
+    ints = lambda v: torch.tensor(v, device="cuda", dtype=torch.int32)
+    cu, cl = ints([0] + list(torch.tensor(q_lens).cumsum(0))), ints(cache_lens)
+    ts, tq = (ints(t) for t in ref.prefill_tiles(q_lens))
+    slopes = torch.linspace(0.01, 0.3, nh, device="cuda") if bias else None
+    out, p, scale = torch.empty_like(q), nat._ptr, d ** -0.5
+    rc = nat.load().lx_attn_prefill_tc(p(q), q.stride(0), T, p(cache), cache.shape[0], p(bt), bt.shape[1], p(cu), p(cl), p(ts), p(tq), ts.shape[0], p(out),
+                                       out.stride(0), nh, nkv, d, window, scale, softcap, p(slopes), wide, p(nat.workspace().status), nat._stream())
+    assert rc == 0
+    nat.workspace().check_status()
+    at = 0
+    for b in range(B):
+        n, m = q_lens[b], q_lens[b] + cache_lens[b]
+        pos, key = cache_lens[b] + torch.arange(n, device="cuda")[:, None], torch.arange(m, device="cuda")
+        for h in range(nh):
+            k, v = cache[bt[b].long()][:, h * nkv // nh].transpose(0, 1).reshape(2, -1, d)[:, :m].double()
+            s = q[at: at + n, h * d: (h + 1) * d].double() @ k.t() * scale
+            s = softcap * torch.tanh(s / softcap) if softcap else s
+            s = s + slopes[h].double() * key if bias else s
+            s = s.masked_fill((key > pos) | ((pos - key >= window) if window else (key < 0)), float("-inf"))
+            assert _rel_err(out[at: at + n, h * d: (h + 1) * d], torch.softmax(s, -1) @ v) < (2 ** -9 if wide else 2 ** -8)
+        at += n
+
+
 def _by_blocks(q, k, v, first, scale, block=128):
     """Attention of one head in float64 the way prompt attention forms it: keys in blocks, weights rounded to bf16 relative to the largest
     score up to and including their block, divided by the sum of the unrounded weights.  q [n, d] at positions first .., k and v [m, d]."""
