@@ -82,9 +82,10 @@ struct GemmParams {
   const __nv_bfloat16* lora_arena;     // the slots' blobs
   const __nv_bfloat16* lora_x;         // the step's activations [T, K] (operand B of the GEMM), row stride lora_ldx
   long long lora_ldx;
-  int lora_max_r;                      // largest rank * parts of a resident adapter: bounds the 8-row blocks of a shrink unit
   int lora_inline_shrink;              // 1: the epilogue warps compute the shrink during the first K loop (0: a launch in front did)
   int* lora_sync;                      // [2] CTAs of this launch that have finished / whose shrink units are done; zero between launches
+  float* lora_kparts;                  // [grid][16 ranks][8 rows] fp32 sums of shrink units whose K several CTAs share (nullptr: none do)
+  int* lora_kcounters;                 // [grid] arrivals at such a unit, zero between launches
   int lora_arena_maps;                 // 1: B_cat tiles come through the four arena-wide maps of the launch (LoraBMaps), not the slots' own
   int lora_tables_const;               // tables and adapters may be read before the wait for the kernel in front
   int lora_fence_maps;                 // 1: acquire-fence a slot's B_cat map before every use (0: never; measurement only)
@@ -264,7 +265,8 @@ constexpr int kShrinkRows = 8;          // rows of x per mma (its N); a unit has
 // Rows of x per shrink unit.  Decode-sized steps have few rows per adapter: one group of eight.  Long steps (prefill) have whole
 // entries of 32 rows: four groups share every load of the A_cat block, which halves the bytes a unit of work moves.
 LX_DEVICE int lora_shrink_unit_rows(const GemmParams& p) { return p.lora_T > 512 ? 4 * kShrinkRows : kShrinkRows; }
-LX_DEVICE void lora_group_prefix(const GemmParams& p, const LoraEnt* ents, unsigned short* gstart) {
+// Units before each entry; gstart[num_tiles] is the number of all (at most 512 entries x 4 groups x 12 blocks of ranks).
+LX_DEVICE void lora_unit_prefix(const GemmParams& p, const LoraEnt* ents, unsigned short* gstart) {
   const int unit_rows = lora_shrink_unit_rows(p);
   const int lane = threadIdx.x & 31;
   int run = 0;
@@ -273,7 +275,7 @@ LX_DEVICE void lora_group_prefix(const GemmParams& p, const LoraEnt* ents, unsig
     int cnt = 0;
     if (lt < p.lora_num_tiles) {
       const LoraEnt e = ents[lt];
-      if (e.slot >= 0 && e.r > 0) cnt = (e.nrows + unit_rows - 1) / unit_rows;
+      if (e.slot >= 0 && e.r > 0) cnt = (e.nrows + unit_rows - 1) / unit_rows * (e.r * p.lora_nparts >> 4);
     }
     int incl = cnt;
 #pragma unroll
@@ -289,28 +291,31 @@ LX_DEVICE void lora_group_prefix(const GemmParams& p, const LoraEnt* ents, unsig
 
 struct ShrinkUnit {
   int lt, t0, nt, r, j;          // entry, first row, rows (<= 8 or 32), rank of the slot, first of the unit's 16 rank rows (part * r + i)
+  int u, part, b0, b1;
   const __nv_bfloat16* a;        // A_cat row j
 };
 
-LX_DEVICE bool decode_shrink_unit(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, int u, int nblk, int unit_rows,
-                                  ShrinkUnit& s) {
-  const int g = u / nblk, jb = u - g * nblk;
-  int lo = 0, hi = p.lora_num_tiles;                     // last entry with gstart <= g
+// Part `part` of `parts` of unit u, whose batches of K blocks are [b0, b1) of nbatch.
+LX_DEVICE void decode_shrink_unit(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, int u, int part, int parts, int nbatch,
+                                  int unit_rows, ShrinkUnit& s) {
+  int lo = 0, hi = p.lora_num_tiles;                     // last entry with gstart <= u: the one that has the unit
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if ((int)gstart[mid] <= g) lo = mid; else hi = mid;
+    if ((int)gstart[mid] <= u) lo = mid; else hi = mid;
   }
   const LoraEnt e = ents[lo];
-  if (e.slot < 0 || e.r <= 0) return false;
-  const int sub = g - (int)gstart[lo];
-  if (sub * unit_rows >= e.nrows || jb * 16 >= e.r * p.lora_nparts) return false;
+  const int nblk = e.r * p.lora_nparts >> 4, local = u - (int)gstart[lo];
+  const int sub = local / nblk, jb = local - sub * nblk;
   s.lt = lo;
   s.t0 = e.row0 + sub * unit_rows;
   s.nt = min(unit_rows, e.row0 + e.nrows - s.t0);
   s.r = e.r;
   s.j = jb * 16;
+  s.u = u;
+  s.part = part;
+  s.b0 = nbatch * part / parts;
+  s.b1 = nbatch * (part + 1) / parts;
   s.a = p.lora_arena + (long long)e.boff * 8 + (long long)e.r * (p.lora_off_a - p.lora_off_b) + (long long)s.j * p.K;
-  return true;
 }
 
 LX_DEVICE void mma_bf16_16x8x16(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -342,33 +347,64 @@ LX_DEVICE void shrink_loads(const GemmParams& p, const ShrinkUnit& s, int batch,
   }
 }
 
+// This CTA's sums over its part of a unit's K, in the four warps' slices of `red`, join the other parts'.  True in the CTA that arrived last:
+// the first slice then holds the unit's sums, the others zeros.
+LX_DEVICE bool lora_join_kparts(const GemmParams& p, const ShrinkUnit& s, int parts, float* red, int* flag, int tid4) {
+  float* mine = p.lora_kparts + ((long long)s.u * parts + s.part) * 128;
+  __stcg(mine + tid4, red[tid4] + red[128 + tid4] + red[256 + tid4] + red[384 + tid4]);
+  __threadfence();
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (tid4 == 0) {
+    const int prev = atomicAdd(&p.lora_kcounters[s.u], 1);
+    *flag = prev == parts - 1;
+    if (prev == parts - 1) p.lora_kcounters[s.u] = 0;      // ready for the next launch
+  }
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (*flag == 0) return false;
+  __threadfence();
+  const float* first = p.lora_kparts + (long long)s.u * parts * 128 + tid4;
+  float sum = 0.f;
+  for (int i = 0; i < parts; ++i) sum += __ldcg(first + i * 128);
+  red[tid4] = sum;
+  red[128 + tid4] = red[256 + tid4] = red[384 + tid4] = 0.f;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  return true;
+}
+
 template <int NG, int SB>
 LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, float* red, int ewarp, int lane) {
   const int tid4 = ewarp * 32 + lane;
-  const int nblk = (p.lora_max_r + 15) >> 4;
-  const int U = (int)gstart[p.lora_num_tiles] * nblk;
+  const int U = (int)gstart[p.lora_num_tiles];
   const int nbatch = ((p.K + 31) / 32 + 4 * SB - 1) / (4 * SB);    // batches of SB blocks per warp
   constexpr int kUnitRows = NG * kShrinkRows;
-  ShrinkUnit cur;
-  int u = (int)blockIdx.x;
-  while (u < U && !decode_shrink_unit(p, ents, gstart, u, nblk, kUnitRows, cur)) u += (int)gridDim.x;
-  if (u < U) {
-    int b = 0, par = 0;
+  // Few units: several CTAs share the K of each, and the last of them to arrive sums their parts in order.  A unit moves 32 KB per 1024 of K
+  // into its SM, beside the base tiles that every SM takes in at its full rate, in batches that wait for one another: with one row in the step
+  // the one to three CTAs that had a unit were done 10 us (K = 4096) to 21 us (14336) behind the wait, and every tile's expand waited for them.
+  int parts = 1;
+  if (NG == 1 && p.lora_kparts != nullptr && U > 0) parts = max(1, min((int)gridDim.x / U, nbatch));
+  const int total = U * parts;
+  int x = (int)blockIdx.x;
+  if (x < total) {
+    ShrinkUnit cur;
+    decode_shrink_unit(p, ents, gstart, x / parts, x % parts, parts, nbatch, kUnitRows, cur);
+    int b = cur.b0, par = 0;
     uint4 ra[SB], rb[SB], rx[NG][SB];
-    shrink_loads<NG, SB>(p, cur, 0, ewarp, lane, ra, rb, rx);
+    shrink_loads<NG, SB>(p, cur, b, ewarp, lane, ra, rb, rx);
     float acc[NG][4];
 #pragma unroll
     for (int q = 0; q < NG; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
     while (true) {
       // the batch after this one: the next of the unit, or the first of the CTA's next unit
       ShrinkUnit nxt = cur;
-      int nb = b + 1, nu = u;
+      int nb = b + 1;
       bool more = true;
-      if (nb == nbatch) {
-        nb = 0;
-        nu = u + (int)gridDim.x;
-        while (nu < U && !decode_shrink_unit(p, ents, gstart, nu, nblk, kUnitRows, nxt)) nu += (int)gridDim.x;
-        more = nu < U;
+      if (nb == cur.b1) {
+        x += (int)gridDim.x;
+        more = x < total;
+        if (more) {
+          decode_shrink_unit(p, ents, gstart, x / parts, x % parts, parts, nbatch, kUnitRows, nxt);
+          nb = nxt.b0;
+        }
       }
       uint4 na[SB], nbv[SB], nx[NG][SB];
       if (more) shrink_loads<NG, SB>(p, nxt, nb, ewarp, lane, na, nbv, nx);
@@ -382,7 +418,7 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
           }
         }
       }
-      if (b == nbatch - 1) {
+      if (b == cur.b1 - 1) {
         // the unit is complete: 16 ranks x up to 8 rows per group.  This warp holds (rank g, rows 2t, 2t+1) and (rank g + 8, same
         // rows) of every group; the groups go through the two staging buffers one after the other.
         const LoraEnt e = ents[cur.lt];
@@ -402,7 +438,9 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
             mine[(g + 8) * 8 + 2 * t] = acc[q][2];
             mine[(g + 8) * 8 + 2 * t + 1] = acc[q][3];
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (tid4 < 2 * ntg) {
+            bool whole = true;
+            if (NG == 1 && parts > 1) whole = lora_join_kparts(p, cur, parts, red + par * 4 * 128, reinterpret_cast<int*>(red + 2 * 4 * 128), tid4);
+            if (whole && tid4 < 2 * ntg) {
               // thread -> (row rq of the group, 8 ranks ch): one 16-byte chunk of the image
               const int rq = tid4 >> 1, ch = tid4 & 1;
               const float* r0 = red + par * 4 * 128;
@@ -420,7 +458,7 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
             const int z_lo = (t0g == e.row0) ? e.row0 - w0 : 0;
             const int z_hi = (t0g + ntg == e.row0 + e.nrows) ? e.row0 + e.nrows - w0 : wn;
             const int zrows = z_lo + (wn - z_hi);
-            if (tid4 >= 32 && tid4 - 32 < 2 * zrows) {
+            if (whole && tid4 >= 32 && tid4 - 32 < 2 * zrows) {
               const int cz = (tid4 - 32) >> 1, ch = (tid4 - 32) & 1;
               const int row = cz < z_lo ? cz : z_hi + (cz - z_lo);
               *reinterpret_cast<uint4*>(img + row * 16 + (ch << 3)) = make_uint4(0, 0, 0, 0);
@@ -431,7 +469,7 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
         }
       }
       if (!more) break;
-      cur = nxt; b = nb; u = nu;
+      cur = nxt; b = nb;
 #pragma unroll
       for (int i = 0; i < SB; ++i) {
         ra[i] = na[i]; rb[i] = nbv[i];
@@ -597,7 +635,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   int* n_live = reinterpret_cast<int*>(tmem_base_slot + 3);             // live entries of the LoRA table
   LoraEnt* ents = reinterpret_cast<LoraEnt*>(smem + STAGES * S::kStageBytes + S::kBarrierBytes);
   LoraUnit* ulist_p = reinterpret_cast<LoraUnit*>(ents + kLoraMaxEntries);      // producer warp's expand units of the current token tile
-  unsigned short* gstart = reinterpret_cast<unsigned short*>(ulist_p + kLoraListCap);   // [entries + 1] four-row groups before an entry
+  unsigned short* gstart = reinterpret_cast<unsigned short*>(ulist_p + kLoraListCap);   // [entries + 1] shrink units before an entry
   __nv_bfloat16* epi_stage = reinterpret_cast<__nv_bfloat16*>(smem + STAGES * S::kStageBytes + S::kBarrierBytes + S::kEntBytes);
 
   const int warp = threadIdx.x >> 5;
@@ -642,7 +680,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       if (!p.lora_tables_const) pdl_wait();
       load_lora_entries(p, ents, n_live);
       __syncthreads();
-      if (p.lora_inline_shrink && warp == 2) lora_group_prefix(p, ents, gstart);
+      if (p.lora_inline_shrink && warp == 2) lora_unit_prefix(p, ents, gstart);
       if (warp == 0 && !(p.lora_skip & 2)) {
         // the producer warp builds the unit list of its first tile now, under the tail of the kernel in front, and pulls that
         // tile's B_cat rows (adapter weights, which no kernel of the step writes) into L2
@@ -1655,9 +1693,10 @@ struct LxLoraFused {
   int fence_maps;
   const void* arena; long long off_a;      // A_cat of the group and layer: arena + slot_base + rank * off_a (elements)
   long long off_b, arena_elems;            // B_cat likewise; the arena's size bounds the arena-wide maps
-  int* sync;                               // two ints, zero before the first launch (see GemmParams::lora_sync)
+  int* sync;                               // zero before the first launch: two ints (see GemmParams::lora_sync), then lora_kcounters
   int w_const;                             // 1: the kernel in front on the stream does not write w (mode bit 16 of lx_gemm_bf16)
   int tables_const;                        // 1: nor tiles, slot_rank, slot_base, the maps and the arena (in a step copies do)
+  int sync_ints;                           // ints at sync
 };
 
 static int gemm_impl(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
@@ -1768,11 +1807,16 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     p.lora_arena = reinterpret_cast<const __nv_bfloat16*>(lora->arena);
     p.lora_x = reinterpret_cast<const __nv_bfloat16*>(x);
     p.lora_ldx = ldx;
-    p.lora_max_r = lora->nparts * lora->max_rank;
     p.lora_sync = lora->sync;
     // the epilogue warps compute the shrink when every CTA of the launch is resident at once (the expand stages wait for all of
     // them) and the arena-wide maps give the entries their offsets; otherwise a launch in front does
     p.lora_inline_shrink = (lora->sync != nullptr && p.lora_arena_maps && pl.grid <= num_sms && !(p.lora_skip & 1)) ? 1 : 0;
+    // sums of shared shrink units go behind the operand images
+    const long long img_bytes = (long long)lora->num_tiles * lora->nparts * kLoraImgElems * 2;
+    if (lora->sync_ints >= 2 + pl.grid && lora->vimg_bytes - img_bytes >= (long long)pl.grid * 128 * 4) {
+      p.lora_kparts = reinterpret_cast<float*>(static_cast<char*>(lora->vimg) + img_bytes);
+      p.lora_kcounters = lora->sync + 2;
+    }
     {
       const char* e = getenv("LORAX_LORA_INLINE_SHRINK");       // measurement only
       if (e && atoi(e) == 0) p.lora_inline_shrink = 0;

@@ -71,7 +71,7 @@ struct LxLoraFused {
   const void* arena; long long off_a;
   long long off_b, arena_elems;
   int* sync;
-  int w_const, tables_const;
+  int w_const, tables_const, sync_ints;
 };
 int lx_gemm_bf16_lora(const void* x, const void* w, void* out, const void* bias, int T, int N, int K, long long ldx,
                       long long ldw, long long ldo, void* ws, long long ws_bytes, int* counters, int* status, int num_sms,
@@ -128,7 +128,7 @@ struct LxModelDesc {
   // scratch of the GEMM that carries LoRA in its own launch
   void* lora_vimg; long long lora_vimg_bytes; long long arena_elems; int* lora_sync; int lora_fence_maps;
   int tc_prefill, kv_blocks;     // tensor-core prefill attention where the shape allows; blocks of the paged cache
-  int kv_fp8, pad3_;             // the cache holds e4m3 bytes
+  int kv_fp8, lora_sync_ints;    // the cache holds e4m3 bytes; ints at lora_sync
 };
 
 struct LxStepDesc {
@@ -168,7 +168,7 @@ int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDes
     f.slot_rank = m.slot_rank; f.slot_base = m.slot_base; f.num_slots = m.num_slots;
     f.nparts = site.nparts; f.n0 = site.n0; f.n1 = site.n1; f.layer = l.layer_index; f.max_rank = m.max_rank;
     f.vimg = m.lora_vimg; f.vimg_bytes = m.lora_vimg_bytes; f.fence_maps = m.lora_fence_maps;
-    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync; f.w_const = f.tables_const = 1;
+    f.arena = m.arena; f.off_a = site.off_a; f.off_b = site.off_b; f.arena_elems = m.arena_elems; f.sync = m.lora_sync; f.sync_ints = m.lora_sync_ints; f.w_const = f.tables_const = 1;
     const int rc = lx_gemm_bf16_lora(x, w, y, bias, s.T, N, K, ldx, ldw, ldy, m.gemm_ws, m.gemm_ws_bytes, m.gemm_counters, m.status, m.num_sms,
                                      &f, stream);
     if (rc != 1) return rc;          // 1: this step does not fit the fused launch, use the separate kernels below

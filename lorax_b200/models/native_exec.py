@@ -48,7 +48,7 @@ class LxModelDesc(Structure):
                 ("arena", P), ("slot_base", P), ("slot_rank", P), ("slot_tmaps", P),
                 ("num_slots", I), ("max_rank", I), ("groups_per_slot", I), ("fused_lora", I),
                 ("lora_vimg", P), ("lora_vimg_bytes", L), ("arena_elems", L), ("lora_sync", P), ("lora_fence_maps", I),
-                ("tc_prefill", I), ("kv_blocks", I), ("kv_fp8", I), ("pad3_", I)]
+                ("tc_prefill", I), ("kv_blocks", I), ("kv_fp8", I), ("lora_sync_ints", I)]
 
 
 class LxStepDesc(Structure):
@@ -141,7 +141,7 @@ class NativeExecutor:
             m.fused_lora = int(model.fused_lora_max_tokens)        # rows up to which LoRA rides inside the GEMM launch
             m.lora_vimg, m.lora_vimg_bytes = ws.lora_vimg.data_ptr(), ws.lora_vimg.numel() * 2
             m.arena_elems = ad.arena.numel()
-            m.lora_sync = ws.lora_sync.data_ptr()
+            m.lora_sync, m.lora_sync_ints = ws.lora_sync.data_ptr(), ws.lora_sync.numel()
             m.lora_fence_maps = native.LORA_FENCE_MAPS
         self.m = m
         self.layers = (LxLayerDesc * len(model.layers))()

@@ -169,13 +169,14 @@ class Workspace:
         # LoRA expand inside the GEMM launch: bf16 operand images of the shrink results (6 KB per table entry and part)
         self.lora_max_entries = 1024
         self.lora_vimg = torch.zeros(self.lora_max_entries * 3 * 48 * 64, dtype=torch.bfloat16, device=device)
-        self.lora_sync = torch.zeros(2, dtype=torch.int32, device=device)       # launch-wide counters of the in-kernel shrink
         self.fp8_scratch = None              # bf16 image of one fp8 projection (long prefills), allocated on first use
         self.attn_part_tokens = 256
         self.attn_splits = attn_splits
         self.attn_part_o = torch.empty(self.attn_part_tokens * num_heads * attn_splits * head_dim, dtype=torch.float32, device=device)
         self.attn_part_lse = torch.empty(self.attn_part_tokens * num_heads * attn_splits, dtype=torch.float32, device=device)
         self.num_sms = torch.cuda.get_device_properties(device).multi_processor_count
+        # counters of the in-kernel shrink: two of the launch, one per unit whose K several CTAs share (at most one CTA per SM)
+        self.lora_sync = torch.zeros(2 + self.num_sms, dtype=torch.int32, device=device)
 
     def attn_parts(self, wanted: int, rows: int, heads: int, d: int) -> int:
         """Parts of a row's keys (at most `wanted`) whose sums the scratch holds for `rows` rows of `heads` heads of `d`."""
@@ -246,7 +247,7 @@ class LxLoraFused(ctypes.Structure):
                 ("fence_maps", ctypes.c_int),
                 ("arena", ctypes.c_void_p), ("off_a", ctypes.c_longlong),
                 ("off_b", ctypes.c_longlong), ("arena_elems", ctypes.c_longlong), ("sync", ctypes.c_void_p),
-                ("w_const", ctypes.c_int), ("tables_const", ctypes.c_int)]
+                ("w_const", ctypes.c_int), ("tables_const", ctypes.c_int), ("sync_ints", ctypes.c_int)]
 
 
 class LoraFused(NamedTuple):
@@ -280,7 +281,7 @@ def lora_fused_desc(ws: "Workspace", lf: LoraFused, K: int) -> LxLoraFused:
     d.vimg, d.vimg_bytes = ws.lora_vimg.data_ptr(), ws.lora_vimg.numel() * 2
     d.arena, d.off_a = (lf.arena.data_ptr() if lf.arena is not None else None), lf.off_a
     d.off_b, d.arena_elems = lf.off_b, (lf.arena.numel() if lf.arena is not None else 0)
-    d.sync = ws.lora_sync.data_ptr()
+    d.sync, d.sync_ints = ws.lora_sync.data_ptr(), ws.lora_sync.numel()
     d.fence_maps = LORA_FENCE_MAPS
     d.tables_const = int(lf.tables_const)
     return d

@@ -863,6 +863,14 @@ def test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout):
         assert _rel_err(got[untouched], base[untouched]) < 1e-6
 
 
+@pytest.mark.parametrize("T,K,parts,ranks,layout", [(2, 4096, [512, 128, 128], [16], "alternating"), (2, 14336, [512], [64], "alternating"),
+                                                    (5, 3080, [768, 768], [16, 64, 32, 48], "alternating"), (6, 1000, [512], [32, 16], "alternating"),
+                                                    (29, 4096, [4096, 1024, 1024], [16, 32], "runs"), (90, 2048, [512], [16], "runs")])
+def test_gemm_with_lora_of_few_units(nat, T, K, parts, ranks, layout):
+    """Steps with fewer shrink units than CTAs, which share the K of each: one row, K of a part of a batch and of a ragged last one."""
+    test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
+
+
 @pytest.mark.parametrize("T,E,k,H,I,e0,e_local", [(7, 8, 2, 512, 256, 0, 8), (256, 8, 2, 1024, 768, 0, 8), (300, 8, 2, 512, 256, 2, 2),
                                                   (1500, 16, 4, 256, 128, 0, 16), (64, 4, 1, 256, 384, 1, 1)])
 def test_moe_ffn_on_the_device(nat, T, E, k, H, I, e0, e_local):
