@@ -353,8 +353,7 @@ struct DecodeParams {
 // DK, DV: widths of keys and values (a page of one head holds its key plane, then its value plane).
 template <int DK, int DV, int STAGES, bool KV8, int NW, bool WIDE = false>
 __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams p) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+  pdl_wait_ahead();      // every block waits, also those that return early below
   extern __shared__ __align__(1024) uint8_t dsm[];
   static_assert(!KV8 || DK == DV, "e4m3 pages hold keys and values of one width");
   constexpr int PLANE = kPage * DK * 2, VPLANE = kPage * DV * 2;
@@ -525,8 +524,7 @@ template <int D>
 __global__ void __launch_bounds__(D) attn_combine_kernel(const float* part_o, const float* part_lse,
                                                          __nv_bfloat16* __restrict__ out, long long ldo, int nh, int nsplit,
                                                          const AttnTail tail, const int* ctx_lens) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+  pdl_wait_ahead();      // every block waits, also those that return early below
   const int t = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)t * nh + h) * nsplit;
   float M = -INFINITY;

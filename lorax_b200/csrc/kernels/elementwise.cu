@@ -28,8 +28,7 @@ norm_residual_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ residua
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                      __nv_bfloat16* __restrict__ out, int H, long long ldx, long long ldr, long long ldo, float eps,
                      float w_offset, float x_scale) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+  pdl_wait_ahead();      // every block waits, also those that return early below
   const int row = blockIdx.x;
   const int nvec = H / 8;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
@@ -157,8 +156,7 @@ __global__ void __launch_bounds__(256)
 rope_kvwrite_kernel(__nv_bfloat16* __restrict__ qkv, const int* positions, const float* __restrict__ cos_sin,
                     __nv_bfloat16* __restrict__ kv_cache, const int* slots, int nh, int nkv, int d, int rot,
                     int page, long long ldq, int apply_rope, int kv_fp8, float k_inv_scale, float v_inv_scale) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+  pdl_wait_ahead();      // every block waits, also those that return early below
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int slot = slots ? slots[t] : -1;
@@ -257,8 +255,7 @@ LX_DEVICE float act_fn(float x) {
 template <int ACT, bool GATED>
 __global__ void __launch_bounds__(256)
 act_mul_kernel(const __nv_bfloat16* in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec) {
-  pdl_wait();      // every block waits, also those that return early below
-  pdl_trigger();
+  pdl_wait_ahead();      // every block waits, also those that return early below
   const int vec_per_row = I / 8;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total_vec; v += (long long)gridDim.x * blockDim.x) {
     const long long t = v / vec_per_row;
