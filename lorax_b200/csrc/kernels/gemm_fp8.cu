@@ -17,7 +17,7 @@
 // block), tokens the N side in tiles of up to 128.
 #include <cuda_fp8.h>
 
-#include "common.cuh"
+#include "lora_add.cuh"
 
 namespace lx {
 
@@ -280,6 +280,94 @@ __global__ void __launch_bounds__(256) fp8_splitk_reduce_kernel(const float* par
   out[(long long)t * ldo + n] = __float2bfloat16(a);
 }
 
+// The same with the step's adapters: y[t, n] = bf16(sum_s partial[s, t, n] + bias[n] + delta), or without parts (ksplit 0) y += delta.
+// A warp takes 128 features of `run` rows one after the other.  Their B_cat rows lie end to end: lanes side by side read 16 bytes, eight ranks,
+// side by side (a lane with whole rows of its own features touches 32 lines per load: 19 us for 28672 features of 32 rows, rank 32), and the
+// two to eight lanes of a feature join their sums.  Those of the warp's first row are loaded before the wait for the product.
+// The reduction and the expand as launches of their own took 12 to 20 us a projection at 32 rows of 24 adapters.
+constexpr int kAddWarps = 8, kAddAhead = 8;
+__global__ void __launch_bounds__(32 * kAddWarps) lora_add_kernel(const LxLoraAdd a, const float* partial, int ksplit, int T, int N, int run,
+                                                                  const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* out, long long ldo) {
+  __shared__ LoraAddRow rows[kLoraAddRows];
+  __shared__ __align__(16) float deltas[kAddWarps][128];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, f0 = blockIdx.x * 128, n = f0 + lane * 4;
+  const int t_lo = (blockIdx.y * kAddWarps + warp) * run, t_hi = min(t_lo + run, T);
+  if (!a.tables_const) pdl_wait();
+  lora_add_rows(a, T, rows);
+  const int part = lora_add_part(a, f0);
+  uint4 bw[kAddAhead];
+  // loads i0 .. i0 + 7 of the 128 features: 2^sh lanes a feature, those past the rank idle
+  auto load_b = [&](const LoraAddRow& q, int sh, int i0) {
+    const int c = lane & ((1 << sh) - 1);
+#pragma unroll
+    for (int i = 0; i < kAddAhead; ++i) {
+      const int f = ((i0 + i) << (5 - sh)) + (lane >> sh);
+      const __nv_bfloat16* B = q.b + (long long)(f0 + f) * q.r + c * 8;
+      bw[i] = f0 + f < N && c * 8 < q.r ? __ldg(reinterpret_cast<const uint4*>(B + 0)) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto lanes = [](int r) { return r <= 16 ? 1 : r <= 32 ? 2 : r <= 64 ? 3 : r <= 128 ? 4 : 5; };      // log2 of a feature's lanes
+  if (t_lo < t_hi && rows[t_lo].r > 0) load_b(rows[t_lo], lanes(rows[t_lo].r), 0);
+  pdl_wait();      // every block waits, also those that have nothing to do
+  pdl_trigger();
+  for (int t = t_lo; t < t_hi; ++t) {
+    const LoraAddRow q = rows[t];
+    if (ksplit == 0 && q.r == 0) continue;
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+    __nv_bfloat16* at = out + (long long)t * ldo + n;
+    if (n < N) {                       // N is a multiple of four
+      if (ksplit == 0) {
+        const uint2 old = *reinterpret_cast<const uint2*>(at);
+        const float2 o0 = unpack_bf16x2(old.x), o1 = unpack_bf16x2(old.y);
+        y[0] = o0.x; y[1] = o0.y; y[2] = o1.x; y[3] = o1.y;
+      }
+#pragma unroll 4
+      for (int s = 0; s < ksplit; ++s) {
+        const float4 p4 = __ldcg(reinterpret_cast<const float4*>(partial + ((long long)s * T + t) * N + n));
+        y[0] += p4.x; y[1] += p4.y; y[2] += p4.z; y[3] += p4.w;
+      }
+      if (ksplit > 0 && bias != nullptr) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) y[c] += __bfloat162float(bias[n + c]);
+      }
+    }
+    if (q.r > 0) {
+      const int sh = lanes(q.r), c = lane & ((1 << sh) - 1);
+      float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
+      if (c * 8 < q.r) {
+        const float* vv = a.v + (long long)t * a.ldv + part * q.r + c * 8;
+        v0 = *reinterpret_cast<const float4*>(vv);
+        v1 = *reinterpret_cast<const float4*>(vv + 4);
+      }
+      for (int i0 = 0; i0 < (4 << sh); i0 += kAddAhead) {      // 128 features, 32 >> sh at a time
+        if (t > t_lo || i0 > 0) load_b(q, sh, i0);
+#pragma unroll
+        for (int i = 0; i < kAddAhead; ++i) {
+          float d = lora_dot8(bw[i], v0, v1, 0.f);
+          for (int m = 1; m < (1 << sh); m <<= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+          if (c == 0) deltas[warp][((i0 + i) << (5 - sh)) + (lane >> sh)] = d;
+        }
+      }
+      __syncwarp();
+      const float4 d4 = *reinterpret_cast<const float4*>(&deltas[warp][lane * 4]);
+      y[0] += d4.x; y[1] += d4.y; y[2] += d4.z; y[3] += d4.w;
+      __syncwarp();
+    }
+    if (n < N) *reinterpret_cast<uint2*>(at) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
+  }
+}
+
+static int launch_lora_add(const LxLoraAdd& a, const float* partial, int ksplit, int T, int N, const __nv_bfloat16* bias, __nv_bfloat16* out,
+                           long long ldo, int num_sms, cudaStream_t stream) {
+  // rows per warp: as many as leave four blocks an SM
+  const int col_blocks = (N + 127) / 128;
+  int run = (int)((long long)col_blocks * T / (kAddWarps * 4ll * num_sms));
+  run = run < 1 ? 1 : run > 32 ? 32 : run;
+  launch_pdl(lora_add_kernel, dim3(col_blocks, (T + kAddWarps * run - 1) / (kAddWarps * run)), dim3(32 * kAddWarps), 0, stream, a, partial, ksplit, T, N, run,
+             bias, out, ldo);
+  return -(int)cudaGetLastError();
+}
+
 typedef CUresult (*EncodeTiledFn3)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -336,12 +424,20 @@ int lx_quant_act_fp8(const void* x, long long ldx, void* xq, long long ldq, floa
 }
 
 // out[T, N] (bf16) = block-scaled fp8 product of xq[T, K] (scales sa[kb, t]) and wq[N, K] (scales sw[N/128, K/128]) + bias.
-// w_const: the kernel in front on the stream does not write wq.
+// w_const: the kernel in front on the stream does not write wq.  add (nullptr: none): the step's adapters, for at most lx_lora_add_max_rows()
+// rows, N a multiple of four and parts of multiples of 128; their shrink is in front on the stream.
+int lx_lora_add_max_rows() { return lx::kLoraAddRows; }
+int lx_lora_add(const LxLoraAdd* add, void* y, long long ldy, int T, int N, int num_sms, void* stream) {
+  if (T <= 0 || N <= 0) return 0;
+  if (add == nullptr || T > lx::kLoraAddRows || N % 4 != 0 || ldy % 4 != 0 || (add->n0 < N && add->n0 % 128 != 0) || (add->n1 < N && add->n1 % 128 != 0)) return -1;
+  return lx::launch_lora_add(*add, nullptr, 0, T, N, nullptr, reinterpret_cast<__nv_bfloat16*>(y), ldy, num_sms, reinterpret_cast<cudaStream_t>(stream));
+}
 int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_sa, const void* wq, long long ldw, const float* sw,
                          void* out, long long ldo, const void* bias, int T, int N, int K, void* ws, long long ws_bytes, int* status,
-                         int num_sms, int w_const, void* stream_) {
+                         int num_sms, int w_const, const LxLoraAdd* add, void* stream_) {
   using namespace lx;
   if (T <= 0 || N <= 0) return 0;
+  if (add != nullptr && (T > kLoraAddRows || N % 4 != 0 || ldo % 4 != 0 || (add->n0 < N && add->n0 % 128 != 0) || (add->n1 < N && add->n1 % 128 != 0))) return -1001;
   if (K % 16 != 0 || ldq % 16 != 0 || ldw % 16 != 0) return -1000;
   Fp8Params p{};
   p.N = N; p.T = T; p.K = K;
@@ -374,7 +470,9 @@ int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_
   if (bn <= 32) rc = launch_fp8<32, 8>(tw, tx, p, grid, stream);
   else if (bn <= 64) rc = launch_fp8<64, 8>(tw, tx, p, grid, stream);
   else rc = launch_fp8<128, 6>(tw, tx, p, grid, stream);
-  if (rc != 0 || ks == 1) return rc;
+  if (rc != 0) return rc;
+  if (add != nullptr) return launch_lora_add(*add, p.partial, ks == 1 ? 0 : ks, T, N, p.bias, p.out, ldo, num_sms, stream);
+  if (ks == 1) return rc;
   const long long total = (long long)T * N;
   launch_pdl(fp8_splitk_reduce_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, p.partial, ks, T, N, p.bias, p.out, ldo);
   return -(int)cudaGetLastError();

@@ -24,7 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "common.cuh"
+#include "lora_add.cuh"
 
 namespace lx {
 
@@ -110,6 +110,7 @@ struct Wq4Params {
   long long ldx, ldo;
   int T, N, K, group;
   int w_const;                 // the kernel in front on the stream does not write the codes: they are read before the wait for it
+  LxLoraAdd add;               // add.tiles != nullptr: the step's adapters, added to the sums before they are rounded
 };
 
 LX_DEVICE void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -163,6 +164,7 @@ LX_DEVICE Wq4Group wq4_group(__half2 szv) {
 template <int NT, int MT, bool EXACT>                  // token tiles of 8, row tiles of 16
 __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Params p) {
   __shared__ float red[kWqWarps][kWqRows * MT][8 * NT + 1];
+  constexpr int kRows = kWqRows * MT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * kWqRows * MT;
@@ -202,6 +204,18 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
   if (!p.w_const) pdl_wait();
 #pragma unroll
   for (int d = 0; d < AHEAD; ++d) fetch(kb + d * kWqWarps, d);
+  // B_cat of the row whose results this thread will form, as it will walk them below, on its way into L2
+  constexpr int kOuts = (kRows * 8 * NT + kWqWarps * 32 - 1) / (kWqWarps * 32);
+  LoraAddRow lrow[kOuts];
+  if (p.add.tiles != nullptr) {
+    if (p.w_const && !p.add.tables_const) pdl_wait();
+#pragma unroll
+    for (int i = 0; i < kOuts; ++i) {
+      const int o = threadIdx.x + i * kWqWarps * 32;
+      lrow[i] = lora_add_row32(p.add, o / kRows);
+      if (lrow[i].r > 0 && o / kRows < p.T) asm volatile("prefetch.global.L2 [%0];" ::"l"(lrow[i].b + (long long)(n0 + o % kRows) * lrow[i].r) : "memory");
+    }
+  }
   if (p.w_const) pdl_wait();
   pdl_trigger();
   uint4 nx[4];
@@ -286,14 +300,25 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
     }
   }
   __syncthreads();
-  constexpr int kRows = kWqRows * MT;
-  for (int o = threadIdx.x; o < kRows * 8 * NT; o += kWqWarps * 32) {
+#pragma unroll
+  for (int i = 0; i < kOuts; ++i) {
+    const int o = threadIdx.x + i * kWqWarps * 32;
+    if (o >= kRows * 8 * NT) break;
     const int tok = o / kRows, r = o % kRows;          // neighbouring threads write neighbouring features of one token
     if (tok < p.T) {
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < kWqWarps; ++w) v += red[w][r][tok];
       if (p.bias != nullptr) v += __bfloat162float(p.bias[n0 + r]);
+      if (p.add.tiles != nullptr && lrow[i].r > 0) {
+        const LoraAddRow q = lrow[i];
+        const __nv_bfloat16* B = q.b + (long long)(n0 + r) * q.r;
+        const float* vv = p.add.v + (long long)tok * p.add.ldv + lora_add_part(p.add, n0 + r) * q.r;
+        float delta = 0.f;
+        for (int j = 0; j < q.r; j += 8)
+          delta = lora_dot8(__ldg(reinterpret_cast<const uint4*>(B + j)), *reinterpret_cast<const float4*>(vv + j), *reinterpret_cast<const float4*>(vv + j + 4), delta);
+        v += delta;
+      }
       p.out[tok * p.ldo + n0 + r] = __float2bfloat16(v);
     }
   }
@@ -329,8 +354,12 @@ int lx_wq4_max_tokens() { return 32; }
 
 // out[T, N] = x[T, K] . W^T (+ bias) for T <= 32 from affine 4-bit codes.  N % 16 == 0, K % 128 == 0, group % 32 == 0, x rows
 // 16-byte aligned.
+int lx_wq4_gemm_lora(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
+                     int K, int group, int flags, const LxLoraAdd* add, void* stream);
 int lx_wq4_gemm_ex(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
-                   int K, int group, int flags, void* stream);
+                   int K, int group, int flags, void* stream) {
+  return lx_wq4_gemm_lora(x, ldx, codes, sz, bias, out, ldo, T, N, K, group, flags, nullptr, stream);
+}
 
 int lx_wq4_gemm(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
                 int K, int group, void* stream) {
@@ -339,13 +368,15 @@ int lx_wq4_gemm(const void* x, long long ldx, const void* codes, const void* sz,
 
 // `flags` bit 0 promises that every zero point is an integer (GPTQ, AWQ, round-to-nearest; not HQQ): with groups that are
 // multiples of 128 the kernel then multiplies exact integers and scales the partial sums (see EXACT above).  Bit 1: the kernel in front
-// on the stream does not write the codes, scales and zero points, which are then read while it still runs.
-int lx_wq4_gemm_ex(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
-                   int K, int group, int flags, void* stream) {
+// on the stream does not write the codes, scales and zero points, which are then read while it still runs.  `add`: the step's adapters (nullptr:
+// none), whose shrink is in front on the stream.  An expand launch behind the product cost 5 us of its own per projection.
+int lx_wq4_gemm_lora(const void* x, long long ldx, const void* codes, const void* sz, const void* bias, void* out, long long ldo, int T, int N,
+                     int K, int group, int flags, const LxLoraAdd* add, void* stream) {
   using namespace lx;
   if (T <= 0 || T > 32 || N % kWqRows != 0 || K % 128 != 0 || group % 32 != 0 || K % group != 0 || ldx % 8 != 0) return -1;
   Wq4Params p{static_cast<const uint8_t*>(codes), static_cast<const __half2*>(sz), static_cast<const __nv_bfloat16*>(x),
-              static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), ldx, ldo, T, N, K, group, (flags >> 1) & 1};
+              static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), ldx, ldo, T, N, K, group, (flags >> 1) & 1,
+              add != nullptr ? *add : LxLoraAdd{}};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // two row tiles per warp halve the re-reads of the activations (every block reads all of x); with few rows and few tokens
   // the larger grid of single tiles fills the machine better

@@ -457,10 +457,12 @@ class DecoderModel:
         self.quantized = method
         self._native = None
 
-    def _gemm(self, x, w, b, out=None):
+    def _gemm(self, x, w, b, out=None, lora=None):
+        """`lora`: for quantised weights on a GPU, what the shrink returned and the step's tile table: the delta is added with the result."""
+        more = {} if lora is None else dict(lora=lora)
         if isinstance(w, GroupQuantWeight):
             xb = x if x.dtype == torch.bfloat16 or not x.is_cuda else x.to(torch.bfloat16)
-            y = self.ops.gemm_wq(xb, w, bias=b, out=out if out is not None and out.dtype == xb.dtype else None, w_const=True)
+            y = self.ops.gemm_wq(xb, w, bias=b, out=out if out is not None and out.dtype == xb.dtype else None, w_const=True, **more)
             if out is not None and y is not out:
                 out.copy_(y)
                 return out
@@ -468,7 +470,7 @@ class DecoderModel:
         if out is not None and isinstance(w, torch.Tensor):
             return self.ops.gemm(x, w, bias=b, out=out, w_const=True)
         if isinstance(w, Fp8Weight):
-            y = self.ops.gemm_fp8(x if x.dtype == torch.bfloat16 or not x.is_cuda else x.to(torch.bfloat16), w.q, w.scale, bias=b)
+            y = self.ops.gemm_fp8(x if x.dtype == torch.bfloat16 or not x.is_cuda else x.to(torch.bfloat16), w.q, w.scale, bias=b, **more)
             return y if y.dtype == x.dtype else y.to(x.dtype)
         return self.ops.gemm(x, w, bias=b, w_const=True)
 
@@ -493,6 +495,9 @@ class DecoderModel:
             epi = self.adapters.shrink(self.ops, x, ts, group, layer, tiles=inp.lora_tiles)
         if epi is None:
             return self._gemm(x, w, b, out=out)
+        if x.is_cuda and x.dtype == torch.bfloat16 and inp.lora_tiles is not None and isinstance(w, (GroupQuantWeight, Fp8Weight)) \
+                and self.ops.lora_short_step(x.shape[0], inp.lora_tiles.max_rows):
+            return self._gemm(x, w, b, out=out, lora=(epi, inp.lora_tiles))
         y = self._gemm(x, w, b, out=out)
         self.adapters.expand(self.ops, epi, y, tiles=inp.lora_tiles)
         return y

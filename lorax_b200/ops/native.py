@@ -96,11 +96,14 @@ def load() -> ctypes.CDLL:
         "lx_gemm_bf16_lora": ([P, P, P, P, I, I, I, L, L, L, P, L, P, P, I, P, P], I),
         "lx_lora_fused_desc_bytes": ([], I),
         "lx_quant_act_fp8": ([P, L, P, L, P, I, I, I, P], I),
-        "lx_gemm_fp8_block128": ([P, L, P, I, P, L, P, P, L, P, I, I, I, P, L, P, I, I, P], I),
+        "lx_gemm_fp8_block128": ([P, L, P, I, P, L, P, P, L, P, I, I, I, P, L, P, I, I, P, P], I),
+        "lx_lora_add_max_rows": ([], I),
+        "lx_lora_add": ([P, P, L, I, I, I, P], I),
         "lx_fp8_block128_dequant": ([P, L, P, I, P, L, I, I, P], I),
         "lx_wq_dequant": ([P, P, P, P, L, I, I, I, I, P], I),
         "lx_wq4_gemm": ([P, L, P, P, P, P, L, I, I, I, I, P], I),
         "lx_wq4_gemm_ex": ([P, L, P, P, P, P, L, I, I, I, I, I, P], I),
+        "lx_wq4_gemm_lora": ([P, L, P, P, P, P, L, I, I, I, I, I, P, P], I),
         "lx_lora_expand_tiled": ([P, I, L, I, P, I, I, P, P, P, I, L, P, L, I, I, I, I, P, I, P], I),
         "lx_attn_prefill_tc_supported": ([I, I, I, L, L], I),
         "lx_attn_prefill_tc": ([P, L, I, P, I, P, I, P, P, P, P, I, P, L, I, I, I, I, F, F, P, I, P, P], I),
@@ -223,6 +226,20 @@ class LoraEpilogue(NamedTuple):
     unit_off: int
     n0: int
     n1: int
+
+
+class LxLoraAdd(ctypes.Structure):
+    """Mirror of the C struct of the same name (csrc/kernels/lora_add.cuh)."""
+    _fields_ = [("tiles", ctypes.c_void_p), ("num_tiles", ctypes.c_int), ("num_slots", ctypes.c_int), ("arena", ctypes.c_void_p),
+                ("slot_base", ctypes.c_void_p), ("slot_rank", ctypes.c_void_p), ("unit_off", ctypes.c_longlong), ("v", ctypes.c_void_p),
+                ("ldv", ctypes.c_int), ("n0", ctypes.c_int), ("n1", ctypes.c_int), ("tables_const", ctypes.c_int), ("status", ctypes.c_void_p)]
+
+
+def lora_add_desc(epi: LoraEpilogue, tiles, tables_const: bool) -> LxLoraAdd:
+    """The second half of a short step's LoRA for the launch that forms a product's results; `tiles`: the step's table (`LoraTiles`)."""
+    return LxLoraAdd(tiles.table.data_ptr(), tiles.num_tiles, epi.slot_rank.shape[0], epi.arena.data_ptr(), epi.slot_base.data_ptr(),
+                     epi.slot_rank.data_ptr(), epi.unit_off, epi.v.data_ptr(), epi.v.stride(0), epi.n0, epi.n1, int(tables_const),
+                     workspace(epi.v.device).status.data_ptr())
 
 
 # 1 (default): the GEMM that carries LoRA acquire-fences a slot's B_cat tensor map before every use, as a tensor map that lives
@@ -456,9 +473,10 @@ def fp8_expand(wq: torch.Tensor, w_scale: torch.Tensor) -> Optional[torch.Tensor
 
 
 def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Optional[torch.Tensor] = None,
-             out: Optional[torch.Tensor] = None) -> torch.Tensor:
+             out: Optional[torch.Tensor] = None, lora=None) -> torch.Tensor:
     """out[T, N] = x[T, K] @ dequant(wq[N, K], w_scale[N/128, K/128])^T (+ bias): activations are quantised to e4m3 per
-    token and 128-wide K block on the fly, the product runs on the fp8 tensor cores, bf16 out."""
+    token and 128-wide K block on the fly, the product runs on the fp8 tensor cores, bf16 out.  `lora`: (what the shrink returned, the step's
+    tile table), added to the result; copies in front of the step wrote the table and the adapters."""
     assert x.dtype == torch.bfloat16 and wq.dtype in (torch.uint8, torch.float8_e4m3fn) and w_scale.dtype == torch.float32
     T, K = x.shape
     N = wq.shape[0]
@@ -471,12 +489,32 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
         # fp8 tensor-core kernel below is bound by the per-128 promotion of its partial sums at this size
         w16 = fp8_expand(wq, w_scale)
         if w16 is not None:
-            return gemm(x, w16, bias=bias, out=out)
+            return _lora_expand(gemm(x, w16, bias=bias, out=out), lora)
     xq, sa = quant_act_fp8(x)
+    add = _lora_add(out, lora)
     rc = load().lx_gemm_fp8_block128(_ptr(xq), xq.stride(0), _ptr(sa), sa.stride(0), _ptr(wq), wq.stride(0), _ptr(w_scale), _ptr(out),
                                      out.stride(0), _ptr(bias), T, N, K, _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.status),
-                                     ws.num_sms, 1, _stream())      # (the kernel in front is the quantiser, which has waited for whatever wrote wq)
+                                     ws.num_sms, 1, ctypes.byref(add) if add is not None else None,
+                                     _stream())      # (the kernel in front is the quantiser, which has waited for whatever wrote wq)
     _check(rc, "lx_gemm_fp8_block128")
+    return out if add is not None else _lora_expand(out, lora)
+
+
+def _lora_add(out: torch.Tensor, lora, max_rows: Optional[int] = None) -> Optional[LxLoraAdd]:
+    """The descriptor of `lora` where the launch that writes `out` can add it."""
+    if lora is None or out.shape[0] > (load().lx_lora_add_max_rows() if max_rows is None else max_rows):
+        return None
+    N = out.shape[1]
+    if N % 4 or out.stride(0) % 4 or any(n < N and n % 128 for n in (lora[0].n0, lora[0].n1)):
+        return None
+    return lora_add_desc(*lora, tables_const=True)
+
+
+def _lora_expand(out: torch.Tensor, lora) -> torch.Tensor:
+    if lora is not None:
+        epi, tiles = lora
+        lora_expand_tiles(epi.v[: out.shape[0]], tiles.table, tiles.num_tiles, tiles.max_rows, epi.arena, epi.slot_base, epi.slot_rank, epi.unit_off, out,
+                          epi.n0, epi.n1, tables_const=True)
     return out
 
 
@@ -495,10 +533,10 @@ def wq_dequant(w, out: Optional[torch.Tensor] = None) -> torch.Tensor:
 WQ4_DIRECT_MAX_TOKENS = int(os.environ.get("LORAX_WQ4_DIRECT_TOKENS", "32"))
 
 
-def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, w_const: bool = False) -> torch.Tensor:
+def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, w_const: bool = False, lora=None) -> torch.Tensor:
     """out[T, N] = x[T, K] @ dequant(w)^T (+ bias) for a weight-only quantised matrix.  Few tokens and affine 4-bit codes:
     the tensor-core kernel that multiplies straight from the packed codes (HBM traffic = the packed weights).  Otherwise
-    the codes are expanded to bf16 once and the tcgen05 GEMM runs on the expansion.  `w_const` as for `gemm`."""
+    the codes are expanded to bf16 once and the tcgen05 GEMM runs on the expansion.  `w_const` as for `gemm`, `lora` as for `gemm_fp8`."""
     assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1
     T, K = x.shape
     N = w.shape[0]
@@ -512,11 +550,13 @@ def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Option
         w = dataclasses.replace(w, perm=None)
     if (w.bits == 4 and w.table is None and T <= WQ4_DIRECT_MAX_TOKENS and N % 16 == 0 and K % 128 == 0 and w.group % 32 == 0
             and x.stride(0) % 8 == 0):
-        rc = load().lx_wq4_gemm_ex(_ptr(x), x.stride(0), _ptr(w.codes), _ptr(w.sz), _ptr(bias), _ptr(out), out.stride(0), T, N, K, w.group,
-                                   (1 if getattr(w, "int_zero", False) else 0) | (2 if w_const else 0), _stream())
+        add = _lora_add(out, lora, WQ4_DIRECT_MAX_TOKENS)
+        rc = load().lx_wq4_gemm_lora(_ptr(x), x.stride(0), _ptr(w.codes), _ptr(w.sz), _ptr(bias), _ptr(out), out.stride(0), T, N, K, w.group,
+                                     (1 if getattr(w, "int_zero", False) else 0) | (2 if w_const else 0), ctypes.byref(add) if add is not None else None,
+                                     _stream())
         _check(rc, "lx_wq4_gemm")
-        return out
-    return gemm(x, wq_dequant(w), bias=bias, out=out)
+        return out if add is not None else _lora_expand(out, lora)
+    return _lora_expand(gemm(x, wq_dequant(w), bias=bias, out=out), lora)
 
 
 # ------------------------------------------------------------------------------------------------ elementwise

@@ -871,6 +871,62 @@ def test_gemm_with_lora_of_few_units(nat, T, K, parts, ranks, layout):
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
 
 
+@pytest.mark.parametrize("form", ["fp8", "wq4"])
+@pytest.mark.parametrize("T,K,parts,ranks", [(1, 512, [128], [16]), (5, 1024, [256, 128, 128], [16, 64]), (8, 512, [1024], [48]), (9, 2048, [512, 512], [32, 16]),
+                                             (32, 4096, [384, 128, 128], [16, 32, 48, 64]), (77, 512, [256], [32, 16]), (256, 512, [16384], [16, 64]),
+                                             (257, 512, [256, 256], [16])])
+def test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks):
+    """The delta of a short step, added in fp32 before the result is rounded, against the shrink's v in float64 on top of the product alone:
+    rows of the base model in between, entries up to 32 rows, ranks of one to four 16s, with and without splits of K, and a step too long for it.
+    Both sides round their sum to bf16, the reference the product before that: 2^-9 each."""
+    from types import SimpleNamespace
+    from lorax_b200.utils.quant_formats import quantize_weight
+    N, nparts = sum(parts), len(parts)
+    gen = torch.Generator("cuda").manual_seed(T + K)
+    w = torch.randn(N, K, generator=gen, device="cuda").to(torch.bfloat16) / math.sqrt(K)
+    x = torch.randn(T, K, generator=gen, device="cuda").to(torch.bfloat16)
+    unit_off, bases, off = 64, [], 0
+    for r in ranks:
+        bases.append(off)
+        off += r * (unit_off + N)
+    arena = (torch.randn(off, generator=gen, device="cuda") * 0.5).to(torch.bfloat16)
+    slots = [(i // 3) % (len(ranks) + 1) - 1 for i in range(T)] if T < 64 else [(i // 37) % (len(ranks) + 1) - 1 for i in range(T)]
+    if T == 1:
+        slots = [0]
+    tl = ref.build_lora_tiles(slots, 32)
+    table = torch.cat([torch.tensor(tl, device="cuda", dtype=torch.int32).view(-1, 4), torch.full((7, 4), -1, device="cuda", dtype=torch.int32)])
+    tiles = SimpleNamespace(table=table, num_tiles=table.shape[0], max_rows=32, live=len(tl))
+    v = nat.workspace().lora_v
+    v[:T] = torch.randn(T, v.shape[1], generator=gen, device="cuda")
+    n0 = parts[0] if nparts > 1 else N
+    n1 = parts[0] + parts[1] if nparts > 2 else N
+    i64 = torch.tensor(bases, device="cuda", dtype=torch.int64)
+    epi = nat.LoraEpilogue(v, torch.tensor(slots, device="cuda", dtype=torch.int32), arena, i64, torch.tensor(ranks, device="cuda", dtype=torch.int32), unit_off, n0, n1)
+    bias = torch.randn(N, generator=gen, device="cuda").to(torch.bfloat16)
+    if form == "fp8":
+        sw = torch.rand((N + 127) // 128, (K + 127) // 128, generator=gen, device="cuda") * 0.01 + 0.01
+        q = (torch.randn(N, K, generator=gen, device="cuda") * 2).to(torch.float8_e4m3fn)
+        run = lambda **kw: nat.gemm_fp8(x, q, sw, bias=bias, **kw)
+    else:
+        gq = quantize_weight(w, "hqq-4bit", 128)
+        run = lambda **kw: nat.gemm_wq(x, gq, bias=bias, w_const=True, **kw)
+    got, base = run(lora=(epi, tiles)), run()
+    nat.workspace().check_status()
+    want = base.double()
+    edges = [0, n0, n1, N]
+    for t, s in enumerate(slots):
+        if s < 0:
+            continue
+        r = ranks[s]
+        B = arena[bases[s] + r * unit_off:][: N * r].view(N, r).double()
+        for part in range(nparts):
+            lo, hi = edges[part], edges[part + 1] if part + 1 < nparts else N
+            want[t, lo:hi] += B[lo:hi] @ v[t, part * r: (part + 1) * r].double()
+    assert _rel_err(got, want) < 2 ** -8
+    alone = [t for t, s in enumerate(slots) if s < 0]
+    assert torch.equal(got[alone], base[alone])
+
+
 @pytest.mark.parametrize("T,E,k,H,I,e0,e_local", [(7, 8, 2, 512, 256, 0, 8), (256, 8, 2, 1024, 768, 0, 8), (300, 8, 2, 512, 256, 2, 2),
                                                   (1500, 16, 4, 256, 128, 0, 16), (64, 4, 1, 256, 384, 1, 1)])
 def test_moe_ffn_on_the_device(nat, T, E, k, H, I, e0, e_local):
