@@ -91,6 +91,7 @@ struct GemmParams {
   int lora_fence_maps;                 // 1: acquire-fence a slot's B_cat map before every use (0: never; measurement only)
   int lora_skip;                       // measurement only: bit 0 leaves out the shrink launch, bit 1 the expand stages (results are then wrong)
   int lora_T;                          // rows of the step
+  int lora_mask, lora_slice;           // an entry's window begins and ends at multiples of mask + 1 rows; elements of a K slice of an image
 };
 
 // ---- LoRA items ----------------------------------------------------------------------------------------------
@@ -154,15 +155,15 @@ struct ExpandItem {
 };
 // -1: end of the live entries or of those that can meet the tile (they are sorted by row), 0: nothing to add for this
 // entry, 1: `e` is valid.
-LX_DEVICE int decode_expand_item(const LoraEnt* ents, int lt, int j0, int jlim, ExpandItem& e) {
+LX_DEVICE int decode_expand_item(const LoraEnt* ents, int lt, int j0, int jlim, int mask, ExpandItem& e) {
   const LoraEnt t = ents[lt];
   if (t.slot < 0 || t.row0 >= jlim) return -1;
   if (t.r == 0) return 0;
   e.slot = t.slot;
   e.r = t.r;
   e.boff = t.boff;
-  e.w0 = t.row0 & ~15;
-  const int w1 = (t.row0 + t.nrows + 15) & ~15;
+  e.w0 = t.row0 & ~mask;
+  const int w1 = (t.row0 + t.nrows + mask) & ~mask;
   e.c0 = max(e.w0, j0);
   e.c1 = min(w1, jlim);
   if (e.c0 >= e.c1) return 0;
@@ -422,10 +423,10 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
         // the unit is complete: 16 ranks x up to 8 rows per group.  This warp holds (rank g, rows 2t, 2t+1) and (rank g + 8, same
         // rows) of every group; the groups go through the two staging buffers one after the other.
         const LoraEnt e = ents[cur.lt];
-        const int w0 = e.row0 & ~15;
-        const int wn = ((e.row0 + e.nrows + 15) & ~15) - w0;
+        const int w0 = e.row0 & ~p.lora_mask;
+        const int wn = ((e.row0 + e.nrows + p.lora_mask) & ~p.lora_mask) - w0;
         const int pp = cur.j / cur.r, i0 = cur.j - pp * cur.r;
-        __nv_bfloat16* img = p.lora_vimg + ((long long)(pp * 4 + (i0 >> 4)) * p.lora_num_tiles + cur.lt) * kLoraSliceElems;
+        __nv_bfloat16* img = p.lora_vimg + ((long long)(pp * 4 + (i0 >> 4)) * p.lora_num_tiles + cur.lt) * p.lora_slice;
 #pragma unroll
         for (int q = 0; q < NG; ++q) {
           if (q * kShrinkRows < cur.nt) {              // the same for the four warps: they meet at the barrier below
@@ -458,8 +459,8 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
             const int z_lo = (t0g == e.row0) ? e.row0 - w0 : 0;
             const int z_hi = (t0g + ntg == e.row0 + e.nrows) ? e.row0 + e.nrows - w0 : wn;
             const int zrows = z_lo + (wn - z_hi);
-            if (whole && tid4 >= 32 && tid4 - 32 < 2 * zrows) {
-              const int cz = (tid4 - 32) >> 1, ch = (tid4 - 32) & 1;
+            for (int z = tid4 - 32; whole && z >= 0 && z < 2 * zrows; z += 96) {
+              const int cz = z >> 1, ch = z & 1;
               const int row = cz < z_lo ? cz : z_hi + (cz - z_lo);
               *reinterpret_cast<uint4*>(img + row * 16 + (ch << 3)) = make_uint4(0, 0, 0, 0);
             }
@@ -511,13 +512,13 @@ LX_DEVICE bool wait_flag(const int* flag, int want, volatile int* abort_flag) {
 // A unit = one K slice (16 ranks) of one table entry that meets the token tile.  The producer warp and the MMA warp each build
 // the same list in their own shared-memory area, 32 entries at a time (one per lane, ranks -> slices by a warp prefix sum), and
 // keep it while the token tile stays the same: it does not depend on the feature tile.
-// First live entry whose 16-aligned window ends after row j0 (entries are sorted by row and do not overlap).
-LX_DEVICE int lora_first_entry(const LoraEnt* ents, int n_live, int j0) {
+// First live entry whose aligned window ends after row j0 (entries are sorted by row and do not overlap).
+LX_DEVICE int lora_first_entry(const LoraEnt* ents, int n_live, int j0, int mask) {
   int lo = 0, hi = n_live;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
     const LoraEnt t = ents[mid];
-    if (((t.row0 + t.nrows + 15) & ~15) > j0) hi = mid; else lo = mid + 1;
+    if (((t.row0 + t.nrows + mask) & ~mask) > j0) hi = mid; else lo = mid + 1;
   }
   return lo;
 }
@@ -525,7 +526,7 @@ LX_DEVICE int lora_first_entry(const LoraEnt* ents, int n_live, int j0) {
 struct LoraUnit {
   int slot, img;        // img = entry * 4 + slice
   int c0, c1;           // accumulator columns [c0, c1) the unit adds to
-  int w0;               // first row of the entry's 16-aligned window
+  int w0;               // first row of the entry's aligned window
   int boff;             // B_cat of the slot, group and layer in 16-byte steps from the arena's start
   int rclass;           // rank / 16 - 1: which arena-wide map has the slot's row pitch
   int pad_;
@@ -542,7 +543,7 @@ LX_DEVICE int lora_build_units(const GemmParams& p, const LoraEnt* ents, int lt0
   const int lane = threadIdx.x & 31;
   const int lt = lt0 + lane;
   ExpandItem e;
-  const int rc = lt < p.lora_num_tiles ? decode_expand_item(ents, lt, j0, jlim, e) : -1;
+  const int rc = lt < p.lora_num_tiles ? decode_expand_item(ents, lt, j0, jlim, p.lora_mask, e) : -1;
   const unsigned endmask = __ballot_sync(0xffffffffu, rc < 0);
   const int first_end = endmask ? __ffs(endmask) - 1 : 32;
   const int nsl = (rc == 1 && lane < first_end) ? e.r / 16 : 0;
@@ -568,7 +569,7 @@ LX_DEVICE int lora_build_units(const GemmParams& p, const LoraEnt* ents, int lt0
 LX_DEVICE int lora_prebuild_units(const GemmParams& p, const LoraEnt* ents, int n_live, int j0, int jlim, LoraUnit* list) {
   int n = 0;
   bool ended = false;
-  for (int lt0 = lora_first_entry(ents, n_live, j0); !ended && lt0 < p.lora_num_tiles; lt0 += 32) {
+  for (int lt0 = lora_first_entry(ents, n_live, j0, p.lora_mask); !ended && lt0 < p.lora_num_tiles; lt0 += 32) {
     if (n > kLoraListCap - 128) return -1;             // 32 entries yield up to 128 units
     n = lora_build_units(p, ents, lt0, j0, jlim, list, n, ended);
   }
@@ -847,7 +848,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             // more units than the list holds: built and sent in pieces
             int n = 0;
             bool ended = false;
-            for (int lt0 = lora_first_entry(ents, *n_live, j0); ok; lt0 += 32) {
+            for (int lt0 = lora_first_entry(ents, *n_live, j0, p.lora_mask); ok; lt0 += 32) {
               bool last = true;
               if (lt0 < p.lora_num_tiles) {
                 n = lora_build_units(p, ents, lt0, j0, jlim, ulist_p, n, ended);
@@ -1555,6 +1556,35 @@ static int launch_gemm_t(const CUtensorMap& ta, const CUtensorMap& tb, const Lor
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
+}  // namespace lx
+#include "gemm_pair.cuh"
+namespace lx {
+
+// The operand images as rows of 16 ranks: what a copy takes is laid out (and swizzled) as the MMA reads it.
+static int make_tmap_lora_images(CUtensorMap* out, const void* base, uint64_t rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return -1;
+  cuuint64_t dims[2] = {16, rows};
+  cuuint64_t strides[1] = {32};
+  cuuint32_t box[2] = {16, 16};
+  cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(int)r - 100;
+}
+
+template <bool LORA>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ti, const LoraBMaps& bm, const GemmParams& base, int bn, int pairs,
+                       cudaStream_t stream) {
+  GemmParams p = base;
+  p.bn = p.umma_n = bn;
+  const int tiles = (p.a_rows + 255) / 256 * ((p.b_rows + bn - 1) / bn);
+  const int grid = 2 * (tiles < pairs ? tiles : pairs);
+  launch_pdl_cluster(gemm_pair_kernel<LORA>, dim3(grid), dim3(kGemmThreads), dim3(2, 1, 1), (size_t)PairSmem<LORA>::kTotal, stream, ta, tb, ti, bm, p);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -(int)e;
+}
+
 template <int BN, int STAGES>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
   static const LoraBMaps none{};
@@ -1578,6 +1608,7 @@ struct GemmPlan {
 // Steps of thousands of rows lose by an early start of the next kernel (see pdl_trigger).  Where the line lies matters little: passes of 300 to
 // 2500 rows took the same within 1 % with limits of 128, 512 and 2048.
 constexpr int kOverlapMaxTokens = 512;
+constexpr int kPairMinTokens = 512;            // longer steps take pairs of CTAs
 constexpr int kModeConstWeights = 1 << 16;     // of a launch's `mode`: no kernel that may still run writes the weights
 
 constexpr int kClassicSplitTokens = 32;
@@ -1751,6 +1782,7 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     pl_swap = choose_plan_swap(T, N, K, num_sms, usable_ws, have_counters, force_split & 0xffff, force_bn, sk_policy);
     swap = pl_swap.cost <= pl_tok.cost;
   }
+  const int pair_bn = T > kPairMinTokens && N >= 256 && (mode == 0 || has_lora) && force_split == 0 && sk_policy == 0 ? pair_token_tile(T, N, num_sms / 2) : 0;
   p.overlap = T <= kOverlapMaxTokens;
   if (swap) {
     p.a_rows = N; p.b_rows = T;
@@ -1803,6 +1835,8 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       p.lora_skip = e ? atoi(e) : 0;
     }
     p.lora_T = T;
+    p.lora_mask = 15;
+    p.lora_slice = kLoraSliceElems;
     p.lora_off_a = lora->off_a;
     p.lora_arena = reinterpret_cast<const __nv_bfloat16*>(lora->arena);
     p.lora_x = reinterpret_cast<const __nv_bfloat16*>(x);
@@ -1833,12 +1867,33 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       const int rc = launch_lora_shrink_rows(sp, lora->max_rank, num_sms, stream);
       if (rc != 0) return rc;
     }
+    if (pair_bn > 0 && p.lora_inline_shrink && (lora->nparts == 1 || (lora->n0 % 256 == 0 && (lora->nparts == 2 || lora->n1 % 256 == 0))) &&
+        img_bytes / 48 * 64 <= lora->vimg_bytes) {
+      const int pairs = pair_capacity<true>();
+      CUtensorMap ti;
+      if (pairs * 2 >= 2 && make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32)) == 0 && make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair_bn / 2) == 0) {
+        p.lora_mask = 31;
+        p.lora_slice = 64 * 16;
+        p.lora_kparts = nullptr;
+        return launch_pair<true>(ta, tb, ti, bm, p, pair_bn, pairs, stream);
+      }
+    }
     switch (template_bn(bn)) {
       case 16:  return launch_gemm_t<16, 8, true>(ta, tb, bm, p, pl.grid, stream);
       case 32:  return launch_gemm_t<32, 8, true>(ta, tb, bm, p, pl.grid, stream);
       case 64:  return launch_gemm_t<64, 8, true>(ta, tb, bm, p, pl.grid, stream);
       case 128: return launch_gemm_t<128, 6, true>(ta, tb, bm, p, pl.grid, stream);
       default:  return launch_gemm_t<256, 4, true>(ta, tb, bm, p, pl.grid, stream);
+    }
+  }
+  if (pair_bn > 0) {
+    const int pairs = pair_capacity<false>();
+    if (pairs > 0) {
+      if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
+      if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair_bn / 2)) return -1003;
+      p.a_rows = N; p.b_rows = T;
+      p.ldo_a = 1; p.ldo_b = ldo;
+      return launch_pair<false>(ta, tb, ta, LoraBMaps{}, p, pair_bn, pairs, stream);
     }
   }
   switch (template_bn(bn)) {

@@ -1,0 +1,437 @@
+// The bf16 GEMM of gemm_bf16.cu for long steps, by pairs of CTAs (tcgen05 cta_group::2).  Included there, behind the LoRA pieces it shares.
+//
+// A pair takes a tile of 256 output features x up to 256 tokens: each CTA loads 128 rows of the weights and half of the tokens, 32 KB a stage
+// where one CTA on its own tile of 128 x 256 takes 48, and reads half the token operand from its shared memory per MMA: what a single CTA
+// moves in and out of shared memory per product is the limit of gemm_bf16_tcgen05_kernel at these sizes (192 of about 128 B per cycle asked for).
+// Rank 0's MMA thread issues for both; a stage is full when the loads of both CTAs have arrived at rank 0's barrier, and its commits
+// tell both that a stage is free or an accumulator complete.  Tiles are whole (no split of K): the token tile is chosen so that the last
+// wave is nearly full.  LoRA as there: shrink on the epilogue warps of all CTAs during the first K loop, expand by MMAs into the
+// accumulators, whose columns come in steps of 32 here (an entry's window: 64 rows, 32-aligned); each CTA brings its features' B_cat and half of the
+// window's rows.  One row of ranks serves both CTAs, so parts must begin at multiples of 256.
+#pragma once
+
+namespace lx {
+
+constexpr int kPairStages = 6;
+constexpr int kPairUnits = 6;                         // expand units that share a stage
+constexpr int kPairImgBytes = 32 * 32;                // half of a window's rows, 16 ranks
+struct PairHeader {
+  LoraUnit units[kPairUnits];
+  int nu, last, pad_[2];
+};
+template <bool LORA>
+struct PairSmem {
+  static constexpr int kABytes = kBM * kBK * 2, kBBytes = kBM * kBK * 2;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static_assert(kPairUnits * (kLoraBTileBytes + kPairImgBytes) + (int)sizeof(PairHeader) <= kStageBytes, "an expand stage fits");
+  static constexpr int kBarrierBytes = 256;
+  static constexpr int kEntBytes = LORA ? kLoraMaxEntries * (int)sizeof(LoraEnt) + kLoraListCap * 32 + (kLoraMaxEntries + 8) * 2 : 0;
+  static constexpr int kEpiBytes = 4 * 32 * 32 * 2;
+  static constexpr int kTotal = kPairStages * kStageBytes + kBarrierBytes + kEntBytes + kEpiBytes + 1024;
+  static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
+};
+
+LX_DEVICE uint32_t pair_map(const void* smem, uint32_t rank) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(smem)), "r"(rank));
+  return ra;
+}
+LX_DEVICE void pair_load_2d(void* dst, const CUtensorMap* m, uint32_t bar, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+LX_DEVICE void pair_load_2d_hint(void* dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, uint64_t policy) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
+}
+LX_DEVICE void pair_load_3d(void* dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+LX_DEVICE void pair_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// The barrier at this offset in both CTAs, when all MMAs issued so far have completed.
+LX_DEVICE void pair_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+LX_DEVICE void pair_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+
+// mbar_wait for a barrier that the other CTA arrives at.
+LX_DEVICE bool pair_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  uint64_t t0 = 0;
+  uint32_t polls = 0;
+  while (true) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P1, [%1], %2;\n\tselp.u32 %0, 1, 0, P1;\n\t}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((++polls & 2047u) == 0) {
+      if (*abort_flag != 0) return false;
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kWaitBudgetNs) return false;
+    }
+  }
+}
+
+template <bool LORA>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_img,
+                 const __grid_constant__ LoraBMaps bmaps, const GemmParams p) {
+  using S = PairSmem<LORA>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* tiles = smem;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kPairStages * S::kStageBytes);      // (rank 0's are used)
+  uint64_t* empty_bar = full_bar + kPairStages;
+  uint64_t* tmem_full = empty_bar + kPairStages;
+  uint64_t* tmem_empty = tmem_full + 2;                                                       // (rank 0's are used)
+  uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+  int* n_live = reinterpret_cast<int*>(tmem_base_slot + 3);
+  LoraEnt* ents = reinterpret_cast<LoraEnt*>(smem + kPairStages * S::kStageBytes + S::kBarrierBytes);
+  LoraUnit* ulist = reinterpret_cast<LoraUnit*>(ents + kLoraMaxEntries);
+  unsigned short* gstart = reinterpret_cast<unsigned short*>(ulist + kLoraListCap);
+  __nv_bfloat16* epi_stage = reinterpret_cast<__nv_bfloat16*>(smem + kPairStages * S::kStageBytes + S::kBarrierBytes + S::kEntBytes);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  const int tiles_a = (p.a_rows + 2 * kBM - 1) / (2 * kBM), tiles_b = (p.b_rows + p.bn - 1) / p.bn;
+  const int num_tiles = tiles_a * tiles_b;
+  const int kblocks = (p.K + kBK - 1) / kBK;
+  const int half = p.bn >> 1;                          // tokens that this CTA loads
+  const bool lora = LORA && p.lora_tiles != nullptr;
+  int pre_tb = -1, pre_n = 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tmem_full[s], 1); mbar_init(&tmem_empty[s], 8); }
+    *abort_flag = 0;
+    *n_live = LORA ? p.lora_num_tiles : 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                      // both CTAs' barriers and columns are there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_base_slot;
+  if constexpr (LORA) {
+    if (lora) {
+      if (!p.lora_tables_const) pdl_wait();
+      load_lora_entries(p, ents, n_live);
+      __syncthreads();
+      if (warp == 2) lora_unit_prefix(p, ents, gstart);
+      if (warp == 0 && pair < num_tiles) {
+        const int ta0 = pair / tiles_b, tb0 = pair % tiles_b;
+        const int n0 = lora_prebuild_units(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.bn, ulist);
+        if (n0 >= 0) { pre_tb = tb0; pre_n = n0; }
+        if (n0 > 0) lora_prefetch_b(p, ulist, n0, 2 * ta0 + (int)rank);
+      }
+      __syncthreads();
+    }
+  }
+  pdl_wait();
+
+  if (warp == 0) {
+    const uint64_t pol_a = policy_evict_first(), pol_b = policy_evict_last();
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int list_tb = pre_tb, list_n = pre_n;
+    bool first_tile = pre_tb >= 0, shrink_seen = false;
+    for (int tile = pair; tile < num_tiles; tile += pairs) {
+      const int ta = tile / tiles_b, tb = tile % tiles_b;
+      const int i0 = (2 * ta + (int)rank) * kBM, j0 = tb * p.bn, jlim = j0 + p.bn;
+      if constexpr (LORA) {
+        if (lora) {
+          if (list_tb != tb) {
+            const int n0 = lora_prebuild_units(p, ents, *n_live, j0, jlim, ulist);
+            list_tb = n0 >= 0 ? tb : -1;
+            list_n = n0 >= 0 ? n0 : 0;
+          }
+          if (list_tb == tb && list_n > 0 && !first_tile) lora_prefetch_b(p, ulist, list_n, 2 * ta + (int)rank);
+          first_tile = false;
+        }
+      }
+      if (lane == 0 && ok) {
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+            report_status(p.status, kTimeoutEmptyBarrier, tile);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          uint8_t* sa = tiles + stage * S::kStageBytes;
+          const uint32_t bar = pair_map(&full_bar[stage], 0);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)(S::kABytes + half * kBK * 2));
+          pair_load_2d_hint(sa, &tmap_a, bar, kb * kBK, i0, pol_a);
+          pair_load_2d_hint(sa + S::kABytes, &tmap_b, bar, kb * kBK, j0 + (int)rank * half, pol_b);
+          if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+        }
+      }
+      if constexpr (LORA) {
+        if (lora) {
+          __syncwarp();
+          stage = __shfl_sync(0xffffffffu, stage, 0);
+          phase = __shfl_sync(0xffffffffu, phase, 0);
+          ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+          const int pt = min(p.lora_nparts - 1, i0 < p.lora_n0 ? 0 : (i0 < p.lora_n1 ? 1 : 2));
+          const long long img_part = (long long)pt * 4 * p.lora_num_tiles;
+          if (ok && !shrink_seen) {
+            if (lane == 0) {
+              if (!wait_flag(&p.lora_sync[1], (int)gridDim.x, abort_flag)) {
+                report_status(p.status, kTimeoutSplitK, tile);
+                *abort_flag = 1;
+              }
+            }
+            __syncwarp();
+            ok = (*abort_flag == 0);
+            fence_proxy_async_all();       // the images were written with ordinary stores; the loads below are the async proxy's
+            shrink_seen = true;
+          }
+          auto send_stage = [&](int base, int nu, bool last) -> bool {
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+              if (lane == 0) {
+                report_status(p.status, kTimeoutEmptyBarrier, tile);
+                *abort_flag = 1;
+              }
+              return false;
+            }
+            uint8_t* sa = tiles + stage * S::kStageBytes;
+            PairHeader* hdr = reinterpret_cast<PairHeader*>(sa + kPairUnits * (kLoraBTileBytes + kPairImgBytes));
+            LoraUnit q{};
+            if (lane < nu) q = ulist[base + lane];
+            const int rows = lane < nu ? (q.c1 - q.c0) >> 1 : 0;                  // of the window, in each CTA: 16 or 32
+            const int bytes = __reduce_add_sync(0xffffffffu, lane < nu ? kLoraBTileBytes + rows * 32 : 0);
+            const uint32_t bar = pair_map(&full_bar[stage], 0);
+            if (rank == 0) {
+              if (lane < nu) hdr->units[lane] = q;
+              if (lane == 0) { hdr->nu = nu; hdr->last = last ? 1 : 0; }
+              fence_proxy_async_smem();          // the stage's bytes are written by bulk copies at other times
+              __syncwarp();
+              if (lane == 0) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)bytes);
+            }
+            __syncwarp();
+            if (lane < nu) {
+              pair_load_3d(sa + lane * kLoraBTileBytes, &bmaps.m[q.rclass], bar, (q.img & 3) * 16, i0, q.boff);
+              const int row = (int)(img_part + (long long)(q.img & 3) * p.lora_num_tiles + (q.img >> 2)) * 64 + (q.c0 - q.w0) + (int)rank * rows;
+              uint8_t* dst = sa + kPairUnits * kLoraBTileBytes + lane * kPairImgBytes;
+              for (int h = 0; h < rows; h += 16) pair_load_2d(dst + h * 32, &tmap_img, bar, 0, row + h);
+            }
+            if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+            return true;
+          };
+          auto send_run = [&](int n, bool closes) {
+            if (n == 0 && closes) ok = send_stage(0, 0, true);
+            for (int base = 0; ok && base < n; base += kPairUnits) ok = send_stage(base, min(kPairUnits, n - base), closes && base + kPairUnits >= n);
+          };
+          if (!ok) {
+          } else if (list_tb == tb) {
+            send_run(list_n, true);
+          } else {
+            // more units than the list holds: built and sent in pieces
+            int n = 0;
+            bool ended = false;
+            for (int lt0 = lora_first_entry(ents, *n_live, j0, p.lora_mask); ok; lt0 += 32) {
+              bool last = true;
+              if (lt0 < p.lora_num_tiles) {
+                n = lora_build_units(p, ents, lt0, j0, jlim, ulist, n, ended);
+                last = ended || lt0 + 32 >= p.lora_num_tiles;
+                if (n < 128 && !last) continue;
+              }
+              send_run(n, last);
+              if (last) break;
+              n = 0;
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      const uint32_t idesc = make_idesc(2 * kBM, (uint32_t)p.bn, kFmtBF16, kFmtBF16);
+      int stage = 0;
+      uint32_t phase = 0;
+      int acc = 0;
+      uint32_t acc_phase[2] = {0, 0};
+      bool ok = true;
+      for (int tile = pair; ok && tile < num_tiles; tile += pairs) {
+        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * 256);
+        if (!pair_wait(&tmem_empty[acc], acc_phase[acc] ^ 1, abort_flag)) {
+          report_status(p.status, kTimeoutTmemEmpty, tile);
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after();
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+            report_status(p.status, kTimeoutFullBarrier, tile);
+            *abort_flag = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(tiles + stage * S::kStageBytes);
+          const uint64_t da = make_desc_k_sw128(sa), db = make_desc_k_sw128(sa + S::kABytes);
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k) pair_mma(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          pair_commit(&empty_bar[stage]);
+          if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+        }
+        if constexpr (LORA) {
+          bool more = lora && ok;
+          while (more) {
+            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
+              report_status(p.status, kTimeoutFullBarrier, tile);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            uint8_t* sp = tiles + stage * S::kStageBytes;
+            const PairHeader* hdr = reinterpret_cast<const PairHeader*>(sp + kPairUnits * (kLoraBTileBytes + kPairImgBytes));
+            const uint32_t sa = smem_u32(sp);
+            const int nu = min(hdr->nu, kPairUnits), j0 = tile % tiles_b * p.bn;
+            more = hdr->last == 0;
+            for (int u = 0; u < nu; ++u) {
+              const LoraUnit q = hdr->units[u];
+              pair_mma(tmem_d + (uint32_t)(q.c0 - j0), make_desc_k_sw32(sa + (uint32_t)(u * kLoraBTileBytes)),
+                       make_desc_k_sw32(sa + (uint32_t)(kPairUnits * kLoraBTileBytes + u * kPairImgBytes)),
+                       make_idesc(2 * kBM, (uint32_t)(q.c1 - q.c0), kFmtBF16, kFmtBF16), 1u);
+            }
+            pair_commit(&empty_bar[stage]);
+            if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+          }
+        }
+        if (ok) pair_commit(&tmem_full[acc]);
+        acc_phase[acc] ^= 1;
+        acc ^= 1;
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quad = warp & 3;
+    int acc = 0;
+    uint32_t acc_phase[2] = {0, 0};
+    if constexpr (LORA) {
+      if (lora) lora_shrink_units(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
+    }
+    const bool turn = p.ldo_a == 1 && (p.ldo_b & 7) == 0 && (p.a_rows & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+    for (int tile = pair; tile < num_tiles; tile += pairs) {
+      const int ta = tile / tiles_b, tb = tile % tiles_b;
+      if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_flag)) {
+        report_status(p.status, kTimeoutTmemFull, tile);
+        *abort_flag = 1;
+        break;
+      }
+      tc_fence_after();
+      acc_phase[acc] ^= 1;
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
+      const int f0 = (2 * ta + (int)rank) * kBM + quad * 32, i = f0 + lane;
+      const int j0 = tb * p.bn, jend = min(p.b_rows, j0 + p.bn);
+      const float bias_i = (p.bias != nullptr && i < p.a_rows) ? __bfloat162float(p.bias[i]) : 0.f;
+      __nv_bfloat16* st = epi_stage + quad * (32 * 32);
+      const int fbase = f0 + (lane & 3) * 8;
+#pragma unroll 1
+      for (int c = 0; c < p.bn; c += 32) {
+        if (j0 + c >= jend) break;
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(taddr + c, r);
+        tc_wait_ld();
+        if (turn) {
+          // a thread holds one feature of 32 tokens; the warp turns its block around and stores eight features of a token per lane
+#pragma unroll
+          for (int q = 0; q < 32; ++q) st[q * 32 + lane] = __float2bfloat16(__uint_as_float(r[q]) * p.out_scale + bias_i);
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const int tq = h * 8 + (lane >> 2), t = j0 + c + tq;
+            if (t < jend && fbase < p.a_rows)
+              *reinterpret_cast<uint4*>(p.out + (long long)t * p.ldo_b + fbase) = *reinterpret_cast<const uint4*>(st + tq * 32 + (lane & 3) * 8);
+          }
+          __syncwarp();
+        } else if (i < p.a_rows) {
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (j0 + c + q < jend)
+              p.out[(long long)i * p.ldo_a + (long long)(j0 + c + q) * p.ldo_b] = __float2bfloat16(__uint_as_float(r[q]) * p.out_scale + bias_i);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) pair_arrive(pair_map(&tmem_empty[acc], 0));
+      acc ^= 1;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                      // nothing of this pair is on its way to a CTA that has left
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+  if constexpr (LORA) {
+    if (lora && threadIdx.x == 0) {
+      __threadfence();
+      const int prev = atomicAdd(&p.lora_sync[0], 1);
+      if (prev == (int)gridDim.x - 1) {
+        p.lora_sync[0] = 0;
+        p.lora_sync[1] = 0;
+        __threadfence();
+      }
+    }
+  }
+}
+
+// Pairs of CTAs that run at the same time (the wait for the shrink counts on it); 0: the device has none.
+template <bool LORA>
+static int pair_capacity() {
+  static int known[64] = {0};          // capacity + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (known[dev] == 0) {
+    int n = 0;
+    if (cudaFuncSetAttribute(gemm_pair_kernel<LORA>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<LORA>::kTotal) == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2);
+      cfg.blockDim = dim3(kGemmThreads);
+      cfg.dynamicSmemBytes = PairSmem<LORA>::kTotal;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<LORA>, &cfg) != cudaSuccess) n = 0;
+    }
+    cudaGetLastError();
+    known[dev] = n + 1;
+  }
+  return known[dev] - 1;
+}
+
+// The token tile, a multiple of 32, whose waves of whole tiles cost least.  A tile takes as long as its operands take to come in from L2, 128 rows
+// of weights and half its tokens per CTA (their MMAs need less than that), and some for its start.
+static int pair_token_tile(int T, int N, int pairs) {
+  int best = 256;
+  long long cost = -1;
+  for (int bn = 256; bn >= 96; bn -= 32) {
+    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn);
+    const long long c = (tiles + pairs - 1) / pairs * (kBM + bn / 2 + 16);
+    if (cost < 0 || c < cost) { cost = c; best = bn; }
+  }
+  return best;
+}
+
+}  // namespace lx
