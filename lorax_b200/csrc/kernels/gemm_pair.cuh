@@ -174,8 +174,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           uint8_t* sa = tiles + stage * S::kStageBytes;
           const uint32_t bar = pair_map(&full_bar[stage], 0);
           if (rank == 0) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)(S::kABytes + half * kBK * 2));
-          pair_load_2d_hint(sa, &tmap_a, bar, kb * kBK, i0, pol_a);
-          pair_load_2d_hint(sa + S::kABytes, &tmap_b, bar, kb * kBK, j0 + (int)rank * half, pol_b);
+          pair_load_2d(sa, &tmap_a, bar, kb * kBK, i0);
+          pair_load_2d(sa + S::kABytes, &tmap_b, bar, kb * kBK, j0 + (int)rank * half);
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
         }
       }
