@@ -21,7 +21,7 @@
 // on the device, every launch has static shapes (k * tokens rows at most), so a decode step with experts is one CUDA graph.
 // Under expert parallelism a rank owns experts [e0, e0 + e_local): rows routed elsewhere get pos = -1 and the per-rank outputs
 // are summed by the all-reduce that follows.
-#include "common.cuh"
+#include "pair.cuh"
 
 namespace lx {
 
@@ -639,6 +639,165 @@ __global__ void __launch_bounds__(256) moe_grouped_gemm_f32_kernel(const float* 
 
 int make_tmap_bf16_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uint64_t K, uint64_t row_stride_elems, uint32_t box_rows);
 
+// The same for runs of a tile and more, by pairs of CTAs (gemm_pair.cuh has the reasons): a tile is 256 features x up to 256 rows of a run, each CTA
+// brings 128 rows of the weights and half of the tile's rows.  A run's last tile multiplies as many rows as it has (in steps of 32).
+constexpr int kMpMinRows = 192;      // rows a run on average
+constexpr int kMpStages = 6;
+struct MpSmem {
+  static constexpr int kStage = 2 * kMgBM * kMgBK * 2;
+  static constexpr int kEpiBytes = 4 * 32 * 32 * 2;
+  static constexpr int kTotal = kMpStages * kStage + 1024 + kMgTail + kEpiBytes;
+};
+static_assert(MpSmem::kTotal <= 227 * 1024, "shared memory of one CTA");
+
+__global__ void __launch_bounds__(kMgThreads, 1)
+moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const MoeGemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* tiles = smem;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kMpStages * MpSmem::kStage);      // (rank 0's are used)
+  uint64_t* empty_bar = full_bar + kMpStages;
+  uint64_t* tmem_full = empty_bar + kMpStages;
+  uint64_t* tmem_empty = tmem_full + 2;                                                     // (rank 0's are used)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* start_s = reinterpret_cast<int*>(smem + kMpStages * MpSmem::kStage + 1024);          // [runs + 1]
+  int* cum_s = start_s + kMoeMaxRuns + 1;
+  __nv_bfloat16* epi_stage = reinterpret_cast<__nv_bfloat16*>(smem + kMpStages * MpSmem::kStage + kMgTail);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank(), pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  const int kblocks = (p.K + kMgBK - 1) / kMgBK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMpStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tmem_full[s], 1); mbar_init(&tmem_empty[s], 8); }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) pair_tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                      // both CTAs' barriers and columns are there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  if (warp == 0) MgIter::build(p.seg, p.runs, p.rows_cap, p.n_w / (2 * kMgBM), p.bn, start_s, cum_s);
+  __syncthreads();
+  const MgIter it{p.runs, p.n_w / (2 * kMgBM), p.bn, start_s, cum_s};
+  const int shared0 = p.runs - p.shared;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int g = pair; ok && g < it.total(); g += pairs) {
+        int e, ta, tb, row0, nrows;
+        it.decode(g, e, ta, tb, row0, nrows);
+        const int half = ((nrows + 31) & ~31) >> 1;      // rows of the tile that each CTA's part of the operand holds (the box brings more)
+        const int xrow = row0 - (e > shared0 ? (e - shared0) * p.tokens : 0) + rank * half;
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { report_status(p.status, kTimeoutEmptyBarrier, g); *abort_flag = 1; ok = false; break; }
+          uint8_t* sa = tiles + stage * MpSmem::kStage;
+          const uint32_t bar = pair_map(&full_bar[stage], 0);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)((kMgBM + p.bn / 2) * kMgBK * 2));
+          pair_load_2d(sa, &tmap_w, bar, kb * kMgBK, e * p.n_w + (2 * ta + rank) * kMgBM);
+          pair_load_2d(sa + kMgBM * kMgBK * 2, &tmap_x, bar, kb * kMgBK, xrow);
+          if (++stage == kMpStages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase[2] = {0, 0};
+      bool ok = true;
+      for (int g = pair; ok && g < it.total(); g += pairs) {
+        int e, ta, tb, row0, nrows;
+        it.decode(g, e, ta, tb, row0, nrows);
+        const uint32_t idesc = make_idesc(2 * kMgBM, (uint32_t)((nrows + 31) & ~31), kFmtBF16, kFmtBF16);
+        if (!pair_wait(&tmem_empty[acc], acc_phase[acc] ^ 1, abort_flag)) { report_status(p.status, kTimeoutTmemEmpty, g); *abort_flag = 1; break; }
+        tc_fence_after();
+        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * 256);
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { report_status(p.status, kTimeoutFullBarrier, g); *abort_flag = 1; ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(tiles + stage * MpSmem::kStage);
+          const uint64_t da = make_desc_k_sw128(sa), db = make_desc_k_sw128(sa + kMgBM * kMgBK * 2);
+#pragma unroll
+          for (int k = 0; k < kMgBK / 16; ++k) pair_mma(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          pair_commit(&empty_bar[stage]);
+          if (++stage == kMpStages) { stage = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        pair_commit(&tmem_full[acc]);
+        acc_phase[acc] ^= 1;
+        acc ^= 1;
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quad = warp & 3;
+    int acc = 0;
+    uint32_t acc_phase[2] = {0, 0};
+    const bool turn = p.act != kMoeActSwiglu && p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+    __nv_bfloat16* st = epi_stage + quad * (32 * 32);
+    for (int g = pair; g < it.total(); g += pairs) {
+      int e, ta, tb, row0, nrows;
+      it.decode(g, e, ta, tb, row0, nrows);
+      if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_flag)) { report_status(p.status, kTimeoutTmemFull, g); *abort_flag = 1; break; }
+      tc_fence_after();
+      acc_phase[acc] ^= 1;
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
+      const int f0 = (2 * ta + rank) * kMgBM + quad * 32, i = f0 + lane;             // feature of this lane
+#pragma unroll 1
+      for (int c = 0; c < nrows; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(taddr + c, r);
+        tc_wait_ld();
+        if (turn) {
+          // the warp turns its block around and stores eight features of a row per lane
+#pragma unroll
+          for (int q = 0; q < 32; ++q) st[q * 32 + lane] = __float2bfloat16(moe_act(__uint_as_float(r[q]), p.act));
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const int tq = h * 8 + (lane >> 2);
+            if (c + tq < nrows)
+              *reinterpret_cast<uint4*>(p.out + (long long)(row0 + c + tq) * p.ldo + f0 + (lane & 3) * 8) = *reinterpret_cast<const uint4*>(st + tq * 32 + (lane & 3) * 8);
+          }
+          __syncwarp();
+        } else if (p.act == kMoeActSwiglu) {
+          // gate and up of a column sit in neighbouring lanes: each lane of the pair finishes half of the rows
+          const bool odd = lane & 1;
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[q] : r[q + 16]), 1);
+            const float gate = odd ? other : __uint_as_float(r[q]), up = odd ? __uint_as_float(r[q + 16]) : other;
+            const int tok = c + q + (odd ? 16 : 0);
+            if (tok < nrows) p.out[(long long)(row0 + tok) * p.ldo + (i >> 1)] = __float2bfloat16(__fdividef(gate, 1.f + __expf(-gate)) * up);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (c + q < nrows) p.out[(long long)(row0 + c + q) * p.ldo + i] = __float2bfloat16(moe_act(__uint_as_float(r[q]), p.act));
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) pair_arrive(pair_map(&tmem_empty[acc], 0));
+      acc ^= 1;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                      // nothing of this pair is on its way to a CTA that has left
+  if (warp == 1) { tc_fence_after(); pair_tmem_dealloc(tmem_base, 512); }
+}
+
 template <int BN, int STAGES>
 static int launch_moe_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const MoeGemmParams& p, int grid, cudaStream_t stream) {
   using S = MgSmem<BN, STAGES>;
@@ -742,6 +901,18 @@ int lx_moe_grouped_gemm(const void* xg, long long ldx, const void* w, long long 
     launch_pdl(moe_grouped_gemm_f32_kernel, dim3((n_w + 63) / 64, rows_cap / 64 + runs), dim3(256), 0, s, reinterpret_cast<const float*>(xg), ldx,
                reinterpret_cast<const float*>(w), ldw, reinterpret_cast<float*>(out), p);
     return -(int)cudaGetLastError();
+  }
+  if (avg_rows >= kMpMinRows && n_w % (2 * kMgBM) == 0) {
+    static int known[64] = {0};
+    const int pairs = pair_capacity_of(moe_pair_kernel, kMgThreads, MpSmem::kTotal, known);
+    if (pairs > 0) {
+      p.bn = 256;
+      CUtensorMap tw, tx;
+      if (make_tmap_bf16_kmajor(&tw, w, (uint64_t)runs * n_w, K, ldw, kMgBM)) return -2;
+      if (make_tmap_bf16_kmajor(&tx, xg, x_rows, K, ldx, p.bn / 2)) return -3;
+      launch_pdl_cluster(moe_pair_kernel, dim3(2 * pairs), dim3(kMgThreads), dim3(2, 1, 1), (size_t)MpSmem::kTotal, s, tw, tx, p);
+      return -(int)cudaGetLastError();
+    }
   }
   // few rows per expert: a tile twice the average holds most runs whole (a second tile would read the weights again)
   int bn = ((avg_rows < 128 ? 2 * avg_rows : avg_rows) + 15) / 16 * 16;

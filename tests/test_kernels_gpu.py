@@ -927,6 +927,47 @@ def test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks):
     assert torch.equal(got[alone], base[alone])
 
 
+@pytest.mark.parametrize("T,N,K", [(513, 256, 64), (545, 300, 200), (1000, 1000, 136), (2047, 640, 4096), (700, 4360, 72), (1024, 257, 64)])
+def test_products_of_cta_pairs(nat, T, N, K):
+    """Long steps at the edges of tiles: features that do not fill a tile of 256 or begin off 16 bytes in the output, ragged K, a last token tile of
+    a few rows, with a bias.  fp32 sums, rounded to bf16: 2^-9."""
+    g = torch.Generator("cuda").manual_seed(T + N)
+    x = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
+    b = torch.randn(N, generator=g, device="cuda").to(torch.bfloat16)
+    for bias in (b, None):
+        got = nat.gemm(x, w, bias=bias)
+        nat.workspace().check_status()
+        want = x.double() @ w.double().t() + (0 if bias is None else bias.double())
+        assert _rel_err(got, want) < 2 ** -8
+    wide = torch.full((T, N + 24), 7.0, dtype=torch.bfloat16, device="cuda")      # rows of a wider buffer: nothing beside them is written
+    nat.gemm(x, w, out=wide[:, :N])
+    assert torch.equal(wide[:, :N], nat.gemm(x, w)) and (wide[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("act", ["", "relu2", "swiglu"])
+@pytest.mark.parametrize("lengths,n_w,K", [([0, 1, 31, 32, 33, 255, 256, 257, 511, 0], 256, 128), ([700, 3, 290], 512, 72), ([400], 768, 64)])
+def test_expert_products_of_cta_pairs(nat, lengths, n_w, K, act):
+    """Runs around the edges of tiles, empty ones among them, with every activation of the epilogue.  bf16 results: 2^-9."""
+    g = torch.Generator("cuda").manual_seed(n_w + K)
+    rows, E = sum(lengths), len(lengths)
+    x = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, n_w, K, generator=g, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
+    seg = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), device="cuda", dtype=torch.int32)
+    got = nat.moe_grouped_gemm(x, w, seg, 256, act=act)
+    nat.workspace().check_status()
+    at = 0
+    for e, n in enumerate(lengths):
+        y = x[at: at + n].double() @ w[e].double().t()
+        if act == "relu2":
+            y = y.clamp_min(0) ** 2
+        elif act == "swiglu":
+            y = torch.nn.functional.silu(y[:, ::2]) * y[:, 1::2]
+        if n:
+            assert _rel_err(got[at: at + n], y) < 2 ** -8, (e, n)
+        at += n
+
+
 @pytest.mark.parametrize("T,E,k,H,I,e0,e_local", [(7, 8, 2, 512, 256, 0, 8), (256, 8, 2, 1024, 768, 0, 8), (300, 8, 2, 512, 256, 2, 2),
                                                   (1500, 16, 4, 256, 128, 0, 16), (64, 4, 1, 256, 384, 1, 1)])
 def test_moe_ffn_on_the_device(nat, T, E, k, H, I, e0, e_local):
