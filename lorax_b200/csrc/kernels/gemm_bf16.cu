@@ -181,7 +181,7 @@ struct GemmWork {
 
 // A stream-K tile the CTA has parked a partial for: summed after the CTA's last unit of work.
 struct PendingTile {
-  int ta, tb, counter, nparts, part_idx;
+  int i0, tb, counter, nparts, part_idx;      // i0: first of the tile's features (rows of operand A)
   long long red_first, red_base, red_stride;
 };
 
@@ -194,6 +194,12 @@ struct GemmWorkIter {
   __device__ GemmWorkIter(const GemmParams& p, int num_tiles_, int kblocks_)
       : num_tiles(num_tiles_), kblocks(kblocks_), split_k(p.split_k), grid((int)gridDim.x), cta((int)blockIdx.x),
         dp_tiles(p.split_k > 1 ? 0 : p.dp_tiles), sk_ctas(p.sk_ctas), i(0), phase(0) {
+    sk_units = (long long)(num_tiles - dp_tiles) * kblocks;
+    u = u_begin = u_end = 0;
+  }
+  // pair `cta_` of `grid_` pairs of CTAs
+  __device__ GemmWorkIter(const GemmParams& p, int num_tiles_, int kblocks_, int grid_, int cta_)
+      : num_tiles(num_tiles_), kblocks(kblocks_), split_k(1), grid(grid_), cta(cta_), dp_tiles(p.dp_tiles), sk_ctas(p.sk_ctas), i(0), phase(0) {
     sk_units = (long long)(num_tiles - dp_tiles) * kblocks;
     u = u_begin = u_end = 0;
   }
@@ -597,6 +603,93 @@ struct LoraBMaps { CUtensorMap m[4]; };
 
 LX_DEVICE void tensormap_fence_acquire_g(const CUtensorMap* m) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
+}
+
+// A stream-K tile that the CTA has parked a partial for: every contributor sums its share of the columns, 4 rows (16 bytes of every partial) per
+// thread and step (the four epilogue warps).  All contributors are running (one CTA per SM, each a consecutive K range of the same length), so the
+// wait for the others is short; it is bounded like every wait.  False: it ran out.
+LX_DEVICE bool gemm_sum_share(const GemmParams& p, const PendingTile& t, volatile int* abort_flag) {
+        if (threadIdx.x == 64) {
+          uint64_t t0 = 0;
+          uint32_t polls = 0;
+          while ((ld_acquire_gpu(&p.counters[t.counter]) & 0xffff) != t.nparts) {
+            if ((++polls & 255u) == 0) {
+              const uint64_t now = global_timer_ns();
+              if (t0 == 0) t0 = now;
+              else if (now - t0 > kWaitBudgetNs) {
+                report_status(p.status, kTimeoutSplitK, t.counter);
+                *abort_flag = 1;
+                break;
+              }
+            }
+          }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (*abort_flag != 0) return false;
+        const int j0 = t.tb * p.bn;
+        const int ncols = min(min(p.bn, p.umma_n), p.b_rows - j0);
+        const int c_lo = (int)((long long)ncols * t.part_idx / t.nparts), c_hi = (int)((long long)ncols * (t.part_idx + 1) / t.nparts);
+        const int tid4 = (int)threadIdx.x - 64;
+        const int items = (c_hi - c_lo) * (kBM / 4);
+        for (int it0 = tid4; it0 < items; it0 += 128 * 4) {
+          // four items per thread and pass, four partials of each in flight
+          float4 sum[4];
+          long long off[4];
+  #pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int it1 = min(it0 + 128 * e, items - 1);
+            sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+            off[e] = (long long)(c_lo + it1 / (kBM / 4)) * kBM + (it1 % (kBM / 4)) * 4;
+          }
+          for (int sp0 = 0; sp0 < t.nparts; sp0 += 4) {
+            float4 v[4][4];
+  #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int sp = min(sp0 + q, t.nparts - 1);
+              const float* src = p.ws + (sp == 0 ? t.red_first : t.red_base + sp * t.red_stride);
+  #pragma unroll
+              for (int e = 0; e < 4; ++e) v[q][e] = __ldcg(reinterpret_cast<const float4*>(src + off[e]));
+            }
+  #pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              if (sp0 + q < t.nparts) {
+  #pragma unroll
+                for (int e = 0; e < 4; ++e) { sum[e].x += v[q][e].x; sum[e].y += v[q][e].y; sum[e].z += v[q][e].z; sum[e].w += v[q][e].w; }
+              }
+            }
+          }
+  #pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int it1 = it0 + 128 * e;
+            if (it1 >= items) break;
+            const int c = c_lo + it1 / (kBM / 4), r4 = (it1 % (kBM / 4)) * 4;
+            const int i = t.i0 + r4, j = j0 + c;
+            float o[4] = {sum[e].x * p.out_scale, sum[e].y * p.out_scale, sum[e].z * p.out_scale, sum[e].w * p.out_scale};
+            if (p.bias != nullptr) {
+  #pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                if (p.bias_on_a) { if (i + h < p.a_rows) o[h] += __bfloat162float(p.bias[i + h]); }
+                else o[h] += __bfloat162float(p.bias[j]);
+              }
+            }
+            __nv_bfloat16* dst = p.out + (long long)i * p.ldo_a + (long long)j * p.ldo_b;
+            if (p.ldo_a == 1 && i + 4 <= p.a_rows && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+            } else {
+  #pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                if (i + h < p.a_rows) dst[(long long)h * p.ldo_a] = __float2bfloat16(o[h]);
+              }
+            }
+          }
+        }
+        // the last contributor to finish clears the counter for the next launch
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (threadIdx.x == 64) {
+          const int prev = atomicAdd(&p.counters[t.counter], 0x10000);
+          if ((prev >> 16) == t.nparts - 1) p.counters[t.counter] = 0;
+        }
+  return true;
 }
 
 template <int BN, int STAGES, bool LORA>
@@ -1086,7 +1179,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           // Stream-K: the contributors of a tile are different CTAs that finish at about the same time.  Count in now; after
           // its last unit of work every contributor sums its own share of the tile's columns (see below).
           if (threadIdx.x == 64) atomicAdd(&p.counters[w.counter], 1);
-          if (n_pending < 2) pending[n_pending++] = PendingTile{ta, tb, w.counter, w.nparts, w.part_idx, w.red_first, w.red_base, w.red_stride};
+          if (n_pending < 2) pending[n_pending++] = PendingTile{ta * kBM, tb, w.counter, w.nparts, w.part_idx, w.red_first, w.red_base, w.red_stride};
           acc ^= 1;
           continue;
         }
@@ -1155,91 +1248,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       }
       acc ^= 1;
     }
-    // ---- stream-K tiles this CTA contributed to: every contributor sums its share of the columns, 4 rows (16 bytes of
-    // every partial) per thread and step.  All contributors are running (one CTA per SM, each a consecutive K range of the
-    // same length), so the wait for the others is short; it is bounded like every wait.
     for (int pi = 0; alive && pi < n_pending; ++pi) {
-      const PendingTile t = pending[pi];
-      if (threadIdx.x == 64) {
-        uint64_t t0 = 0;
-        uint32_t polls = 0;
-        while ((ld_acquire_gpu(&p.counters[t.counter]) & 0xffff) != t.nparts) {
-          if ((++polls & 255u) == 0) {
-            const uint64_t now = global_timer_ns();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > kWaitBudgetNs) {
-              report_status(p.status, kTimeoutSplitK, t.counter);
-              *abort_flag = 1;
-              break;
-            }
-          }
-        }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (*abort_flag != 0) break;
-      const int j0 = t.tb * p.bn;
-      const int ncols = min(min(p.bn, p.umma_n), p.b_rows - j0);
-      const int c_lo = (int)((long long)ncols * t.part_idx / t.nparts), c_hi = (int)((long long)ncols * (t.part_idx + 1) / t.nparts);
-      const int tid4 = (int)threadIdx.x - 64;
-      const int items = (c_hi - c_lo) * (kBM / 4);
-      for (int it0 = tid4; it0 < items; it0 += 128 * 4) {
-        // four items per thread and pass, four partials of each in flight
-        float4 sum[4];
-        long long off[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int it1 = min(it0 + 128 * e, items - 1);
-          sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-          off[e] = (long long)(c_lo + it1 / (kBM / 4)) * kBM + (it1 % (kBM / 4)) * 4;
-        }
-        for (int sp0 = 0; sp0 < t.nparts; sp0 += 4) {
-          float4 v[4][4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int sp = min(sp0 + q, t.nparts - 1);
-            const float* src = p.ws + (sp == 0 ? t.red_first : t.red_base + sp * t.red_stride);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v[q][e] = __ldcg(reinterpret_cast<const float4*>(src + off[e]));
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (sp0 + q < t.nparts) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) { sum[e].x += v[q][e].x; sum[e].y += v[q][e].y; sum[e].z += v[q][e].z; sum[e].w += v[q][e].w; }
-            }
-          }
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int it1 = it0 + 128 * e;
-          if (it1 >= items) break;
-          const int c = c_lo + it1 / (kBM / 4), r4 = (it1 % (kBM / 4)) * 4;
-          const int i = t.ta * kBM + r4, j = j0 + c;
-          float o[4] = {sum[e].x * p.out_scale, sum[e].y * p.out_scale, sum[e].z * p.out_scale, sum[e].w * p.out_scale};
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              if (p.bias_on_a) { if (i + h < p.a_rows) o[h] += __bfloat162float(p.bias[i + h]); }
-              else o[h] += __bfloat162float(p.bias[j]);
-            }
-          }
-          __nv_bfloat16* dst = p.out + (long long)i * p.ldo_a + (long long)j * p.ldo_b;
-          if (p.ldo_a == 1 && i + 4 <= p.a_rows && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-            *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
-          } else {
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              if (i + h < p.a_rows) dst[(long long)h * p.ldo_a] = __float2bfloat16(o[h]);
-            }
-          }
-        }
-      }
-      // the last contributor to finish clears the counter for the next launch
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (threadIdx.x == 64) {
-        const int prev = atomicAdd(&p.counters[t.counter], 0x10000);
-        if ((prev >> 16) == t.nparts - 1) p.counters[t.counter] = 0;
-      }
+      if (!gemm_sum_share(p, pending[pi], abort_flag)) break;
     }
   }
 
@@ -1556,6 +1566,8 @@ static int launch_gemm_t(const CUtensorMap& ta, const CUtensorMap& tb, const Lor
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
+constexpr double kTileFixedNs = 2500.0;      // what a unit of work pays for its ramp
+
 }  // namespace lx
 #include "gemm_pair.cuh"
 namespace lx {
@@ -1574,12 +1586,16 @@ static int make_tmap_lora_images(CUtensorMap* out, const void* base, uint64_t ro
 }
 
 template <bool LORA>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ti, const LoraBMaps& bm, const GemmParams& base, int bn, int pairs,
-                       cudaStream_t stream) {
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ti, const LoraBMaps& bm, const GemmParams& base, const PairPlan& plan,
+                       int pairs, cudaStream_t stream) {
+  if (pairs < plan.grid) return 1;      // (the plan's pairs run at the same time)
   GemmParams p = base;
-  p.bn = p.umma_n = bn;
-  const int tiles = (p.a_rows + 255) / 256 * ((p.b_rows + bn - 1) / bn);
-  const int grid = 2 * (tiles < pairs ? tiles : pairs);
+  p.bn = p.umma_n = plan.bn;
+  p.split_k = 1;
+  p.dp_tiles = plan.dp_tiles;
+  p.sk_ctas = plan.sk_pairs;
+  p.w_preload = p.w_preload != 0 && p.overlap;
+  const int grid = 2 * plan.grid;
   launch_pdl_cluster(gemm_pair_kernel<LORA>, dim3(grid), dim3(kGemmThreads), dim3(2, 1, 1), (size_t)PairSmem<LORA>::kTotal, stream, ta, tb, ti, bm, p);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -1598,7 +1614,6 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
 // L2 and the last contributor pays the sum.  Constants fitted to sweeps on B200.
 constexpr double kFillBytesPerNs = 95.0;
 constexpr double kFlopPerNs = 11000.0;
-constexpr double kTileFixedNs = 2500.0;
 
 struct GemmPlan {
   int bn, split, dp_tiles, sk_ctas, grid;
@@ -1608,7 +1623,10 @@ struct GemmPlan {
 // Steps of thousands of rows lose by an early start of the next kernel (see pdl_trigger).  Where the line lies matters little: passes of 300 to
 // 2500 rows took the same within 1 % with limits of 128, 512 and 2048.
 constexpr int kOverlapMaxTokens = 512;
-constexpr int kPairMinTokens = 512;            // longer steps take pairs of CTAs
+// Longer steps take pairs of CTAs.  The four projections of a 7B layer, us, one CTA a tile / pairs: 137 rows 133 / 156 (a pair's tile of 160 tokens leaves the
+// weights, which HBM has to bring, too few of the bytes in flight), 200 150 / 149, 256 158 / 156 (with 65 adapters a pass of four layers 1711 / 1677), 384
+// 193 / 197, 512 236 / 222, 1500 535 / 530, 4001 1362 / 1290.
+constexpr int kPairMinTokens = 192;
 constexpr int kModeConstWeights = 1 << 16;     // of a launch's `mode`: no kernel that may still run writes the weights
 
 constexpr int kClassicSplitTokens = 32;
@@ -1782,7 +1800,9 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     pl_swap = choose_plan_swap(T, N, K, num_sms, usable_ws, have_counters, force_split & 0xffff, force_bn, sk_policy);
     swap = pl_swap.cost <= pl_tok.cost;
   }
-  const int pair_bn = T > kPairMinTokens && N >= 256 && (mode == 0 || has_lora) && force_split == 0 && sk_policy == 0 ? pair_token_tile(T, N, num_sms / 2) : 0;
+  PairPlan pair{};
+  if (T > kPairMinTokens && N >= 256 && (mode <= 1 || has_lora) && force_split == 0 && sk_policy == 0)
+    pair = pair_plan(T, N, K, num_sms / 2, usable_ws);
   p.overlap = T <= kOverlapMaxTokens;
   if (swap) {
     p.a_rows = N; p.b_rows = T;
@@ -1867,15 +1887,20 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       const int rc = launch_lora_shrink_rows(sp, lora->max_rank, num_sms, stream);
       if (rc != 0) return rc;
     }
-    if (pair_bn > 0 && p.lora_inline_shrink && (lora->nparts == 1 || (lora->n0 % 256 == 0 && (lora->nparts == 2 || lora->n1 % 256 == 0))) &&
+    if (pair.bn > 0 && p.lora_inline_shrink && (lora->nparts == 1 || (lora->n0 % 256 == 0 && (lora->nparts == 2 || lora->n1 % 256 == 0))) &&
         img_bytes / 48 * 64 <= lora->vimg_bytes) {
       const int pairs = pair_capacity<true>();
-      CUtensorMap ti;
-      if (pairs * 2 >= 2 && make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32)) == 0 && make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair_bn / 2) == 0) {
-        p.lora_mask = 31;
-        p.lora_slice = 64 * 16;
-        p.lora_kparts = nullptr;
-        return launch_pair<true>(ta, tb, ti, bm, p, pair_bn, pairs, stream);
+      CUtensorMap ti, tb2;
+      if (pairs > 0 && make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32)) == 0 && make_tmap_bf16_kmajor(&tb2, x, T, K, ldx, pair.bn / 2) == 0) {
+        GemmParams q = p;
+        q.lora_mask = 31;
+        q.lora_slice = 64 * 16;
+        const long long img64 = img_bytes / 48 * 64, grid = 2ll * pair.grid;
+        const bool shared_k = lora->sync_ints >= 2 + grid && lora->vimg_bytes - img64 >= grid * 128 * 4;
+        q.lora_kparts = shared_k ? reinterpret_cast<float*>(static_cast<char*>(lora->vimg) + img64) : nullptr;
+        q.lora_kcounters = lora->sync + 2;
+        const int rc = launch_pair<true>(ta, tb2, ti, bm, q, pair, pairs, stream);
+        if (rc != 1) return rc;
       }
     }
     switch (template_bn(bn)) {
@@ -1886,14 +1911,17 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       default:  return launch_gemm_t<256, 4, true>(ta, tb, bm, p, pl.grid, stream);
     }
   }
-  if (pair_bn > 0) {
+  if (pair.bn > 0) {
     const int pairs = pair_capacity<false>();
     if (pairs > 0) {
-      if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
-      if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair_bn / 2)) return -1003;
-      p.a_rows = N; p.b_rows = T;
-      p.ldo_a = 1; p.ldo_b = ldo;
-      return launch_pair<false>(ta, tb, ta, LoraBMaps{}, p, pair_bn, pairs, stream);
+      CUtensorMap ta2, tb2;
+      if (make_tmap_bf16_kmajor(&ta2, w, N, K, ldw, kBM)) return -1002;
+      if (make_tmap_bf16_kmajor(&tb2, x, T, K, ldx, pair.bn / 2)) return -1003;
+      GemmParams q = p;
+      q.a_rows = N; q.b_rows = T;
+      q.ldo_a = 1; q.ldo_b = ldo; q.bias_on_a = 1;
+      const int rc = launch_pair<false>(ta2, tb2, ta2, LoraBMaps{}, q, pair, pairs, stream);
+      if (rc != 1) return rc;
     }
   }
   switch (template_bn(bn)) {

@@ -3,9 +3,11 @@
 // A pair takes a tile of 256 output features x up to 256 tokens: each CTA loads 128 rows of the weights and half of the tokens, 32 KB a stage
 // where one CTA on its own tile of 128 x 256 takes 48, and reads half the token operand from its shared memory per MMA: what a single CTA
 // moves in and out of shared memory per product is the limit of gemm_bf16_tcgen05_kernel at these sizes (192 of about 128 B per cycle asked for).
+// 4001 rows, 28672 x 4096: 703 -> 630 us, the tensor pipe 90 % active at the 1.5 GHz that the power limit leaves.  Operands carry no eviction hints: the
+// pairs of a wave share weight tiles and token tiles through L2 (weights evicted early cost 2 to 3 % of a pass).
 // Rank 0's MMA thread issues for both; a stage is full when the loads of both CTAs have arrived at rank 0's barrier, and its commits
-// tell both that a stage is free or an accumulator complete.  Tiles are whole (no split of K): the token tile is chosen so that the last
-// wave is nearly full.  LoRA as there: shrink on the epilogue warps of all CTAs during the first K loop, expand by MMAs into the
+// tell both that a stage is free or an accumulator complete.  Whole tiles and the stream-K remainder as there, each CTA with its half of a tile's
+// partial sums.  LoRA as there: shrink on the epilogue warps of all CTAs during the first K loop, expand by MMAs into the
 // accumulators, whose columns come in steps of 32 here (an entry's window: 64 rows, 32-aligned); each CTA brings its features' B_cat and half of the
 // window's rows.  One row of ranks serves both CTAs, so parts must begin at multiples of 256.
 #pragma once
@@ -32,6 +34,9 @@ struct PairSmem {
   static constexpr int kTotal = kPairStages * kStageBytes + kBarrierBytes + kEntBytes + kEpiBytes + 1024;
   static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
 };
+
+using PairIter = GemmWorkIter<256>;
+constexpr double kPairFillBytesPerNs = 95.0, kPairSumBytesPerNs = 8.0;
 
 template <bool LORA>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -84,8 +89,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       load_lora_entries(p, ents, n_live);
       __syncthreads();
       if (warp == 2) lora_unit_prefix(p, ents, gstart);
-      if (warp == 0 && pair < num_tiles) {
-        const int ta0 = pair / tiles_b, tb0 = pair % tiles_b;
+      PairIter it0(p, num_tiles, kblocks, pairs, pair);
+      GemmWork w0;
+      if (warp == 0 && it0.next(w0) && w0.kb0 == 0) {
+        const int ta0 = w0.tile / tiles_b, tb0 = w0.tile % tiles_b;
         const int n0 = lora_prebuild_units(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.bn, ulist);
         if (n0 >= 0) { pre_tb = tb0; pre_n = n0; }
         if (n0 > 0) lora_prefetch_b(p, ulist, n0, 2 * ta0 + (int)rank);
@@ -93,20 +100,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       __syncthreads();
     }
   }
+  // (see gemm_bf16_tcgen05_kernel: constant weights of the first stages, ahead of the wait)
+  int preloaded = 0;
+  if (threadIdx.x == 0 && p.w_preload) {
+    PairIter it0(p, num_tiles, kblocks, pairs, pair);
+    GemmWork w0;
+    if (it0.next(w0)) {
+      preloaded = min(kPairStages, w0.kb1 - w0.kb0);
+      for (int s = 0; s < preloaded; ++s) {
+        if (rank == 0) mbar_expect_tx(&full_bar[s], 2u * (uint32_t)(S::kABytes + half * kBK * 2));
+        pair_load_2d(tiles + s * S::kStageBytes, &tmap_a, pair_map(&full_bar[s], 0), (w0.kb0 + s) * kBK, (2 * (w0.tile / tiles_b) + (int)rank) * kBM);
+      }
+    }
+  }
   pdl_wait();
 
   if (warp == 0) {
-    const uint64_t pol_a = policy_evict_first(), pol_b = policy_evict_last();
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     int list_tb = pre_tb, list_n = pre_n;
     bool first_tile = pre_tb >= 0, shrink_seen = false;
-    for (int tile = pair; tile < num_tiles; tile += pairs) {
-      const int ta = tile / tiles_b, tb = tile % tiles_b;
+    PairIter it(p, num_tiles, kblocks, pairs, pair);
+    GemmWork w;
+    while (it.next(w)) {
+      const int tile = w.tile, ta = tile / tiles_b, tb = tile % tiles_b;
       const int i0 = (2 * ta + (int)rank) * kBM, j0 = tb * p.bn, jlim = j0 + p.bn;
       if constexpr (LORA) {
-        if (lora) {
+        if (lora && w.kb0 == 0) {
           if (list_tb != tb) {
             const int n0 = lora_prebuild_units(p, ents, *n_live, j0, jlim, ulist);
             list_tb = n0 >= 0 ? tb : -1;
@@ -117,8 +138,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
       }
       if (lane == 0 && ok) {
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+          const bool have = preloaded > 0;
+          if (have) {
+            --preloaded;
+          } else if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
             report_status(p.status, kTimeoutEmptyBarrier, tile);
             *abort_flag = 1;
             ok = false;
@@ -126,14 +150,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           uint8_t* sa = tiles + stage * S::kStageBytes;
           const uint32_t bar = pair_map(&full_bar[stage], 0);
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)(S::kABytes + half * kBK * 2));
-          pair_load_2d(sa, &tmap_a, bar, kb * kBK, i0);
+          if (rank == 0 && !have) mbar_expect_tx(&full_bar[stage], 2u * (uint32_t)(S::kABytes + half * kBK * 2));
+          if (!have) pair_load_2d(sa, &tmap_a, bar, kb * kBK, i0);
           pair_load_2d(sa + S::kABytes, &tmap_b, bar, kb * kBK, j0 + (int)rank * half);
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
         }
       }
       if constexpr (LORA) {
-        if (lora) {
+        if (lora && w.kb0 == 0) {
           __syncwarp();
           stage = __shfl_sync(0xffffffffu, stage, 0);
           phase = __shfl_sync(0xffffffffu, phase, 0);
@@ -211,6 +235,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
     __syncwarp();
+    if (p.overlap) pdl_launch_dependents();      // the last loads of this CTA are on their way: the next kernel's blocks may be set up
   } else if (warp == 1) {
     if (rank == 0 && lane == 0) {
       const uint32_t idesc = make_idesc(2 * kBM, (uint32_t)p.bn, kFmtBF16, kFmtBF16);
@@ -219,7 +244,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       int acc = 0;
       uint32_t acc_phase[2] = {0, 0};
       bool ok = true;
-      for (int tile = pair; ok && tile < num_tiles; tile += pairs) {
+      PairIter it(p, num_tiles, kblocks, pairs, pair);
+      GemmWork w;
+      while (ok && it.next(w)) {
+        const int tile = w.tile;
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * 256);
         if (!pair_wait(&tmem_empty[acc], acc_phase[acc] ^ 1, abort_flag)) {
           report_status(p.status, kTimeoutTmemEmpty, tile);
@@ -227,7 +255,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           break;
         }
         tc_fence_after();
-        for (int kb = 0; kb < kblocks; ++kb) {
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
             report_status(p.status, kTimeoutFullBarrier, tile);
             *abort_flag = 1;
@@ -238,12 +266,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           const uint32_t sa = smem_u32(tiles + stage * S::kStageBytes);
           const uint64_t da = make_desc_k_sw128(sa), db = make_desc_k_sw128(sa + S::kABytes);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) pair_mma(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; ++k) pair_mma(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
           pair_commit(&empty_bar[stage]);
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
         }
         if constexpr (LORA) {
-          bool more = lora && ok;
+          bool more = lora && ok && w.kb0 == 0;
           while (more) {
             if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
               report_status(p.status, kTimeoutFullBarrier, tile);
@@ -281,16 +309,48 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (lora) lora_shrink_units(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
     }
     const bool turn = p.ldo_a == 1 && (p.ldo_b & 7) == 0 && (p.a_rows & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-    for (int tile = pair; tile < num_tiles; tile += pairs) {
-      const int ta = tile / tiles_b, tb = tile % tiles_b;
+    PendingTile pending[2];
+    int n_pending = 0;
+    bool alive = true;
+    PairIter it(p, num_tiles, kblocks, pairs, pair);
+    GemmWork w;
+    while (it.next(w)) {
+      const int tile = w.tile, ta = tile / tiles_b, tb = tile % tiles_b;
       if (!mbar_wait(&tmem_full[acc], acc_phase[acc], abort_flag)) {
         report_status(p.status, kTimeoutTmemFull, tile);
         *abort_flag = 1;
+        alive = false;
         break;
       }
       tc_fence_after();
       acc_phase[acc] ^= 1;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256);
+      if (w.nparts > 0) {
+        // part of a tile's K: both CTAs park their half, [column][128 features] fp32, and count in; the sums follow behind the last unit
+        constexpr long long kPart = 256ll * kBM;
+        float* wsp = p.ws + 2 * w.part_off + rank * kPart + quad * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < p.bn; c += 32) {
+          if (tb * p.bn + c >= p.b_rows) break;
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(taddr + c, r);
+          tc_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 32; ++q) __stcg(wsp + (long long)(c + q) * kBM, __uint_as_float(r[q]));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) pair_arrive(pair_map(&tmem_empty[acc], 0));
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int counter = 2 * w.counter + (int)rank;
+        if (threadIdx.x == 64) atomicAdd(&p.counters[counter], 1);
+        if (n_pending < 2)
+          pending[n_pending++] = PendingTile{(2 * ta + (int)rank) * kBM, tb, counter, w.nparts, w.part_idx, 2 * w.red_first + rank * kPart,
+                                             2 * w.red_base + rank * kPart, 2 * w.red_stride};
+        acc ^= 1;
+        continue;
+      }
       const int f0 = (2 * ta + (int)rank) * kBM + quad * 32, i = f0 + lane;
       const int j0 = tb * p.bn, jend = min(p.b_rows, j0 + p.bn);
       const float bias_i = (p.bias != nullptr && i < p.a_rows) ? __bfloat162float(p.bias[i]) : 0.f;
@@ -326,6 +386,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (lane == 0) pair_arrive(pair_map(&tmem_empty[acc], 0));
       acc ^= 1;
     }
+    for (int i = 0; alive && i < n_pending; ++i) alive = gemm_sum_share(p, pending[i], abort_flag);
   }
 
   tc_fence_before();
@@ -355,15 +416,32 @@ static int pair_capacity() {
   return pair_capacity_of(gemm_pair_kernel<LORA>, kGemmThreads, PairSmem<LORA>::kTotal, known);
 }
 
-// The token tile, a multiple of 32, whose waves of whole tiles cost least.  A tile takes as long as its operands take to come in from L2, 128 rows
-// of weights and half its tokens per CTA (their MMAs need less than that), and some for its start.
-static int pair_token_tile(int T, int N, int pairs) {
-  int best = 256;
-  long long cost = -1;
-  for (int bn = 256; bn >= 96; bn -= 32) {
-    const long long tiles = (long long)((N + 255) / 256) * ((T + bn - 1) / bn);
-    const long long c = (tiles + pairs - 1) / pairs * (kBM + bn / 2 + 16);
-    if (cost < 0 || c < cost) { cost = c; best = bn; }
+struct PairPlan {
+  int bn, dp_tiles, sk_pairs, grid;      // token tile (0: no plan); whole tiles; pairs that share the K of the others; pairs
+  double cost;                           // ns
+};
+// The token tile, a multiple of 32, that costs least.  A k-block takes as long as its operands take to come in from L2, 128 rows of weights and
+// half its tokens per CTA (their MMAs need less than that); a tile has a start, and the sums of a shared one their trips through L2.
+// (ws_bytes: scratch of the sums; without it all tiles are whole.)
+static PairPlan pair_plan(int T, int N, int K, int pairs, long long ws_bytes) {
+  PairPlan best{};
+  best.cost = 1e30;
+  const int kblocks = (K + kBK - 1) / kBK, tiles_a = (N + 255) / 256;
+  const int top = (T + 31) / 32 * 32 < 256 ? (T + 31) / 32 * 32 : 256;
+  for (int bn = top; bn >= 32; bn -= 32) {
+    const long long tiles = (long long)tiles_a * ((T + bn - 1) / bn);
+    const double block = (kBM + bn / 2) * 128.0 / kPairFillBytesPerNs, start = kTileFixedNs;
+    const long long full = tiles / pairs, rest = tiles - full * pairs;
+    PairPlan w{bn, (int)tiles, 0, (int)(tiles < pairs ? tiles : pairs), (double)(full + (rest ? 1 : 0)) * (kblocks * block + start)};
+    if (w.cost < best.cost) best = w;
+    if (rest == 0) continue;
+    long long sk = pairs;
+    if (sk > rest * kblocks / 2) sk = rest * kblocks / 2;
+    if (sk > 15 * rest) sk = 15 * rest;
+    if (sk <= rest || sk * 4 * 256 * kBM * 4 > ws_bytes) continue;
+    const double parts = (double)kBM * bn * 4.0 / kPairSumBytesPerNs + 2500.0;
+    PairPlan q{bn, (int)(full * pairs), (int)sk, full ? pairs : (int)sk, full * (kblocks * block + start) + (double)rest * kblocks / sk * block + start + parts};
+    if (q.cost < best.cost) best = q;
   }
   return best;
 }

@@ -865,7 +865,7 @@ def test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout):
 
 @pytest.mark.parametrize("T,K,parts,ranks,layout", [(2, 4096, [512, 128, 128], [16], "alternating"), (2, 14336, [512], [64], "alternating"),
                                                     (5, 3080, [768, 768], [16, 64, 32, 48], "alternating"), (6, 1000, [512], [32, 16], "alternating"),
-                                                    (29, 4096, [4096, 1024, 1024], [16, 32], "runs"), (90, 2048, [512], [16], "runs")])
+                                                    (29, 4096, [4096, 1024, 1024], [16, 32], "runs"), (90, 2048, [512], [16], "runs"), (210, 4096, [2048, 512, 512], [16, 64, 32, 16], "blocks")])
 def test_gemm_with_lora_of_few_units(nat, T, K, parts, ranks, layout):
     """Steps with fewer shrink units than CTAs, which share the K of each: one row, K of a part of a batch and of a ragged last one."""
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
@@ -927,9 +927,9 @@ def test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks):
     assert torch.equal(got[alone], base[alone])
 
 
-@pytest.mark.parametrize("T,N,K", [(513, 256, 64), (545, 300, 200), (1000, 1000, 136), (2047, 640, 4096), (700, 4360, 72), (1024, 257, 64)])
+@pytest.mark.parametrize("T,N,K", [(193, 256, 64), (200, 6144, 4096), (256, 4096, 14336), (320, 28672, 256), (513, 256, 64), (545, 300, 200), (1000, 1000, 136), (2047, 640, 4096), (700, 4360, 72), (1024, 257, 64)])
 def test_products_of_cta_pairs(nat, T, N, K):
-    """Long steps at the edges of tiles: features that do not fill a tile of 256 or begin off 16 bytes in the output, ragged K, a last token tile of
+    """Long steps at the edges of tiles, whole ones and shared: features that do not fill a tile of 256 or begin off 16 bytes in the output, ragged K, a last token tile of
     a few rows, with a bias.  fp32 sums, rounded to bf16: 2^-9."""
     g = torch.Generator("cuda").manual_seed(T + N)
     x = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
