@@ -1,8 +1,8 @@
 // Ragged causal prefill attention over the paged KV cache on the 5th-generation tensor cores.
 //
 // One CTA = one 64-query tile of one sequence x TWO or FOUR query heads of the same KV group: the 128 rows of a tcgen05 M tile are
-// (head, query) pairs of two heads, a CTA has NT = 1 or 2 such tiles (two where the group's heads divide by four), and a K / V block is
-// staged once for all of them.  Keys are walked in blocks of 128 (four cache pages):
+// (head, query) pairs of two heads, a CTA has NT = 1 or 2 such tiles (two where the group's heads divide by four and there is more than
+// a wave of them), and a K / V block is staged once for all of them.  Keys are walked in blocks of 128 (four cache pages):
 //
 //   loader  (warp 0, one lane)  Q by TMA from the projection output; K and V pages by TMA straight from the paged cache
 //                               through one 5-D tensor map {d, slot, K|V, kv head, block}: the block table supplies the last
@@ -18,7 +18,7 @@
 // the tensor core (S 950: at N = 128 both operands come from shared memory at its full rate; P V 600).  One tile per CTA has them in a chain
 // (S, softmax, P V, S, ...), 4700 cycles with P through shared memory; two tiles fill each other's gaps, and P in TMEM spares the stores and
 // half of P V's shared memory.  32 heads, 8 KV heads, one tile per CTA and P in shared memory -> this: 8192 tokens 1021 -> 579 us, seven prompts
-// of together 4001 134 -> 70, three of 1700 57 -> 31, 137 tokens 15.9 -> 14.0 (products alone: 368 us of the 579).
+// of together 4001 132 -> 77, three of 1700 56 -> 34, 137 tokens 11.5 -> 10.6 (products alone: 368 us of the 579).
 //
 // WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, side by side in
 // TMEM, and P V is two products into the same accumulator (the layer-by-layer designs ask for it).
@@ -600,9 +600,13 @@ static int launch_fa_t(const CUtensorMap& tq, const CUtensorMap& tkv, const FaPa
   launch_pdl(attn_prefill_tc_kernel<WIDE, NT>, dim3(p.nh / (2 * NT), num_tiles), dim3(S::kThreads), (size_t)S::kTotal, s, tq, tkv, p);
   return -(int)cudaGetLastError();
 }
+// Two tiles a CTA where the group allows it and single ones would take more than one wave.  In one wave a tile on its own is quicker: 123 tokens of 32
+// heads 11.6 -> 8.7 us, 500 18.3 -> 14.4; 15 tiles of 64 queries of three prompts, 240 CTAs, 15.2 with two tiles against 19.6.
+constexpr long long kFaSpreadTiles = 148;
 template <bool WIDE>
 static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const FaParams& p, int num_tiles, cudaStream_t s) {
-  return p.group % 4 == 0 ? launch_fa_t<WIDE, 2>(tq, tkv, p, num_tiles, s) : launch_fa_t<WIDE, 1>(tq, tkv, p, num_tiles, s);
+  return p.group % 4 == 0 && (long long)num_tiles * (p.nh / 2) > kFaSpreadTiles ? launch_fa_t<WIDE, 2>(tq, tkv, p, num_tiles, s)
+                                                                               : launch_fa_t<WIDE, 1>(tq, tkv, p, num_tiles, s);
 }
 
 static int attn_prefill_tc(const void* q, long long ldq, int T, const void* kv, int num_blocks, const int* block_tables, int max_blocks,
