@@ -608,7 +608,7 @@ LX_DEVICE void tensormap_fence_acquire_g(const CUtensorMap* m) {
 // A stream-K tile that the CTA has parked a partial for: every contributor sums its share of the columns, 4 rows (16 bytes of every partial) per
 // thread and step (the four epilogue warps).  All contributors are running (one CTA per SM, each a consecutive K range of the same length), so the
 // wait for the others is short; it is bounded like every wait.  False: it ran out.
-LX_DEVICE bool gemm_sum_share(const GemmParams& p, const PendingTile& t, volatile int* abort_flag) {
+LX_DEVICE bool gemm_sum_share(const GemmParams& p, const PendingTile t, volatile int* abort_flag) {
         if (threadIdx.x == 64) {
           uint64_t t0 = 0;
           uint32_t polls = 0;
