@@ -306,8 +306,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;      // later tiles of a sequence see more keys: start the long ones first
-  const int hc = blockIdx.x * 2 * NT;            // first of the CTA's query heads
+  const int head_groups = p.nh / (2 * NT);
+  const int tile = ((int)gridDim.x - 1 - (int)blockIdx.x) / head_groups;      // later tiles of a sequence see more keys: start the long ones first
+  const int hc = (int)blockIdx.x % head_groups * 2 * NT;      // first of the CTA's query heads
   const int kvh = hc / p.group;
 
   if (threadIdx.x == 0) {
@@ -597,7 +598,7 @@ static int launch_fa_t(const CUtensorMap& tq, const CUtensorMap& tkv, const FaPa
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   // the heads of a query tile run side by side (they share its keys' pages where they share a KV head), long tiles first
-  launch_pdl(attn_prefill_tc_kernel<WIDE, NT>, dim3(p.nh / (2 * NT), num_tiles), dim3(S::kThreads), (size_t)S::kTotal, s, tq, tkv, p);
+  launch_pdl(attn_prefill_tc_kernel<WIDE, NT>, dim3(num_tiles * (p.nh / (2 * NT))), dim3(S::kThreads), (size_t)S::kTotal, s, tq, tkv, p);
   return -(int)cudaGetLastError();
 }
 // Two tiles a CTA where the group allows it and single ones would take more than one wave.  In one wave a tile on its own is quicker: 123 tokens of 32
