@@ -583,16 +583,23 @@ LX_DEVICE int lora_prebuild_units(const GemmParams& p, const LoraEnt* ents, int 
   return n;
 }
 
+// Bytes of B_cat that the features of tile `ta` have at rank r; none where all N features lie in front of the tile, as they may for the second CTA
+// of a pair.
+__host__ __device__ constexpr uint32_t lora_tile_bytes(int N, int ta, int r) {
+  const int rows = N - ta * kBM;
+  return rows <= 0 ? 0u : (uint32_t)((rows < kBM ? rows : kBM) * r * 2);
+}
+
 // Pulls the B_cat rows that feature tile `ta` needs for the units of `list` into L2 (whole warp; adapter weights, which no kernel
 // of a step writes, so this may run before the kernel in front has drained).
 LX_DEVICE void lora_prefetch_b(const GemmParams& p, const LoraUnit* list, int n, int ta) {
-  const int rows = min(kBM, p.a_rows - ta * kBM);
+  if (lora_tile_bytes(p.a_rows, ta, 16) == 0) return;
   for (int u = threadIdx.x & 31; u < n; u += 32) {
     const LoraUnit q = list[u];
     if ((q.img & 3) == 0) {
       const int r = (q.rclass + 1) * 16;
       const char* src = reinterpret_cast<const char*>(p.lora_arena) + (long long)q.boff * 16 + (long long)ta * kBM * r * 2;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"((uint32_t)(rows * r * 2)) : "memory");
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(lora_tile_bytes(p.a_rows, ta, r)) : "memory");
     }
   }
 }
@@ -1940,6 +1947,9 @@ int lx_gemm_plan(int T, int N, int K, int num_sms, long long ws_bytes, int force
   out5[0] = pl.bn; out5[1] = pl.split; out5[2] = pl.dp_tiles; out5[3] = pl.sk_ctas; out5[4] = pl.grid;
   return 0;
 }
+
+// Bytes of B_cat (rank r, N features) that the CTA with feature tile `tile` of 128 prefetches.
+unsigned lx_lora_tile_bytes(int N, int tile, int r) { return lx::lora_tile_bytes(N, tile, r); }
 
 // out[T, N] = x[T, K] @ w[N, K]^T (+ bias[N]).  `ldx`, `ldw`, `ldo` are row strides in elements.
 // mode: low byte 0 = choose, 1 = force weights on the M side (small T), 2 = force activations on the M side; bits 8..9 the

@@ -54,3 +54,13 @@ def test_triggers_stand_behind_the_wait():
 def test_classic_split_only_where_it_measured_quicker(T, N, K, parts):
     from lorax_b200.ops import native
     assert native.gemm_plan(T, N, K)["split"] == parts
+
+
+@pytest.mark.parametrize("r", [16, 64])
+@pytest.mark.parametrize("N", [128, 256, 320, 384, 448, 896, 1600, 2880, 4096])
+def test_prefetches_of_adapter_rows_stay_inside(N, r):
+    """A pair of CTAs covers 256 features, 128 each: past the last feature there is nothing to fetch, and what the tiles fetch is B_cat once."""
+    from lorax_b200.ops import native
+    sizes = [native.load().lx_lora_tile_bytes(N, tile, r) for tile in range((N + 255) // 256 * 2)]
+    assert sum(sizes) == N * r * 2
+    assert all(size % 16 == 0 and tile * 128 * r * 2 + size <= N * r * 2 for tile, size in enumerate(sizes) if size)

@@ -871,6 +871,15 @@ def test_gemm_with_lora_of_few_units(nat, T, K, parts, ranks, layout):
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
 
 
+@pytest.mark.parametrize("T,K,parts,ranks,layout", [(200, 256, [320], [16, 32], "runs"), (257, 1024, [384], [64, 16], "blocks"), (300, 512, [448], [16, 48, 64, 32], "alternating"),
+                                                    (520, 136, [512, 256, 320], [16, 64], "runs"), (600, 256, [12864], [32, 16], "runs"), (600, 128, [12800, 200], [16], "blocks"),
+                                                    (700, 4096, [2880], [16, 64, 32], "runs")])
+def test_gemm_with_lora_of_ragged_pairs(nat, T, K, parts, ranks, layout):
+    """Pairs of CTAs whose last tile of 256 features is not full, the second CTA's half partly or all past the last feature: one part and several, a tile a
+    pair and more."""
+    test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
+
+
 @pytest.mark.parametrize("form", ["fp8", "wq4"])
 @pytest.mark.parametrize("T,K,parts,ranks", [(1, 512, [128], [16]), (5, 1024, [256, 128, 128], [16, 64]), (8, 512, [1024], [48]), (9, 2048, [512, 512], [32, 16]),
                                              (32, 4096, [384, 128, 128], [16, 32, 48, 64]), (77, 512, [256], [32, 16]), (256, 512, [16384], [16, 64]),
