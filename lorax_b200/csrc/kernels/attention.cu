@@ -49,7 +49,7 @@ int lx_attn_page_size() { return lx::kPage; }
 // part_o / part_lse are only touched when nsplit > 1: sizes T*nh*nsplit*D and T*nh*nsplit floats.
 int lx_attn_decode_alibi(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
                          void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                         float softcap, int nsplit, const float* alibi, void* stream);
+                         float softcap, int nsplit, const float* alibi, int ahead, void* stream);
 int lx_attn_prefill_alibi(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* cu_q,
                           const int* cache_lens, const int* tile_seq, const int* tile_q0, int num_tiles, void* out, long long ldo, int nh,
                           int nkv, int d, int window, float scale, float softcap, const float* alibi, void* stream);
@@ -58,12 +58,12 @@ int lx_attn_decode(const void* q, long long ldq, const void* kv, const int* bloc
                    void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
                    float softcap, int nsplit, void* stream) {
   return lx_attn_decode_alibi(q, ldq, kv, block_tables, max_blocks, ctx_lens, out, ldo, part_o, part_lse, T, nh, nkv, d, window, scale,
-                              softcap, nsplit, nullptr, stream);
+                              softcap, nsplit, nullptr, 0, stream);
 }
 
 static int attn_decode_impl(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
                             void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                            float softcap, int nsplit, const float* alibi, bool kv8, float k_scale, float v_scale, void* stream) {
+                            float softcap, int nsplit, const float* alibi, bool kv8, float k_scale, float v_scale, int ahead, void* stream) {
   using namespace lx;
   if (T <= 0) return 0;
   if (nh % nkv != 0) return -1;
@@ -77,6 +77,7 @@ static int attn_decode_impl(const void* q, long long ldq, const void* kv, const 
   p.window = window; p.scale = kv8 ? scale * k_scale : scale; p.softcap = softcap; p.alibi = alibi;
   p.v_scale = v_scale;
   p.nsplit = nsplit < 1 ? 1 : nsplit;
+  p.ahead = ahead;
   if (p.nsplit > 1 && (part_o == nullptr || part_lse == nullptr)) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (kv8) {
@@ -89,20 +90,20 @@ static int attn_decode_impl(const void* q, long long ldq, const void* kv, const 
   return -3;
 }
 
-// `alibi`: [nh] fp32 slopes on the device (BLOOM, MPT), or null.
+// `alibi`: [nh] fp32 slopes on the device (BLOOM, MPT), or null.  `ahead` as for lx_norm_residual.
 int lx_attn_decode_alibi(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
                          void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                         float softcap, int nsplit, const float* alibi, void* stream) {
+                         float softcap, int nsplit, const float* alibi, int ahead, void* stream) {
   return attn_decode_impl(q, ldq, kv, block_tables, max_blocks, ctx_lens, out, ldo, part_o, part_lse, T, nh, nkv, d, window, scale, softcap,
-                          nsplit, alibi, false, 1.f, 1.f, stream);
+                          nsplit, alibi, false, 1.f, 1.f, ahead, stream);
 }
 
 // The same over an e4m3 cache: stored value * k_scale (v_scale) is the key (value).
 int lx_attn_decode_kv8(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
                        void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                       float softcap, int nsplit, const float* alibi, float k_scale, float v_scale, void* stream) {
+                       float softcap, int nsplit, const float* alibi, float k_scale, float v_scale, int ahead, void* stream) {
   return attn_decode_impl(q, ldq, kv, block_tables, max_blocks, ctx_lens, out, ldo, part_o, part_lse, T, nh, nkv, d, window, scale, softcap,
-                          nsplit, alibi, true, k_scale, v_scale, stream);
+                          nsplit, alibi, true, k_scale, v_scale, ahead, stream);
 }
 
 int lx_attn_prefill(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* cu_q,

@@ -345,6 +345,7 @@ struct DecodeParams {
   int nsplit;
   const float* alibi;         // [nh] ALiBi slopes, or null
   float v_scale;              // fp8 cache: multiplies the output (the K scale is folded into `scale` by the host)
+  int ahead;                  // the launch may trigger in front of its wait (pdl_wait_ahead)
   AttnTail tail;
 };
 
@@ -353,7 +354,7 @@ struct DecodeParams {
 // DK, DV: widths of keys and values (a page of one head holds its key plane, then its value plane).
 template <int DK, int DV, int STAGES, bool KV8, int NW, bool WIDE = false>
 __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams p) {
-  pdl_wait_ahead();      // every block waits, also those that return early below
+  pdl_wait_ahead(p.ahead);      // every block waits, also those that return early below
   extern __shared__ __align__(1024) uint8_t dsm[];
   static_assert(!KV8 || DK == DV, "e4m3 pages hold keys and values of one width");
   constexpr int PLANE = kPage * DK * 2, VPLANE = kPage * DV * 2;
@@ -523,8 +524,8 @@ __global__ void __launch_bounds__(32 * NW) attn_decode_kernel(const DecodeParams
 template <int D>
 __global__ void __launch_bounds__(D) attn_combine_kernel(const float* part_o, const float* part_lse,
                                                          __nv_bfloat16* __restrict__ out, long long ldo, int nh, int nsplit,
-                                                         const AttnTail tail, const int* ctx_lens) {
-  pdl_wait_ahead();      // every block waits, also those that return early below
+                                                         const AttnTail tail, const int* ctx_lens, int ahead) {
+  pdl_wait_ahead(ahead);      // every block waits, also those that return early below
   const int t = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)t * nh + h) * nsplit;
   float M = -INFINITY;
@@ -717,7 +718,7 @@ static int launch_decode_nw(const DecodeParams& p, int T, cudaStream_t s) {
   launch_pdl(attn_decode_kernel<DK, DV, STAGES, KV8, NW, WIDE>, grid, dim3(32 * NW), (size_t)SMEM, s, p);
   if (p.nsplit > 1) {
     dim3 g2(T, p.nh);
-    launch_pdl(attn_combine_kernel<DV>, g2, dim3(DV), 0, s, p.part_o, p.part_lse, p.out, p.ldo, p.nh, p.nsplit, p.tail, p.ctx_lens);
+    launch_pdl(attn_combine_kernel<DV>, g2, dim3(DV), 0, s, p.part_o, p.part_lse, p.out, p.ldo, p.nh, p.nsplit, p.tail, p.ctx_lens, p.ahead);
   }
   return -(int)cudaGetLastError();
 }

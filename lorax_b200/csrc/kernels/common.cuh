@@ -115,11 +115,13 @@ LX_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_fla
 // it.  pdl_trigger() lets the successor's blocks be scheduled as soon as all of this grid's blocks have called it or exited;
 // without it they are when this grid's have exited.  It stands
 //   * behind the block's own pdl_wait() in general: no more than one kernel is then unfinished in front of the successor's set-up;
-//   * in front of it, by pdl_wait_ahead(), in the short kernels between the products of a step (norms, RoPE, decode attention, activations) where
-//     they have no more than a block per SM: what they wait for is a product's tail, and their successor, mostly the next product, is then set up
-//     under that tail too, block by block as the product's blocks leave their SMs.  A chain of such kernels may be unfinished in front of a
-//     set-up, so a launch that says `const` of weights, tables or adapters says that no kernel writes them that any of these chains could
-//     still have in flight: in a step only copies do, and a chain cannot begin before a copy in front of it has ended;
+//   * in front of it, by pdl_wait_ahead(), in the short kernels between the products of a step (norms, RoPE, decode attention, activations) whose
+//     launch says `ahead`, where they have no more than a block per SM: what they wait for is a product's tail, and their successor, mostly the
+//     next product, is then set up under that tail too, block by block as the product's blocks leave their SMs.  Whatever these kernels
+//     wait for may be unfinished in front of that set-up as well.  A launch that says `const` of weights, tables or adapters vouches for the kernel
+//     directly in front of it; one that says `ahead` vouches for those that it waits for itself: they write nothing that its successor reads as
+//     constant.  A model's step does (only copies write weights, tables and adapters, and its first kernel, the embedding, waits before it
+//     triggers); calls on their own do not say it;
 //   * behind the block's tensor memory allocation, if it has one: a successor's block on the same SM might take the columns first, and
 //     would hold them until this kernel has completed.
 // A successor's pdl_wait() returns when its predecessor has completed, which that one does behind its own wait: all in front of it have too.
@@ -139,11 +141,11 @@ LX_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The wait of a short kernel between products, with its trigger.  Passes of four 7B layers with adapters: 1 row 607 -> 598 us, 13 rows 722 -> 693; with
 // 256 rows, whose kernels have more blocks than the GPU has SMs, it made no difference.
 constexpr unsigned kAheadBlocks = 148;
-LX_DEVICE void pdl_wait_ahead() {
-  const bool ahead = gridDim.x * gridDim.y * gridDim.z <= kAheadBlocks;
-  if (ahead) pdl_launch_dependents();
+LX_DEVICE void pdl_wait_ahead(int ahead) {
+  const bool early = ahead && gridDim.x * gridDim.y * gridDim.z <= kAheadBlocks;
+  if (early) pdl_launch_dependents();
   pdl_wait();
-  if (!ahead) pdl_trigger();
+  if (!early) pdl_trigger();
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -27,8 +27,8 @@ __global__ void __launch_bounds__(kNormThreads)
 norm_residual_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ residual,
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                      __nv_bfloat16* __restrict__ out, int H, long long ldx, long long ldr, long long ldo, float eps,
-                     float w_offset, float x_scale) {
-  pdl_wait_ahead();      // every block waits, also those that return early below
+                     float w_offset, float x_scale, int ahead) {
+  pdl_wait_ahead(ahead);      // every block waits, also those that return early below
   const int row = blockIdx.x;
   const int nvec = H / 8;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
@@ -155,8 +155,8 @@ LX_DEVICE uint32_t bf16x4_to_e4m3x4(uint2 w, float inv_scale) {
 __global__ void __launch_bounds__(256)
 rope_kvwrite_kernel(__nv_bfloat16* __restrict__ qkv, const int* positions, const float* __restrict__ cos_sin,
                     __nv_bfloat16* __restrict__ kv_cache, const int* slots, int nh, int nkv, int d, int rot,
-                    int page, long long ldq, int apply_rope, int kv_fp8, float k_inv_scale, float v_inv_scale) {
-  pdl_wait_ahead();      // every block waits, also those that return early below
+                    int page, long long ldq, int apply_rope, int kv_fp8, float k_inv_scale, float v_inv_scale, int ahead) {
+  pdl_wait_ahead(ahead);      // every block waits, also those that return early below
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int slot = slots ? slots[t] : -1;
@@ -254,8 +254,8 @@ LX_DEVICE float act_fn(float x) {
 }
 template <int ACT, bool GATED>
 __global__ void __launch_bounds__(256)
-act_mul_kernel(const __nv_bfloat16* in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec) {
-  pdl_wait_ahead();      // every block waits, also those that return early below
+act_mul_kernel(const __nv_bfloat16* in, __nv_bfloat16* __restrict__ out, int I, long long ldi, long long ldo, long long total_vec, int ahead) {
+  pdl_wait_ahead(ahead);      // every block waits, also those that return early below
   const int vec_per_row = I / 8;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total_vec; v += (long long)gridDim.x * blockDim.x) {
     const long long t = v / vec_per_row;
@@ -517,8 +517,10 @@ prefill_metadata_kernel(const int* cu_q, const int* cache_lens, const int* seq_s
 
 extern "C" {
 
+// `ahead` (here, and of lx_rope_kvwrite_kv8, lx_act_mul and the decode attention): the kernels in front on the stream write nothing that the next
+// launch reads as constant, so this one may let it be set up while they run (pdl_wait_ahead).
 int lx_norm_residual(const void* x, void* residual, const void* w, const void* b, void* out, int T, int H, long long ldx,
-                     long long ldr, long long ldo, float eps, float w_offset, float x_scale, int layernorm, void* stream) {
+                     long long ldr, long long ldo, float eps, float w_offset, float x_scale, int layernorm, int ahead, void* stream) {
   using namespace lx;
   if (T <= 0) return 0;
   if (H % 8 != 0 || H > kNormThreads * kNormMaxVec * 8) return -1;
@@ -531,7 +533,7 @@ int lx_norm_residual(const void* x, void* residual, const void* w, const void* b
   const int nv = (H / 8 + kNormThreads - 1) / kNormThreads;
 #define LX_NORM(NV)                                                                                                                     \
   launch_pdl(layernorm ? norm_residual_kernel<true, NV> : norm_residual_kernel<false, NV>, dim3(T), dim3(kNormThreads), 0, s, X, R, W, Bv, O, \
-             H, ldx, ldr, ldo, eps, w_offset, x_scale)
+             H, ldx, ldr, ldo, eps, w_offset, x_scale, ahead)
   if (nv <= 1) LX_NORM(1);
   else if (nv <= 2) LX_NORM(2);
   else if (nv <= 4) LX_NORM(4);
@@ -543,23 +545,23 @@ int lx_norm_residual(const void* x, void* residual, const void* w, const void* b
 // kv_fp8 != 0: the cache holds e4m3 bytes, value / k_scale for keys and value / v_scale for values (same layout).
 int lx_rope_kvwrite_kv8(void* qkv, const int* positions, const float* cos_sin, void* kv_cache, const int* slots, int T, int nh,
                         int nkv, int d, int rot, int page, long long ldq, int apply_rope, int kv_fp8, float k_scale, float v_scale,
-                        void* stream) {
+                        int ahead, void* stream) {
   using namespace lx;
   if (T <= 0) return 0;
   if (d % 8 != 0 || rot % 8 != 0 || rot > d) return -1;
   if (kv_fp8 && (k_scale <= 0.f || v_scale <= 0.f)) return -2;
   launch_pdl(rope_kvwrite_kernel, dim3(T), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<__nv_bfloat16*>(qkv), positions, cos_sin, reinterpret_cast<__nv_bfloat16*>(kv_cache), slots, nh, nkv, d,
-      rot, page, ldq, apply_rope, kv_fp8, kv_fp8 ? 1.f / k_scale : 1.f, kv_fp8 ? 1.f / v_scale : 1.f);
+      rot, page, ldq, apply_rope, kv_fp8, kv_fp8 ? 1.f / k_scale : 1.f, kv_fp8 ? 1.f / v_scale : 1.f, ahead);
   return -(int)cudaGetLastError();
 }
 
 int lx_rope_kvwrite(void* qkv, const int* positions, const float* cos_sin, void* kv_cache, const int* slots, int T, int nh,
                     int nkv, int d, int rot, int page, long long ldq, int apply_rope, void* stream) {
-  return lx_rope_kvwrite_kv8(qkv, positions, cos_sin, kv_cache, slots, T, nh, nkv, d, rot, page, ldq, apply_rope, 0, 1.f, 1.f, stream);
+  return lx_rope_kvwrite_kv8(qkv, positions, cos_sin, kv_cache, slots, T, nh, nkv, d, rot, page, ldq, apply_rope, 0, 1.f, 1.f, 0, stream);
 }
 
-int lx_act_mul(const void* in, void* out, int T, int I, long long ldi, long long ldo, int act, int gated, void* stream) {
+int lx_act_mul(const void* in, void* out, int T, int I, long long ldi, long long ldo, int act, int gated, int ahead, void* stream) {
   using namespace lx;
   if (T <= 0) return 0;
   if (I % 8 != 0) return -1;
@@ -569,8 +571,8 @@ int lx_act_mul(const void* in, void* out, int T, int I, long long ldi, long long
   auto X = reinterpret_cast<const __nv_bfloat16*>(in);
   auto O = reinterpret_cast<__nv_bfloat16*>(out);
 #define LX_ACT(A)                                                                         \
-  if (gated) launch_pdl(act_mul_kernel<A, true>, dim3(grid), dim3(256), 0, s, X, O, I, ldi, ldo, total);      \
-  else launch_pdl(act_mul_kernel<A, false>, dim3(grid), dim3(256), 0, s, X, O, I, ldi, ldo, total);
+  if (gated) launch_pdl(act_mul_kernel<A, true>, dim3(grid), dim3(256), 0, s, X, O, I, ldi, ldo, total, ahead);      \
+  else launch_pdl(act_mul_kernel<A, false>, dim3(grid), dim3(256), 0, s, X, O, I, ldi, ldo, total, ahead);
   switch (act) {
     case kSilu: LX_ACT(kSilu); break;
     case kGelu: LX_ACT(kGelu); break;

@@ -17,22 +17,22 @@ extern "C" {
 
 // launchers of this library (defined in the other translation units)
 int lx_norm_residual(const void* x, void* residual, const void* w, const void* b, void* out, int T, int H, long long ldx,
-                     long long ldr, long long ldo, float eps, float w_offset, float x_scale, int layernorm, void* stream);
+                     long long ldr, long long ldo, float eps, float w_offset, float x_scale, int layernorm, int ahead, void* stream);
 int lx_rope_kvwrite(void* qkv, const int* positions, const float* cos_sin, void* kv_cache, const int* slots, int T, int nh,
                     int nkv, int d, int rot, int page, long long ldq, int apply_rope, void* stream);
-int lx_act_mul(const void* in, void* out, int T, int I, long long ldi, long long ldo, int act, int gated, void* stream);
-int lx_attn_decode(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
-                   void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                   float softcap, int nsplit, void* stream);
+int lx_act_mul(const void* in, void* out, int T, int I, long long ldi, long long ldo, int act, int gated, int ahead, void* stream);
+int lx_attn_decode_alibi(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
+                         void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
+                         float softcap, int nsplit, const float* alibi, int ahead, void* stream);
 int lx_attn_prefill(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* cu_q,
                     const int* cache_lens, const int* tile_seq, const int* tile_q0, int num_tiles, void* out, long long ldo, int nh,
                     int nkv, int d, int window, float scale, float softcap, void* stream);
 int lx_rope_kvwrite_kv8(void* qkv, const int* positions, const float* cos_sin, void* kv_cache, const int* slots, int T, int nh,
                         int nkv, int d, int rot, int page, long long ldq, int apply_rope, int kv_fp8, float k_scale, float v_scale,
-                        void* stream);
+                        int ahead, void* stream);
 int lx_attn_decode_kv8(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* ctx_lens,
                        void* out, long long ldo, float* part_o, float* part_lse, int T, int nh, int nkv, int d, int window, float scale,
-                       float softcap, int nsplit, const float* alibi, float k_scale, float v_scale, void* stream);
+                       float softcap, int nsplit, const float* alibi, float k_scale, float v_scale, int ahead, void* stream);
 int lx_attn_prefill_kv8(const void* q, long long ldq, const void* kv, const int* block_tables, int max_blocks, const int* cu_q,
                         const int* cache_lens, const int* tile_seq, const int* tile_q0, int num_tiles, void* out, long long ldo, int nh,
                         int nkv, int d, int window, float scale, float softcap, const float* alibi, float k_scale, float v_scale,
@@ -155,6 +155,8 @@ namespace {
     if (rc_ != 0) return rc_;   \
   } while (0)
 
+constexpr int kStep = 1;      // `ahead` of the short kernels: no kernel of a step writes weights, tables or adapters
+
 // y[T, N] = x[T, K] w^T (+ bias) (+ LoRA delta of the site)
 int linear_with_lora(const LxModelDesc& m, const LxLayerDesc& l, const LxStepDesc& s, int site_idx, const void* x, long long ldx,
                      const void* w, long long ldw, const void* bias, void* y, long long ldy, int N, int K, void* stream) {
@@ -223,14 +225,14 @@ int lx_layer_attention(const LxModelDesc* m, const LxLayerDesc* l, const LxStepD
   if (T <= 0) return 0;
   if (x_in != nullptr) {
     LX_TRY(lx_norm_residual(x_in, residual, l->input_norm_w, l->input_norm_b, s->normed, T, H, H, H, H, m->eps, m->norm_offset, x_scale,
-                            m->layernorm, stream));
+                            m->layernorm, kStep, stream));
   } else {
     LX_TRY(lx_norm_residual(residual, nullptr, l->input_norm_w, l->input_norm_b, s->normed, T, H, H, 0, H, m->eps, m->norm_offset, 1.f,
-                            m->layernorm, stream));
+                            m->layernorm, kStep, stream));
   }
   LX_TRY(linear_with_lora(*m, *l, *s, 0, s->normed, H, l->qkv_w, l->ld_qkv, l->qkv_b, s->qkv, m->n_qkv, m->n_qkv, H, stream));
   LX_TRY(lx_rope_kvwrite_kv8(s->qkv, s->positions, m->cos_sin, l->kv_cache, s->slots, T, m->nh, m->nkv, m->d, m->rot, m->page, m->n_qkv,
-                             m->apply_rope, m->kv_fp8, l->k_scale, l->v_scale, stream));
+                             m->apply_rope, m->kv_fp8, l->k_scale, l->v_scale, kStep, stream));
   const int nd = s->n_decode;
   const long long ldq = m->n_qkv, lda = m->n_o_in;
   char* q = reinterpret_cast<char*>(s->qkv);
@@ -242,10 +244,10 @@ int lx_layer_attention(const LxModelDesc* m, const LxLayerDesc* l, const LxStepD
     if (m->kv_fp8) {
       LX_TRY(lx_attn_decode_kv8(q, ldq, l->kv_cache, s->dec_block_tables, s->dec_max_blocks, s->ctx_lens, a, lda, m->attn_part_o,
                                 m->attn_part_lse, nd, m->nh, m->nkv, m->d, l->window, m->attn_scale, m->softcap, nsplit, nullptr,
-                                l->k_scale, l->v_scale, stream));
+                                l->k_scale, l->v_scale, kStep, stream));
     } else {
-      LX_TRY(lx_attn_decode(q, ldq, l->kv_cache, s->dec_block_tables, s->dec_max_blocks, s->ctx_lens, a, lda, m->attn_part_o, m->attn_part_lse,
-                            nd, m->nh, m->nkv, m->d, l->window, m->attn_scale, m->softcap, nsplit, stream));
+      LX_TRY(lx_attn_decode_alibi(q, ldq, l->kv_cache, s->dec_block_tables, s->dec_max_blocks, s->ctx_lens, a, lda, m->attn_part_o,
+                                  m->attn_part_lse, nd, m->nh, m->nkv, m->d, l->window, m->attn_scale, m->softcap, nsplit, nullptr, kStep, stream));
     }
   }
   if (T > nd) {
@@ -274,10 +276,10 @@ int lx_layer_mlp(const LxModelDesc* m, const LxLayerDesc* l, const LxStepDesc* s
   const int T = s->T, H = m->H;
   if (T <= 0) return 0;
   LX_TRY(lx_norm_residual(x_in, residual, l->post_norm_w, l->post_norm_b, s->normed, T, H, H, H, H, m->eps, m->norm_offset, x_scale,
-                          m->layernorm, stream));
+                          m->layernorm, kStep, stream));
   LX_TRY(linear_with_lora(*m, *l, *s, 2, s->normed, H, l->gate_up_w, l->ld_gate_up, l->gate_up_b, s->gate_up, m->n_gate_up, m->n_gate_up, H,
                           stream));
-  LX_TRY(lx_act_mul(s->gate_up, s->act, T, m->inter, m->n_gate_up, m->inter, m->act, m->gated, stream));
+  LX_TRY(lx_act_mul(s->gate_up, s->act, T, m->inter, m->n_gate_up, m->inter, m->act, m->gated, kStep, stream));
   return linear_with_lora(*m, *l, *s, 3, s->act, m->inter, l->down_w, l->ld_down, l->down_b, out, H, H, m->n_down_in, stream);
 }
 

@@ -418,7 +418,7 @@ class DecoderModel:
     def _norm(self, x, residual, w, b=None, x_scale: float = 1.0):
         c = self.config
         return self.ops.norm_residual(x, residual, w, c.rms_norm_eps, bias=b, weight_offset=c.norm_weight_offset,
-                                      x_scale=x_scale, layernorm=c.norm_type.startswith("layernorm"))
+                                      x_scale=x_scale, layernorm=c.norm_type.startswith("layernorm"), ahead=True)
 
     def quantize_fp8(self):
         """Replace the dense projection matrices of every layer by block-scaled fp8 (e4m3, 128 x 128 scales) for the
@@ -660,7 +660,7 @@ class DecoderModel:
             qkv.clamp_(-c.clip_qkv, c.clip_qkv)
         kvs = {"kv_scale": self.kv_scales[li]} if (self.kv_scales and kv.dtype == torch.float8_e4m3fn) else {}
         ops.rope_kvwrite(qkv, inp.positions, self.cos_sin, kv, inp.slots, self.nh, self.nkv, self.d, c.rotary_dim,
-                         not (c.learned_positions or c.alibi), **kvs)
+                         not (c.learned_positions or c.alibi), ahead=True, **kvs)
         ali = {"alibi": self.alibi_slopes} if self.alibi_slopes is not None else {}
         ali.update(kvs)
         window = c.sliding_window or 0
@@ -671,7 +671,7 @@ class DecoderModel:
             nd = inp.n_decode
             attn = torch.empty(qkv.shape[0], self.nh * self.d, dtype=qkv.dtype, device=qkv.device)
             a = ops.attn_decode(qkv[:nd], kv, inp.dec_block_tables, inp.ctx_lens, self.nh, self.nkv, self.d, c.attn_scale, window,
-                                softcap, inp.attn_nsplit, out=attn[:nd], **ali)
+                                softcap, inp.attn_nsplit, out=attn[:nd], ahead=True, **ali)
             b = ops.attn_prefill(qkv[nd:], kv, inp.block_tables, inp.cu_q, inp.cache_lens, inp.tile_seq, inp.tile_q0,
                                  self.nh, self.nkv, self.d, c.attn_scale, window, softcap, out=attn[nd:], **ali)
             if a.data_ptr() != attn.data_ptr():      # ops that ignore `out`
@@ -682,13 +682,13 @@ class DecoderModel:
                                     self.nh, self.nkv, self.d, c.attn_scale, window, softcap, **ali)
         else:
             attn = ops.attn_decode(qkv, kv, inp.block_tables, inp.ctx_lens, self.nh, self.nkv, self.d, c.attn_scale, window,
-                                   softcap, inp.attn_nsplit, **ali)
+                                   softcap, inp.attn_nsplit, ahead=True, **ali)
         return self._row_parallel(attn, lw.o_w, lw.o_b, "o", li, inp)
 
     def _mlp(self, x, lw: LayerWeights, li: int, inp: StepInputs):
         c, ops = self.config, self.ops
         gu = self._linear(x, lw.gate_up_w, lw.gate_up_b, "gate_up", li, inp)
-        act = ops.act_mul(gu, self.inter, c.hidden_act, gated=self.gated)
+        act = ops.act_mul(gu, self.inter, c.hidden_act, gated=self.gated, ahead=True)
         return self._row_parallel(act, lw.down_w, lw.down_b, "down", li, inp)
 
     def _moe(self, x, lw: LayerWeights, li: int, inp: StepInputs):

@@ -153,7 +153,7 @@ class EncoderModel:
         if self.type_emb is not None:
             tt = token_type_ids.long() if token_type_ids is not None else torch.zeros(T, dtype=torch.long, device=self.device)
             h = h + self.type_emb[tt]
-        h = ops.norm_residual(h.contiguous(), None, self.emb_ln_w, c.layer_norm_eps, bias=self.emb_ln_b, layernorm=True)
+        h = ops.norm_residual(h.contiguous(), None, self.emb_ln_w, c.layer_norm_eps, bias=self.emb_ln_b, layernorm=True, ahead=True)
         H = c.hidden_size
         act = "gelu" if c.hidden_act in ("gelu", "gelu_new") else c.hidden_act
         for lw in self.layers:
@@ -164,10 +164,10 @@ class EncoderModel:
                 attn[a:b] = F.scaled_dot_product_attention(q, k, v).transpose(0, 1).reshape(b - a, H)
             o = ops.gemm(attn, lw.o_w, bias=lw.o_b)
             # post-LN: h <- LN(h + o); norm_residual adds into `h` (the residual stream) and returns the normed value
-            h = ops.norm_residual(o, h, lw.attn_ln_w, c.layer_norm_eps, bias=lw.attn_ln_b, layernorm=True)
-            f = ops.act_mul(ops.gemm(h, lw.ffn1_w, bias=lw.ffn1_b), c.intermediate_size, act, gated=False)
+            h = ops.norm_residual(o, h, lw.attn_ln_w, c.layer_norm_eps, bias=lw.attn_ln_b, layernorm=True, ahead=True)
+            f = ops.act_mul(ops.gemm(h, lw.ffn1_w, bias=lw.ffn1_b), c.intermediate_size, act, gated=False, ahead=True)
             f = ops.gemm(f, lw.ffn2_w, bias=lw.ffn2_b)
-            h = ops.norm_residual(f, h, lw.out_ln_w, c.layer_norm_eps, bias=lw.out_ln_b, layernorm=True)
+            h = ops.norm_residual(f, h, lw.out_ln_w, c.layer_norm_eps, bias=lw.out_ln_b, layernorm=True, ahead=True)
         return h
 
     def embed(self, seqs: Sequence[Sequence[int]]) -> List[List[float]]:

@@ -560,7 +560,7 @@ class MixerLayer:
         y = torch.empty(T, m.out_dim + self.ff, dtype=h.dtype, device=h.device)
         m.run(model, h, views, y, inp, cache)
         if self.ff:
-            ops.act_mul(views["mlp"], self.ff, model.config.hidden_act, gated=True, out=y[:, m.out_dim:])
+            ops.act_mul(views["mlp"], self.ff, model.config.hidden_act, gated=True, out=y[:, m.out_dim:], ahead=True)
         return ops.gemm(y, self.out_w, w_const=True)
 
 
@@ -593,7 +593,7 @@ class DenseMlp:
         """-> the same and the projection beside (or None)."""
         ops, n = model.ops, len(self.names) * self.fp
         u = ops.gemm(h, self.up, bias=self.up_b, w_const=True)
-        a = ops.act_mul(u, self.fp, self.act or model.config.hidden_act, gated=self.gated, **self.act_args)
+        a = ops.act_mul(u, self.fp, self.act or model.config.hidden_act, gated=self.gated, ahead=True, **self.act_args)
         return ops.gemm(a, self.down, w_const=True), None, u[:, n:] if self.up_b is not None else None
 
 

@@ -59,7 +59,7 @@ def moe_forward(model, x: torch.Tensor, lw, li: int, inp) -> torch.Tensor:
         we = w[:, e]
         if T <= DENSE_MAX_TOKENS:
             gu = model._gemm(x, lw.experts_w13[j], None)
-            a = ops.act_mul(gu, I, c.hidden_act, gated=True)
+            a = ops.act_mul(gu, I, c.hidden_act, gated=True, ahead=True)
             dn = model._gemm(a, lw.experts_w2[j], None)
             out.addcmul_(dn.float(), we[:, None])
         else:
@@ -68,7 +68,7 @@ def moe_forward(model, x: torch.Tensor, lw, li: int, inp) -> torch.Tensor:
                 continue
             xe = x.index_select(0, idx).contiguous()
             gu = model._gemm(xe, lw.experts_w13[j], None)
-            a = ops.act_mul(gu, I, c.hidden_act, gated=True)
+            a = ops.act_mul(gu, I, c.hidden_act, gated=True, ahead=True)
             dn = model._gemm(a, lw.experts_w2[j], None)
             out.index_add_(0, idx, dn.float() * we.index_select(0, idx)[:, None])
     out = out.to(x.dtype)

@@ -69,9 +69,9 @@ def load() -> ctypes.CDLL:
         "lx_lora_tile_bytes": ([I, I, I], ctypes.c_uint),
         "lx_gemm_plan": ([I, I, I, I, L, I, I, P], I),
         "lx_gemm_bf16": ([P, P, P, P, I, I, I, L, L, L, F, P, L, P, P, I, I, I, P], I),
-        "lx_norm_residual": ([P, P, P, P, P, I, I, L, L, L, F, F, F, I, P], I),
+        "lx_norm_residual": ([P, P, P, P, P, I, I, L, L, L, F, F, F, I, I, P], I),
         "lx_rope_kvwrite": ([P, P, P, P, P, I, I, I, I, I, I, L, I, P], I),
-        "lx_act_mul": ([P, P, I, I, L, L, I, I, P], I),
+        "lx_act_mul": ([P, P, I, I, L, L, I, I, I, P], I),
         "lx_embed": ([P, P, P, I, I, I, I, F, P], I),
         "lx_place_rows": ([P, I, I, P, P, P, P, P], I),
         "lx_argmax_logprob": ([P, L, I, I, P, P, F, P], I),
@@ -80,10 +80,10 @@ def load() -> ctypes.CDLL:
         "lx_attn_page_size": ([], I),
         "lx_attn_decode": ([P, L, P, P, I, P, P, L, P, P, I, I, I, I, I, F, F, I, P], I),
         "lx_attn_prefill": ([P, L, P, P, I, P, P, P, P, I, P, L, I, I, I, I, F, F, P], I),
-        "lx_attn_decode_alibi": ([P, L, P, P, I, P, P, L, P, P, I, I, I, I, I, F, F, I, P, P], I),
+        "lx_attn_decode_alibi": ([P, L, P, P, I, P, P, L, P, P, I, I, I, I, I, F, F, I, P, I, P], I),
         "lx_attn_prefill_alibi": ([P, L, P, P, I, P, P, P, P, I, P, L, I, I, I, I, F, F, P, P], I),
-        "lx_rope_kvwrite_kv8": ([P, P, P, P, P, I, I, I, I, I, I, L, I, I, F, F, P], I),
-        "lx_attn_decode_kv8": ([P, L, P, P, I, P, P, L, P, P, I, I, I, I, I, F, F, I, P, F, F, P], I),
+        "lx_rope_kvwrite_kv8": ([P, P, P, P, P, I, I, I, I, I, I, L, I, I, F, F, I, P], I),
+        "lx_attn_decode_kv8": ([P, L, P, P, I, P, P, L, P, P, I, I, I, I, I, F, F, I, P, F, F, I, P], I),
         "lx_attn_prefill_kv8": ([P, L, P, P, I, P, P, P, P, I, P, L, I, I, I, I, F, F, P, F, F, P], I),
         "lx_lora_shrink": ([P, L, P, P, P, P, I, L, I, P, I, I, I, I, P, P], I),
         "lx_lora_expand": ([P, I, P, P, P, P, I, L, P, L, I, I, I, I, P, P], I),
@@ -308,7 +308,8 @@ def lora_fused_desc(ws: "Workspace", lf: LoraFused, K: int) -> LxLoraFused:
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
          out_scale: float = 1.0, mode: int = 0, force_split: int = 0, w_const: bool = False) -> torch.Tensor:
     """out[T, N] = x[T, K] @ w[N, K]^T (+ bias).  bf16 in, fp32 accumulate on tcgen05, bf16 out (fp32 in: true fp32 throughout).
-    `w_const`: the kernel in front on the stream does not write `w` (a model's weights), which is then read while it still runs."""
+    `w_const`: the kernel in front on the stream does not write `w` (a model's weights), which is then read while it still runs (a kernel launched
+    `ahead` vouches for those in front of it)."""
     if x.dtype == torch.float32:
         return gemm_f32(x, w, out=out, out_scale=out_scale, bias=bias)
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.dim() == 2 and w.dim() == 2
@@ -442,7 +443,7 @@ def moe_ffn(x: torch.Tensor, router_w: torch.Tensor, w13: torch.Tensor, w2: torc
     r = moe_route(x, router_w, k, e0, e_local)
     avg = max(1, (T * k + E - 1) // E)
     gu = moe_grouped_gemm(r.xg, w13, r.seg, avg)
-    a = act_mul(gu, two_i // 2, act, gated=True)
+    a = act_mul(gu, two_i // 2, act, gated=True, ahead=True)      # (expert products read nothing before their wait)
     y = moe_grouped_gemm(a, w2, r.seg, avg)
     return moe_combine(y, r.pos, r.topk_w, k, torch.empty(T, H, dtype=torch.bfloat16, device=x.device))
 
@@ -563,21 +564,23 @@ def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Option
 # ------------------------------------------------------------------------------------------------ elementwise
 def norm_residual(x: torch.Tensor, residual: Optional[torch.Tensor], weight: torch.Tensor, eps: float,
                   bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, weight_offset: float = 0.0,
-                  x_scale: float = 1.0, layernorm: bool = False) -> torch.Tensor:
-    """h = x * x_scale (+ residual); residual <- h (in place); returns norm(h) * (weight + offset) (+ bias)."""
+                  x_scale: float = 1.0, layernorm: bool = False, ahead: bool = False) -> torch.Tensor:
+    """h = x * x_scale (+ residual); residual <- h (in place); returns norm(h) * (weight + offset) (+ bias).
+    `ahead` (here, and of `rope_kvwrite`, `act_mul` and `attn_decode`), said inside a model's step: the kernels in front on the stream write
+    nothing that the next launch may read as constant (`w_const`, `tables_const`), which then may be set up while they run."""
     T, H = x.shape
     if out is None:
         out = torch.empty_like(x)
     rc = load().lx_norm_residual(_ptr(x), _ptr(residual), _ptr(weight), _ptr(bias), _ptr(out), T, H, x.stride(0),
                                  residual.stride(0) if residual is not None else 0, out.stride(0), eps, weight_offset,
-                                 x_scale, int(layernorm), _stream())
+                                 x_scale, int(layernorm), int(ahead), _stream())
     _check(rc, "lx_norm_residual")
     return out
 
 
 def rope_kvwrite(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor, kv_cache: torch.Tensor,
                  slots: Optional[torch.Tensor], nh: int, nkv: int, d: int, rot: int, apply_rope: bool = True,
-                 kv_scale: Optional[Tuple[float, float]] = None):
+                 kv_scale: Optional[Tuple[float, float]] = None, ahead: bool = False):
     """RoPE in place on q and k, then k and v into the paged cache.  A `torch.float8_e4m3fn` cache takes value / scale as e4m3
     (`kv_scale` = (k scale, v scale), default 1)."""
     T = qkv.shape[0]
@@ -585,7 +588,7 @@ def rope_kvwrite(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tens
     fp8 = kv_cache.dtype == torch.float8_e4m3fn
     ks, vs = kv_scale if (fp8 and kv_scale) else (1.0, 1.0)
     rc = load().lx_rope_kvwrite_kv8(_ptr(qkv), _ptr(positions), _ptr(cos_sin), _ptr(kv_cache), _ptr(slots), T, nh, nkv, d, rot,
-                                    page, qkv.stride(0), int(apply_rope), int(fp8), ks, vs, _stream())
+                                    page, qkv.stride(0), int(apply_rope), int(fp8), ks, vs, int(ahead), _stream())
     _check(rc, "lx_rope_kvwrite")
 
 
@@ -593,7 +596,7 @@ _ACTS = {"silu": 0, "swish": 0, "gelu": 1, "gelu_new": 2, "gelu_pytorch_tanh": 2
 
 
 def act_mul(x: torch.Tensor, inter: int, act: str = "silu", gated: bool = True, out: Optional[torch.Tensor] = None,
-            limit: float = 0.0) -> torch.Tensor:
+            limit: float = 0.0, ahead: bool = False) -> torch.Tensor:
     T = x.shape[0]
     if out is None:
         out = torch.empty(T, inter, dtype=x.dtype, device=x.device)
@@ -604,7 +607,7 @@ def act_mul(x: torch.Tensor, inter: int, act: str = "silu", gated: bool = True, 
     if x.dtype == torch.float32:
         _check(load().lx_act_mul_f32(_ptr(x), _ptr(out), T, inter, x.stride(0), out.stride(0), _ACTS[act], int(gated), _stream()), "lx_act_mul_f32")
         return out
-    rc = load().lx_act_mul(_ptr(x), _ptr(out), T, inter, x.stride(0), out.stride(0), _ACTS[act], int(gated), _stream())
+    rc = load().lx_act_mul(_ptr(x), _ptr(out), T, inter, x.stride(0), out.stride(0), _ACTS[act], int(gated), int(ahead), _stream())
     _check(rc, "lx_act_mul")
     return out
 
@@ -665,7 +668,7 @@ def prefill_metadata(cu_q: torch.Tensor, cache_lens: torch.Tensor, seq_slot: tor
 def attn_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_tables: torch.Tensor, ctx_lens: torch.Tensor, nh: int, nkv: int,
                 d: int, scale: float, window: int = 0, softcap: float = 0.0, nsplit: int = 1,
                 out: Optional[torch.Tensor] = None, alibi: Optional[torch.Tensor] = None,
-                kv_scale: Optional[Tuple[float, float]] = None) -> torch.Tensor:
+                kv_scale: Optional[Tuple[float, float]] = None, ahead: bool = False) -> torch.Tensor:
     """q: [T, >= nh*d] (row stride arbitrary), one query token per row.  Returns [T, nh*d].  `alibi`: [nh] fp32 slopes.
     An e4m3 cache is read as stored value * scale (`kv_scale` = (k scale, v scale))."""
     T = q.shape[0]
@@ -677,12 +680,12 @@ def attn_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_tables: torch.Ten
         ks, vs = kv_scale or (1.0, 1.0)
         rc = load().lx_attn_decode_kv8(_ptr(q), q.stride(0), _ptr(kv_cache), _ptr(block_tables), block_tables.shape[1], _ptr(ctx_lens),
                                        _ptr(out), out.stride(0), _ptr(ws.attn_part_o), _ptr(ws.attn_part_lse), T, nh, nkv, d, window,
-                                       scale, softcap, nsplit, _ptr(alibi), ks, vs, _stream())
+                                       scale, softcap, nsplit, _ptr(alibi), ks, vs, int(ahead), _stream())
         _check(rc, "lx_attn_decode_kv8")
         return out
     rc = load().lx_attn_decode_alibi(_ptr(q), q.stride(0), _ptr(kv_cache), _ptr(block_tables), block_tables.shape[1], _ptr(ctx_lens),
                                      _ptr(out), out.stride(0), _ptr(ws.attn_part_o), _ptr(ws.attn_part_lse), T, nh, nkv, d, window,
-                                     scale, softcap, nsplit, _ptr(alibi), _stream())
+                                     scale, softcap, nsplit, _ptr(alibi), int(ahead), _stream())
     _check(rc, "lx_attn_decode")
     return out
 

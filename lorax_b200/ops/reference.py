@@ -91,7 +91,7 @@ def gemm_fp8(x, wq, w_scale, bias=None, out=None):
 
 
 def norm_residual(x, residual, weight, eps, bias=None, out=None, weight_offset: float = 0.0, x_scale: float = 1.0,
-                  layernorm: bool = False):
+                  layernorm: bool = False, ahead: bool = False):
     h = x.float() * x_scale
     if residual is not None:
         h = h + residual.float()
@@ -128,7 +128,8 @@ def _to_e4m3_bytes(x, scale):
     return (x.float() / scale).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
 
 
-def rope_kvwrite(qkv, positions, cos_sin, kv_cache, slots, nh, nkv, d, rot, apply_rope_flag: bool = True, kv_scale=None):
+def rope_kvwrite(qkv, positions, cos_sin, kv_cache, slots, nh, nkv, d, rot, apply_rope_flag: bool = True, kv_scale=None,
+                 ahead: bool = False):
     """In place on qkv [T, (nh+2nkv)*d]; kv_cache [blocks, nkv, 2, page, d] (bf16 / fp32, or e4m3 holding value / scale)."""
     T = qkv.shape[0]
     page = kv_cache.shape[3]
@@ -171,7 +172,7 @@ def _act(x, act):
 CLAMPED_SWIGLU_ALPHA = 1.702
 
 
-def act_mul(x, inter, act="silu", gated=True, out=None, limit: float = 0.0):
+def act_mul(x, inter, act="silu", gated=True, out=None, limit: float = 0.0, ahead: bool = False):
     """act(gate) * up of rows [gate | up], or act(gate).  "clamped_swiglu" (gated): gate at most `limit`, up within +-limit,
     gate * sigmoid(1.702 gate) * (up + 1)."""
     g = x[:, :inter].float()
@@ -279,7 +280,7 @@ def _attend(q, k, v, q_pos, scale, window, softcap, slope=None):
 
 
 def attn_decode(q, kv_cache, block_tables, ctx_lens, nh, nkv, d, scale, window=0, softcap=0.0, nsplit=1, out=None, alibi=None,
-                kv_scale=None):
+                kv_scale=None, ahead: bool = False):
     T = q.shape[0]
     res = torch.zeros(T, nh * d, dtype=q.dtype, device=q.device)
     g = nh // nkv

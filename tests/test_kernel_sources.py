@@ -47,6 +47,24 @@ def test_triggers_stand_behind_the_wait():
         assert not at or 0 <= body.find("pdl_wait()") < min(at) or "shrink_rows_part" in body, kernel
 
 
+def test_triggers_ahead_of_the_wait_are_asked_for():
+    """Only launches that say so trigger in front of their wait: those of a model's step, whose first kernel waits before it triggers.  By default
+    what a caller's kernels wrote two launches in front of a product is there when it reads its weights."""
+    import inspect
+
+    from lorax_b200.ops import native, reference
+    ahead = {kernel.split(":")[1] for kernel, params, body in _kernels() if "pdl_wait_ahead(" in body}
+    assert ahead == {"norm_residual_kernel", "rope_kvwrite_kernel", "act_mul_kernel", "attn_decode_kernel", "attn_combine_kernel"}
+    for kernel, params, body in _kernels():
+        calls = re.findall(r"pdl_wait_ahead\((.*?)\);", body)
+        assert calls in ([], ["ahead"], ["p.ahead"]) and ("pdl_wait" in body or "pdl_trigger" not in body), kernel
+        if "embed_kernel" in kernel or "embed_peer" in kernel or "embed_stream" in kernel:
+            assert not calls, kernel
+    for name in ("norm_residual", "rope_kvwrite", "act_mul", "attn_decode"):
+        for ops in (native, reference):
+            assert inspect.signature(getattr(ops, name)).parameters["ahead"].default is False, name
+
+
 @pytest.mark.parametrize("T,N,K,parts", [
     (13, 4096, 4096, 4), (32, 4096, 2048, 4), (1, 4096, 1984, 1), (13, 6144, 4096, 3), (16, 5504, 1536, 3), (16, 5504, 1472, 1), (17, 5504, 3072, 3),
     (17, 5504, 3008, 1), (13, 8192, 2048, 2), (13, 9216, 1984, 1), (32, 8192, 3072, 2), (32, 8192, 3008, 1),

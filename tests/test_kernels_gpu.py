@@ -586,6 +586,32 @@ def test_gemm_reads_constant_weights_early(nat, T, N, K, mode, split):
     nat.workspace().check_status()
 
 
+@pytest.mark.parametrize("between", ["norm", "act", "rope", "attention"])
+@pytest.mark.parametrize("T,N,K", [(3, 4096, 1024), (64, 2048, 4096), (300, 1024, 512)])
+def test_constant_weights_come_from_two_kernels_in_front(nat, T, N, K, between):
+    """A kernel that lets its successor start early writes a product's weights, a short one that does not touch them stands in between: the
+    one in front of the product does not write them, so it may say that they are constant."""
+    torch.manual_seed(T + N)
+    srcs = [torch.randn(N, 2 * K, device="cuda", dtype=torch.bfloat16) * (1 + i) for i in range(2)]
+    w, x = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16), torch.randn(T, K, device="cuda", dtype=torch.bfloat16)
+    small, ones = torch.randn(4, 1024, device="cuda", dtype=torch.bfloat16), torch.ones(1024, device="cuda", dtype=torch.bfloat16)
+    cache, bt = _make_cache(4, 64, 2, 128)
+    ints = lambda *v: torch.tensor(v, device="cuda", dtype=torch.int32)
+    pos, slots, ctx, cos = ints(0, 1, 2, 3), ints(-1, -1, -1, -1), ints(5, 33, 64, 1), torch.rand(8, 128, device="cuda")
+    step = dict(norm=lambda: nat.norm_residual(small, None, ones, 1e-5), act=lambda: nat.act_mul(small, 512),
+                rope=lambda: nat.rope_kvwrite(small, pos, cos, cache, slots, 4, 2, 128, 128),
+                attention=lambda: nat.attn_decode(small, cache, bt, ctx, 4, 2, 128, 0.1))[between]
+    outs = []
+    for i in range(6):
+        nat.act_mul(srcs[i % 2], K, "silu", out=w)
+        step()
+        outs.append(nat.gemm(x, w, w_const=True))
+    torch.cuda.synchronize()
+    nat.workspace().check_status()
+    want = [nat.gemm(x, nat.act_mul(s, K, "silu")) for s in srcs]
+    assert all(torch.equal(o, want[i % 2]) for i, o in enumerate(outs))
+
+
 @pytest.mark.parametrize("T,N,K,group", [(1, 4096, 1024, 128), (5, 28672, 4096, 128), (8, 8192, 384, 64), (9, 512, 2048, 128), (17, 1024, 256, 32), (32, 256, 128, 128)])
 def test_packed_products_read_constant_codes_early(nat, T, N, K, group):
     from lorax_b200.utils.quant_formats import quantize_rtn
