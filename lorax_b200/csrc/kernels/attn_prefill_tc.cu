@@ -8,17 +8,18 @@
 //                               through one 5-D tensor map {d, slot, K|V, kv head, block}: the block table supplies the last
 //                               coordinate, so pages need not be contiguous; rings of two stages for K and for V
 //   MMA     (warp 1)            S = Q K^T into TMEM, O_j = P_j V_j into TMEM; P is a TMEM operand in the columns that its scores had.
-//                               The tiles take turns: P V and the next S of one run while the other's softmax does
+//                               Two tiles take turns: P V and the next S of one run while the other's softmax does.  A single tile has
+//                               two buffers of S and of O in their place: the next S and P V run while its softmax does
 //   softmax (a warpgroup per tile)  one thread per row: scores from TMEM with tcgen05.ld, scale / softcap / ALiBi / causal and
 //                               window mask, running max and sum, exp2, P as bf16 back into TMEM; the per-block products O_j come
 //                               from TMEM and are folded into fp32 registers with the usual rescaling, so nothing in TMEM ever has
-//                               to be rescaled.  O_j is folded while the tensor core forms S_{j+1}
+//                               to be rescaled
 //
 // What bounds it: per tile and block 128 x 128 exponentials take 1024 cycles of the special function units and the products about 1550 of
-// the tensor core (S 950: at N = 128 both operands come from shared memory at its full rate; P V 600).  One tile per CTA has them in a chain
-// (S, softmax, P V, S, ...), 4700 cycles with P through shared memory; two tiles fill each other's gaps, and P in TMEM spares the stores and
-// half of P V's shared memory.  32 heads, 8 KV heads, one tile per CTA and P in shared memory -> this: 8192 tokens 1021 -> 579 us, seven prompts
-// of together 4001 132 -> 77, three of 1700 56 -> 34, 137 tokens 11.5 -> 10.6 (products alone: 368 us of the 579).
+// the tensor core (S 950: at N = 128 both operands come from shared memory at its full rate; P V 600).  Two tiles fill each other's gaps, and P in
+// TMEM spares the stores and half of P V's shared memory.  Launches in a row, 32 heads, one tile per CTA and P through shared memory -> this: 8 KV
+// heads, 8192 tokens 1022 -> 597 us, seven prompts of 571 106 -> 62, three of 570 52 -> 32 (two tiles a CTA); 500 tokens 19.8 -> 15.0, 123 10.4 -> 9.5;
+// 16 KV heads, 8192 tokens 1046 -> 798, capped 1640 -> 1430, with a bias 3000 -> 2510 (one).  8192 tokens on their own 579, 368 without the softmax.
 //
 // WIDE: the softmax weights stay fp32 up to the value product: each is split into two bf16 terms, value and remainder, side by side in
 // TMEM, and P V is two products into the same accumulator (the layer-by-layer designs ask for it).
@@ -61,7 +62,8 @@ struct FaShape {
   static constexpr int kKBytes = kFaKeys * kFaD * 2;
   static constexpr int kVBytes = kFaKeys * kFaD * 2;
   static constexpr int kTotal = NT * kQBytes + 2 * (kKBytes + kVBytes) + 512 + 1024;
-  static constexpr uint32_t kTmemCols = NT * 256;            // S (later P) of every tile, then O of every tile
+  static constexpr uint32_t kTmemCols = 512;                 // S (later P) of every tile, or of a tile's even and odd blocks, then O alike
+  static constexpr int kAhead = 3 - NT;                      // blocks of a tile whose scores may be under way
 };
 
 // 5-D tiled load: the paged cache {d, slot in page, K|V, kv head, block}.
@@ -173,80 +175,63 @@ LX_DEVICE void fa_block_mask(uint32_t ts, int kb0, const FaBounds& bd) {
 }
 
 // Maximum over the 128 scores of a row (log2 domain).  Without a bias the scores grow with the products (scale > 0), so the largest product
-// gives it; MASK: keys outside the bounds do not count.
+// gives it.  Plain products have their masked keys at -inf already; MASK: keys outside the bounds do not count.  The code of capped and biased scores
+// here and in fa_block_probs is a rolled loop: a CTA of a short prompt fetches all its code for a block or two (unrolled, with and without masks:
+// 250 tokens of 32 heads with a bias 19 us -> 27).  Blocks that all rows see whole take capped scores without a mask (with it, 8192 tokens of 16 KV heads
+// 1640 us -> 2030); those with a bias, which are formed twice, gain nothing by that.
 template <int MODE, bool MASK>
 LX_DEVICE float fa_block_max(uint32_t ts, int kb0, const FaBounds& bd, const FaScore& sc) {
   float bm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  auto take = [&](const uint32_t (&r)[32], int c, bool mask) {
-    const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
+  if constexpr (MODE != kFaBias && !MASK) {
+    auto take = [&](const uint32_t (&r)[32]) {
 #pragma unroll
-    for (int q = 0; q < 32; q += 2) {
-      float t[2];
+      for (int q = 0; q < 32; q += 2) bm[(q >> 1) & 3] = fa_max3(bm[(q >> 1) & 3], __uint_as_float(r[q]), __uint_as_float(r[q + 1]));
+    };
+    uint32_t ra[32], rb[32];
+    tmem_ld_32x32b_x32(ts, ra);
+    fa_wait_ld(ra);
+    tmem_ld_32x32b_x32(ts + 32u, rb);
+    take(ra);
+    fa_wait_ld(rb);
+    tmem_ld_32x32b_x32(ts + 64u, ra);
+    take(rb);
+    fa_wait_ld(ra);
+    tmem_ld_32x32b_x32(ts + 96u, rb);
+    take(ra);
+    fa_wait_ld(rb);
+    take(rb);
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < kFaKeys; c += 32) {
+      if (bd.none(kb0 + c, 32)) continue;
+      const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
+      fa_wait_ld(r);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        t[u] = MODE == kFaBias ? sc.of<MODE>(__uint_as_float(r[q + u]), kb0 + c + q + u) : __uint_as_float(r[q + u]);
-        if (mask) t[u] = (q + u >= lo && q + u < hi) ? t[u] : -INFINITY;
+      for (int q = 0; q < 32; q += 2) {
+        float t[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          t[u] = MODE == kFaBias ? sc.of<MODE>(__uint_as_float(r[q + u]), kb0 + c + q + u) : __uint_as_float(r[q + u]);
+          t[u] = (q + u >= lo && q + u < hi) ? t[u] : -INFINITY;
+        }
+        bm[(q >> 1) & 3] = fa_max3(bm[(q >> 1) & 3], t[0], t[1]);
       }
-      bm[(q >> 1) & 3] = fa_max3(bm[(q >> 1) & 3], t[0], t[1]);
     }
-  };
-  auto chunk = [&](const uint32_t (&r)[32], int c) {
-    if (!MASK || bd.all(kb0 + c, 32)) take(r, c, false);
-    else if (!bd.none(kb0 + c, 32)) take(r, c, true);
-  };
-  uint32_t ra[32], rb[32];
-  tmem_ld_32x32b_x32(ts, ra);
-  fa_wait_ld(ra);
-  tmem_ld_32x32b_x32(ts + 32u, rb);
-  chunk(ra, 0);
-  fa_wait_ld(rb);
-  tmem_ld_32x32b_x32(ts + 64u, ra);
-  chunk(rb, 32);
-  fa_wait_ld(ra);
-  tmem_ld_32x32b_x32(ts + 96u, rb);
-  chunk(ra, 64);
-  fa_wait_ld(rb);
-  chunk(rb, 96);
+  }
   const float m = fmaxf(fa_max3(bm[0], bm[1], bm[2]), bm[3]);
   return MODE == kFaBias || m == -INFINITY ? m : sc.of<MODE>(m, 0);
 }
 
 // p = exp2(score - m_new) for the 128 keys of the block -> bf16 as a TMEM operand in the columns of the scores: those of 16 keys give
-// eight columns of weights (WIDE: and eight of the remainders).  Returns the row sum.  The exponentials of the next 16 keys are under way
-// while those before are summed, rounded and stored (one after the other 2360 cycles a block, 1024 of them the special function unit's).
+// eight columns of weights (WIDE: and eight of the remainders).  Returns the row sum.  Plain scores: the exponentials of the next 16 keys are
+// under way while those before are summed, rounded and stored (one after the other 2360 cycles a block, 1024 of them the special function unit's).
 template <int MODE, bool MASK, bool WIDE>
 LX_DEVICE float fa_block_probs(uint32_t ts, int kb0, const FaBounds& bd, float m_new, const FaScore& sc) {
   float sum = 0.f;
   const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
-  const unsigned long long scale2 = fa_pair(sc.scale_l2, sc.scale_l2), neg2 = fa_pair(neg_m, neg_m);
-  auto exps = [&](const uint32_t (&r)[16], int c, float (&e)[16]) {
-#pragma unroll
-    for (int q = 0; q < 16; q += 2) {
-      const float s0 = __uint_as_float(r[q]), s1 = __uint_as_float(r[q + 1]);
-      if (MODE == kFaPlain) {
-        const float2 x = fa_unpair(fa_fma2(fa_pair(s0, s1), scale2, neg2));
-        e[q] = fa_ex2(x.x);
-        e[q + 1] = fa_ex2(x.y);
-      } else {
-        e[q] = fa_ex2(sc.of<MODE>(s0, kb0 + c + q) + neg_m);
-        e[q + 1] = fa_ex2(sc.of<MODE>(s1, kb0 + c + q + 1) + neg_m);
-      }
-    }
-  };
-  auto chunk = [&](const uint32_t (&r)[16], int c, float (&e)[16]) {
-    if (MASK && bd.none(kb0 + c, 16)) {
-#pragma unroll
-      for (int q = 0; q < 16; ++q) e[q] = 0.f;
-      return;
-    }
-    exps(r, c, e);
-    if (MASK && !bd.all(kb0 + c, 16)) {
-      const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) e[q] = (q >= lo && q < hi) ? e[q] : 0.f;
-    }
-  };
-  auto finish = [&](const float (&e)[16], int c) {
+  auto finish = [&](const float* e, int c) {
     uint32_t pk[8], rest[8];
 #pragma unroll
     for (int q = 0; q < 16; q += 2) {
@@ -260,27 +245,59 @@ LX_DEVICE float fa_block_probs(uint32_t ts, int kb0, const FaBounds& bd, float m
     tmem_st_32x32b_x8(ts + (uint32_t)c, pk);
     if constexpr (WIDE) tmem_st_32x32b_x8(ts + (uint32_t)(c + 8), rest);
   };
-  uint32_t ra[16], rb[16];
-  float ea[16], eb[16];
-  tmem_ld_32x32b_x16(ts, ra);
-  fa_wait_ld(ra);
-  tmem_ld_32x32b_x16(ts + 16u, rb);
-  chunk(ra, 0, ea);
-#pragma unroll 1
-  for (int c = 0; c < kFaKeys - 32; c += 32) {
-    fa_wait_ld(rb);
-    tmem_ld_32x32b_x16(ts + (uint32_t)(c + 32), ra);
-    chunk(rb, c + 16, eb);
-    finish(ea, c);
+  if constexpr (MODE == kFaPlain) {
+    const unsigned long long scale2 = fa_pair(sc.scale_l2, sc.scale_l2), neg2 = fa_pair(neg_m, neg_m);
+    auto exps = [&](const uint32_t (&r)[16], float (&e)[16]) {
+#pragma unroll
+      for (int q = 0; q < 16; q += 2) {
+        const float2 x = fa_unpair(fa_fma2(fa_pair(__uint_as_float(r[q]), __uint_as_float(r[q + 1])), scale2, neg2));
+        e[q] = fa_ex2(x.x);
+        e[q + 1] = fa_ex2(x.y);
+      }
+    };
+    uint32_t ra[16], rb[16];
+    float ea[16], eb[16];
+    tmem_ld_32x32b_x16(ts, ra);
     fa_wait_ld(ra);
-    tmem_ld_32x32b_x16(ts + (uint32_t)(c + 48), rb);
-    chunk(ra, c + 32, ea);
-    finish(eb, c + 16);
+    tmem_ld_32x32b_x16(ts + 16u, rb);
+    exps(ra, ea);
+#pragma unroll 1
+    for (int c = 0; c < kFaKeys - 32; c += 32) {
+      fa_wait_ld(rb);
+      tmem_ld_32x32b_x16(ts + (uint32_t)(c + 32), ra);
+      exps(rb, eb);
+      finish(ea, c);
+      fa_wait_ld(ra);
+      tmem_ld_32x32b_x16(ts + (uint32_t)(c + 48), rb);
+      exps(ra, ea);
+      finish(eb, c + 16);
+    }
+    fa_wait_ld(rb);
+    exps(rb, eb);
+    finish(ea, kFaKeys - 32);
+    finish(eb, kFaKeys - 16);
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < kFaKeys; c += 32) {
+      float e[32];
+      if (MASK && bd.none(kb0 + c, 32)) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q) e[q] = 0.f;
+      } else {
+        const int lo = bd.lo - (kb0 + c), hi = bd.hi - (kb0 + c);
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(ts + (uint32_t)c, r);
+        fa_wait_ld(r);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          const float x = fa_ex2(sc.of<MODE>(__uint_as_float(r[q]), kb0 + c + q) + neg_m);
+          e[q] = !MASK || (q >= lo && q < hi) ? x : 0.f;
+        }
+      }
+      finish(e, c);
+      finish(e + 16, c + 16);
+    }
   }
-  fa_wait_ld(rb);
-  chunk(rb, kFaKeys - 16, eb);
-  finish(ea, kFaKeys - 32);
-  finish(eb, kFaKeys - 16);
   return sum;
 }
 
@@ -299,9 +316,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   uint64_t* k_empty = bars + 3;       // 2
   uint64_t* v_full = bars + 5;        // 2
   uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // per tile
-  uint64_t* p_full = bars + 11;       // per tile, an arrival per softmax warp: weights written, the product before them folded
-  uint64_t* pv_full = bars + 13;      // per tile
+  uint64_t* s_full = bars + 9;        // per tile; of a single tile, of its even and its odd blocks
+  uint64_t* p_full = bars + 11;       // alike, an arrival per softmax warp: weights written, the product before in their columns' O folded
+  uint64_t* pv_full = bars + 13;      // alike
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -385,16 +402,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         if (leader) report_status(p.status, code, tile);
         *abort_flag = 1;
       };
-      // S of tile t and block j.  It takes the columns of the weights that the product issued before it reads: one thread's MMAs run in order.
+      // S of tile t and block j.  It takes the columns of the weights that a product issued before it reads: one thread's MMAs run in order.
       auto issue_s = [&](int t, int j) {
+        const int at_s = NT == 2 ? t : j & 1;
         const uint64_t da = dq + (uint64_t)((t * S::kQBytes) >> 4), db = dk + (uint64_t)(((j & 1) * S::kKBytes) >> 4);
         if (leader) {
 #pragma unroll
           for (int ks = 0; ks < kFaD / 16; ++ks) {
             const uint64_t at = (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * 2);
-            umma_f16_ss(tmem_base + (uint32_t)(t * 128), da + at, db + at, idesc_s, ks > 0 ? 1u : 0u);
+            umma_f16_ss(tmem_base + (uint32_t)(at_s * 128), da + at, db + at, idesc_s, ks > 0 ? 1u : 0u);
           }
-          tc_commit(&s_full[t]);
+          tc_commit(&s_full[at_s]);
           if (t == NT - 1) tc_commit(&k_empty[j & 1]);
         }
         __syncwarp();
@@ -406,16 +424,23 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 #pragma unroll
       for (int t = 0; t < NT; ++t)
         if (ok) issue_s(t, 0);
+      if (NT == 1 && ok && nblk > 1) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&k_full[1], 0, abort_flag));
+        if (!ok) give_up(kTimeoutFullBarrier);
+        tc_fence_after();
+        if (ok) issue_s(0, 1);
+      }
       for (int j = 0; ok && j < nblk; ++j) {
         ok = __all_sync(0xffffffffu, mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag));
         if (!ok) { give_up(kTimeoutFullBarrier); break; }
         const uint64_t dvj = dv + (uint64_t)(((j & 1) * S::kVBytes) >> 4);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&p_full[t], j & 1, abort_flag));
+          const int at_s = NT == 2 ? t : j & 1;
+          ok = __all_sync(0xffffffffu, mbar_wait(&p_full[at_s], NT == 2 ? j & 1 : (j >> 1) & 1, abort_flag));
           if (!ok) { give_up(kTimeoutTmemEmpty); break; }
           tc_fence_after();
-          const uint32_t tmem_p = tmem_base + (uint32_t)(t * 128), tmem_o = tmem_base + (uint32_t)(NT * 128 + t * 128);
+          const uint32_t tmem_p = tmem_base + (uint32_t)(at_s * 128), tmem_o = tmem_base + (uint32_t)(256 + at_s * 128);
           if (leader) {
 #pragma unroll
             for (int ks = 0; ks < kFaKeys / 16; ++ks) {
@@ -423,17 +448,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
               umma_f16_ts(tmem_o, tmem_p + (uint32_t)(ks * 16), db, idesc_pv, ks > 0 ? 1u : 0u);
               if constexpr (WIDE) umma_f16_ts(tmem_o, tmem_p + (uint32_t)(ks * 16 + 8), db, idesc_pv, 1u);
             }
-            tc_commit(&pv_full[t]);
+            tc_commit(&pv_full[at_s]);
             if (t == NT - 1) tc_commit(&v_empty[j & 1]);
           }
           __syncwarp();
-          if (j + 1 < nblk) {
+          const int next = j + S::kAhead;
+          if (next < nblk) {
             if (t == 0) {
-              ok = __all_sync(0xffffffffu, mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag));
+              ok = __all_sync(0xffffffffu, mbar_wait(&k_full[next & 1], (next >> 1) & 1, abort_flag));
               if (!ok) { give_up(kTimeoutFullBarrier); break; }
               tc_fence_after();
             }
-            issue_s(t, j + 1);
+            issue_s(t, next);
           }
         }
       }
@@ -460,14 +486,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     // (the plain forms take the largest product for the largest score)
     const int mode = p.alibi != nullptr || !(p.scale > 0.f) ? kFaBias : p.softcap > 0.f ? kFaCap : kFaPlain;
     const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t ts = trow + (uint32_t)(t * 128), to = trow + (uint32_t)(NT * 128 + t * 128);
+    // where block j's scores and product lie, and which of the tile's barriers (and what parity) say that they are complete
+    auto part = [&](int j) { return NT == 2 ? t : j & 1; };
+    auto parity = [&](int j) { return (uint32_t)(NT == 2 ? j & 1 : (j >> 1) & 1); };
 
     float m = -INFINITY, l = 0.f;
     unsigned long long o[kFaD / 2];           // pairs of columns
 #pragma unroll
     for (int i = 0; i < kFaD / 2; ++i) o[i] = 0ull;
-    // o += the product of the block before, while the tensor core forms the next scores
-    auto fold = [&]() {
+    // o += the product of block j, relative to the largest score up to it
+    auto fold = [&](int j) {
+      if (!mbar_wait(&pv_full[part(j)], parity(j), abort_flag)) return false;
+      tc_fence_after();
+      const uint32_t to = trow + (uint32_t)(256 + part(j) * 128);
       auto add = [&](const uint32_t (&r)[32], int c) {
 #pragma unroll
         for (int q = 0; q < 32; q += 2) o[(c + q) >> 1] = fa_add2(o[(c + q) >> 1], fa_pair(__uint_as_float(r[q]), __uint_as_float(r[q + 1])));
@@ -485,36 +516,42 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       add(ra, 64);
       fa_wait_ld(rb);
       add(rb, 96);
+      return true;
     };
     bool alive = nblk > 0;
+    auto give_up = [&]() {
+      report_status(p.status, kTimeoutTmemFull, tile);
+      *abort_flag = 1;
+      alive = false;
+    };
 
     for (int j = 0; j < nblk && alive; ++j) {
       const int kb0 = (t_lo + j) * kFaKeys;
-      if (j > 0) {
-        if (!mbar_wait(&pv_full[t], (j - 1) & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
-        tc_fence_after();
-        fold();
-      }
-      if (!mbar_wait(&s_full[t], j & 1, abort_flag)) { report_status(p.status, kTimeoutTmemFull, tile); *abort_flag = 1; alive = false; break; }
+      // (two tiles: the product of the block before has to leave its columns first, and the other tile's runs meanwhile)
+      if (NT == 2 && j > 0 && !fold(j - 1)) { give_up(); break; }
+      if (!mbar_wait(&s_full[part(j)], parity(j), abort_flag)) { give_up(); break; }
       tc_fence_after();
+      const uint32_t ts = trow + (uint32_t)(part(j) * 128);
       // pass 1: block maximum of this row (log2 domain).  Plain scores have their masked keys set to -inf first, the others are masked chunk
       // by chunk: a capped -inf is finite
-      if (mode == kFaPlain && !bd.all(kb0, kFaKeys)) fa_block_mask(ts, kb0, bd);
+      const bool inside = bd.all(kb0, kFaKeys);
+      if (mode == kFaPlain && !inside) fa_block_mask(ts, kb0, bd);
       float bm;
       if (mode == kFaPlain) bm = fa_block_max<kFaPlain, false>(ts, kb0, bd, sc);
-      else if (mode == kFaCap) bm = fa_block_max<kFaCap, true>(ts, kb0, bd, sc);
+      else if (mode == kFaCap) bm = inside ? fa_block_max<kFaCap, false>(ts, kb0, bd, sc) : fa_block_max<kFaCap, true>(ts, kb0, bd, sc);
       else bm = fa_block_max<kFaBias, true>(ts, kb0, bd, sc);
       const float m_new = fmaxf(m, bm);
       const float alpha = (m_new == -INFINITY) ? 1.f : fa_ex2(m - m_new);
       // pass 2: weights -> bf16 operand, row sum
       float sum;
       if (mode == kFaPlain) sum = fa_block_probs<kFaPlain, false, WIDE>(ts, kb0, bd, m_new, sc);
-      else if (mode == kFaCap) sum = fa_block_probs<kFaCap, true, WIDE>(ts, kb0, bd, m_new, sc);
+      else if (mode == kFaCap) sum = inside ? fa_block_probs<kFaCap, false, WIDE>(ts, kb0, bd, m_new, sc) : fa_block_probs<kFaCap, true, WIDE>(ts, kb0, bd, m_new, sc);
       else sum = fa_block_probs<kFaBias, true, WIDE>(ts, kb0, bd, m_new, sc);
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
+      if (lane == 0) mbar_arrive(&p_full[part(j)]);
+      if (NT == 1 && j > 0 && !fold(j - 1)) { give_up(); break; }
       l = l * alpha + sum;
       if (j > 0 && !__all_sync(0xffffffffu, alpha == 1.f)) {      // some row of the warp saw a new maximum
         const unsigned long long alpha2 = fa_pair(alpha, alpha);
@@ -524,8 +561,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       m = m_new;
     }
     if (alive) {
-      if (mbar_wait(&pv_full[t], (nblk - 1) & 1, abort_flag)) {
+      if (mbar_wait(&pv_full[part(nblk - 1)], parity(nblk - 1), abort_flag)) {
         tc_fence_after();
+        const uint32_t to = trow + (uint32_t)(256 + part(nblk - 1) * 128);
         const float inv = l > 0.f ? attn_denominator(p.tail, head, m, l) * p.tail.scale : 0.f;
         const __nv_bfloat16* grow = p.tail.gate != nullptr ? p.tail.gate + (long long)(tok_base + qi) * p.tail.ldg + (long long)head * kFaD : nullptr;
         __nv_bfloat16* orow = p.out + (long long)(tok_base + qi) * p.ldo + (long long)head * kFaD;
@@ -601,8 +639,10 @@ static int launch_fa_t(const CUtensorMap& tq, const CUtensorMap& tkv, const FaPa
   launch_pdl(attn_prefill_tc_kernel<WIDE, NT>, dim3(num_tiles * (p.nh / (2 * NT))), dim3(S::kThreads), (size_t)S::kTotal, s, tq, tkv, p);
   return -(int)cudaGetLastError();
 }
-// Two tiles a CTA where the group allows it and single ones would take more than one wave.  In one wave a tile on its own is quicker: 123 tokens of 32
-// heads 11.6 -> 8.7 us, 500 18.3 -> 14.4; 15 tiles of 64 queries of three prompts, 240 CTAs, 15.2 with two tiles against 19.6.
+// Two tiles a CTA where the group allows it and single ones would take more than one wave.  In one wave a tile on its own is quicker, in two it is not:
+// 32 heads, us, one / two tiles a CTA: 123 tokens 9.5 / 12.3, 500 (128 CTAs of one) 15.0 / 18.8, capped 20.5 / 28.4; three prompts of 300 (240) 20.5 /
+// 16.4, capped 25.0 / 22.2; five of 100 behind 500 keys (160) 30.4 / 22.7.  One prompt of 640 to 1000 (160 to 256), whose CTAs are of unequal length, 17.6 / 21.1 to
+// 28.1 / 29.3.
 constexpr long long kFaSpreadTiles = 148;
 template <bool WIDE>
 static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tkv, const FaParams& p, int num_tiles, cudaStream_t s) {

@@ -384,6 +384,16 @@ def test_attn_prefill_tensor_core_tiles_and_masks(nat, nh, nkv, window, softcap,
         at += n
 
 
+@pytest.mark.parametrize("wide", [0, 1])
+@pytest.mark.parametrize("nh,nkv,window,softcap,bias", [(32, 8, 0, 0.0, False), (32, 8, 100, 0.0, False), (32, 8, 0, 20.0, False), (32, 8, 60, 20.0, False),
+                                                        (32, 8, 0, 0.0, True), (32, 4, 200, 15.0, True),
+                                                        (32, 16, 0, 0.0, False), (24, 4, 0, 20.0, False), (12, 2, 300, 20.0, False), (32, 16, 0, 0.0, True)])
+def test_attn_prefill_tensor_core_of_many_tiles(nat, nh, nkv, window, softcap, bias, wide):
+    """More tiles than SMs: two a CTA where a group has four heads or eight, one with two buffers of scores where it has two or six; one to eleven
+    blocks of keys, blocks that all rows see whole among them."""
+    test_attn_prefill_tensor_core_tiles_and_masks(nat, nh, nkv, window, softcap, bias, [1, 63, 64, 65, 129, 300, 40, 513], [0, 0, 127, 128, 300, 31, 1000, 900], wide)
+
+
 def _by_blocks(q, k, v, first, scale, block=128):
     """Attention of one head in float64 the way prompt attention forms it: keys in blocks, weights rounded to bf16 relative to the largest
     score up to and including their block, divided by the sum of the unrounded weights.  q [n, d] at positions first .., k and v [m, d]."""
