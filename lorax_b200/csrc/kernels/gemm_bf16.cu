@@ -1595,8 +1595,7 @@ static int make_tmap_lora_images(CUtensorMap* out, const void* base, uint64_t ro
 
 template <bool LORA>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ti, const LoraBMaps& bm, const GemmParams& base, const PairPlan& plan,
-                       int pairs, cudaStream_t stream) {
-  if (pairs < plan.grid) return 1;      // (the plan's pairs run at the same time)
+                       cudaStream_t stream) {
   GemmParams p = base;
   p.bn = p.umma_n = plan.bn;
   p.split_k = 1;
@@ -1631,9 +1630,8 @@ struct GemmPlan {
 // Steps of thousands of rows lose by an early start of the next kernel (see pdl_trigger).  Where the line lies matters little: passes of 300 to
 // 2500 rows took the same within 1 % with limits of 128, 512 and 2048.
 constexpr int kOverlapMaxTokens = 512;
-// Longer steps take pairs of CTAs.  The four projections of a 7B layer, us, one CTA a tile / pairs: 137 rows 133 / 156 (a pair's tile of 160 tokens leaves the
-// weights, which HBM has to bring, too few of the bytes in flight), 200 150 / 149, 256 158 / 156 (with 65 adapters a pass of four layers 1711 / 1677), 384
-// 193 / 197, 512 236 / 222, 1500 535 / 530, 4001 1362 / 1290.
+// Longer steps may take pairs of CTAs (below it a pair's tile leaves the weights, which HBM has to bring, too few of the bytes in flight: the four
+// projections of a 7B layer at 137 rows 133 us one CTA a tile, 156 by pairs).
 constexpr int kPairMinTokens = 192;
 constexpr int kModeConstWeights = 1 << 16;     // of a launch's `mode`: no kernel that may still run writes the weights
 
@@ -1731,6 +1729,20 @@ static GemmPlan choose_plan_swap(int T, int N, int K, int num_sms, long long ws_
   return best;
 }
 
+// Tokens on the M side: the feature tile (UMMA N) whose tile count wastes the fewest SM slots in the last wave;
+// 32-wide steps keep the epilogue's 16-byte stores whole.
+static GemmPlan choose_plan_tokens(int T, int N, int K, int num_sms, long long ws_bytes, bool have_counters, int force_bn, int sk_policy) {
+  const int tiles_t = (T + kBM - 1) / kBM, kblocks = (K + kBK - 1) / kBK;
+  GemmPlan best{};
+  best.cost = 1e30;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    if (force_bn >= 32 && force_bn <= 256 && force_bn % 32 == 0 && bn != force_bn) continue;
+    const GemmPlan pl = plan_tiles(tiles_t * ((N + bn - 1) / bn), kblocks, K, bn, num_sms, ws_bytes, have_counters, sk_policy);
+    if (pl.cost < best.cost) best = pl;
+  }
+  return best.cost < 1e30 ? best : plan_tiles(tiles_t * ((N + 255) / 256), kblocks, K, 256, num_sms, ws_bytes, have_counters, sk_policy);
+}
+
 }  // namespace lx
 
 extern "C" {
@@ -1779,38 +1791,25 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
   p.out_scale = out_scale;
   p.split_k = 1;
   CUtensorMap ta, tb;
-  int bn;
   const bool has_lora = (lora != nullptr && lora->tiles != nullptr && lora->num_tiles > 0);
   const int force_bn = force_split >> 16;
-  const int kblocks_all = (K + kBK - 1) / kBK;
-  // Tokens on the M side: the feature tile (UMMA N) whose tile count wastes the fewest SM slots in the last wave;
-  // 32-wide steps keep the epilogue's 16-byte stores whole.
-  GemmPlan pl_tok{};
-  pl_tok.cost = 1e30;
-  {
-    const int tiles_t = (T + kBM - 1) / kBM;
-    for (int cand = 256; cand >= 64; cand -= 32) {
-      if (force_bn >= 32 && force_bn <= 256 && force_bn % 32 == 0 && cand != force_bn) continue;
-      GemmPlan c = plan_tiles(tiles_t * ((N + cand - 1) / cand), kblocks_all, K, cand, num_sms, usable_ws, have_counters, sk_policy);
-      if (c.cost < pl_tok.cost) pl_tok = c;
-    }
-    if (pl_tok.cost >= 1e30) pl_tok = plan_tiles(tiles_t * ((N + 255) / 256), kblocks_all, K, 256, num_sms, usable_ws, have_counters, sk_policy);
-  }
   // Orientation.  Up to 128 tokens the weights take the M side (no padded MMA rows, the token tile is the small
   // operand).  Above that both plans are costed.  The LoRA stages are written for weights on M.
-  bool swap;
-  GemmPlan pl_swap{};
-  if (mode == 1 || has_lora || (mode == 0 && T <= 128)) {
-    swap = true;
-  } else if (mode == 2) {
-    swap = false;
-  } else {
-    pl_swap = choose_plan_swap(T, N, K, num_sms, usable_ws, have_counters, force_split & 0xffff, force_bn, sk_policy);
-    swap = pl_swap.cost <= pl_tok.cost;
+  bool swap = mode == 1 || has_lora || (mode == 0 && T <= 128);
+  if (mode != 2 || has_lora) pl = choose_plan_swap(T, N, K, num_sms, usable_ws, have_counters, force_split & 0xffff, force_bn, sk_policy);
+  if (!swap) {
+    const GemmPlan pl_tok = choose_plan_tokens(T, N, K, num_sms, usable_ws, have_counters, force_bn, sk_policy);
+    swap = mode != 2 && pl.cost <= pl_tok.cost;
+    if (!swap) pl = pl_tok;
   }
+  // Pairs of CTAs, where they are quicker than that
   PairPlan pair{};
-  if (T > kPairMinTokens && N >= 256 && (mode <= 1 || has_lora) && force_split == 0 && sk_policy == 0)
-    pair = pair_plan(T, N, K, num_sms / 2, usable_ws);
+  if (T > kPairMinTokens && N >= 256 && (mode <= 1 || has_lora) && force_split == 0 && sk_policy == 0) {
+    const int fit = has_lora ? pair_capacity<true>() : pair_capacity<false>();
+    if (fit < 0) return fit;
+    const int pairs = fit < num_sms / 2 ? fit : num_sms / 2;
+    if (pairs > 0) pair = choose_pair(T, N, K, pairs, usable_ws, pl.cost, has_lora ? lora->max_rank : 0);
+  }
   p.overlap = T <= kOverlapMaxTokens;
   if (swap) {
     p.a_rows = N; p.b_rows = T;
@@ -1819,25 +1818,16 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     p.hint_a_first = 1;
     p.w_preload = w_const && p.overlap ? 1 : 0;
     p.b_fastest = 1;          // token tiles of one weight tile run side by side: the weight tile leaves HBM once
-    pl = choose_plan_swap(T, N, K, num_sms, usable_ws, have_counters, force_split & 0xffff, force_split >> 16, sk_policy);
-    bn = pl.bn;
-    p.umma_n = bn;
-    if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
-    if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, bn)) return -1003;
   } else {
-    pl = pl_tok;
-    bn = pl.bn;
     p.a_rows = T; p.b_rows = N;
-    p.umma_n = bn;
     p.ldo_a = ldo; p.ldo_b = 1;
     p.bias_on_a = 0;
     p.hint_a_first = 0;
     p.w_preload = w_const && p.overlap ? 2 : 0;
     p.b_fastest = 0;
-    if (make_tmap_bf16_kmajor(&ta, x, T, K, ldx, kBM)) return -1002;
-    if (make_tmap_bf16_kmajor(&tb, w, N, K, ldw, bn)) return -1003;
   }
-  p.bn = bn;
+  const int bn = pl.bn;
+  p.bn = p.umma_n = bn;
   p.split_k = pl.split;
   p.dp_tiles = pl.dp_tiles;
   p.sk_ctas = pl.sk_ctas;
@@ -1897,20 +1887,20 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     }
     if (pair.bn > 0 && p.lora_inline_shrink && (lora->nparts == 1 || (lora->n0 % 256 == 0 && (lora->nparts == 2 || lora->n1 % 256 == 0))) &&
         img_bytes / 48 * 64 <= lora->vimg_bytes) {
-      const int pairs = pair_capacity<true>();
-      CUtensorMap ti, tb2;
-      if (pairs > 0 && make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32)) == 0 && make_tmap_bf16_kmajor(&tb2, x, T, K, ldx, pair.bn / 2) == 0) {
-        GemmParams q = p;
-        q.lora_mask = 31;
-        q.lora_slice = 64 * 16;
-        const long long img64 = img_bytes / 48 * 64, grid = 2ll * pair.grid;
-        const bool shared_k = lora->sync_ints >= 2 + grid && lora->vimg_bytes - img64 >= grid * 128 * 4;
-        q.lora_kparts = shared_k ? reinterpret_cast<float*>(static_cast<char*>(lora->vimg) + img64) : nullptr;
-        q.lora_kcounters = lora->sync + 2;
-        const int rc = launch_pair<true>(ta, tb2, ti, bm, q, pair, pairs, stream);
-        if (rc != 1) return rc;
-      }
+      CUtensorMap ti;
+      if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
+      if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair.bn / 2)) return -1003;
+      if (make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32))) return -1004;
+      p.lora_mask = 31;
+      p.lora_slice = 64 * 16;
+      const long long img64 = img_bytes / 48 * 64, grid = 2ll * pair.grid;
+      const bool shared_k = lora->sync_ints >= 2 + grid && lora->vimg_bytes - img64 >= grid * 128 * 4;
+      p.lora_kparts = shared_k ? reinterpret_cast<float*>(static_cast<char*>(lora->vimg) + img64) : nullptr;
+      p.lora_kcounters = lora->sync + 2;
+      return launch_pair<true>(ta, tb, ti, bm, p, pair, stream);
     }
+    if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
+    if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, bn)) return -1003;
     switch (template_bn(bn)) {
       case 16:  return launch_gemm_t<16, 8, true>(ta, tb, bm, p, pl.grid, stream);
       case 32:  return launch_gemm_t<32, 8, true>(ta, tb, bm, p, pl.grid, stream);
@@ -1920,18 +1910,14 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
     }
   }
   if (pair.bn > 0) {
-    const int pairs = pair_capacity<false>();
-    if (pairs > 0) {
-      CUtensorMap ta2, tb2;
-      if (make_tmap_bf16_kmajor(&ta2, w, N, K, ldw, kBM)) return -1002;
-      if (make_tmap_bf16_kmajor(&tb2, x, T, K, ldx, pair.bn / 2)) return -1003;
-      GemmParams q = p;
-      q.a_rows = N; q.b_rows = T;
-      q.ldo_a = 1; q.ldo_b = ldo; q.bias_on_a = 1;
-      const int rc = launch_pair<false>(ta2, tb2, ta2, LoraBMaps{}, q, pair, pairs, stream);
-      if (rc != 1) return rc;
-    }
+    p.a_rows = N; p.b_rows = T;
+    p.ldo_a = 1; p.ldo_b = ldo; p.bias_on_a = 1;
+    if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
+    if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair.bn / 2)) return -1003;
+    return launch_pair<false>(ta, tb, ta, LoraBMaps{}, p, pair, stream);
   }
+  if (make_tmap_bf16_kmajor(&ta, swap ? w : x, swap ? N : T, K, swap ? ldw : ldx, kBM)) return -1002;
+  if (make_tmap_bf16_kmajor(&tb, swap ? x : w, swap ? T : N, K, swap ? ldx : ldw, bn)) return -1003;
   switch (template_bn(bn)) {
     case 16:  return launch_gemm<16, 8>(ta, tb, p, pl.grid, stream);
     case 32:  return launch_gemm<32, 8>(ta, tb, p, pl.grid, stream);
@@ -1950,6 +1936,18 @@ int lx_gemm_plan(int T, int N, int K, int num_sms, long long ws_bytes, int force
 
 // Bytes of B_cat (rank r, N features) that the CTA with feature tile `tile` of 128 prefetches.
 unsigned lx_lora_tile_bytes(int N, int tile, int r) { return lx::lora_tile_bytes(N, tile, r); }
+
+// The plan of pairs of CTAs for a shape and its largest adapter rank (0: none), at most `pairs` at once: out4 = {token tile (0: single CTAs are
+// quicker), whole tiles, pairs that share the others, pairs}.
+int lx_gemm_pair_plan(int T, int N, int K, int num_sms, int pairs, long long ws_bytes, int lora_rank, int* out4) {
+  using namespace lx;
+  GemmPlan pl = choose_plan_swap(T, N, K, num_sms, ws_bytes, ws_bytes > 0, 0, 0, 0);
+  const GemmPlan pl_tok = choose_plan_tokens(T, N, K, num_sms, ws_bytes, ws_bytes > 0, 0, 0);
+  if (lora_rank == 0 && pl_tok.cost < pl.cost) pl = pl_tok;
+  const PairPlan pair = choose_pair(T, N, K, pairs, ws_bytes, pl.cost, lora_rank);
+  out4[0] = pair.bn; out4[1] = pair.dp_tiles; out4[2] = pair.sk_pairs; out4[3] = pair.grid;
+  return 0;
+}
 
 // out[T, N] = x[T, K] @ w[N, K]^T (+ bias[N]).  `ldx`, `ldw`, `ldo` are row strides in elements.
 // mode: low byte 0 = choose, 1 = force weights on the M side (small T), 2 = force activations on the M side; bits 8..9 the

@@ -446,4 +446,20 @@ static PairPlan pair_plan(int T, int N, int K, int pairs, long long ws_bytes) {
   return best;
 }
 
+// The same, with token tile 0 where single CTAs (a plan of `single_cost`) are as quick.  Both costs leave out what every launch has, and pairs have more
+// of it (two barriers of the cluster, columns allocated for both): 4 us and 15 % of the pairs' cost is where they are worth it over 2960 shapes of 193
+// to 4001 rows, 256 to 28672 features, K 128 to 14336.  Where the rule takes pairs they win up to 1.5x (4001 rows, us, single / pairs: 28672 x 4096 1.10x,
+// 4096 x 14336 1.12x; 512 rows 1.19x both), 18 shapes lose 3 to 11 %; always pairs lost more than 3 % in 1550 (K = 256, 1000 rows: 20 %; 11008 x 4096, 320
+// rows: 29 %).
+// With adapters of rank `lora_rank` the first tile of a pair waits for the shrink, and a pair holds twice the tile: only where most pairs have
+// three tiles or a feature tile of their own, K of 2048 and ranks of up to 32 (r 16, one adapter / 24: 28672 x 4096 of 256 rows 1.07x / 1.03x, of 2000 1.07x / 1.06x;
+// without these lines 4096 x 14336 of 1000 rows 0.90x, rank 64 with 24 adapters 0.85 to 0.97x nearly everywhere).
+constexpr double kPairCostFactor = 1.15, kPairCostMore = 4000.0;
+static PairPlan choose_pair(int T, int N, int K, int pairs, long long ws_bytes, double single_cost, int lora_rank) {
+  PairPlan plan = pair_plan(T, N, K, pairs, ws_bytes);
+  const int tiles_a = (N + 255) / 256, tiles = plan.bn > 0 ? tiles_a * ((T + plan.bn - 1) / plan.bn) : 0;
+  if (plan.cost * kPairCostFactor + kPairCostMore >= single_cost || (lora_rank > 0 && (lora_rank > 32 || K < 2048 || (tiles_a < pairs && tiles < 3 * pairs)))) plan.bn = 0;
+  return plan;
+}
+
 }  // namespace lx

@@ -82,3 +82,19 @@ def test_prefetches_of_adapter_rows_stay_inside(N, r):
     sizes = [native.load().lx_lora_tile_bytes(N, tile, r) for tile in range((N + 255) // 256 * 2)]
     assert sum(sizes) == N * r * 2
     assert all(size % 16 == 0 and tile * 128 * r * 2 + size <= N * r * 2 for tile, size in enumerate(sizes) if size)
+
+
+@pytest.mark.parametrize("T,N,K,rank,taken", [
+    (4001, 28672, 4096, 0, True), (256, 4096, 14336, 0, True), (512, 28672, 4096, 0, True),
+    (1000, 4096, 256, 0, False), (2048, 512, 1024, 0, False), (320, 11008, 4096, 0, False), (193, 256, 64, 0, False),      # 20, 10, 29 % slower by pairs
+    (256, 28672, 4096, 16, True), (4001, 4096, 4096, 32, True),
+    (1000, 4096, 14336, 16, False), (800, 17920, 1536, 16, False), (200, 28672, 4096, 64, False)])                          # 10, 8, 6 %
+def test_pairs_of_ctas_only_where_they_measured_quicker(T, N, K, rank, taken):
+    import ctypes
+
+    from lorax_b200.ops import native
+    out = (ctypes.c_int * 4)()
+    native.load().lx_gemm_pair_plan(T, N, K, 148, 74, 64 << 20, rank, out)
+    assert (out[0] > 0) == taken
+    native.load().lx_gemm_pair_plan(T, N, K, 148, 40, 64 << 20, rank, out)
+    assert out[3] <= 40 and out[2] <= 40

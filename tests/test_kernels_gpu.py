@@ -1,4 +1,5 @@
 """Numerics of every CUDA kernel against the fp32 PyTorch statement of the same operator."""
+import ctypes
 import math
 
 import pytest
@@ -907,12 +908,20 @@ def test_gemm_with_lora_of_few_units(nat, T, K, parts, ranks, layout):
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
 
 
-@pytest.mark.parametrize("T,K,parts,ranks,layout", [(200, 256, [320], [16, 32], "runs"), (257, 1024, [384], [64, 16, 48, 32], "blocks"), (300, 512, [448], [16, 48, 64, 32], "alternating"),
-                                                    (520, 136, [512, 256, 320], [16, 64], "runs"), (600, 256, [12864], [32, 16], "runs"), (600, 128, [12800, 200], [16], "alternating"),
-                                                    (700, 4096, [2880], [16, 64, 32], "runs")])
+def _pair_tile(nat, T, N, K, rank=0):
+    """Token tile of a product that pairs of CTAs take, 0 where single CTAs do."""
+    ws, out = nat.workspace(), (ctypes.c_int * 4)()
+    nat.load().lx_gemm_pair_plan(T, N, K, ws.num_sms, ws.num_sms // 2, ws.gemm_ws.numel(), rank, out)
+    return out[0]
+
+
+@pytest.mark.parametrize("T,K,parts,ranks,layout", [(200, 2048, [19264], [16, 32], "runs"), (257, 4096, [19072], [32, 16], "alternating"),
+                                                    (300, 4096, [12800, 6208], [16], "alternating"), (520, 2048, [4096, 15168], [32, 16], "runs"),
+                                                    (6000, 2048, [3264], [16, 32], "runs"), (5000, 2048, [4096, 1024, 320], [16, 32, 16, 32], "blocks")])
 def test_gemm_with_lora_of_ragged_pairs(nat, T, K, parts, ranks, layout):
     """Pairs of CTAs whose last tile of 256 features is not full, the second CTA's half partly or all past the last feature: one part and several, a tile a
     pair and more."""
+    assert _pair_tile(nat, T, sum(parts), K, max(ranks)) > 0 and sum(parts) % 256
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
 
 
@@ -988,6 +997,13 @@ def test_products_of_cta_pairs(nat, T, N, K):
     wide = torch.full((T, N + 24), 7.0, dtype=torch.bfloat16, device="cuda")      # rows of a wider buffer: nothing beside them is written
     nat.gemm(x, w, out=wide[:, :N])
     assert torch.equal(wide[:, :N], nat.gemm(x, w)) and (wide[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("T,N,K", [(193, 28700, 4096), (256, 4100, 14336), (545, 6144, 8192), (700, 4360, 8200), (2047, 640, 14344), (3000, 2880, 2880), (4001, 4096, 1024)])
+def test_products_that_pairs_of_ctas_take(nat, T, N, K):
+    """The same where the plan prefers pairs: whole tiles in one wave and several, and all tiles shared."""
+    assert _pair_tile(nat, T, N, K) > 0
+    test_products_of_cta_pairs(nat, T, N, K)
 
 
 @pytest.mark.parametrize("act", ["", "relu2", "swiglu"])
