@@ -379,6 +379,14 @@ LX_DEVICE bool lora_join_kparts(const GemmParams& p, const ShrinkUnit& s, int pa
   return true;
 }
 
+// Parts of a unit's K where `ctas` CTAs share `units` units of `nbatch` batches: as many as there are CTAs for, where that takes three batches or more
+// off the chain.  With fewer the sums' way through L2 costs as much as it saves (one of the two of K = 1536, two of the four of 4096, 1 to 64 rows: 3 to
+// 9 % slower; three of four 1 to 9 % quicker, ten of fourteen 8 to 14 %).
+__host__ __device__ constexpr int lora_shrink_k_parts(int ctas, int units, int nbatch) {
+  const int most = units > 0 ? ctas / units : 0, parts = most < nbatch ? most : nbatch;
+  return parts > 1 && nbatch - (nbatch + parts - 1) / parts >= 3 ? parts : 1;
+}
+
 template <int NG, int SB>
 LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, float* red, int ewarp, int lane) {
   const int tid4 = ewarp * 32 + lane;
@@ -388,8 +396,7 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
   // Few units: several CTAs share the K of each, and the last of them to arrive sums their parts in order.  A unit moves 32 KB per 1024 of K
   // into its SM, beside the base tiles that every SM takes in at its full rate, in batches that wait for one another: with one row in the step
   // the one to three CTAs that had a unit were done 10 us (K = 4096) to 21 us (14336) behind the wait, and every tile's expand waited for them.
-  int parts = 1;
-  if (NG == 1 && p.lora_kparts != nullptr && U > 0) parts = max(1, min((int)gridDim.x / U, nbatch));
+  const int parts = NG == 1 && p.lora_kparts != nullptr ? lora_shrink_k_parts((int)gridDim.x, U, nbatch) : 1;
   const int total = U * parts;
   int x = (int)blockIdx.x;
   if (x < total) {
@@ -1936,6 +1943,9 @@ int lx_gemm_plan(int T, int N, int K, int num_sms, long long ws_bytes, int force
 
 // Bytes of B_cat (rank r, N features) that the CTA with feature tile `tile` of 128 prefetches.
 unsigned lx_lora_tile_bytes(int N, int tile, int r) { return lx::lora_tile_bytes(N, tile, r); }
+
+// Parts of K of each of a short step's `units` shrink units in a launch of `ctas` CTAs.
+int lx_lora_fused_k_parts(int ctas, int units, int K) { return lx::lora_shrink_k_parts(ctas, units, ((K + 31) / 32 + 31) / 32); }
 
 // The plan of pairs of CTAs for a shape and its largest adapter rank (0: none), at most `pairs` at once: out4 = {token tile (0: single CTAs are
 // quicker), whole tiles, pairs that share the others, pairs}.
