@@ -92,11 +92,12 @@ struct GemmParams {
   int lora_fence_maps;                 // 1: acquire-fence a slot's B_cat map before every use (0: never; measurement only)
   int lora_skip;                       // measurement only: bit 0 leaves out the shrink launch, bit 1 the expand stages (results are then wrong)
   int lora_T;                          // rows of the step
-  int lora_mask, lora_slice;           // an entry's window begins and ends at multiples of mask + 1 rows; elements of a K slice of an image
 };
 
 // ---- LoRA items ----------------------------------------------------------------------------------------------
 constexpr int kLoraWin = 48;            // a run of <= 32 rows lies inside a 16-aligned window of at most 48 rows
+// (pairs of CTAs, whose accumulators are cut in steps of 32 columns: windows of 64 rows that begin and end at multiples of 32)
+constexpr int kLoraPairWin = 64;
 constexpr int kLoraSliceElems = kLoraWin * 16;      // one K slice (16 ranks) of an image: 48 rows of 32 bytes
 constexpr int kLoraSliceBytes = kLoraSliceElems * 2;
 constexpr int kLoraImgElems = 4 * kLoraSliceElems;  // ranks up to 64
@@ -156,7 +157,9 @@ struct ExpandItem {
 };
 // -1: end of the live entries or of those that can meet the tile (they are sorted by row), 0: nothing to add for this
 // entry, 1: `e` is valid.
-LX_DEVICE int decode_expand_item(const LoraEnt* ents, int lt, int j0, int jlim, int mask, ExpandItem& e) {
+template <int WIN>
+LX_DEVICE int decode_expand_item(const LoraEnt* ents, int lt, int j0, int jlim, ExpandItem& e) {
+  constexpr int mask = WIN - 33;
   const LoraEnt t = ents[lt];
   if (t.slot < 0 || t.row0 >= jlim) return -1;
   if (t.r == 0) return 0;
@@ -387,7 +390,7 @@ __host__ __device__ constexpr int lora_shrink_k_parts(int ctas, int units, int n
   return parts > 1 && nbatch - (nbatch + parts - 1) / parts >= 3 ? parts : 1;
 }
 
-template <int NG, int SB>
+template <int NG, int SB, int WIN>
 LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, float* red, int ewarp, int lane) {
   const int tid4 = ewarp * 32 + lane;
   const int U = (int)gstart[p.lora_num_tiles];
@@ -413,7 +416,8 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
       ShrinkUnit nxt = cur;
       int nb = b + 1;
       bool more = true;
-      if (nb == cur.b1) {
+      const int last = NG == 1 ? cur.b1 : nbatch;
+      if (nb == last) {
         x += (int)gridDim.x;
         more = x < total;
         if (more) {
@@ -433,14 +437,15 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
           }
         }
       }
-      if (b == cur.b1 - 1) {
+      if (b == last - 1) {
         // the unit is complete: 16 ranks x up to 8 rows per group.  This warp holds (rank g, rows 2t, 2t+1) and (rank g + 8, same
         // rows) of every group; the groups go through the two staging buffers one after the other.
         const LoraEnt e = ents[cur.lt];
-        const int w0 = e.row0 & ~p.lora_mask;
-        const int wn = ((e.row0 + e.nrows + p.lora_mask) & ~p.lora_mask) - w0;
+        constexpr int mask = WIN - 33;
+        const int w0 = e.row0 & ~mask;
+        const int wn = ((e.row0 + e.nrows + mask) & ~mask) - w0;
         const int pp = cur.j / cur.r, i0 = cur.j - pp * cur.r;
-        __nv_bfloat16* img = p.lora_vimg + ((long long)(pp * 4 + (i0 >> 4)) * p.lora_num_tiles + cur.lt) * p.lora_slice;
+        __nv_bfloat16* img = p.lora_vimg + ((long long)(pp * 4 + (i0 >> 4)) * p.lora_num_tiles + cur.lt) * (WIN * 16);
 #pragma unroll
         for (int q = 0; q < NG; ++q) {
           if (q * kShrinkRows < cur.nt) {              // the same for the four warps: they meet at the barrier below
@@ -473,10 +478,14 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
             const int z_lo = (t0g == e.row0) ? e.row0 - w0 : 0;
             const int z_hi = (t0g + ntg == e.row0 + e.nrows) ? e.row0 + e.nrows - w0 : wn;
             const int zrows = z_lo + (wn - z_hi);
-            for (int z = tid4 - 32; whole && z >= 0 && z < 2 * zrows; z += 96) {
+            auto clear = [&](int z) {
               const int cz = z >> 1, ch = z & 1;
               const int row = cz < z_lo ? cz : z_hi + (cz - z_lo);
               *reinterpret_cast<uint4*>(img + row * 16 + (ch << 3)) = make_uint4(0, 0, 0, 0);
+            };
+            if (whole && tid4 >= 32) {
+              if (tid4 - 32 < 2 * zrows) clear(tid4 - 32);
+              if (4 * mask > 96 && tid4 + 64 < 2 * zrows) clear(tid4 + 64);
             }
             par ^= 1;
             acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
@@ -502,9 +511,10 @@ LX_DEVICE void lora_shrink_units_t(const GemmParams& p, const LoraEnt* ents, con
   }
 }
 
+template <int WIN>
 LX_DEVICE void lora_shrink_units(const GemmParams& p, const LoraEnt* ents, const unsigned short* gstart, float* red, int ewarp, int lane) {
-  if (lora_shrink_unit_rows(p) == kShrinkRows) lora_shrink_units_t<1, 8>(p, ents, gstart, red, ewarp, lane);
-  else lora_shrink_units_t<4, 4>(p, ents, gstart, red, ewarp, lane);
+  if (lora_shrink_unit_rows(p) == kShrinkRows) lora_shrink_units_t<1, 8, WIN>(p, ents, gstart, red, ewarp, lane);
+  else lora_shrink_units_t<4, 4, WIN>(p, ents, gstart, red, ewarp, lane);
 }
 
 // Bounded wait for *flag == want.  False when the budget ran out.
@@ -527,7 +537,9 @@ LX_DEVICE bool wait_flag(const int* flag, int want, volatile int* abort_flag) {
 // the same list in their own shared-memory area, 32 entries at a time (one per lane, ranks -> slices by a warp prefix sum), and
 // keep it while the token tile stays the same: it does not depend on the feature tile.
 // First live entry whose aligned window ends after row j0 (entries are sorted by row and do not overlap).
-LX_DEVICE int lora_first_entry(const LoraEnt* ents, int n_live, int j0, int mask) {
+template <int WIN>
+LX_DEVICE int lora_first_entry(const LoraEnt* ents, int n_live, int j0) {
+  constexpr int mask = WIN - 33;
   int lo = 0, hi = n_live;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
@@ -553,11 +565,12 @@ struct LoraStageHeader {
   int nu, last, pad_[2];
 };
 constexpr int kLoraListCap = 256;       // units a list holds; it is worked off whenever it holds 128 or more
+template <int WIN>
 LX_DEVICE int lora_build_units(const GemmParams& p, const LoraEnt* ents, int lt0, int j0, int jlim, LoraUnit* list, int n, bool& ended) {
   const int lane = threadIdx.x & 31;
   const int lt = lt0 + lane;
   ExpandItem e;
-  const int rc = lt < p.lora_num_tiles ? decode_expand_item(ents, lt, j0, jlim, p.lora_mask, e) : -1;
+  const int rc = lt < p.lora_num_tiles ? decode_expand_item<WIN>(ents, lt, j0, jlim, e) : -1;
   const unsigned endmask = __ballot_sync(0xffffffffu, rc < 0);
   const int first_end = endmask ? __ffs(endmask) - 1 : 32;
   const int nsl = (rc == 1 && lane < first_end) ? e.r / 16 : 0;
@@ -580,12 +593,13 @@ LX_DEVICE int lora_build_units(const GemmParams& p, const LoraEnt* ents, int lt0
 
 // The complete unit list of token tile [j0, jlim), if it fits the list: built ahead of time (before the kernel waits for its
 // predecessor) for the CTA's first tile.  Returns the number of units, or -1 when the list would not hold them all.
+template <int WIN>
 LX_DEVICE int lora_prebuild_units(const GemmParams& p, const LoraEnt* ents, int n_live, int j0, int jlim, LoraUnit* list) {
   int n = 0;
   bool ended = false;
-  for (int lt0 = lora_first_entry(ents, n_live, j0, p.lora_mask); !ended && lt0 < p.lora_num_tiles; lt0 += 32) {
+  for (int lt0 = lora_first_entry<WIN>(ents, n_live, j0); !ended && lt0 < p.lora_num_tiles; lt0 += 32) {
     if (n > kLoraListCap - 128) return -1;             // 32 entries yield up to 128 units
-    n = lora_build_units(p, ents, lt0, j0, jlim, list, n, ended);
+    n = lora_build_units<WIN>(p, ents, lt0, j0, jlim, list, n, ended);
   }
   return n;
 }
@@ -798,7 +812,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         if (it0.next(w0) && w0.kb0 == 0) {
           const int ta0 = p.b_fastest ? w0.tile / tiles_b : w0.tile % tiles_a;
           const int tb0 = p.b_fastest ? w0.tile % tiles_b : w0.tile / tiles_a;
-          const int n0 = lora_prebuild_units(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.umma_n, ulist_p);
+          const int n0 = lora_prebuild_units<kLoraWin>(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.umma_n, ulist_p);
           if (n0 >= 0) { pre_tb = tb0; pre_n = n0; }
           if (n0 > 0 && p.lora_arena_maps) lora_prefetch_b(p, ulist_p, n0, ta0);
         }
@@ -850,7 +864,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           // the whole warp, while the ring still holds the stages of the tile before: this tile's unit list (kept while the token
           // tile stays the same) and its B_cat rows on their way into L2 under the base k-blocks
           if (list_tb != tb) {
-            const int n0 = lora_prebuild_units(p, ents, *n_live, tb * p.bn, tb * p.bn + p.umma_n, ulist_p);
+            const int n0 = lora_prebuild_units<kLoraWin>(p, ents, *n_live, tb * p.bn, tb * p.bn + p.umma_n, ulist_p);
             list_tb = n0 >= 0 ? tb : -1;
             list_n = n0 >= 0 ? n0 : 0;
           }
@@ -956,10 +970,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             // more units than the list holds: built and sent in pieces
             int n = 0;
             bool ended = false;
-            for (int lt0 = lora_first_entry(ents, *n_live, j0, p.lora_mask); ok; lt0 += 32) {
+            for (int lt0 = lora_first_entry<kLoraWin>(ents, *n_live, j0); ok; lt0 += 32) {
               bool last = true;
               if (lt0 < p.lora_num_tiles) {
-                n = lora_build_units(p, ents, lt0, j0, jlim, ulist_p, n, ended);
+                n = lora_build_units<kLoraWin>(p, ents, lt0, j0, jlim, ulist_p, n, ended);
                 last = ended || lt0 + 32 >= p.lora_num_tiles;
                 if (n < 128 && !last) continue;
               }
@@ -1060,7 +1074,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     PendingTile pending[2];
     int n_pending = 0;
     if constexpr (LORA) {
-      if (lora && p.lora_inline_shrink) lora_shrink_units(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
+      if (lora && p.lora_inline_shrink) lora_shrink_units<kLoraWin>(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
     }
     GemmWorkIter<BN> it(p, num_tiles, kblocks);
     GemmWork w;
@@ -1860,8 +1874,6 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       p.lora_skip = e ? atoi(e) : 0;
     }
     p.lora_T = T;
-    p.lora_mask = 15;
-    p.lora_slice = kLoraSliceElems;
     p.lora_off_a = lora->off_a;
     p.lora_arena = reinterpret_cast<const __nv_bfloat16*>(lora->arena);
     p.lora_x = reinterpret_cast<const __nv_bfloat16*>(x);
@@ -1893,14 +1905,12 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
       if (rc != 0) return rc;
     }
     if (pair.bn > 0 && p.lora_inline_shrink && (lora->nparts == 1 || (lora->n0 % 256 == 0 && (lora->nparts == 2 || lora->n1 % 256 == 0))) &&
-        img_bytes / 48 * 64 <= lora->vimg_bytes) {
+        img_bytes / kLoraWin * kLoraPairWin <= lora->vimg_bytes) {
       CUtensorMap ti;
       if (make_tmap_bf16_kmajor(&ta, w, N, K, ldw, kBM)) return -1002;
       if (make_tmap_bf16_kmajor(&tb, x, T, K, ldx, pair.bn / 2)) return -1003;
       if (make_tmap_lora_images(&ti, lora->vimg, (uint64_t)(lora->vimg_bytes / 32))) return -1004;
-      p.lora_mask = 31;
-      p.lora_slice = 64 * 16;
-      const long long img64 = img_bytes / 48 * 64, grid = 2ll * pair.grid;
+      const long long img64 = img_bytes / kLoraWin * kLoraPairWin, grid = 2ll * pair.grid;
       const bool shared_k = lora->sync_ints >= 2 + grid && lora->vimg_bytes - img64 >= grid * 128 * 4;
       p.lora_kparts = shared_k ? reinterpret_cast<float*>(static_cast<char*>(lora->vimg) + img64) : nullptr;
       p.lora_kcounters = lora->sync + 2;

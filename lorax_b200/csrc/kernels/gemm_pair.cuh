@@ -93,7 +93,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       GemmWork w0;
       if (warp == 0 && it0.next(w0) && w0.kb0 == 0) {
         const int ta0 = w0.tile / tiles_b, tb0 = w0.tile % tiles_b;
-        const int n0 = lora_prebuild_units(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.bn, ulist);
+        const int n0 = lora_prebuild_units<kLoraPairWin>(p, ents, *n_live, tb0 * p.bn, tb0 * p.bn + p.bn, ulist);
         if (n0 >= 0) { pre_tb = tb0; pre_n = n0; }
         if (n0 > 0) lora_prefetch_b(p, ulist, n0, 2 * ta0 + (int)rank);
       }
@@ -129,7 +129,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if constexpr (LORA) {
         if (lora && w.kb0 == 0) {
           if (list_tb != tb) {
-            const int n0 = lora_prebuild_units(p, ents, *n_live, j0, jlim, ulist);
+            const int n0 = lora_prebuild_units<kLoraPairWin>(p, ents, *n_live, j0, jlim, ulist);
             list_tb = n0 >= 0 ? tb : -1;
             list_n = n0 >= 0 ? n0 : 0;
           }
@@ -201,7 +201,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             __syncwarp();
             if (lane < nu) {
               pair_load_3d(sa + lane * kLoraBTileBytes, &bmaps.m[q.rclass], bar, (q.img & 3) * 16, i0, q.boff);
-              const int row = (int)(img_part + (long long)(q.img & 3) * p.lora_num_tiles + (q.img >> 2)) * 64 + (q.c0 - q.w0) + (int)rank * rows;
+              const int row = (int)(img_part + (long long)(q.img & 3) * p.lora_num_tiles + (q.img >> 2)) * kLoraPairWin + (q.c0 - q.w0) + (int)rank * rows;
               uint8_t* dst = sa + kPairUnits * kLoraBTileBytes + lane * kPairImgBytes;
               for (int h = 0; h < rows; h += 16) pair_load_2d(dst + h * 32, &tmap_img, bar, 0, row + h);
             }
@@ -219,10 +219,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             // more units than the list holds: built and sent in pieces
             int n = 0;
             bool ended = false;
-            for (int lt0 = lora_first_entry(ents, *n_live, j0, p.lora_mask); ok; lt0 += 32) {
+            for (int lt0 = lora_first_entry<kLoraPairWin>(ents, *n_live, j0); ok; lt0 += 32) {
               bool last = true;
               if (lt0 < p.lora_num_tiles) {
-                n = lora_build_units(p, ents, lt0, j0, jlim, ulist, n, ended);
+                n = lora_build_units<kLoraPairWin>(p, ents, lt0, j0, jlim, ulist, n, ended);
                 last = ended || lt0 + 32 >= p.lora_num_tiles;
                 if (n < 128 && !last) continue;
               }
@@ -306,7 +306,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     int acc = 0;
     uint32_t acc_phase[2] = {0, 0};
     if constexpr (LORA) {
-      if (lora) lora_shrink_units(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
+      if (lora) lora_shrink_units<kLoraPairWin>(p, ents, gstart, reinterpret_cast<float*>(epi_stage), warp - 2, lane);
     }
     const bool turn = p.ldo_a == 1 && (p.ldo_b & 7) == 0 && (p.a_rows & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
     PendingTile pending[2];
