@@ -1828,7 +1828,7 @@ static int gemm_impl(const void* x, const void* w, void* out, const void* bias, 
   if (T > kPairMinTokens && N >= 256 && (mode <= 1 || has_lora) && force_split == 0 && sk_policy == 0) {
     const int fit = has_lora ? pair_capacity<true>() : pair_capacity<false>();
     if (fit < 0) return fit;
-    const int pairs = fit < num_sms / 2 ? fit : num_sms / 2;
+    const int pairs = pairs_on(num_sms, fit);
     if (pairs > 0) pair = choose_pair(T, N, K, pairs, usable_ws, pl.cost, has_lora ? lora->max_rank : 0);
   }
   p.overlap = T <= kOverlapMaxTokens;
@@ -1956,6 +1956,9 @@ unsigned lx_lora_tile_bytes(int N, int tile, int r) { return lx::lora_tile_bytes
 
 // Parts of K of each of a short step's `units` shrink units in a launch of `ctas` CTAs.
 int lx_lora_fused_k_parts(int ctas, int units, int K) { return lx::lora_shrink_k_parts(ctas, units, ((K + 31) / 32 + 31) / 32); }
+
+// Pairs of CTAs that a launch on num_sms SMs takes where `fit` run at the same time.
+int lx_pairs_on(int num_sms, int fit) { return lx::pairs_on(num_sms, fit); }
 
 // The plan of pairs of CTAs for a shape and its largest adapter rank (0: none), at most `pairs` at once: out4 = {token tile (0: single CTAs are
 // quicker), whole tiles, pairs that share the others, pairs}.

@@ -904,7 +904,9 @@ int lx_moe_grouped_gemm(const void* xg, long long ldx, const void* w, long long 
   }
   if (avg_rows >= kMpMinRows && n_w % (2 * kMgBM) == 0) {
     static int known[64] = {0};
-    const int pairs = pair_capacity_of(moe_pair_kernel, kMgThreads, MpSmem::kTotal, known);
+    const int fit = pair_capacity_of(moe_pair_kernel, kMgThreads, MpSmem::kTotal, known);
+    if (fit < 0) return fit;
+    const int pairs = pairs_on(num_sms, fit);
     if (pairs > 0) {
       p.bn = 256;
       CUtensorMap tw, tx;

@@ -59,29 +59,37 @@ LX_DEVICE void pair_tmem_dealloc(uint32_t base, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 
-// Pairs of CTAs of `kernel` that run at the same time on the current device; 0: none.  `known` is the caller's, one per kernel.
+// Pairs of CTAs that a launch may take: as many as run at the same time (`fit`), on the SMs it is given.
+inline int pairs_on(int num_sms, int fit) { return fit < num_sms / 2 ? fit : num_sms / 2; }
+
+// Pairs of CTAs of `kernel` that run at the same time on the current device (0: none), or the negative error of a query that failed, which the
+// next call makes again.  `known` is the caller's, one per kernel.
 template <typename K>
 inline int pair_capacity_of(K kernel, int threads, int smem, int (&known)[64]) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (known[dev] == 0) {
-    int n = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(2);
-      cfg.blockDim = dim3(threads);
-      cfg.dynamicSmemBytes = smem;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
-    }
-    cudaGetLastError();
-    known[dev] = n + 1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev >= 64) return 0;
+  if (e == cudaSuccess && known[dev] != 0) return known[dev] - 1;
+  int n = 0;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   }
-  return known[dev] - 1;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return -(int)e;
+  }
+  known[dev] = n + 1;
+  return n;
 }
 
 }  // namespace lx

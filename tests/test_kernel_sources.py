@@ -105,3 +105,12 @@ def test_pairs_of_ctas_only_where_they_measured_quicker(T, N, K, rank, taken):
 def test_shrink_units_share_their_k_only_where_it_measured_quicker(units, K, parts):
     from lorax_b200.ops import native
     assert native.load().lx_lora_fused_k_parts(148, units, K) == parts
+
+
+def test_pairs_of_ctas_stay_on_the_sms_they_are_given():
+    """As many as run at the same time and no more than the launch's SMs hold, in both users; a plan is made for that number."""
+    from lorax_b200.ops import native
+    assert [native.load().lx_pairs_on(*a) for a in ((148, 74), (148, 70), (100, 74), (21, 74), (1, 74), (148, 0))] == [74, 70, 50, 10, 0, 0]
+    for name in ("gemm_bf16.cu", "moe.cu"):
+        text = (KERNELS / name).read_text()
+        assert "pairs_on(num_sms, fit)" in text and "if (fit < 0) return fit;" in text

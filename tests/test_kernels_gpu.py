@@ -1029,6 +1029,20 @@ def test_expert_products_of_cta_pairs(nat, lengths, n_w, K, act):
         at += n
 
 
+@pytest.mark.parametrize("num_sms", [2, 21, 148])
+def test_expert_products_of_pairs_on_some_of_the_sms(nat, num_sms):
+    """Fewer pairs walk more tiles each: the same bits."""
+    g, E, n_w, K, rows = torch.Generator("cuda").manual_seed(num_sms), 3, 512, 256, 900
+    x = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, n_w, K, generator=g, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
+    seg, ws = torch.tensor([0, 400, 401, 900], device="cuda", dtype=torch.int32), nat.workspace()
+    out = torch.empty(rows, n_w, dtype=torch.bfloat16, device="cuda")
+    p = nat._ptr
+    assert nat.load().lx_moe_grouped_gemm(p(x), K, p(w), K, p(out), n_w, p(seg), E, rows, rows, n_w, K, 300, 0, 0, 0, 0, p(ws.status), num_sms, nat._stream()) == 0
+    ws.check_status()
+    assert torch.equal(out, nat.moe_grouped_gemm(x, w, seg, 300))
+
+
 @pytest.mark.parametrize("T,E,k,H,I,e0,e_local", [(7, 8, 2, 512, 256, 0, 8), (256, 8, 2, 1024, 768, 0, 8), (300, 8, 2, 512, 256, 2, 2),
                                                   (1500, 16, 4, 256, 128, 0, 16), (64, 4, 1, 256, 384, 1, 1)])
 def test_moe_ffn_on_the_device(nat, T, E, k, H, I, e0, e_local):
