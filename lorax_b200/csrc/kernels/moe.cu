@@ -641,7 +641,13 @@ int make_tmap_bf16_kmajor(CUtensorMap* out, const void* base, uint64_t rows, uin
 
 // The same for runs of a tile and more, by pairs of CTAs (gemm_pair.cuh has the reasons): a tile is 256 features x up to 256 rows of a run, each CTA
 // brings 128 rows of the weights and half of the tile's rows.  A run's last tile multiplies as many rows as it has (in steps of 32).
-constexpr int kMpMinRows = 192;      // rows a run on average
+// From 192 rows a run on average: below it a tile of 256 rows is mostly padding.  Against single CTAs, eleven shapes of 4 to 64 experts, runs even or
+// uneven, 192 to 1500 rows: 1.0 to 2.1x (eight of 28672 x 4096 192 rows 1.39x, 300 1.02x, 1500 1.03x).  Gated results, which leave as two bytes a lane, only with
+// K of 3072: there a tile's products take long enough to hide them (K = 4096, 7168, 14336 0.96 to 1.6x, 3072 0.97 to 1.3x; 2048 down to 0.88x, 256 0.71x).
+constexpr int kMpMinRows = 192, kMpGatedMinK = 3072;
+static bool moe_by_pairs(int avg_rows, int n_w, int K, int act) {
+  return avg_rows >= kMpMinRows && n_w % (2 * kMgBM) == 0 && (act != kMoeActSwiglu || K >= kMpGatedMinK);
+}
 constexpr int kMpStages = 6;
 struct MpSmem {
   static constexpr int kStage = 2 * kMgBM * kMgBK * 2;
@@ -883,6 +889,9 @@ int lx_moe_combine(const void* y, long long ldy, const int* pos, const float* w,
   return -(int)cudaGetLastError();
 }
 
+// 1: pairs of CTAs take a grouped product of this shape (lx_moe_grouped_gemm).
+int lx_moe_by_pairs(int avg_rows, int n_w, int K, int act) { return lx::moe_by_pairs(avg_rows, n_w, K, act) ? 1 : 0; }
+
 // out[q, :] = act(xg[q, :] @ W_e(q)^T) for every sorted row q, e(q) the run that holds q.  w: the experts' matrices stacked
 // [runs * n_w, K]; n_w must be a multiple of 128.  The last `shared` runs all read the `tokens` rows at the beginning of the first of
 // them (0: every run has input rows of its own).  x_rows / rows_cap: rows of xg / of out.  avg_rows (rows per expert the caller
@@ -902,7 +911,7 @@ int lx_moe_grouped_gemm(const void* xg, long long ldx, const void* w, long long 
                reinterpret_cast<const float*>(w), ldw, reinterpret_cast<float*>(out), p);
     return -(int)cudaGetLastError();
   }
-  if (avg_rows >= kMpMinRows && n_w % (2 * kMgBM) == 0) {
+  if (moe_by_pairs(avg_rows, n_w, K, act)) {
     static int known[64] = {0};
     const int fit = pair_capacity_of(moe_pair_kernel, kMgThreads, MpSmem::kTotal, known);
     if (fit < 0) return fit;

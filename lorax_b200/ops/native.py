@@ -68,6 +68,7 @@ def load() -> ctypes.CDLL:
         "lx_gemm_max_tiles": ([], I),
         "lx_lora_fused_k_parts": ([I, I, I], I),
         "lx_lora_tile_bytes": ([I, I, I], ctypes.c_uint),
+        "lx_moe_by_pairs": ([I, I, I, I], I),
         "lx_pairs_on": ([I, I], I),
         "lx_gemm_pair_plan": ([I, I, I, I, I, L, I, P], I),
         "lx_gemm_plan": ([I, I, I, I, L, I, I, P], I),

@@ -114,3 +114,10 @@ def test_pairs_of_ctas_stay_on_the_sms_they_are_given():
     for name in ("gemm_bf16.cu", "moe.cu"):
         text = (KERNELS / name).read_text()
         assert "pairs_on(num_sms, fit)" in text and "if (fit < 0) return fit;" in text
+
+
+@pytest.mark.parametrize("avg_rows,n_w,K,act,pairs", [(192, 256, 64, "", 1), (191, 4096, 4096, "", 0), (700, 384, 4096, "", 0), (300, 512, 256, "relu2", 1), (300, 28672, 4096, "swiglu", 1),
+                                                      (300, 4096, 3072, "swiglu", 1), (300, 2816, 2048, "swiglu", 0), (192, 512, 1024, "swiglu", 0)])      # 6 and 20 % slower by pairs
+def test_expert_products_by_pairs_only_where_they_measured_quicker(avg_rows, n_w, K, act, pairs):
+    from lorax_b200.ops import native
+    assert native.load().lx_moe_by_pairs(avg_rows, n_w, K, native._MOE_ACTS[act]) == pairs

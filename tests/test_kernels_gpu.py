@@ -1029,6 +1029,13 @@ def test_expert_products_of_cta_pairs(nat, lengths, n_w, K, act):
         at += n
 
 
+@pytest.mark.parametrize("lengths,n_w", [([700, 3, 290, 0, 257], 256), ([33, 255, 512], 512)])
+def test_gated_expert_products_of_cta_pairs(nat, lengths, n_w):
+    """The gated epilogue of pairs, which take it from K of 3072 on."""
+    assert nat.load().lx_moe_by_pairs(256, n_w, 3080, 2) == 1
+    test_expert_products_of_cta_pairs(nat, lengths, n_w, 3080, "swiglu")
+
+
 @pytest.mark.parametrize("num_sms", [2, 21, 148])
 def test_expert_products_of_pairs_on_some_of_the_sms(nat, num_sms):
     """Fewer pairs walk more tiles each: the same bits."""
