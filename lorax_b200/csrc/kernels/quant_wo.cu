@@ -161,7 +161,9 @@ LX_DEVICE Wq4Group wq4_group(__half2 szv) {
 // EXACT: every 128-wide k-block lies inside one group and the zero points are integers.  The codes then go to the tensor cores as
 // the exact integers (code - zero); the k-block's partial product is scaled by the group's fp16 scale in fp32 on its way into the
 // accumulator: no fma per pair of weights and no bf16 rounding of the scale.
-template <int NT, int MT, bool EXACT>                  // token tiles of 8, row tiles of 16
+// LORA: the step's adapters are added to the sums.  A kernel of its own: what it holds for them costs the registers of the products of 9 to 16 rows
+// (without adapters, 4096 x 4096 12 rows 8 % slower with it, 4096 x 14336 12 %).
+template <int NT, int MT, bool EXACT, bool LORA>       // token tiles of 8, row tiles of 16
 __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Params p) {
   __shared__ float red[kWqWarps][kWqRows * MT][8 * NT + 1];
   constexpr int kRows = kWqRows * MT;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
   // B_cat of the row whose results this thread will form, as it will walk them below, on its way into L2
   constexpr int kOuts = (kRows * 8 * NT + kWqWarps * 32 - 1) / (kWqWarps * 32);
   LoraAddRow lrow[kOuts];
-  if (p.add.tiles != nullptr) {
+  if (LORA && p.add.tiles != nullptr) {
     if (p.w_const && !p.add.tables_const) pdl_wait();
 #pragma unroll
     for (int i = 0; i < kOuts; ++i) {
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
 #pragma unroll
       for (int w = 0; w < kWqWarps; ++w) v += red[w][r][tok];
       if (p.bias != nullptr) v += __bfloat162float(p.bias[n0 + r]);
-      if (p.add.tiles != nullptr && lrow[i].r > 0) {
+      if (LORA && p.add.tiles != nullptr && lrow[i].r > 0) {
         const LoraAddRow q = lrow[i];
         const __nv_bfloat16* B = q.b + (long long)(n0 + r) * q.r;
         const float* vv = p.add.v + (long long)tok * p.add.ldv + lora_add_part(p.add, n0 + r) * q.r;
@@ -326,7 +328,9 @@ __global__ void __launch_bounds__(kWqWarps * 32, 2) wq4_mma_kernel(const Wq4Para
 
 template <int NT, int MT>
 int wq4_launch(const Wq4Params& p, bool exact, cudaStream_t s) {
-  launch_pdl(exact ? wq4_mma_kernel<NT, MT, true> : wq4_mma_kernel<NT, MT, false>, dim3(p.N / (kWqRows * MT)), dim3(kWqWarps * 32), 0, s, p);
+  auto kernel = p.add.tiles != nullptr ? (exact ? wq4_mma_kernel<NT, MT, true, true> : wq4_mma_kernel<NT, MT, false, true>)
+                                       : (exact ? wq4_mma_kernel<NT, MT, true, false> : wq4_mma_kernel<NT, MT, false, false>);
+  launch_pdl(kernel, dim3(p.N / (kWqRows * MT)), dim3(kWqWarps * 32), 0, s, p);
   return -(int)cudaGetLastError();
 }
 
