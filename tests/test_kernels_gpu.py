@@ -925,6 +925,24 @@ def test_gemm_with_lora_of_ragged_pairs(nat, T, K, parts, ranks, layout):
     test_gemm_with_lora_in_the_same_launch(nat, T, K, parts, ranks, layout)
 
 
+def test_leaving_out_the_expand_leaves_it_out_of_long_steps(nat, monkeypatch):
+    """The measurement switch means the same where pairs of CTAs would take the product: the base product alone."""
+    T, N, K, r, gen = 200, 19072, 2048, 16, torch.Generator("cuda").manual_seed(3)
+    assert _pair_tile(nat, T, N, K, r) > 0
+    x, w = (torch.randn(n, K, generator=gen, device="cuda").to(torch.bfloat16) / (1 if n == T else math.sqrt(K)) for n in (T, N))
+    arena = torch.randn(r * (K + N), generator=gen, device="cuda").to(torch.bfloat16)
+    maps = torch.zeros(2 * 128, dtype=torch.uint8).pin_memory()
+    nat.lora_encode_tmap(maps, arena.data_ptr(), K, r, r * (K + N), 1)
+    nat.lora_encode_tmap_b(maps[128:], arena.data_ptr() + r * K * 2, r, N, r * (K + N), 1)
+    tiles = torch.tensor(ref.build_lora_tiles([0] * T, 32), device="cuda", dtype=torch.int32).view(-1, 4)
+    rank, base = torch.tensor([r], device="cuda", dtype=torch.int32), torch.tensor([0], device="cuda", dtype=torch.int64)
+    lf = nat.LoraFused(tiles, tiles.shape[0], tiles.shape[0], maps.cuda(), 2, 0, 1, rank, base, 1, N, N, 0, r, arena, 0, K)
+    with_adapters, alone = nat.gemm_lora_fused(x, w, lf), nat.gemm(x, w, mode=1)
+    monkeypatch.setenv("LORAX_LORA_SKIP", "2")
+    assert _rel_err(nat.gemm_lora_fused(x, w, lf), alone) < 2 ** -8 and _rel_err(with_adapters, alone) > 1
+    nat.workspace().check_status()
+
+
 @pytest.mark.parametrize("form", ["fp8", "wq4"])
 @pytest.mark.parametrize("T,K,parts,ranks", [(1, 512, [128], [16]), (5, 1024, [256, 128, 128], [16, 64]), (8, 512, [1024], [48]), (9, 2048, [512, 512], [32, 16]),
                                              (32, 4096, [384, 128, 128], [16, 32, 48, 64]), (77, 512, [256], [32, 16]), (256, 512, [16384], [16, 64]),
