@@ -497,7 +497,7 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
         if w16 is not None:
             return _lora_expand(gemm(x, w16, bias=bias, out=out), lora)
     xq, sa = quant_act_fp8(x)
-    add = _lora_add(out, lora)
+    add = _lora_add(out, lora, T <= load().lx_lora_add_max_rows() and (T <= LORA_ADD_FP8_ROWS or T * N <= LORA_ADD_FP8_RESULTS))
     rc = load().lx_gemm_fp8_block128(_ptr(xq), xq.stride(0), _ptr(sa), sa.stride(0), _ptr(wq), wq.stride(0), _ptr(w_scale), _ptr(out),
                                      out.stride(0), _ptr(bias), T, N, K, _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.status),
                                      ws.num_sms, 1, ctypes.byref(add) if add is not None else None,
@@ -506,9 +506,17 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
     return out if add is not None else _lora_expand(out, lora)
 
 
-def _lora_add(out: torch.Tensor, lora, max_rows: Optional[int] = None) -> Optional[LxLoraAdd]:
-    """The descriptor of `lora` where the launch that writes `out` can add it."""
-    if lora is None or out.shape[0] > (load().lx_lora_add_max_rows() if max_rows is None else max_rows):
+# Steps whose adapters join the launch that forms a quantised product's results, by their number of results; larger ones take the expand
+# launch behind it, which has a row's B_cat in registers for up to 32 rows.  Measured against it with one adapter / as many as rows, up to 24, of ranks 16 to
+# 64.  Behind fp8 products: 28672 features of 32 rows 1.18 to 1.61x / 1.02 to 1.09x, of 64 0.85 to 0.92x with 24 and of 256 0.54x; 6144 of 128 1.33x up / 1.05x up, of 160
+# 0.90x; 4096 of 128 1.48x up / 1.03x up, of 160 0.92x.  In 4-bit products, a lane of which reads whole rows of B_cat: 28672 of 5 rows 1.04x up / 0.97x up, of 16
+# 0.95x / 0.86x; 17920 of 8 1.28x up / 1.08x up, of 16 0.91x; 6144 of 16 1.08x up, of 24 0.93x; 4096 of 32 1.03x up.
+LORA_ADD_FP8_ROWS, LORA_ADD_FP8_RESULTS, LORA_ADD_WQ4_RESULTS = 32, 589824, 143360
+
+
+def _lora_add(out: torch.Tensor, lora, quicker: bool) -> Optional[LxLoraAdd]:
+    """The descriptor of `lora` where the launch that writes `out` can add it and is `quicker` with it."""
+    if lora is None or not quicker:
         return None
     N = out.shape[1]
     if N % 4 or out.stride(0) % 4 or any(n < N and n % 128 for n in (lora[0].n0, lora[0].n1)):
@@ -556,7 +564,7 @@ def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Option
         w = dataclasses.replace(w, perm=None)
     if (w.bits == 4 and w.table is None and T <= WQ4_DIRECT_MAX_TOKENS and N % 16 == 0 and K % 128 == 0 and w.group % 32 == 0
             and x.stride(0) % 8 == 0):
-        add = _lora_add(out, lora, WQ4_DIRECT_MAX_TOKENS)
+        add = _lora_add(out, lora, T * N <= LORA_ADD_WQ4_RESULTS)
         rc = load().lx_wq4_gemm_lora(_ptr(x), x.stride(0), _ptr(w.codes), _ptr(w.sz), _ptr(bias), _ptr(out), out.stride(0), T, N, K, w.group,
                                      (1 if getattr(w, "int_zero", False) else 0) | (2 if w_const else 0), ctypes.byref(add) if add is not None else None,
                                      _stream())

@@ -121,3 +121,28 @@ def test_pairs_of_ctas_stay_on_the_sms_they_are_given():
 def test_expert_products_by_pairs_only_where_they_measured_quicker(avg_rows, n_w, K, act, pairs):
     from lorax_b200.ops import native
     assert native.load().lx_moe_by_pairs(avg_rows, n_w, K, native._MOE_ACTS[act]) == pairs
+
+
+@pytest.mark.parametrize("form,T,N,taken", [
+    ("fp8", 32, 28672, True), ("fp8", 64, 28672, False), ("fp8", 256, 28672, False), ("fp8", 96, 6144, True), ("fp8", 160, 6144, False), ("fp8", 144, 4096, True),
+    ("fp8", 256, 1536, True), ("fp8", 257, 512, False),
+    ("wq4", 5, 28672, True), ("wq4", 16, 28672, False), ("wq4", 16, 6144, True), ("wq4", 24, 6144, False), ("wq4", 32, 4096, True)])
+def test_adapters_join_quantised_products_only_where_it_measured_quicker(monkeypatch, form, T, N, taken):
+    """Which steps ask the product's launch to add the adapters: read off what the wrappers ask for, with the library's calls left out."""
+    import torch
+    from types import SimpleNamespace as NS
+
+    from lorax_b200.ops import native
+    asked = []
+    lib = NS(lx_lora_add_max_rows=native.load().lx_lora_add_max_rows, lx_gemm_fp8_block128=lambda *a: 0, lx_quant_act_fp8=lambda *a: 0, lx_wq4_gemm_lora=lambda *a: 0)
+    ws = NS(gemm_ws=torch.empty(8), status=torch.empty(2), num_sms=148)
+    for name, value in dict(load=lambda: lib, workspace=lambda dev: ws, _stream=lambda: None, _lora_expand=lambda out, lora: out,
+                            _lora_add=lambda out, lora, quicker: asked.append(quicker)).items():
+        monkeypatch.setattr(native, name, value)
+    x, lora = torch.empty(T, 128, dtype=torch.bfloat16), (None, None)
+    if form == "fp8":
+        native.gemm_fp8(x, torch.empty(N, 128, dtype=torch.uint8), torch.empty(N // 128, 1), lora=lora)
+    else:
+        w = NS(shape=(N, 128), bits=4, table=None, group=128, perm=None, codes=torch.empty(1, dtype=torch.uint8), sz=torch.empty(1), int_zero=False)
+        native.gemm_wq(x, w, lora=lora)
+    assert asked == [taken]

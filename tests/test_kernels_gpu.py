@@ -999,6 +999,13 @@ def test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks):
     assert torch.equal(got[alone], base[alone])
 
 
+@pytest.mark.parametrize("form,T,K,parts,ranks", [("fp8", 32, 512, [28672, 28672], [16, 64]), ("fp8", 32, 1024, [28672], [32, 48]), ("fp8", 144, 256, [4096], [16, 64, 32]),
+                                                  ("wq4", 5, 512, [14336, 14336], [16, 64]), ("wq4", 32, 1024, [4096], [48, 16])])
+def test_quantised_products_add_the_adapters_of_many_features(nat, form, T, K, parts, ranks):
+    """At the ends of the range in which they do: several rows a warp of the kernel behind fp8 products among them."""
+    test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks)
+
+
 @pytest.mark.parametrize("T,N,K", [(193, 256, 64), (200, 6144, 4096), (256, 4096, 14336), (320, 28672, 256), (513, 256, 64), (545, 300, 200), (1000, 1000, 136), (2047, 640, 4096), (700, 4360, 72), (1024, 257, 64)])
 def test_products_of_cta_pairs(nat, T, N, K):
     """Long steps at the edges of tiles, whole ones and shared: features that do not fill a tile of 256 or begin off 16 bytes in the output, ragged K, a last token tile of
