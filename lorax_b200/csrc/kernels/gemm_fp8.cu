@@ -425,7 +425,7 @@ int lx_quant_act_fp8(const void* x, long long ldx, void* xq, long long ldq, floa
 
 // out[T, N] (bf16) = block-scaled fp8 product of xq[T, K] (scales sa[kb, t]) and wq[N, K] (scales sw[N/128, K/128]) + bias.
 // w_const: the kernel in front on the stream does not write wq.  add (nullptr: none): the step's adapters, for at most lx_lora_add_max_rows()
-// rows, N a multiple of four and parts of multiples of 128; their shrink is in front on the stream.
+// rows, N and ldo multiples of four, out at 8 bytes and parts of multiples of 128; their shrink is in front on the stream.
 int lx_lora_add_max_rows() { return lx::kLoraAddRows; }
 int lx_lora_add(const LxLoraAdd* add, void* y, long long ldy, int T, int N, int num_sms, void* stream) {
   if (T <= 0 || N <= 0) return 0;
@@ -437,7 +437,9 @@ int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_
                          int num_sms, int w_const, const LxLoraAdd* add, void* stream_) {
   using namespace lx;
   if (T <= 0 || N <= 0) return 0;
-  if (add != nullptr && (T > kLoraAddRows || N % 4 != 0 || ldo % 4 != 0 || (add->n0 < N && add->n0 % 128 != 0) || (add->n1 < N && add->n1 % 128 != 0))) return -1001;
+  if (add != nullptr && (T > kLoraAddRows || N % 4 != 0 || ldo % 4 != 0 || (reinterpret_cast<uintptr_t>(out) & 7) != 0 || !lora_add_aligned(*add) ||
+                         (add->n0 < N && add->n0 % 128 != 0) || (add->n1 < N && add->n1 % 128 != 0)))
+    return -1001;
   if (K % 16 != 0 || ldq % 16 != 0 || ldw % 16 != 0) return -1000;
   Fp8Params p{};
   p.N = N; p.T = T; p.K = K;

@@ -23,6 +23,9 @@ struct LxLoraAdd {
 
 namespace lx {
 
+// v is read 16 bytes at a time (part * rank is a multiple of 16 columns).
+inline bool lora_add_aligned(const LxLoraAdd& a) { return a.ldv % 4 == 0 && (reinterpret_cast<uintptr_t>(a.v) & 15) == 0; }
+
 constexpr int kLoraAddRows = 256;
 struct LoraAddRow {
   const __nv_bfloat16* b;    // B_cat of the row's adapter

@@ -378,6 +378,7 @@ int lx_wq4_gemm_lora(const void* x, long long ldx, const void* codes, const void
                      int K, int group, int flags, const LxLoraAdd* add, void* stream) {
   using namespace lx;
   if (T <= 0 || T > 32 || N % kWqRows != 0 || K % 128 != 0 || group % 32 != 0 || K % group != 0 || ldx % 8 != 0) return -1;
+  if (add != nullptr && !lora_add_aligned(*add)) return -2;
   Wq4Params p{static_cast<const uint8_t*>(codes), static_cast<const __half2*>(sz), static_cast<const __nv_bfloat16*>(x),
               static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), ldx, ldo, T, N, K, group, (flags >> 1) & 1,
               add != nullptr ? *add : LxLoraAdd{}};

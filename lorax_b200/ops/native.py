@@ -519,7 +519,7 @@ def _lora_add(out: torch.Tensor, lora, quicker: bool) -> Optional[LxLoraAdd]:
     if lora is None or not quicker:
         return None
     N = out.shape[1]
-    if N % 4 or out.stride(0) % 4 or any(n < N and n % 128 for n in (lora[0].n0, lora[0].n1)):
+    if N % 4 or out.stride(0) % 4 or out.data_ptr() % 8 or any(n < N and n % 128 for n in (lora[0].n0, lora[0].n1)):
         return None
     return lora_add_desc(*lora, tables_const=True)
 

@@ -146,3 +146,15 @@ def test_adapters_join_quantised_products_only_where_it_measured_quicker(monkeyp
         w = NS(shape=(N, 128), bits=4, table=None, group=128, perm=None, codes=torch.empty(1, dtype=torch.uint8), sz=torch.empty(1), int_zero=False)
         native.gemm_wq(x, w, lora=lora)
     assert asked == [taken]
+
+
+@pytest.mark.parametrize("out,ldo,v,ldv", [(0x1004, 512, 0x2000, 192), (0x1000, 510, 0x2000, 192), (0x1000, 512, 0x2008, 192), (0x1000, 512, 0x2000, 190)])
+def test_adapters_beside_quantised_products_are_refused_off_their_alignment(out, ldo, v, ldv):
+    """Four results are written and four sums read at a time: what does not lie that way is refused before anything is launched."""
+    import ctypes
+
+    from lorax_b200.ops import native
+    add = native.LxLoraAdd(0x3000, 1, 1, 0x4000, 0x5000, 0x6000, 0, v, ldv, 512, 512, 1, 0x7000)
+    assert native.load().lx_gemm_fp8_block128(0x8000, 512, 0x9000, 16, 0xA000, 512, 0xB000, out, ldo, None, 1, 512, 512, None, 0, 0xC000, 148, 1, ctypes.byref(add), None) == -1001
+    if v % 16 or ldv % 4:      # (the 4-bit kernel writes single results)
+        assert native.load().lx_wq4_gemm_lora(0x8000, 512, 0x9000, 0xA000, None, out, ldo, 1, 512, 512, 128, 0, ctypes.byref(add), None) == -2
