@@ -638,86 +638,86 @@ LX_DEVICE void tensormap_fence_acquire_g(const CUtensorMap* m) {
 // thread and step (the four epilogue warps).  All contributors are running (one CTA per SM, each a consecutive K range of the same length), so the
 // wait for the others is short; it is bounded like every wait.  False: it ran out.
 LX_DEVICE bool gemm_sum_share(const GemmParams& p, const PendingTile t, volatile int* abort_flag) {
-        if (threadIdx.x == 64) {
-          uint64_t t0 = 0;
-          uint32_t polls = 0;
-          while ((ld_acquire_gpu(&p.counters[t.counter]) & 0xffff) != t.nparts) {
-            if ((++polls & 255u) == 0) {
-              const uint64_t now = global_timer_ns();
-              if (t0 == 0) t0 = now;
-              else if (now - t0 > kWaitBudgetNs) {
-                report_status(p.status, kTimeoutSplitK, t.counter);
-                *abort_flag = 1;
-                break;
-              }
-            }
-          }
+  if (threadIdx.x == 64) {
+    uint64_t t0 = 0;
+    uint32_t polls = 0;
+    while ((ld_acquire_gpu(&p.counters[t.counter]) & 0xffff) != t.nparts) {
+      if ((++polls & 255u) == 0) {
+        const uint64_t now = global_timer_ns();
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > kWaitBudgetNs) {
+          report_status(p.status, kTimeoutSplitK, t.counter);
+          *abort_flag = 1;
+          break;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (*abort_flag != 0) return false;
-        const int j0 = t.tb * p.bn;
-        const int ncols = min(min(p.bn, p.umma_n), p.b_rows - j0);
-        const int c_lo = (int)((long long)ncols * t.part_idx / t.nparts), c_hi = (int)((long long)ncols * (t.part_idx + 1) / t.nparts);
-        const int tid4 = (int)threadIdx.x - 64;
-        const int items = (c_hi - c_lo) * (kBM / 4);
-        for (int it0 = tid4; it0 < items; it0 += 128 * 4) {
-          // four items per thread and pass, four partials of each in flight
-          float4 sum[4];
-          long long off[4];
-  #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int it1 = min(it0 + 128 * e, items - 1);
-            sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-            off[e] = (long long)(c_lo + it1 / (kBM / 4)) * kBM + (it1 % (kBM / 4)) * 4;
-          }
-          for (int sp0 = 0; sp0 < t.nparts; sp0 += 4) {
-            float4 v[4][4];
-  #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int sp = min(sp0 + q, t.nparts - 1);
-              const float* src = p.ws + (sp == 0 ? t.red_first : t.red_base + sp * t.red_stride);
-  #pragma unroll
-              for (int e = 0; e < 4; ++e) v[q][e] = __ldcg(reinterpret_cast<const float4*>(src + off[e]));
-            }
-  #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              if (sp0 + q < t.nparts) {
-  #pragma unroll
-                for (int e = 0; e < 4; ++e) { sum[e].x += v[q][e].x; sum[e].y += v[q][e].y; sum[e].z += v[q][e].z; sum[e].w += v[q][e].w; }
-              }
-            }
-          }
-  #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int it1 = it0 + 128 * e;
-            if (it1 >= items) break;
-            const int c = c_lo + it1 / (kBM / 4), r4 = (it1 % (kBM / 4)) * 4;
-            const int i = t.i0 + r4, j = j0 + c;
-            float o[4] = {sum[e].x * p.out_scale, sum[e].y * p.out_scale, sum[e].z * p.out_scale, sum[e].w * p.out_scale};
-            if (p.bias != nullptr) {
-  #pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                if (p.bias_on_a) { if (i + h < p.a_rows) o[h] += __bfloat162float(p.bias[i + h]); }
-                else o[h] += __bfloat162float(p.bias[j]);
-              }
-            }
-            __nv_bfloat16* dst = p.out + (long long)i * p.ldo_a + (long long)j * p.ldo_b;
-            if (p.ldo_a == 1 && i + 4 <= p.a_rows && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
-            } else {
-  #pragma unroll
-              for (int h = 0; h < 4; ++h) {
-                if (i + h < p.a_rows) dst[(long long)h * p.ldo_a] = __float2bfloat16(o[h]);
-              }
-            }
-          }
+      }
+    }
+  }
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (*abort_flag != 0) return false;
+  const int j0 = t.tb * p.bn;
+  const int ncols = min(min(p.bn, p.umma_n), p.b_rows - j0);
+  const int c_lo = (int)((long long)ncols * t.part_idx / t.nparts), c_hi = (int)((long long)ncols * (t.part_idx + 1) / t.nparts);
+  const int tid4 = (int)threadIdx.x - 64;
+  const int items = (c_hi - c_lo) * (kBM / 4);
+  for (int it0 = tid4; it0 < items; it0 += 128 * 4) {
+    // four items per thread and pass, four partials of each in flight
+    float4 sum[4];
+    long long off[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int it1 = min(it0 + 128 * e, items - 1);
+      sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      off[e] = (long long)(c_lo + it1 / (kBM / 4)) * kBM + (it1 % (kBM / 4)) * 4;
+    }
+    for (int sp0 = 0; sp0 < t.nparts; sp0 += 4) {
+      float4 v[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int sp = min(sp0 + q, t.nparts - 1);
+        const float* src = p.ws + (sp == 0 ? t.red_first : t.red_base + sp * t.red_stride);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[q][e] = __ldcg(reinterpret_cast<const float4*>(src + off[e]));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (sp0 + q < t.nparts) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { sum[e].x += v[q][e].x; sum[e].y += v[q][e].y; sum[e].z += v[q][e].z; sum[e].w += v[q][e].w; }
         }
-        // the last contributor to finish clears the counter for the next launch
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (threadIdx.x == 64) {
-          const int prev = atomicAdd(&p.counters[t.counter], 0x10000);
-          if ((prev >> 16) == t.nparts - 1) p.counters[t.counter] = 0;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int it1 = it0 + 128 * e;
+      if (it1 >= items) break;
+      const int c = c_lo + it1 / (kBM / 4), r4 = (it1 % (kBM / 4)) * 4;
+      const int i = t.i0 + r4, j = j0 + c;
+      float o[4] = {sum[e].x * p.out_scale, sum[e].y * p.out_scale, sum[e].z * p.out_scale, sum[e].w * p.out_scale};
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (p.bias_on_a) { if (i + h < p.a_rows) o[h] += __bfloat162float(p.bias[i + h]); }
+          else o[h] += __bfloat162float(p.bias[j]);
         }
+      }
+      __nv_bfloat16* dst = p.out + (long long)i * p.ldo_a + (long long)j * p.ldo_b;
+      if (p.ldo_a == 1 && i + 4 <= p.a_rows && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+      } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (i + h < p.a_rows) dst[(long long)h * p.ldo_a] = __float2bfloat16(o[h]);
+        }
+      }
+    }
+  }
+  // the last contributor to finish clears the counter for the next launch
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (threadIdx.x == 64) {
+    const int prev = atomicAdd(&p.counters[t.counter], 0x10000);
+    if ((prev >> 16) == t.nparts - 1) p.counters[t.counter] = 0;
+  }
   return true;
 }
 

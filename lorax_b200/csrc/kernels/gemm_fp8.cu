@@ -423,15 +423,11 @@ int lx_quant_act_fp8(const void* x, long long ldx, void* xq, long long ldq, floa
   return -(int)cudaGetLastError();
 }
 
+int lx_lora_add_max_rows() { return lx::kLoraAddRows; }
+
 // out[T, N] (bf16) = block-scaled fp8 product of xq[T, K] (scales sa[kb, t]) and wq[N, K] (scales sw[N/128, K/128]) + bias.
 // w_const: the kernel in front on the stream does not write wq.  add (nullptr: none): the step's adapters, for at most lx_lora_add_max_rows()
 // rows, N and ldo multiples of four, out at 8 bytes and parts of multiples of 128; their shrink is in front on the stream.
-int lx_lora_add_max_rows() { return lx::kLoraAddRows; }
-int lx_lora_add(const LxLoraAdd* add, void* y, long long ldy, int T, int N, int num_sms, void* stream) {
-  if (T <= 0 || N <= 0) return 0;
-  if (add == nullptr || T > lx::kLoraAddRows || N % 4 != 0 || ldy % 4 != 0 || (add->n0 < N && add->n0 % 128 != 0) || (add->n1 < N && add->n1 % 128 != 0)) return -1;
-  return lx::launch_lora_add(*add, nullptr, 0, T, N, nullptr, reinterpret_cast<__nv_bfloat16*>(y), ldy, num_sms, reinterpret_cast<cudaStream_t>(stream));
-}
 int lx_gemm_fp8_block128(const void* xq, long long ldq, const float* sa, int ld_sa, const void* wq, long long ldw, const float* sw,
                          void* out, long long ldo, const void* bias, int T, int N, int K, void* ws, long long ws_bytes, int* status,
                          int num_sms, int w_const, const LxLoraAdd* add, void* stream_) {

@@ -103,7 +103,6 @@ def load() -> ctypes.CDLL:
         "lx_quant_act_fp8": ([P, L, P, L, P, I, I, I, P], I),
         "lx_gemm_fp8_block128": ([P, L, P, I, P, L, P, P, L, P, I, I, I, P, L, P, I, I, P, P], I),
         "lx_lora_add_max_rows": ([], I),
-        "lx_lora_add": ([P, P, L, I, I, I, P], I),
         "lx_fp8_block128_dequant": ([P, L, P, I, P, L, I, I, P], I),
         "lx_wq_dequant": ([P, P, P, P, L, I, I, I, I, P], I),
         "lx_wq4_gemm": ([P, L, P, P, P, P, L, I, I, I, I, P], I),
