@@ -281,15 +281,17 @@ __global__ void __launch_bounds__(256) fp8_splitk_reduce_kernel(const float* par
 }
 
 // The same with the step's adapters: y[t, n] = bf16(sum_s partial[s, t, n] + bias[n] + delta), or without parts (ksplit 0) y += delta.
-// A warp takes 128 features of `run` rows one after the other.  Their B_cat rows lie end to end: lanes side by side read 16 bytes, eight ranks,
-// side by side (a lane with whole rows of its own features touches 32 lines per load: 19 us for 28672 features of 32 rows, rank 32), and the
-// two to eight lanes of a feature join their sums.  Those of the warp's first row are loaded before the wait for the product.
+// A warp takes 128 features of `run` rows, up to G neighbours of one adapter at a time.  Their B_cat rows lie end to end: lanes side by side read 16
+// bytes, eight ranks, side by side (a lane with whole rows of its own features touches 32 lines per load: 19 us for 28672 features of 32 rows, rank 32),
+// and the two to eight lanes of a feature join their sums.  Those of the warp's first row are loaded before the wait for the product.
 // The reduction and the expand as launches of their own took 12 to 20 us a projection at 32 rows of 24 adapters.
 constexpr int kAddWarps = 8, kAddAhead = 8;
-__global__ void __launch_bounds__(32 * kAddWarps) lora_add_kernel(const LxLoraAdd a, const float* partial, int ksplit, int T, int N, int run,
+template <int G>
+__global__ void __launch_bounds__(32 * kAddWarps, 2) lora_add_kernel(const LxLoraAdd a, const float* partial, int ksplit, int T, int N, int run,
                                                                   const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* out, long long ldo) {
+  static_assert(G == 1 || G == 4, "sums of a row on their own, or of four rows together");
   __shared__ LoraAddRow rows[kLoraAddRows];
-  __shared__ __align__(16) float deltas[kAddWarps][128];
+  __shared__ __align__(16) float deltas[kAddWarps][G][128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, f0 = blockIdx.x * 128, n = f0 + lane * 4;
   const int t_lo = (blockIdx.y * kAddWarps + warp) * run, t_hi = min(t_lo + run, T);
   if (!a.tables_const) pdl_wait();
@@ -310,61 +312,95 @@ __global__ void __launch_bounds__(32 * kAddWarps) lora_add_kernel(const LxLoraAd
   if (t_lo < t_hi && rows[t_lo].r > 0) load_b(rows[t_lo], lanes(rows[t_lo].r), 0);
   pdl_wait();      // every block waits, also those that have nothing to do
   pdl_trigger();
-  for (int t = t_lo; t < t_hi; ++t) {
+  for (int t = t_lo, cnt; t < t_hi; t += cnt) {
     const LoraAddRow q = rows[t];
+    for (cnt = 1; cnt < G && t + cnt < t_hi && rows[t + cnt].b == q.b;) ++cnt;
     if (ksplit == 0 && q.r == 0) continue;
-    float y[4] = {0.f, 0.f, 0.f, 0.f};
-    __nv_bfloat16* at = out + (long long)t * ldo + n;
-    if (n < N) {                       // N is a multiple of four
-      if (ksplit == 0) {
-        const uint2 old = *reinterpret_cast<const uint2*>(at);
-        const float2 o0 = unpack_bf16x2(old.x), o1 = unpack_bf16x2(old.y);
-        y[0] = o0.x; y[1] = o0.y; y[2] = o1.x; y[3] = o1.y;
-      }
-#pragma unroll 4
-      for (int s = 0; s < ksplit; ++s) {
-        const float4 p4 = __ldcg(reinterpret_cast<const float4*>(partial + ((long long)s * T + t) * N + n));
-        y[0] += p4.x; y[1] += p4.y; y[2] += p4.z; y[3] += p4.w;
-      }
-      if (ksplit > 0 && bias != nullptr) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) y[c] += __bfloat162float(bias[n + c]);
-      }
-    }
     if (q.r > 0) {
       const int sh = lanes(q.r), c = lane & ((1 << sh) - 1);
-      float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
-      if (c * 8 < q.r) {
-        const float* vv = a.v + (long long)t * a.ldv + part * q.r + c * 8;
-        v0 = *reinterpret_cast<const float4*>(vv);
-        v1 = *reinterpret_cast<const float4*>(vv + 4);
+      float4 v0[G], v1[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        v0[g] = v1[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g < cnt && c * 8 < q.r) {
+          const float* vv = a.v + (long long)(t + g) * a.ldv + part * q.r + c * 8;
+          v0[g] = *reinterpret_cast<const float4*>(vv);
+          v1[g] = *reinterpret_cast<const float4*>(vv + 4);
+        }
       }
       for (int i0 = 0; i0 < (4 << sh); i0 += kAddAhead) {      // 128 features, 32 >> sh at a time
         if (t > t_lo || i0 > 0) load_b(q, sh, i0);
 #pragma unroll
         for (int i = 0; i < kAddAhead; ++i) {
-          float d = lora_dot8(bw[i], v0, v1, 0.f);
-          for (int m = 1; m < (1 << sh); m <<= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
-          if (c == 0) deltas[warp][((i0 + i) << (5 - sh)) + (lane >> sh)] = d;
+          const int f = ((i0 + i) << (5 - sh)) + (lane >> sh);
+          float d[G];
+#pragma unroll
+          for (int g = 0; g < G; ++g) d[g] = lora_dot8(bw[i], v0[g], v1[g], 0.f);
+          if constexpr (G == 1) {
+            for (int m = 1; m < (1 << sh); m <<= 1) d[0] += __shfl_xor_sync(0xffffffffu, d[0], m);
+            if (c == 0) deltas[warp][0][f] = d[0];
+          } else {
+            // every exchange leaves a lane half of the rows it has: 4 to 6 shuffles for the four instead of 4 to 20, the sums in the same order
+            const bool o1 = lane & 1, o2 = lane & 2;
+            const float k0 = (o1 ? d[2] : d[0]) + __shfl_xor_sync(0xffffffffu, o1 ? d[0] : d[2], 1);
+            const float k1 = (o1 ? d[3] : d[1]) + __shfl_xor_sync(0xffffffffu, o1 ? d[1] : d[3], 1);
+            if (sh == 1) {
+              deltas[warp][2 * c][f] = k0;
+              deltas[warp][2 * c + 1][f] = k1;
+            } else {
+              float k = (o2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, o2 ? k0 : k1, 2);
+              for (int m = 4; m < (1 << sh); m <<= 1) k += __shfl_xor_sync(0xffffffffu, k, m);
+              if (c < 4) deltas[warp][(o1 ? 2 : 0) + (o2 ? 1 : 0)][f] = k;
+            }
+          }
         }
       }
       __syncwarp();
-      const float4 d4 = *reinterpret_cast<const float4*>(&deltas[warp][lane * 4]);
-      y[0] += d4.x; y[1] += d4.y; y[2] += d4.z; y[3] += d4.w;
-      __syncwarp();
     }
-    if (n < N) *reinterpret_cast<uint2*>(at) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (g < cnt && n < N) {                       // N is a multiple of four
+        float y[4] = {0.f, 0.f, 0.f, 0.f};
+        __nv_bfloat16* at = out + (long long)(t + g) * ldo + n;
+        if (ksplit == 0) {
+          const uint2 old = *reinterpret_cast<const uint2*>(at);
+          const float2 o0 = unpack_bf16x2(old.x), o1 = unpack_bf16x2(old.y);
+          y[0] = o0.x; y[1] = o0.y; y[2] = o1.x; y[3] = o1.y;
+        }
+#pragma unroll 4
+        for (int s = 0; s < ksplit; ++s) {
+          const float4 p4 = __ldcg(reinterpret_cast<const float4*>(partial + ((long long)s * T + t + g) * N + n));
+          y[0] += p4.x; y[1] += p4.y; y[2] += p4.z; y[3] += p4.w;
+        }
+        if (ksplit > 0 && bias != nullptr) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) y[c] += __bfloat162float(bias[n + c]);
+        }
+        if (q.r > 0) {
+          const float4 d4 = *reinterpret_cast<const float4*>(&deltas[warp][g][lane * 4]);
+          y[0] += d4.x; y[1] += d4.y; y[2] += d4.z; y[3] += d4.w;
+        }
+        *reinterpret_cast<uint2*>(at) = make_uint2(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]));
+      }
+    }
+    __syncwarp();
   }
 }
 
+// Steps of more than 32 rows whose entries have eight on average take rows by fours (prompts: B_cat is read once for the four): 256 rows of 28672 features,
+// rank 64, product and sums 368 -> 229 us; prompts of together 250 rows, a pass of two layers 1520 -> 1141 us, 180 rows 992 -> 880.  Short entries would leave a warp
+// several adapters one after the other: 64 rows of 24, 6144 features, 26 -> 44 us.
+static bool lora_add_by_fours(int T, int num_tiles) { return T > 32 && T >= 8 * num_tiles; }
 static int launch_lora_add(const LxLoraAdd& a, const float* partial, int ksplit, int T, int N, const __nv_bfloat16* bias, __nv_bfloat16* out,
                            long long ldo, int num_sms, cudaStream_t stream) {
   // rows per warp: as many as leave four blocks an SM
   const int col_blocks = (N + 127) / 128;
+  const bool fours = lora_add_by_fours(T, a.num_tiles);
   int run = (int)((long long)col_blocks * T / (kAddWarps * 4ll * num_sms));
   run = run < 1 ? 1 : run > 32 ? 32 : run;
-  launch_pdl(lora_add_kernel, dim3(col_blocks, (T + kAddWarps * run - 1) / (kAddWarps * run)), dim3(32 * kAddWarps), 0, stream, a, partial, ksplit, T, N, run,
-             bias, out, ldo);
+  if (fours) run = (run + 3) & ~3;
+  launch_pdl(fours ? lora_add_kernel<4> : lora_add_kernel<1>, dim3(col_blocks, (T + kAddWarps * run - 1) / (kAddWarps * run)), dim3(32 * kAddWarps), 0, stream, a,
+             partial, ksplit, T, N, run, bias, out, ldo);
   return -(int)cudaGetLastError();
 }
 

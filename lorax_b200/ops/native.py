@@ -496,7 +496,8 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
         if w16 is not None:
             return _lora_expand(gemm(x, w16, bias=bias, out=out), lora)
     xq, sa = quant_act_fp8(x)
-    add = _lora_add(out, lora, T <= load().lx_lora_add_max_rows() and (T <= LORA_ADD_FP8_ROWS or T * N <= LORA_ADD_FP8_RESULTS))
+    add = None if lora is None else _lora_add(out, lora, T <= load().lx_lora_add_max_rows() and (
+        T <= LORA_ADD_FP8_ROWS or T * N <= (LORA_ADD_FP8_LONG if T >= 8 * lora[1].num_tiles else LORA_ADD_FP8_RESULTS)))
     rc = load().lx_gemm_fp8_block128(_ptr(xq), xq.stride(0), _ptr(sa), sa.stride(0), _ptr(wq), wq.stride(0), _ptr(w_scale), _ptr(out),
                                      out.stride(0), _ptr(bias), T, N, K, _ptr(ws.gemm_ws), ws.gemm_ws.numel(), _ptr(ws.status),
                                      ws.num_sms, 1, ctypes.byref(add) if add is not None else None,
@@ -505,12 +506,16 @@ def gemm_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, bias: Opt
     return out if add is not None else _lora_expand(out, lora)
 
 
-# Steps whose adapters join the launch that forms a quantised product's results, by their number of results; larger ones take the expand
-# launch behind it, which has a row's B_cat in registers for up to 32 rows.  Measured against it with one adapter / as many as rows, up to 24, of ranks 16 to
-# 64.  Behind fp8 products: 28672 features of 32 rows 1.18 to 1.61x / 1.02 to 1.09x, of 64 0.85 to 0.92x with 24 and of 256 0.54x; 6144 of 128 1.33x up / 1.05x up, of 160
-# 0.90x; 4096 of 128 1.48x up / 1.03x up, of 160 0.92x.  In 4-bit products, a lane of which reads whole rows of B_cat: 28672 of 5 rows 1.04x up / 0.97x up, of 16
-# 0.95x / 0.86x; 17920 of 8 1.28x up / 1.08x up, of 16 0.91x; 6144 of 16 1.08x up, of 24 0.93x; 4096 of 32 1.03x up.
-LORA_ADD_FP8_ROWS, LORA_ADD_FP8_RESULTS, LORA_ADD_WQ4_RESULTS = 32, 589824, 143360
+# Steps whose adapters join the launch that forms a quantised product's results, by their rows and results; larger ones take the expand launch behind it, which
+# has a row's B_cat in registers for up to 32 rows.  Measured against it (GPU time) with as many adapters as rows, up to 24, of ranks 16 to 64.  Behind fp8 products:
+# 28672 features of 32 rows 1.05 to 1.2x, of 64 0.99x, of 128 0.8 to 0.9x; 6144 of 96 0.96 to 1.10x, of 151 0.99x.  In 4-bit products, a lane of which reads whole rows of B_cat:
+# 28672 of 5 rows 1.04x up / 0.97x up, of 16 0.95x / 0.86x (8: a pass of four layers 473 us either way); 17920 of 8 1.28x up / 1.08x up, of 16 0.91x; 6144 of 16 1.08x up,
+# of 24 0.93x; 4096 of 32 1.03x up.
+# Steps whose entries have eight rows and more on average, mostly prompts: fp8 takes their rows by fours and is quicker up to 97 rows of 28672 features, 1.06 to 1.5x
+# (from 128 rows 0.82 to 1.0x), and for 1536 to 6144 at any number of rows, 1.0 to 2.0x.  Such steps are eager, and a launch less is 10 us of the host's: 4-bit products take
+# all (28 rows, a pass of four layers 1240 -> 1128 us).
+LORA_ADD_FP8_ROWS, LORA_ADD_FP8_RESULTS, LORA_ADD_FP8_LONG = 32, 589824, 2785280
+LORA_ADD_WQ4_ROWS, LORA_ADD_WQ4_RESULTS = 8, 143360
 
 
 def _lora_add(out: torch.Tensor, lora, quicker: bool) -> Optional[LxLoraAdd]:
@@ -563,7 +568,8 @@ def gemm_wq(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, out: Option
         w = dataclasses.replace(w, perm=None)
     if (w.bits == 4 and w.table is None and T <= WQ4_DIRECT_MAX_TOKENS and N % 16 == 0 and K % 128 == 0 and w.group % 32 == 0
             and x.stride(0) % 8 == 0):
-        add = _lora_add(out, lora, T * N <= LORA_ADD_WQ4_RESULTS)
+        add = None if lora is None else _lora_add(
+            out, lora, T <= LORA_ADD_WQ4_ROWS or T * N <= LORA_ADD_WQ4_RESULTS or T >= 8 * lora[1].num_tiles)
         rc = load().lx_wq4_gemm_lora(_ptr(x), x.stride(0), _ptr(w.codes), _ptr(w.sz), _ptr(bias), _ptr(out), out.stride(0), T, N, K, w.group,
                                      (1 if getattr(w, "int_zero", False) else 0) | (2 if w_const else 0), ctypes.byref(add) if add is not None else None,
                                      _stream())

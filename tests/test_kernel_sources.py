@@ -123,11 +123,12 @@ def test_expert_products_by_pairs_only_where_they_measured_quicker(avg_rows, n_w
     assert native.load().lx_moe_by_pairs(avg_rows, n_w, K, native._MOE_ACTS[act]) == pairs
 
 
-@pytest.mark.parametrize("form,T,N,taken", [
-    ("fp8", 32, 28672, True), ("fp8", 64, 28672, False), ("fp8", 256, 28672, False), ("fp8", 96, 6144, True), ("fp8", 160, 6144, False), ("fp8", 144, 4096, True),
-    ("fp8", 256, 1536, True), ("fp8", 257, 512, False),
-    ("wq4", 5, 28672, True), ("wq4", 16, 28672, False), ("wq4", 16, 6144, True), ("wq4", 24, 6144, False), ("wq4", 32, 4096, True)])
-def test_adapters_join_quantised_products_only_where_it_measured_quicker(monkeypatch, form, T, N, taken):
+@pytest.mark.parametrize("form,T,N,entry,taken", [
+    ("fp8", 32, 28672, 1, True), ("fp8", 64, 28672, 1, False), ("fp8", 256, 28672, 1, False), ("fp8", 96, 6144, 1, True), ("fp8", 160, 6144, 1, False), ("fp8", 144, 4096, 1, True),
+    ("fp8", 256, 1536, 1, True), ("fp8", 257, 512, 1, False),
+    ("fp8", 160, 6144, 7, False), ("fp8", 160, 6144, 8, True), ("fp8", 96, 28672, 32, True), ("fp8", 128, 28672, 32, False), ("fp8", 256, 6144, 16, True), ("fp8", 288, 6144, 32, False),
+    ("wq4", 5, 28672, 1, True), ("wq4", 8, 28672, 1, True), ("wq4", 9, 28672, 1, False), ("wq4", 16, 6144, 1, True), ("wq4", 24, 6144, 1, False), ("wq4", 32, 4096, 1, True), ("wq4", 28, 28672, 14, True)])
+def test_adapters_join_quantised_products_only_where_it_measured_quicker(monkeypatch, form, T, N, entry, taken):
     """Which steps ask the product's launch to add the adapters: read off what the wrappers ask for, with the library's calls left out."""
     import torch
     from types import SimpleNamespace as NS
@@ -139,7 +140,7 @@ def test_adapters_join_quantised_products_only_where_it_measured_quicker(monkeyp
     for name, value in dict(load=lambda: lib, workspace=lambda dev: ws, _stream=lambda: None, _lora_expand=lambda out, lora: out,
                             _lora_add=lambda out, lora, quicker: asked.append(quicker)).items():
         monkeypatch.setattr(native, name, value)
-    x, lora = torch.empty(T, 128, dtype=torch.bfloat16), (None, None)
+    x, lora = torch.empty(T, 128, dtype=torch.bfloat16), (None, NS(num_tiles=-(-T // entry)))
     if form == "fp8":
         native.gemm_fp8(x, torch.empty(N, 128, dtype=torch.uint8), torch.empty(N // 128, 1), lora=lora)
     else:

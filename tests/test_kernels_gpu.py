@@ -1006,6 +1006,12 @@ def test_quantised_products_add_the_adapters_of_many_features(nat, form, T, K, p
     test_quantised_products_add_the_adapters(nat, form, T, K, parts, ranks)
 
 
+@pytest.mark.parametrize("T,K,parts,ranks", [(64, 512, [16384, 1024], [16, 64]), (96, 512, [256, 128], [16, 32, 64]), (255, 256, [4096], [48, 16]), (33, 1024, [260], [32])])
+def test_quantised_products_add_the_adapters_of_prompts(nat, T, K, parts, ranks):
+    """Entries of eight rows and more on average, whose rows are taken by fours: several such groups a warp and one, groups that end at an entry's end or the step's."""
+    test_quantised_products_add_the_adapters(nat, "fp8", T, K, parts, ranks)
+
+
 @pytest.mark.parametrize("T,N,K", [(193, 256, 64), (200, 6144, 4096), (256, 4096, 14336), (320, 28672, 256), (513, 256, 64), (545, 300, 200), (1000, 1000, 136), (2047, 640, 4096), (700, 4360, 72), (1024, 257, 64)])
 def test_products_of_cta_pairs(nat, T, N, K):
     """Long steps at the edges of tiles, whole ones and shared: features that do not fill a tile of 256 or begin off 16 bytes in the output, ragged K, a last token tile of
