@@ -7,7 +7,7 @@
 // Both operands are "K-major", which is how activations [tokens, K] and nn.Linear weights [N, K] already sit in
 // memory, so either can take the UMMA M side:
 //   * prefill (many tokens):  A = activations, B = weights, 128 x 256 tiles, compute bound;
-//     (from 193 tokens on pairs of CTAs take the product, weights on the M side: gemm_pair.cuh);
+//     (from 193 tokens on pairs of CTAs take the product where they are quicker, weights on the M side: gemm_pair.cuh);
 //   * decode (few tokens):    A = weights (128 output features per tile), B = activations (UMMA N = tokens
 //     rounded up to 16), so the tensor core does no work for padding rows and each weight byte is read from
 //     HBM exactly once.  Small grids are widened with split-K; the last CTA to finish a tile reduces the

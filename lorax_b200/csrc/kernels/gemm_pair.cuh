@@ -3,8 +3,8 @@
 // A pair takes a tile of 256 output features x up to 256 tokens: each CTA loads 128 rows of the weights and half of the tokens, 32 KB a stage
 // where one CTA on its own tile of 128 x 256 takes 48, and reads half the token operand from its shared memory per MMA: what a single CTA
 // moves in and out of shared memory per product is the limit of gemm_bf16_tcgen05_kernel at these sizes (192 of about 128 B per cycle asked for).
-// 4001 rows, 28672 x 4096: 703 -> 630 us, the tensor pipe 90 % active at the 1.5 GHz that the power limit leaves.  Operands carry no eviction hints: the
-// pairs of a wave share weight tiles and token tiles through L2 (weights evicted early cost 2 to 3 % of a pass).
+// 4001 rows, 28672 x 4096: 703 -> 630 to 680 us with the clock, the tensor pipe 90 % active at the 1.5 GHz that the power limit leaves.  Operands carry
+// no eviction hints: the pairs of a wave share weight tiles and token tiles through L2 (weights evicted early cost 2 to 3 % of a pass).
 // Rank 0's MMA thread issues for both; a stage is full when the loads of both CTAs have arrived at rank 0's barrier, and its commits
 // tell both that a stage is free or an accumulator complete.  Whole tiles and the stream-K remainder as there, each CTA with its half of a tile's
 // partial sums.  LoRA as there: shrink on the epilogue warps of all CTAs during the first K loop, expand by MMAs into the
@@ -451,14 +451,21 @@ static PairPlan pair_plan(int T, int N, int K, int pairs, long long ws_bytes) {
 // to 4001 rows, 256 to 28672 features, K 128 to 14336.  Where the rule takes pairs they win up to 1.5x (4001 rows, us, single / pairs: 28672 x 4096 1.10x,
 // 4096 x 14336 1.12x; 512 rows 1.19x both), 18 shapes lose 3 to 11 %; always pairs lost more than 3 % in 1550 (K = 256, 1000 rows: 20 %; 11008 x 4096, 320
 // rows: 29 %).
-// With adapters of rank `lora_rank` the first tile of a pair waits for the shrink, and a pair holds twice the tile: only where most pairs have
-// three tiles or a feature tile of their own, K of 2048 and ranks of up to 32 (r 16, one adapter / 24: 28672 x 4096 of 256 rows 1.07x / 1.03x, of 2000 1.07x / 1.06x;
-// without these lines 4096 x 14336 of 1000 rows 0.90x, rank 64 with 24 adapters 0.85 to 0.97x nearly everywhere).
+// In one wave of a model's step, where a product follows a short kernel, pairs are quicker than in a loop of products: decode of 256 rows, four layers without
+// adapters 1042 -> 1029 us, with a hundred 1715 -> 1662 (in a loop 4096 to 8192 features x 4096 lose 2 to 4 %, 11008 and 13824 win 8 to 11 %).
+// With adapters of rank `lora_rank` the first tile of a pair waits for the shrink, and a pair holds twice the tile: K of 2048 and ranks of up to 32, and one wave
+// (300 rows of one adapter, a pass 1114 -> 1094 us; 200 rows of eight 1184 -> 1146), or the cheaper plan where most pairs have a tile and a half or a
+// feature tile of their own (2000 rows 3830 -> 3750; 1000 rows, whose tiles are less, 2190 -> 2225 with pairs everywhere, of rank 64 2440 -> 2520).
+constexpr int kPairWaveTokens = 256, kPairWaveLoraTokens = 512;
 constexpr double kPairCostFactor = 1.15, kPairCostMore = 4000.0;
 static PairPlan choose_pair(int T, int N, int K, int pairs, long long ws_bytes, double single_cost, int lora_rank) {
   PairPlan plan = pair_plan(T, N, K, pairs, ws_bytes);
   const int tiles_a = (N + 255) / 256, tiles = plan.bn > 0 ? tiles_a * ((T + plan.bn - 1) / plan.bn) : 0;
-  if (plan.cost * kPairCostFactor + kPairCostMore >= single_cost || (lora_rank > 0 && (lora_rank > 32 || K < 2048 || (tiles_a < pairs && tiles < 3 * pairs)))) plan.bn = 0;
+  const bool cheaper = plan.cost * kPairCostFactor + kPairCostMore < single_cost;
+  const bool wave = K >= 2048 && tiles_a >= 16 && tiles <= pairs && ws_bytes > 0 && T <= (lora_rank > 0 ? kPairWaveLoraTokens : kPairWaveTokens);
+  bool take = cheaper || wave;
+  if (lora_rank > 0) take = lora_rank <= 32 && K >= 2048 && (wave || (cheaper && (tiles_a >= pairs || 2 * tiles >= 3 * pairs)));
+  if (!take) plan.bn = 0;
   return plan;
 }
 

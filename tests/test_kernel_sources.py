@@ -87,7 +87,8 @@ def test_prefetches_of_adapter_rows_stay_inside(N, r):
 @pytest.mark.parametrize("T,N,K,rank,taken", [
     (4001, 28672, 4096, 0, True), (256, 4096, 14336, 0, True), (512, 28672, 4096, 0, True),
     (1000, 4096, 256, 0, False), (2048, 512, 1024, 0, False), (320, 11008, 4096, 0, False), (193, 256, 64, 0, False),      # 20, 10, 29 % slower by pairs
-    (256, 28672, 4096, 16, True), (4001, 4096, 4096, 32, True),
+    (256, 28672, 4096, 16, True), (4001, 4096, 4096, 32, True), (256, 6144, 4096, 16, True), (300, 4096, 14336, 32, True), (512, 1536, 4096, 16, False), (700, 6144, 4096, 16, False),
+    (256, 11008, 4096, 0, True), (257, 6144, 4096, 0, False), (256, 6144, 1984, 0, False),
     (1000, 4096, 14336, 16, False), (800, 17920, 1536, 16, False), (200, 28672, 4096, 64, False)])                          # 10, 8, 6 %
 def test_pairs_of_ctas_only_where_they_measured_quicker(T, N, K, rank, taken):
     import ctypes
