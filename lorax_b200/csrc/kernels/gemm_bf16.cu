@@ -382,12 +382,13 @@ LX_DEVICE bool lora_join_kparts(const GemmParams& p, const ShrinkUnit& s, int pa
   return true;
 }
 
-// Parts of a unit's K where `ctas` CTAs share `units` units of `nbatch` batches: as many as there are CTAs for, where that takes three batches or more
-// off the chain.  With fewer the sums' way through L2 costs as much as it saves (one of the two of K = 1536, two of the four of 4096, 1 to 64 rows: 3 to
-// 9 % slower; three of four 1 to 9 % quicker, ten of fourteen 8 to 14 %).
+// Parts of a unit's K where `ctas` CTAs share `units` units of `nbatch` batches: as many as there are CTAs for, where that takes two batches or more
+// off the chain.  One does not pay for the sums' way through L2 (one of the two of K = 1536, 1 to 64 rows: 3 to 9 % slower).  Two of the four of K = 4096 do
+// in a model's step (64 rows of 24 adapters, a pass of four layers 883 -> 877 us; 32 rows 765 either way), though not in a loop of products (32 rows 25.7 -> 29.4
+// us); three of four 1 to 9 % quicker, ten of fourteen 8 to 14 %.
 __host__ __device__ constexpr int lora_shrink_k_parts(int ctas, int units, int nbatch) {
   const int most = units > 0 ? ctas / units : 0, parts = most < nbatch ? most : nbatch;
-  return parts > 1 && nbatch - (nbatch + parts - 1) / parts >= 3 ? parts : 1;
+  return parts > 1 && nbatch - (nbatch + parts - 1) / parts >= 2 ? parts : 1;
 }
 
 template <int NG, int SB, int WIN>

@@ -101,8 +101,8 @@ def test_pairs_of_ctas_only_where_they_measured_quicker(T, N, K, rank, taken):
     assert out[3] <= 40 and out[2] <= 40
 
 
-@pytest.mark.parametrize("units,K,parts", [(1, 14336, 14), (24, 14336, 6), (72, 14336, 2), (74, 14336, 2), (75, 14336, 1), (3, 4096, 4), (36, 4096, 4), (48, 4096, 1), (72, 4096, 1),
-                                           (1, 1536, 1), (12, 1536, 1), (1, 2880, 1), (2, 3080, 4), (0, 4096, 1)])      # 1536: two batches, 4096: four
+@pytest.mark.parametrize("units,K,parts", [(1, 14336, 14), (24, 14336, 6), (72, 14336, 2), (74, 14336, 2), (75, 14336, 1), (3, 4096, 4), (36, 4096, 4), (48, 4096, 3), (72, 4096, 2), (75, 4096, 1),
+                                           (1, 1536, 1), (12, 1536, 1), (1, 2880, 3), (50, 2880, 1), (2, 3080, 4), (0, 4096, 1)])      # 1536: two batches, 4096: four
 def test_shrink_units_share_their_k_only_where_it_measured_quicker(units, K, parts):
     from lorax_b200.ops import native
     assert native.load().lx_lora_fused_k_parts(148, units, K) == parts
